@@ -1,12 +1,13 @@
 """Builds libarap_gb300.so (the C ABI of include/arap_gpu.h) for sm_103a.
 
-Six translation units compiled in parallel, then linked with the static CUDA
+Seven translation units compiled in parallel, then linked with the static CUDA
 runtime:
   csrc/arap_kernels.cu   the sm_103a kernels (nvcc)
   csrc/arap_context.cu   context state and the C ABI (nvcc)
   csrc/arap_noalloc.cu   cotan weights with static scratch (nvcc)
   csrc/arap_batch.cu     many poses of one mesh in one pass (nvcc)
   csrc/arap_symbolic.cpp host symbolic analysis (g++)
+  csrc/arap_strata.cpp   dense phases of the solves, host plan (g++)
   csrc/arap_server.cpp   the request scheduler of arap_srv_* (g++)
 The library is built in-tree (next to this file) and is git-ignored.
 """
@@ -40,9 +41,11 @@ SOURCES = [
     ("nvcc", CSRC / "arap_noalloc.cu"),
     ("nvcc", CSRC / "arap_batch.cu"),
     ("g++", CSRC / "arap_symbolic.cpp"),
+    ("g++", CSRC / "arap_strata.cpp"),
     ("g++", CSRC / "arap_server.cpp"),
 ]
-HEADERS = [CSRC / "arap_kernels.h", CSRC / "arap_symbolic.h", CSRC / "arap_device.cuh", CSRC / "arap_server.h",
+HEADERS = [CSRC / "arap_kernels.h", CSRC / "arap_strata.h", CSRC / "arap_strata.cuh", CSRC / "arap_btop.cuh",
+           CSRC / "arap_wsolve.cuh", CSRC / "arap_btop_plan.h", CSRC / "arap_symbolic.h", CSRC / "arap_device.cuh", CSRC / "arap_server.h",
            ROOT / "include" / "arap_gpu.h"]
 
 

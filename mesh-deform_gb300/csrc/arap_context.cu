@@ -182,13 +182,22 @@ struct arap_ctx {
     int solve_schedule = kSolveScheduleDefault;  // ARAP_SOLVE_PERSISTENT or ARAP_SOLVE_LEVELS
     int solve_blocks = kSolveBlocksDefault;      // largest solve block (columns), 0: none
     SolveBlocks sb;                              // the blocks of the current analysis (use_sb)
-    bool use_sb = false;
+    bool use_sb = false, sb_built = false;
     DevSym dss;                                  // the single-request sweeps' layout with the blocks
     DevBuf ssn, slevel_sn, sbitems, sbmembers;
     // launch shape of the local step, RHS and residual (arap_set_vertex_launch)
     VertexLaunch vlaunch[kVertexKernels] = {{1, 256}, {1, 256}, {1, 256}};
     size_t dense_inv_smem[2] = {0, 0};  // configured limits (FP32, FP64)
     DevBuf top_col, top_gptr, top_gidx, tdpos, top_items, Ttop, ytop;
+    // dense-phase solves (arap_strata.h): the plan of the current analysis and
+    // precision (0: none yet), what of the current analysis is on the device,
+    // and which solve arrays hold the current factorisation
+    Strata strata;
+    int strata_bits = 0;
+    StrataDev std_{};
+    bool strata_ready = false, sweeps_ready = false;
+    bool strata_formed = false, sweeps_formed = false;
+    DevBuf st_tiles, st_sn, st_col, st_gptr, st_gidx, st_items, st_top_gptr, st_top_gidx, st_m, st_y, st_ytop;
     int ordering = ARAP_ORDER_PER_CONSTRAINT_SET;
     arap_done_fn done_fn = nullptr;  // called from a CUDA thread when an async deform finished
     void *done_user = nullptr;
@@ -222,7 +231,8 @@ struct arap_ctx {
                 &vnorm, &btargets, &bpc64, &bpc32, &bR, &bbfixed, &bb, &bsol, &buvec, &bout, &bftop, &bytop, &bws,
                 &batile,
                 &bticket, &bflags, &top_col, &top_gptr, &top_gidx, &tdpos, &top_items, &Ttop, &ytop, &Lval32,
-                &Dinv32, &ssn, &slevel_sn, &sbitems, &sbmembers};
+                &Dinv32, &ssn, &slevel_sn, &sbitems, &sbmembers, &st_tiles, &st_sn, &st_col, &st_gptr, &st_gidx,
+                &st_items, &st_top_gptr, &st_top_gidx, &st_m, &st_y, &st_ytop};
     }
 };
 
@@ -300,10 +310,47 @@ int analyze_symbolic(arap_ctx *ctx) {
     bool singular = false;
     if (!build_symbolic(ctx->topo, ctx->cmask, ctx->sym, err, singular, ctx->ordering == ARAP_ORDER_MESH))
         return fail(ctx, singular ? ARAP_ERR_NOT_SPD : ARAP_ERR_CUDA, err);
-    ctx->use_sb = ctx->solve_blocks > 0 && build_solve_blocks(ctx->sym, ctx->solve_blocks, ctx->sb);
-    if (!ctx->use_sb) ctx->sb = SolveBlocks();
+    ctx->use_sb = ctx->sb_built = false;
+    ctx->strata_bits = 0;
     ctx->sym_host = true;
     return ARAP_OK;
+}
+
+// The solve blocks of the supernodal sweeps, built when something runs them.
+void build_blocks(arap_ctx *ctx) {
+    if (ctx->sb_built) return;
+    ctx->use_sb = ctx->solve_blocks > 0 && build_solve_blocks(ctx->sym, ctx->solve_blocks, ctx->sb);
+    if (!ctx->use_sb) ctx->sb = SolveBlocks();
+    ctx->sb_built = true;
+}
+
+int device_sms() {
+    static const int sms = [] {  // initialised once, thread-safe
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return 152;
+        return v;
+    }();
+    return sms;
+}
+
+// Whether the single-request solves run as dense phases: with every option of
+// the supernodal sweeps at its default (an explicit dense-top cap, cluster
+// threshold, warp-row limit, solve-block size or level schedule asks for the
+// sweeps) and fronts that fit the phases' kernels. Builds the plan.
+bool use_strata(arap_ctx *ctx, bool fp64) {
+    if (ctx->dense_cols != 0 || ctx->top_bytes != 0 || ctx->warp_rows != kWarpRowsDefault ||
+        ctx->solve_schedule != kSolveScheduleDefault || ctx->solve_blocks != kSolveBlocksDefault)
+        return false;
+    const int bits = fp64 ? 64 : 32;
+    if (ctx->strata_bits != bits) {
+        ctx->strata_ready = ctx->strata_formed = false;
+        if (build_strata(ctx->sym, fp64, device_sms(), ctx->strata) && !strata_fits(ctx->strata, bits / 8))
+            ctx->strata.ok = false;
+        ctx->strata_bits = bits;
+    }
+    return ctx->strata.ok;
 }
 
 // The dense top of the tree: the most top levels whose supernodes hold at most
@@ -343,9 +390,12 @@ int dense_cap(const arap_ctx *ctx) {
 
 // Bytes of every device buffer the setup of precision T (and, for n_poses > 0,
 // arap_deform_poses with that many poses) holds, buffer by buffer.
+// sweeps / phases: the solve arrays of the supernodal sweeps / dense phases.
 template <typename T>
-void planned_sizes(arap_ctx *ctx, int n_poses, std::vector<std::pair<DevBuf *, size_t>> &out) {
+void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
+                   std::vector<std::pair<DevBuf *, size_t>> &out) {
     const Symbolic &s = ctx->sym;
+    if (sweeps) build_blocks(ctx);
     const size_t V = (size_t)s.V, m1 = (size_t)std::max(s.m, 1), nnz = s.dcol.size(), S1 = (size_t)std::max(s.S, 1);
     out.clear();
     auto add = [&](DevBuf &b, size_t bytes) { out.push_back({&b, bytes}); };
@@ -362,8 +412,10 @@ void planned_sizes(arap_ctx *ctx, int n_poses, std::vector<std::pair<DevBuf *, s
     add(ctx->child, s.child.size() * 4);
     add(ctx->level_sn, s.level_sn.size() * 4);
     add(ctx->fitems, s.fitems.size() * sizeof(FItem));
-    add(ctx->ticket, kTickets * sizeof(unsigned long long));
-    add(ctx->flags, 2 * sizeof(unsigned) * S1);
+    if (sweeps) {
+        add(ctx->ticket, kTickets * sizeof(unsigned long long));
+        add(ctx->flags, 2 * sizeof(unsigned) * S1);
+    }
     // iteration state and factor (setup_alloc)
     const bool f32 = sizeof(T) == 4;
     add(ctx->w64, nnz * sizeof(double));
@@ -388,7 +440,27 @@ void planned_sizes(arap_ctx *ctx, int n_poses, std::vector<std::pair<DevBuf *, s
     add(ctx->Lval, (size_t)std::max<int64_t>(s.panel_size, 1) * fs);
     add(ctx->Dinv, (size_t)std::max<int64_t>(s.dinv_size, 1) * fs);
     add(ctx->Upd, (size_t)std::max<int64_t>(s.upd_size, 1) * fs);
-    // the solve arrays, with the solve blocks after the supernodes' own
+    if (f64f) {
+        add(ctx->Lval32, (size_t)std::max<int64_t>(s.panel_size, 1) * sizeof(float));
+        add(ctx->Dinv32, (size_t)std::max<int64_t>(s.dinv_size, 1) * sizeof(float));
+    }
+    if (phases) {
+        const Strata &p = ctx->strata;
+        add(ctx->Xinv, (size_t)std::max<int64_t>(s.x_size, 1) * sizeof(T));
+        add(ctx->st_y, m1 * sizeof(Vec4<T>));
+        add(ctx->st_m, (size_t)p.m_size * sizeof(T));
+        add(ctx->st_ytop, std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16));
+        add(ctx->st_tiles, p.tiles.size() * sizeof(StTile));
+        add(ctx->st_sn, p.sn.size() * sizeof(StSn));
+        add(ctx->st_col, p.col.size() * 4);
+        add(ctx->st_gptr, p.gptr.size() * 4);
+        add(ctx->st_gidx, p.gidx.size() * 4);
+        add(ctx->st_items, p.items.size() * 4);
+        add(ctx->st_top_gptr, p.top_gptr.size() * 4);
+        add(ctx->st_top_gidx, p.top_gidx.size() * 8);
+    }
+    if (!sweeps) return;
+    // the sweeps' solve arrays, with the solve blocks after the supernodes' own
     const int64_t xs = ctx->use_sb ? ctx->sb.x_size : s.x_size, l21s = ctx->use_sb ? ctx->sb.l21_size : s.l21_size,
                   l21ts = ctx->use_sb ? ctx->sb.l21t_size : s.l21t_size;
     add(ctx->Xinv, (size_t)std::max<int64_t>(xs, 1) * sizeof(T));
@@ -396,10 +468,6 @@ void planned_sizes(arap_ctx *ctx, int n_poses, std::vector<std::pair<DevBuf *, s
     add(ctx->L21T, (size_t)std::max<int64_t>(l21ts, 1) * sizeof(T));
     const int nt = choose_dense_top(s, dense_cap(ctx)).ncols;
     add(ctx->Ttop, std::max<size_t>(nt > 0 ? dense_top_elems(nt) : 0, 1) * sizeof(T));
-    if (f64f) {
-        add(ctx->Lval32, (size_t)std::max<int64_t>(s.panel_size, 1) * sizeof(float));
-        add(ctx->Dinv32, (size_t)std::max<int64_t>(s.dinv_size, 1) * sizeof(float));
-    }
     add(ctx->ytop, std::max<size_t>(top_vec_bytes(nt, sizeof(T)), 16));  // y_top, the tiles' partials, counters
     if (n_poses > 0) {
         const size_t P = (size_t)n_poses, VP = V * P, MP = m1 * P, nc = V - (size_t)s.m;
@@ -573,6 +641,7 @@ int prepare_symbolic(arap_ctx *ctx) {
     Symbolic &s = ctx->sym;
     cudaStream_t st = ctx->stream;
     ctx->gen++;
+    ctx->strata_formed = ctx->sweeps_formed = false;
     CK(upload(ctx->drow, s.drow, st));
     CK(upload(ctx->dcol, s.dcol, st));
     CK(upload(ctx->dent, s.dent, st));
@@ -585,12 +654,6 @@ int prepare_symbolic(arap_ctx *ctx) {
     CK(upload(ctx->child, s.child, st));
     CK(upload(ctx->level_sn, s.level_sn, st));
     CK(upload(ctx->fitems, s.fitems, st));
-    // solve scheduling state: ticket counters and per-supernode flags start at 0
-    // counters: forward / backward of the lower levels, then of the top levels
-    CK(ctx->ticket.ensure(kTickets * sizeof(unsigned long long)));
-    CK(ctx->flags.ensure(2 * sizeof(unsigned) * (size_t)std::max(s.S, 1)));
-    CK(cudaMemsetAsync(ctx->ticket.p, 0, kTickets * sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(unsigned) * (size_t)std::max(s.S, 1), st));
     // the solve kernels stream a front's matrices through chunk buffers
     // (whole columns for fronts of one pass, row segments of each pass for
     // larger ones, so columns may have any length) and keep the front's
@@ -604,6 +667,51 @@ int prepare_symbolic(arap_ctx *ctx) {
                     "supernode front of " + std::to_string(max_rows) + " rows (" + std::to_string(s.max_ncol) +
                         " columns) exceeds the solve kernels' shared memory");
     ctx->fp64_solves = b64 <= kSmemMax;
+    DevSym &d = ctx->ds;
+    d = DevSym{};
+    d.V = s.V;
+    d.m = s.m;
+    d.S = s.S;
+    d.s_sched = s.S;
+    for (int k = 0; k < kVertexKernels; ++k) d.vlaunch[k] = ctx->vlaunch[k];
+    d.nnz = (int)s.dcol.size();
+    d.max_ldx = s.max_ldx;
+    d.max_ld21 = s.max_ld21;
+    d.max_ncol = s.max_ncol;
+    d.overlap = ctx->solve_cap <= 0;
+    d.drow = ctx->drow.as<int32_t>();
+    d.dcol = ctx->dcol.as<int32_t>();
+    d.dent = ctx->dent.as<int32_t>();
+    d.oldidx = ctx->oldidx.as<int32_t>();
+    d.amap = ctx->amap.as<int64_t>();
+    d.dmap = ctx->dmap.as<int64_t>();
+    d.sn = ctx->sn.as<SnInfo>();
+    d.rows = ctx->rows.as<int32_t>();
+    d.relind = ctx->relind.as<int32_t>();
+    d.child = ctx->child.as<int32_t>();
+    d.level_sn = ctx->level_sn.as<int32_t>();
+    ctx->strata_ready = ctx->sweeps_ready = false;
+    ctx->sym_valid = true;
+    return ARAP_OK;
+}
+
+// The supernodal sweeps' layout and scheduling state for the current analysis
+// (pose batches, and single requests that ask for the sweeps).
+int prepare_sweeps(arap_ctx *ctx) {
+    if (ctx->sweeps_ready) return ARAP_OK;
+    build_blocks(ctx);
+    const Symbolic &s = ctx->sym;
+    cudaStream_t st = ctx->stream;
+    ctx->gen++;
+    ctx->sweeps_formed = false;
+    constexpr size_t kSmemMax = 227 * 1024;
+    const size_t b32 = solve_smem_bytes(s.max_ldx, s.max_ld21, 4), b64 = solve_smem_bytes(s.max_ldx, s.max_ld21, 8);
+    // solve scheduling state: ticket counters and per-supernode flags start at 0
+    // counters: forward / backward of the lower levels, then of the top levels
+    CK(ctx->ticket.ensure(kTickets * sizeof(unsigned long long)));
+    CK(ctx->flags.ensure(2 * sizeof(unsigned) * (size_t)std::max(s.S, 1)));
+    CK(cudaMemsetAsync(ctx->ticket.p, 0, kTickets * sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(unsigned) * (size_t)std::max(s.S, 1), st));
     if (b32 > ctx->smem_f32 || (ctx->fp64_solves && b64 > ctx->smem_f64)) {
         CK(configure_solve_smem((int)b32, ctx->fp64_solves ? (int)b64 : 0));
         ctx->smem_f32 = b32;
@@ -723,26 +831,6 @@ int prepare_symbolic(arap_ctx *ctx) {
             }
         }
     }
-    d.V = s.V;
-    d.m = s.m;
-    d.S = s.S;
-    d.s_sched = s.S;
-    for (int k = 0; k < kVertexKernels; ++k) d.vlaunch[k] = ctx->vlaunch[k];
-    d.nnz = (int)s.dcol.size();
-    d.max_ldx = s.max_ldx;
-    d.max_ld21 = s.max_ld21;
-    d.max_ncol = s.max_ncol;
-    d.drow = ctx->drow.as<int32_t>();
-    d.dcol = ctx->dcol.as<int32_t>();
-    d.dent = ctx->dent.as<int32_t>();
-    d.oldidx = ctx->oldidx.as<int32_t>();
-    d.amap = ctx->amap.as<int64_t>();
-    d.dmap = ctx->dmap.as<int64_t>();
-    d.sn = ctx->sn.as<SnInfo>();
-    d.rows = ctx->rows.as<int32_t>();
-    d.relind = ctx->relind.as<int32_t>();
-    d.child = ctx->child.as<int32_t>();
-    d.level_sn = ctx->level_sn.as<int32_t>();
     d.top_col = ctx->top_col.as<int32_t>();
     d.top_gptr = ctx->top_gptr.as<int32_t>();
     d.top_gidx = ctx->top_gidx.as<int64_t>();
@@ -752,7 +840,53 @@ int prepare_symbolic(arap_ctx *ctx) {
         const int rc_b = prepare_solve_blocks(ctx);
         if (rc_b != ARAP_OK) return rc_b;
     }
-    ctx->sym_valid = true;
+    ctx->sweeps_ready = true;
+    return ARAP_OK;
+}
+
+// The dense phases' plan on the device, their matrices cleared (the inversion
+// never writes their zeros).
+template <typename T>
+int prepare_strata(arap_ctx *ctx) {
+    if (ctx->strata_ready) return ARAP_OK;
+    const Strata &p = ctx->strata;
+    cudaStream_t st = ctx->stream;
+    ctx->gen++;
+    ctx->strata_formed = false;
+    CK(configure_strata(p, sizeof(T)));
+    CK(upload(ctx->st_tiles, p.tiles, st));
+    CK(upload(ctx->st_sn, p.sn, st));
+    CK(upload(ctx->st_col, p.col, st));
+    CK(upload(ctx->st_gptr, p.gptr, st));
+    CK(upload(ctx->st_gidx, p.gidx, st));
+    CK(upload(ctx->st_items, p.items, st));
+    CK(upload(ctx->st_top_gptr, p.top_gptr, st));
+    CK(upload(ctx->st_top_gidx, p.top_gidx, st));
+    CK(ctx->st_m.ensure((size_t)p.m_size * sizeof(T)));
+    CK(cudaMemsetAsync(ctx->st_m.p, 0, (size_t)p.m_size * sizeof(T), st));
+    // the big top's arrival counters start at zero (each launch resets them)
+    CK(ctx->st_ytop.ensure(std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16)));
+    CK(cudaMemsetAsync(ctx->st_ytop.p, 0, ctx->st_ytop.cap, st));
+    StrataDev d{};
+    d.nph = (int)p.ph.size();
+    for (int k = 0; k < d.nph; ++k) d.ph[k] = p.ph[k];
+    d.grid_cap = ctx->solve_cap;
+    d.overlap = ctx->solve_cap <= 0;
+    d.big_n = p.big_n;
+    d.big_off = p.big_off;
+    d.big_pair32 = p.big_n > 0 && (int64_t)top_tiles(p.big_n) > top_tile_resident_ctas(4);
+    d.big_pair64 = p.big_n > 0 && (int64_t)top_tiles(p.big_n) > top_tile_resident_ctas(8);
+    d.tiles = ctx->st_tiles.as<StTile>();
+    d.sn = ctx->st_sn.as<StSn>();
+    d.col = ctx->st_col.as<int32_t>();
+    d.gptr = ctx->st_gptr.as<int32_t>();
+    d.gidx = ctx->st_gidx.as<int32_t>();
+    d.items = ctx->st_items.as<int32_t>();
+    d.top_col = d.col + p.big_col;
+    d.top_gptr = ctx->st_top_gptr.as<int32_t>();
+    d.top_gidx = ctx->st_top_gidx.as<int64_t>();
+    ctx->std_ = d;
+    ctx->strata_ready = true;
     return ARAP_OK;
 }
 
@@ -760,9 +894,9 @@ int prepare_symbolic(arap_ctx *ctx) {
 // Allocates (or keeps) every buffer the setup and the iterations of precision
 // T use. Any reallocation bumps ctx->gen so captured graphs are rebuilt.
 template <typename T>
-int setup_alloc(arap_ctx *ctx) {
+int setup_alloc(arap_ctx *ctx, bool sweeps, bool phases) {
     std::vector<std::pair<DevBuf *, size_t>> plan;
-    planned_sizes<T>(ctx, 0, plan);
+    planned_sizes<T>(ctx, 0, sweeps, phases, plan);
     bool moved = false;
     for (auto &pb : plan) {
         void *before = pb.first->p;
@@ -835,6 +969,39 @@ int factor_inverses(arap_ctx *ctx, const TI *Lval, const TI *Dinv, TI *X, TI *L2
     return ARAP_OK;
 }
 
+// The dense phases' matrices (arap_strata.h) from a factor in the solves'
+// precision: X = inv(L11) per supernode, then M = [X; W] per group.
+template <typename TI>
+int form_strata(arap_ctx *ctx, const TI *Lval, const TI *Dinv) {
+    const DevSym &d = ctx->ds;
+    cudaStream_t st = ctx->stream;
+    TI *X = ctx->Xinv.as<TI>();
+    for (const FactorLaunch &fl : ctx->sym.fplan) {
+        if (fl.kind != kFx) continue;
+        Prof pr(ctx, ARAP_K_FACTOR);
+        launch_factor_step<TI>(d, fl, ctx->fitems.as<FItem>(), const_cast<TI *>(Lval), nullptr, const_cast<TI *>(Dinv),
+                               X, nullptr, nullptr, ctx->errw.as<int>(), st);
+        ctx->launches += 1;
+    }
+    {
+        Prof pr(ctx, ARAP_K_FACTOR);
+        launch_strata_inverse<TI>(ctx->std_, d, X, Lval, ctx->st_m.as<TI>(), st);
+    }
+    ctx->launches += ctx->std_.nph;
+    CK(cudaGetLastError());
+    return ARAP_OK;
+}
+
+// The solve arrays of the current factorisation, for the dense phases or for
+// the sweeps.
+template <typename T>
+int form_solves(arap_ctx *ctx, bool phases) {
+    const bool demoted = sizeof(T) == 4 && ctx->factor_bits == 64;
+    const T *L = (demoted ? ctx->Lval32 : ctx->Lval).as<T>(), *D = (demoted ? ctx->Dinv32 : ctx->Dinv).as<T>();
+    if (phases) return form_strata<T>(ctx, L, D);
+    return factor_inverses<T>(ctx, L, D, ctx->Xinv.as<T>(), ctx->L21.as<T>(), ctx->L21T.as<T>(), ctx->Ttop.as<T>());
+}
+
 // Enqueues the dirty-deform setup in precision T (FP64: T = double for
 // everything; MIXED: T = float for the local step, RHS and solves, with the
 // factor in FP64 unless factor_bits is 32):
@@ -842,7 +1009,7 @@ int factor_inverses(arap_ctx *ctx, const TI *Lval, const TI *Dinv, TI *X, TI *L2
 // bFixed assembly, the factorisation plan. No host synchronisation; a failed
 // pivot shows up in the device error word.
 template <typename T>
-int setup_enqueue(arap_ctx *ctx) {
+int setup_enqueue(arap_ctx *ctx, bool phases) {
     const Symbolic &s = ctx->sym;
     const DevSym &d = ctx->ds;
     cudaStream_t st = ctx->stream;
@@ -850,10 +1017,12 @@ int setup_enqueue(arap_ctx *ctx) {
     // the solves' scheduling counters and flags restart with every set-up: a
     // launch consumes tickets in proportion to its grid, which differs
     // between the precisions
-    CK(cudaMemsetAsync(ctx->ticket.p, 0, kTickets * sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(unsigned) * (size_t)std::max(s.S, 1), st));
-    // and the dense top's arrival counters
-    if (ctx->ytop.p) CK(cudaMemsetAsync(ctx->ytop.p, 0, ctx->ytop.cap, st));
+    if (!phases) {
+        CK(cudaMemsetAsync(ctx->ticket.p, 0, kTickets * sizeof(unsigned long long), st));
+        CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(unsigned) * (size_t)std::max(s.S, 1), st));
+        // and the dense top's arrival counters
+        if (ctx->ytop.p) CK(cudaMemsetAsync(ctx->ytop.p, 0, ctx->ytop.cap, st));
+    }
     // cotan weights (arap.h:182-239)
     {
         Prof pr(ctx, ARAP_K_WEIGHTS);
@@ -888,18 +1057,29 @@ int setup_enqueue(arap_ctx *ctx) {
                 launch_demote(2, src, dst, n, st);
                 ctx->launches += 1;
             }
-            rc = factor_inverses<float>(ctx, ctx->Lval32.as<float>(), ctx->Dinv32.as<float>(), ctx->Xinv.as<float>(),
-                                        ctx->L21.as<float>(), ctx->L21T.as<float>(), ctx->Ttop.as<float>());
-            if (rc != ARAP_OK) return rc;
         } else {
             rc = factor_numeric<T>(ctx, ctx->Lval.as<T>(), ctx->Upd.as<T>(), ctx->Dinv.as<T>());
             if (rc != ARAP_OK) return rc;
-            rc = factor_inverses<T>(ctx, ctx->Lval.as<T>(), ctx->Dinv.as<T>(), ctx->Xinv.as<T>(), ctx->L21.as<T>(),
-                                    ctx->L21T.as<T>(), ctx->Ttop.as<T>());
-            if (rc != ARAP_OK) return rc;
         }
+        rc = form_solves<T>(ctx, phases);
+        if (rc != ARAP_OK) return rc;
     }
     CK(cudaGetLastError());
+    return ARAP_OK;
+}
+
+// Plan, buffers and solve arrays of the resident factorisation for what runs
+// next, where an earlier call left only the other kind (a pose batch the
+// sweeps' arrays, a deform the dense phases').
+template <typename T>
+int ensure_solves(arap_ctx *ctx, bool phases) {
+    if (phases ? ctx->strata_ready && ctx->strata_formed : ctx->sweeps_ready && ctx->sweeps_formed) return ARAP_OK;
+    int rc = phases ? prepare_strata<T>(ctx) : prepare_sweeps(ctx);
+    if (rc == ARAP_OK) rc = setup_alloc<T>(ctx, !phases, phases);
+    if (rc == ARAP_OK && ctx->sym.m > 0) rc = form_solves<T>(ctx, phases);
+    if (rc != ARAP_OK) return rc;
+    if (!phases && ctx->ytop.p) CK(cudaMemsetAsync(ctx->ytop.p, 0, ctx->ytop.cap, ctx->stream));
+    (phases ? ctx->strata_formed : ctx->sweeps_formed) = true;
     return ARAP_OK;
 }
 
@@ -985,6 +1165,7 @@ int run_iterations<double>(arap_ctx *ctx, int iterations) {
     cudaStream_t st = ctx->stream;
     unsigned long long *tk = ctx->ticket.as<unsigned long long>();
     unsigned *fl = ctx->flags.as<unsigned>();
+    const bool phases = use_strata(ctx, true);
     for (int it = 0; it < iterations; ++it) {
         {
             Prof pr(ctx, ARAP_K_LOCAL);
@@ -997,6 +1178,20 @@ int run_iterations<double>(arap_ctx *ctx, int iterations) {
             Prof pr(ctx, ARAP_K_RHS);
             launch_rhs<double>(d, ctx->w64.as<double>(), ctx->p64.as<Vec4<double>>(), ctx->R.as<Vec4<double>>(),
                                ctx->bfixed.as<Vec4<double>>(), ctx->sol.as<Vec4<double>>(), st);
+        }
+        if (phases) {
+            {
+                Prof pr(ctx, ARAP_K_SOLVE_FWD);
+                launch_strata_fwd<double>(ctx->std_, ctx->st_m.as<double>(), ctx->sol.as<Vec4<double>>(),
+                                          ctx->st_y.as<Vec4<double>>(), ctx->uvec.as<Vec4<double>>(),
+                                          ctx->st_ytop.as<Vec4<double>>(), ctx->errw.as<int>(), st);
+            }
+            Prof pr(ctx, ARAP_K_SOLVE_BWD);
+            launch_strata_bwd<double>(ctx->std_, d, ctx->st_m.as<double>(), ctx->sol.as<Vec4<double>>(),
+                                      ctx->st_y.as<Vec4<double>>(), ctx->st_ytop.as<Vec4<double>>(),
+                                      ctx->pc64.as<Vec4<double>>(), nullptr, 0, ctx->errw.as<int>(), st);
+            ctx->launches += strata_launches(ctx->std_, true) + strata_launches(ctx->std_, false) + 1;
+            continue;
         }
         {
             Prof pr(ctx, ARAP_K_SOLVE_FWD);
@@ -1025,6 +1220,7 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
     cudaStream_t st = ctx->stream;
     unsigned long long *tk = ctx->ticket.as<unsigned long long>();
     unsigned *fl = ctx->flags.as<unsigned>();
+    const bool phases = use_strata(ctx, false);
     for (int it = 0; it < iterations; ++it) {
         {
             Prof pr(ctx, ARAP_K_LOCAL);
@@ -1045,6 +1241,21 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
                 Prof pr(ctx, ARAP_K_RESIDUAL);
                 launch_residual(d, ctx->w64.as<double>(), ctx->diag64.as<double>(), ctx->bfixed.as<Vec4<double>>(),
                                 ctx->b.as<Vec4<float>>(), ctx->pc64.as<Vec4<double>>(), ctx->sol.as<Vec4<float>>(), st);
+            }
+            if (phases) {
+                {
+                    Prof pr(ctx, ARAP_K_SOLVE_FWD);
+                    launch_strata_fwd<float>(ctx->std_, ctx->st_m.as<float>(), ctx->sol.as<Vec4<float>>(),
+                                             ctx->st_y.as<Vec4<float>>(), ctx->uvec.as<Vec4<float>>(),
+                                             ctx->st_ytop.as<Vec4<float>>(), ctx->errw.as<int>(), st);
+                }
+                Prof pr(ctx, ARAP_K_SOLVE_BWD);
+                launch_strata_bwd<float>(ctx->std_, d, ctx->st_m.as<float>(), ctx->sol.as<Vec4<float>>(),
+                                         ctx->st_y.as<Vec4<float>>(), ctx->st_ytop.as<Vec4<float>>(),
+                                         ctx->pc64.as<Vec4<double>>(), ctx->pc32.as<Vec4<float>>(), 1,
+                                         ctx->errw.as<int>(), st);
+                ctx->launches += strata_launches(ctx->std_, true) + strata_launches(ctx->std_, false) + 1;
+                continue;
             }
             {
                 Prof pr(ctx, ARAP_K_SOLVE_FWD);
@@ -1411,15 +1622,22 @@ int arap_deform_poses_async(arap_ctx *ctx, int32_t n_poses, const double *target
         if (!ctx->sym_cache) ctx->sym_host = ctx->sym_valid = false;  // analyse again, as SimplicialLDLT::compute
         int rc = prepare_symbolic(ctx);
         if (rc != ARAP_OK) return rc;
-        rc = setup_alloc<float>(ctx);
+        rc = prepare_sweeps(ctx);
         if (rc != ARAP_OK) return rc;
-        rc = setup_enqueue<float>(ctx);
+        rc = setup_alloc<float>(ctx, true, false);
         if (rc != ARAP_OK) return rc;
+        rc = setup_enqueue<float>(ctx, false);
+        if (rc != ARAP_OK) return rc;
+        ctx->sweeps_formed = true;
+        ctx->strata_formed = false;
         // a failed pivot is reported by arap_wait (the device error word)
         ctx->retarget = false;
         ctx->state_prec = ARAP_PRECISION_MIXED;
         ctx->have_rotations = true;
         ctx->dirty = false;
+    } else {
+        const int rc = ensure_solves<float>(ctx, false);
+        if (rc != ARAP_OK) return rc;
     }
     const Symbolic &s = ctx->sym;
     const DevSym &d = ctx->use_sb ? ctx->dss : ctx->ds;  // the batched sweeps' layout (with the solve blocks)
@@ -1675,19 +1893,31 @@ int arap_deform_async(arap_ctx *ctx, int32_t iterations, double *out_xyz) {
             return fail(ctx, ARAP_ERR_UNSUPPORTED,
                         "supernode fronts too large for the FP64 solves' shared memory (the mixed form handles them)");
         h1 = HClock::now();
-        rc = fp64 ? setup_alloc<double>(ctx) : setup_alloc<float>(ctx);
+        const bool phases = use_strata(ctx, fp64);
+        if (!phases) rc = prepare_sweeps(ctx);
+        else rc = fp64 ? prepare_strata<double>(ctx) : prepare_strata<float>(ctx);
+        if (rc != ARAP_OK) return rc;
+        rc = fp64 ? setup_alloc<double>(ctx, !phases, phases) : setup_alloc<float>(ctx, !phases, phases);
         if (rc != ARAP_OK) return rc;
         h2 = HClock::now();
-        const int64_t key[4] = {ctx->gen, fp64 ? 1 : 2, fp64 ? 64 : ctx->factor_bits, 0};
+        const int64_t key[4] = {ctx->gen, fp64 ? 1 : 2, fp64 ? 64 : ctx->factor_bits, phases ? 1 : 0};
         rc = graph_or_direct(ctx, ctx->g_setup, ctx->g_setup_key, key, ctx->g_setup_launches, [&] {
-            return fp64 ? setup_enqueue<double>(ctx) : setup_enqueue<float>(ctx);
+            return fp64 ? setup_enqueue<double>(ctx, phases) : setup_enqueue<float>(ctx, phases);
         });
         if (rc != ARAP_OK) return rc;
+        ctx->strata_formed = phases;
+        ctx->sweeps_formed = !phases;
         ctx->state_prec = fp64 ? ARAP_PRECISION_FP64 : ARAP_PRECISION_MIXED;
         ctx->have_rotations = true;
         ctx->dirty = false;
         ctx->retarget = false;
-    } else if (ctx->retarget) {
+    } else {
+        const bool st64 = ctx->state_prec == ARAP_PRECISION_FP64;
+        const bool phases = use_strata(ctx, st64);
+        const int rc = st64 ? ensure_solves<double>(ctx, phases) : ensure_solves<float>(ctx, phases);
+        if (rc != ARAP_OK) return rc;
+    }
+    if (ctx->retarget) {
         const int rc = ctx->state_prec == ARAP_PRECISION_FP64 ? retarget_enqueue<double>(ctx)
                                                                : retarget_enqueue<float>(ctx);
         if (rc != ARAP_OK) return rc;
@@ -2189,8 +2419,10 @@ int arap_plan_bytes(arap_ctx *ctx, int32_t n_poses, int64_t *bytes) {
     if (!ctx->cidx.empty()) {
         const int rc = analyze_symbolic(ctx);
         if (rc != ARAP_OK) return rc;
-        if (ctx->precision == ARAP_PRECISION_FP64 && n_poses == 0) planned_sizes<double>(ctx, 0, plan);
-        else planned_sizes<float>(ctx, n_poses, plan);
+        const bool fp64 = ctx->precision == ARAP_PRECISION_FP64 && n_poses == 0;
+        const bool phases = use_strata(ctx, fp64);
+        if (fp64) planned_sizes<double>(ctx, 0, !phases, phases, plan);
+        else planned_sizes<float>(ctx, n_poses, !phases || n_poses > 0, phases, plan);
     }
     for (DevBuf *b : ctx->buffers()) {
         size_t want = b->cap;
@@ -2307,7 +2539,10 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         break;
     case ARAP_K_SOLVE_FWD:
     case ARAP_K_SOLVE_BWD:
-        if (ctx->model_batched) {  // lower matrices once per pose tile, T once, vectors once per pose
+        if (!ctx->model_batched && use_strata(ctx, sz == 8.0)) {  // the groups' matrices once, vectors in and out
+            B = ctx->strata.entries * sz + (m + ctx->strata.nb_sum) * 3 * sz * 2;
+            FL = ctx->strata.entries * 6;
+        } else if (ctx->model_batched) {  // lower matrices once per pose tile, T once, vectors once per pose
             B = (T * (xlow_lo + l21_lo) + tri) * sz + P * vec;
             FL = P * (xlow_lo + l21_lo + tri) * 6;
         } else {

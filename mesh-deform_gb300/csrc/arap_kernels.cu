@@ -792,7 +792,7 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
             const int c = cg * 4 + cc, i = i0 + r;
             if (c >= wj) continue;
             X[(int64_t)(j0 + c) * ldx + i] = v[cc];
-            if (i >= j0 + c) XT[(int64_t)i * ldx + j0 + c] = v[cc];
+            if (L21all && i >= j0 + c) XT[(int64_t)i * ldx + j0 + c] = v[cc];
         }
     };
     {
@@ -852,6 +852,7 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
         __syncthreads();  // Ts and Ds are rewritten by the next block row
     }
     // rows of X above the block column stay as set up: zero (X is lower triangular)
+    if (!L21all) return;  // the dense phases read X alone
     TF *L21 = L21all + d.l21_off, *L21T = L21Tall + d.l21t_off;
     const int ld21 = d.ld21;
     for (int q = tid; q < wj * nb; q += kFactorThreads) {
@@ -2029,6 +2030,9 @@ k_solve_bwd_top(int S, int Z, SolveSmem lay, const int32_t *__restrict__ order, 
 }
 
 // ---------------------------------------------------------------------------
+#include "arap_strata.cuh"
+
+// ---------------------------------------------------------------------------
 // Dense top of the elimination tree. The top levels hold few supernodes, and
 // each is one CTA's task on the sweeps' critical path. For them the factor's
 // restriction L_top (n_top <= a few thousand columns, in elimination order)
@@ -3173,6 +3177,183 @@ cudaError_t configure_dense_smem(int inv32, int inv64) {
     if (e == cudaSuccess) e = raise_smem_limit((const void *)k_top_pair_bwd<double>, (int)top_pair_smem(8));
     return e;
 }
+
+// ---------------------------------------------------------------------------
+// dense-phase solves
+
+static int st_ldf(const StPhase &p) { return (p.nmax + 127) & ~127; }
+static size_t st_fwd_smem(const StPhase &p, int sb) { return (size_t)3 * st_ldf(p) * sb; }
+static size_t st_bwd_smem(const StPhase &p, int sb) {
+    return (size_t)p.vmax * 4 * sb + (size_t)kStThreads * (16 / sb) * 4 * sb;
+}
+// columns per pass of the inversion whose buffers fit shared memory (0: none)
+static int st_inv_cols(const StPhase &p, int sb) {
+    for (int rc = kStInvCols; rc >= 2; rc /= 2)
+        if (dense_inverse_smem_bytes(p.ldx, p.ld21, sb, rc) <= 200 * 1024) return rc;
+    return 0;
+}
+
+bool strata_fits(const Strata &st, int sb) {
+    for (const StPhase &p : st.ph)
+        if (st_inv_cols(p, sb) == 0 || (!p.big && (st_fwd_smem(p, sb) > 200 * 1024 || st_bwd_smem(p, sb) > 200 * 1024)))
+            return false;
+    return true;
+}
+
+template <typename T, int G, int RW> static cudaError_t raise_st_fwd(int bytes) {
+    return raise_smem_limit((const void *)k_strata_fwd<T, G, RW>, bytes);
+}
+template <typename T> static cudaError_t configure_strata_t(const Strata &st) {
+    size_t f = 0, b = 0, v = 0;
+    for (const StPhase &p : st.ph) {
+        v = std::max(v, dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), st_inv_cols(p, sizeof(T))));
+        if (p.big) continue;
+        f = std::max(f, st_fwd_smem(p, sizeof(T)));
+        b = std::max(b, st_bwd_smem(p, sizeof(T)));
+    }
+    cudaError_t e = cudaSuccess;
+    auto up = [&](cudaError_t r) {
+        if (e == cudaSuccess) e = r;
+    };
+    if constexpr (sizeof(T) == 8) {
+        up(raise_st_fwd<T, 1, 1>((int)f));
+        up(raise_st_fwd<T, 4, 1>((int)f));
+    } else {
+        up(raise_st_fwd<T, 8, 2>((int)f));
+        up(raise_st_fwd<T, 8, 4>((int)f));
+        up(raise_st_fwd<T, 32, 2>((int)f));
+        up(raise_st_fwd<T, 32, 4>((int)f));
+    }
+    up(raise_st_fwd<T, 8, 1>((int)f));
+    up(raise_st_fwd<T, 32, 1>((int)f));
+    up(raise_smem_limit((const void *)k_strata_bwd<T, 4>, (int)b));
+    up(raise_smem_limit((const void *)k_strata_bwd<T, 8>, (int)b));
+    up(raise_smem_limit((const void *)k_strata_bwd<T, 16>, (int)b));
+    up(raise_smem_limit((const void *)k_strata_bwd<T, 32>, (int)b));
+    up(raise_smem_limit((const void *)k_strata_bwd<T, 64>, (int)b));
+    up(raise_smem_limit((const void *)k_strata_inverse<T, 8>, (int)v));
+    up(raise_smem_limit((const void *)k_strata_inverse<T, 4>, (int)v));
+    up(raise_smem_limit((const void *)k_strata_inverse<T, 2>, (int)v));
+    if (st.big_n > 0) {
+        up(raise_smem_limit((const void *)k_top_pair_fwd<T>, (int)top_pair_smem(sizeof(T))));
+        up(raise_smem_limit((const void *)k_top_pair_bwd<T>, (int)top_pair_smem(sizeof(T))));
+    }
+    return e;
+}
+cudaError_t configure_strata(const Strata &st, int sb) {
+    return sb == 4 ? configure_strata_t<float>(st) : configure_strata_t<double>(st);
+}
+
+int strata_launches(const StrataDev &d, bool forward) {
+    int n = d.nph;
+    for (int k = 1; forward && k < d.nph; ++k) n += !d.ph[k].big;
+    return n;
+}
+
+template <typename T>
+void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *X, const T *Lval, T *M, cudaStream_t st) {
+    for (int k = d.nph - 1; k >= 0; --k) {
+        const StPhase &p = d.ph[k];
+        const int rc = st_inv_cols(p, sizeof(T));
+        const size_t smem = dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), rc);
+#define ARAP_STINV(R)                                                                                              \
+    k_strata_inverse<T, R><<<p.in, kStThreads, smem, st>>>(d.items + 2 * (size_t)p.i0, s.sn, d.sn, s.relind, X, Lval, \
+                                                           p.ldx, p.ld21, M)
+        switch (rc) {
+        case 8: ARAP_STINV(8); break;
+        case 4: ARAP_STINV(4); break;
+        default: ARAP_STINV(2); break;
+        }
+#undef ARAP_STINV
+    }
+}
+
+template <typename T>
+void launch_strata_fwd(const StrataDev &d, const T *M, Vec4<T> *sol, Vec4<T> *y, Vec4<T> *uvec, Vec4<T> *ytop,
+                       int *err, cudaStream_t st) {
+    for (int k = 0; k < d.nph; ++k) {
+        const StPhase &p = d.ph[k];
+        if (p.big) {
+            const int n = d.big_n, ldt = dense_ld(n);
+            Vec4<T> *part = ytop + ldt;
+            unsigned *cnt = reinterpret_cast<unsigned *>(part + top_tiles(n) * kTopTile);
+            if ((sizeof(T) == 4 ? d.big_pair32 : d.big_pair64) != 0)
+                launch_pdl(k_top_pair_fwd<T>, d.overlap != 0, (int)top_pairs(n), 256, top_pair_smem(sizeof(T)), st, n,
+                           ldt, top_blocks(n), M + d.big_off, d.top_col, d.top_gptr, d.top_gidx, (const Vec4<T> *)sol,
+                           (const Vec4<T> *)uvec, part, cnt, ytop, err);
+            else
+                launch_pdl(k_top_tile_fwd<T>, d.overlap != 0, (int)top_tiles(n), 256, 0, st, n, ldt, M + d.big_off,
+                           d.top_col, d.top_gptr, d.top_gidx, (const Vec4<T> *)sol, (const Vec4<T> *)uvec, part, cnt,
+                           ytop);
+            continue;
+        }
+        if (k > 0)  // no update lands on the first stratum
+            launch_pdl(k_strata_gather<T>, d.overlap != 0, blocks_for(4 * (int64_t)p.cn, kStThreads), kStThreads, 0, st, p.c0, p.cn,
+                       d.col, d.gptr, d.gidx, (const Vec4<T> *)uvec, sol);
+        const int grid = d.grid_cap > 0 ? std::min(d.grid_cap, (int)p.fn) : p.fn;
+        const size_t smem = st_fwd_smem(p, sizeof(T));
+#define ARAP_STF(G, RW)                                                                                        \
+    launch_pdl(k_strata_fwd<T, G, RW>, d.overlap != 0, grid, kStThreads, smem, st, (int)p.fn, st_ldf(p),       \
+               d.tiles + p.f0, M, d.col, (const Vec4<T> *)sol, y, uvec)
+        if constexpr (sizeof(T) == 8) {  // one row per lane group (build_strata)
+            if (p.G == 1) ARAP_STF(1, 1);
+            else if (p.G == 4) ARAP_STF(4, 1);
+            else if (p.G == 8) ARAP_STF(8, 1);
+            else ARAP_STF(32, 1);
+        } else if (p.G == 8) {
+            if (p.RW == 4) ARAP_STF(8, 4);
+            else if (p.RW == 2) ARAP_STF(8, 2);
+            else ARAP_STF(8, 1);
+        } else {
+            if (p.RW == 4) ARAP_STF(32, 4);
+            else if (p.RW == 2) ARAP_STF(32, 2);
+            else ARAP_STF(32, 1);
+        }
+#undef ARAP_STF
+    }
+}
+
+template <typename T>
+void launch_strata_bwd(const StrataDev &d, const DevSym &s, const T *M, Vec4<T> *sol, const Vec4<T> *y,
+                       const Vec4<T> *ytop, Vec4<double> *pc64, Vec4<float> *pc32, int mode, int *err,
+                       cudaStream_t st) {
+    for (int k = d.nph - 1; k >= 0; --k) {
+        const StPhase &p = d.ph[k];
+        if (p.big) {
+            const int n = d.big_n, ldt = dense_ld(n);
+            Vec4<T> *part = const_cast<Vec4<T> *>(ytop) + ldt;
+            unsigned *cnt = reinterpret_cast<unsigned *>(part + top_tiles(n) * kTopTile);
+            if ((sizeof(T) == 4 ? d.big_pair32 : d.big_pair64) != 0)
+                launch_pdl(k_top_pair_bwd<T>, d.overlap != 0, (int)top_pairs(n), 256, top_pair_smem(sizeof(T)), st, n,
+                           ldt, top_blocks(n), M + d.big_off, ytop, part, cnt, d.top_col, sol, pc64, pc32, mode, err);
+            else
+                launch_pdl(k_top_tile_bwd<T>, d.overlap != 0, (int)top_tiles(n), 256, 0, st, n, ldt, top_blocks(n),
+                           M + d.big_off, ytop, part, cnt, d.top_col, sol, pc64, pc32, mode);
+            continue;
+        }
+        const int grid = d.grid_cap > 0 ? std::min(d.grid_cap, (int)p.bn) : p.bn;
+        const size_t smem = st_bwd_smem(p, sizeof(T));
+#define ARAP_STB(TC)                                                                                             \
+    launch_pdl(k_strata_bwd<T, TC>, d.overlap != 0, grid, kStThreads, smem, st, (int)p.bn, (int)p.vmax,          \
+               d.tiles + p.b0, M, d.col, s.rows, y, sol, pc64, mode)
+        if (p.TC == 64) ARAP_STB(64);
+        else if (p.TC == 32) ARAP_STB(32);
+        else if (p.TC == 16) ARAP_STB(16);
+        else if (p.TC == 8) ARAP_STB(8);
+        else ARAP_STB(4);
+#undef ARAP_STB
+    }
+}
+
+#define ARAP_ST_INST(T)                                                                                              \
+    template void launch_strata_inverse<T>(const StrataDev &, const DevSym &, const T *, const T *, T *, cudaStream_t); \
+    template void launch_strata_fwd<T>(const StrataDev &, const T *, Vec4<T> *, Vec4<T> *, Vec4<T> *, Vec4<T> *, int *, \
+                                       cudaStream_t);                                                                \
+    template void launch_strata_bwd<T>(const StrataDev &, const DevSym &, const T *, Vec4<T> *, const Vec4<T> *,     \
+                                       const Vec4<T> *, Vec4<double> *, Vec4<float> *, int, int *, cudaStream_t)
+ARAP_ST_INST(float);
+ARAP_ST_INST(double);
+#undef ARAP_ST_INST
 
 int energy_partials(int V) { return std::max(1, blocks_for(V, kEnergyThreads)); }
 

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "arap_strata.h"
 #include "arap_symbolic.h"
 
 namespace arapgpu {
@@ -210,6 +211,35 @@ void launch_solve_bwd(const DevSym &s, const T *X, const T *L21T, Vec4<T> *sol, 
 // above the diagonal), followed by T^T in the same layout
 template <typename T>
 void launch_top_inverse(const DevSym &s, const T *X, const T *L21, T *Tt, cudaStream_t st);
+// ---- the dense-phase solves (arap_strata.h)
+struct StrataDev {
+    int nph;
+    StPhase ph[kStMaxPhases];
+    int grid_cap;  // most CTAs per launch (0: a CTA per tile)
+    int overlap;   // as DevSym::overlap
+    int big_n, big_pair32, big_pair64;
+    int64_t big_off;
+    const StTile *tiles;
+    const StSn *sn;
+    const int32_t *col, *gptr, *gidx, *items;
+    const int32_t *top_col, *top_gptr;
+    const int64_t *top_gidx;
+};
+// whether the phases' kernels can hold their vectors, and their shared-memory limits
+bool strata_fits(const Strata &p, int scalar_bytes);
+cudaError_t configure_strata(const Strata &p, int scalar_bytes);
+int strata_launches(const StrataDev &d, bool forward);
+// M of every group from the supernodes' X (k_fx) and panels; M's zeros stay as they are
+template <typename T>
+void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *X, const T *Lval, T *M, cudaStream_t st);
+// sol: right-hand side in, solution out; y: the forward sweep's result
+template <typename T>
+void launch_strata_fwd(const StrataDev &d, const T *M, Vec4<T> *sol, Vec4<T> *y, Vec4<T> *uvec, Vec4<T> *ytop,
+                       int *err, cudaStream_t st);
+template <typename T>
+void launch_strata_bwd(const StrataDev &d, const DevSym &s, const T *M, Vec4<T> *sol, const Vec4<T> *y,
+                       const Vec4<T> *ytop, Vec4<double> *pc64, Vec4<float> *pc32, int mode, int *err,
+                       cudaStream_t st);
 size_t dense_inverse_smem_bytes(int ldx_max, int ld21_max, int scalar_bytes, int rc);
 // columns per pass of the inversion whose buffers fit shared memory (0: none)
 int dense_inverse_rhs(int ldx_max, int ld21_max, int scalar_bytes);

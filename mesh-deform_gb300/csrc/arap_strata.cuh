@@ -1,0 +1,475 @@
+// arap_strata.cuh -- kernels of the dense-phase triangular solves
+// (arap_strata.h): forward and backward products of one stratum's groups, the
+// gather of a stratum's right-hand sides, and the groups' matrices from the
+// factor. Included by arap_kernels.cu.
+
+// 16 bytes of T
+template <typename T> struct StPack;
+template <> struct StPack<float> {
+    static constexpr int E = 4;
+    float v[4];
+    __device__ __forceinline__ void load(const float *p) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    }
+    __device__ __forceinline__ void lds(const float *p) {
+        const float4 q = *reinterpret_cast<const float4 *>(p);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    }
+};
+template <> struct StPack<double> {
+    static constexpr int E = 2;
+    double v[2];
+    __device__ __forceinline__ void load(const double *p) {
+        const double2 q = __ldg(reinterpret_cast<const double2 *>(p));
+        v[0] = q.x; v[1] = q.y;
+    }
+    __device__ __forceinline__ void lds(const double *p) {
+        const double2 q = *reinterpret_cast<const double2 *>(p);
+        v[0] = q.x; v[1] = q.y;
+    }
+};
+
+__device__ __forceinline__ StTile st_tile(const StTile *p) {
+    const int4 *q = reinterpret_cast<const int4 *>(p);
+    const int4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+    StTile t;
+    t.m_off = (int64_t)(unsigned)a.x | ((int64_t)a.y << 32);
+    t.n = a.z; t.r = a.w;
+    t.ld = b.x; t.first = b.y; t.count = b.z; t.col_off = b.w;
+    t.row_off = c.x; t.u_off = c.y;
+    t.base = c.z;
+    t.pad = 0;
+    return t;
+}
+
+// Sums NV values over the G lanes of an aligned lane group by recursive
+// halving: while values are left to split, each exchange halves the values a
+// lane carries, so NV values cost about NV additions instead of NV log2 G
+// (FP64 additions are the scarce instructions here). Afterwards a lane holds
+// st_held values from st_base on; true: a copy of another lane's.
+template <int NV, int G, typename T>
+__device__ __forceinline__ bool st_reduce(T (&v)[NV], int lane) {
+    bool dup = false;
+    int h = NV;
+#pragma unroll
+    for (int off = G / 2; off >= 1; off >>= 1) {
+        if (h > 1) {
+            h >>= 1;
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < NV / 2; ++i)
+                if (i < h) {
+                    const T send = up ? v[i] : v[i + h];
+                    const T keep = up ? v[i + h] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+            dup = dup || (lane & off) != 0;
+        }
+    }
+    return dup;
+}
+// index of the first value a lane holds afterwards, and how many it holds
+template <int NV, int G>
+__device__ __forceinline__ int st_base(int lane) {
+    int base = 0, h = NV;
+#pragma unroll
+    for (int off = G / 2; off >= 1; off >>= 1)
+        if (h > 1) {
+            h >>= 1;
+            if (lane & off) base += h;
+        }
+    return base;
+}
+template <int NV, int G> constexpr int st_held() {
+    int h = NV, off = G;
+    while (h > 1 && off > 1) {
+        h /= 2;
+        off /= 2;
+    }
+    return h;
+}
+
+// b[k] += the update entries of column k, for a stratum's columns, as a launch
+// of its own: four threads per column, each an index quad at a time (its
+// entries' loads in flight together), so that no thread runs a long chain of
+// additions. 2.8 us on the bar's second stratum (10,538 columns); gathered
+// inside the forward product instead, once per row tile, that product took
+// 10.3 us against 7 (and in FP64 60% of its additions).
+template <typename T>
+__global__ void __launch_bounds__(kStThreads)
+k_strata_gather(int c0, int cn, const int32_t *__restrict__ gcol, const int32_t *__restrict__ gptr,
+                const int32_t *__restrict__ gidx, const Vec4<T> *uvec, Vec4<T> *b) {
+    pdl_trigger();
+    const int c = (blockIdx.x * kStThreads + threadIdx.x) >> 2, j = threadIdx.x & 3;
+    int q0 = 0, q1 = 0, k = 0;
+    int4 id{-1, -1, -1, -1};
+    const int4 *gq = reinterpret_cast<const int4 *>(gidx);
+    if (c < cn) {
+        k = gcol[c0 + c];
+        q0 = gptr[c0 + c] + j;
+        q1 = gptr[c0 + c + 1];
+        if (q0 < q1) id = __ldg(gq + q0);
+    }
+    pdl_wait();
+    const Vec4<T> zero{(T)0, (T)0, (T)0, (T)0};
+    Vec4<T> v = (j == 0 && c < cn) ? ldcg4(b + k) : zero;
+    for (int q = q0; q < q1; q += 4) {
+        if (q > q0) id = __ldg(gq + q);
+        const Vec4<T> u0 = ldcg4(uvec + id.x);
+        const Vec4<T> u1 = id.y >= 0 ? ldcg4(uvec + id.y) : zero;
+        const Vec4<T> u2 = id.z >= 0 ? ldcg4(uvec + id.z) : zero;
+        const Vec4<T> u3 = id.w >= 0 ? ldcg4(uvec + id.w) : zero;
+        v.x += (u0.x + u1.x) + (u2.x + u3.x);
+        v.y += (u0.y + u1.y) + (u2.y + u3.y);
+        v.z += (u0.z + u1.z) + (u2.z + u3.z);
+    }
+#pragma unroll
+    for (int off = 1; off <= 2; off <<= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+        v.z += __shfl_xor_sync(0xffffffffu, v.z, off);
+    }
+    if (j == 0 && c < cn) b[k] = v;
+}
+
+// Forward product of a stratum: out = M f for the rows of a tile, y = X f
+// into y and u = -W f into the update vectors. A group of G lanes takes RW
+// rows at a time, each lane 16 bytes of every row per step (consecutive lanes
+// consecutive columns), with f as three arrays in shared memory so that a
+// lane's four (two) columns come with one 16-byte load per component. A CTA's
+// first loads of M (which only the factorisation writes) are issued before it
+// waits for the kernel before it.
+// FP32: bound by the launch's latency chain (tile, vector, product, store),
+// not by L2: the bar's first stratum, 12 MB in 7.7 us. Eight CTAs per SM with
+// four loads in flight per lane beat four with eight (bar 164 -> 145 us per
+// iteration). FP64: bound by FP64 issue (about 64 clocks per warp instruction
+// and scheduler), so lanes that share a row are as few as fill the device.
+template <typename T, int G, int RW>
+__global__ void __launch_bounds__(kStThreads, 8)
+k_strata_fwd(int ntiles, int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
+             const int32_t *__restrict__ gcol, const Vec4<T> *__restrict__ b, Vec4<T> *__restrict__ y,
+             Vec4<T> *__restrict__ uvec) {
+    extern __shared__ __align__(128) unsigned char st_raw[];
+    constexpr int E = StPack<T>::E;
+    constexpr int NB = 4 / RW;  // steps of one batch of loads: four 16-byte loads in flight per lane
+    constexpr int kRows = kStThreads / G * RW;
+    T *fx = reinterpret_cast<T *>(st_raw), *fy = fx + ldf, *fz = fy + ldf;
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, l = tid % G, grp = tid / G;
+    bool waited = false;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const StTile d = st_tile(tiles + t);
+        const T *M = Mall + d.m_off;
+        const int rend = d.first + d.count;
+        // X is lower triangular: a warp's columns end at its last row's
+        auto cols_to = [&](int last) {
+            const int nc = last > d.n ? d.n : last;
+            return (nc + G * E - 1) / (G * E) * (G * E);
+        };
+        const int ncol = rend > d.n ? d.n : rend, fspan = cols_to(rend);
+        int span = cols_to(min(rend, d.first + (grp | (32 / G - 1)) * RW + RW));
+        // column c of the group: consecutive ones in the first phase (whole subtrees)
+        auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
+        StPack<T> m[NB][RW];
+        auto load = [&](int row, int c) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+#pragma unroll
+                for (int i = 0; i < RW; ++i) {
+                    const int cc = c + k * G * E;
+                    if (cc < d.ld && cc < span && row + i < rend) m[k][i].load(M + (int64_t)(row + i) * d.ld + cc);
+                    else
+#pragma unroll
+                        for (int e = 0; e < E; ++e) m[k][i].v[e] = (T)0;
+                }
+        };
+        int row = d.first + grp * RW;
+        load(row, l * E);
+        // the places of f before the wait, f after it
+        constexpr int kPre = 2;
+        int at[kPre];
+#pragma unroll
+        for (int i = 0; i < kPre; ++i) at[i] = tid + i * kStThreads < ncol ? column(tid + i * kStThreads) : -1;
+        if (!waited) {
+            pdl_wait();
+            waited = true;
+        }
+        auto put = [&](int c, int k) {
+            const Vec4<T> v = k >= 0 ? ldcg4(b + k) : Vec4<T>{(T)0, (T)0, (T)0, (T)0};
+            fx[c] = v.x;
+            fy[c] = v.y;
+            fz[c] = v.z;
+        };
+#pragma unroll
+        for (int i = 0; i < kPre; ++i)
+            if (tid + i * kStThreads < fspan) put(tid + i * kStThreads, at[i]);
+        for (int c = tid + kPre * kStThreads; c < fspan; c += kStThreads) put(c, c < ncol ? column(c) : -1);
+        __syncthreads();
+        for (int r0 = d.first; r0 < rend; r0 += kRows) {
+            row = r0 + grp * RW;
+            span = cols_to(min(rend, r0 + (grp | (32 / G - 1)) * RW + RW));
+            constexpr int H = st_held<RW * 4, G>();
+            // the value(s) this lane will hold after the reduction go to one row
+            const int orow = row + (st_base<RW * 4, G>(lane) >> 2);
+            const int ocol = orow < rend && orow < d.n ? column(orow) : 0;
+            T acc[RW * 4];
+#pragma unroll
+            for (int i = 0; i < RW * 4; ++i) acc[i] = (T)0;
+            for (int c = l * E; c < span; c += NB * G * E) {
+                if (r0 > d.first || c >= NB * G * E) load(row, c);
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const int cc = c + k * G * E;
+                    if (cc >= span) break;
+                    StPack<T> px, py, pz;
+                    px.lds(fx + cc);
+                    py.lds(fy + cc);
+                    pz.lds(fz + cc);
+#pragma unroll
+                    for (int i = 0; i < RW; ++i)
+#pragma unroll
+                        for (int e = 0; e < E; ++e) {
+                            acc[4 * i] += m[k][i].v[e] * px.v[e];
+                            acc[4 * i + 1] += m[k][i].v[e] * py.v[e];
+                            acc[4 * i + 2] += m[k][i].v[e] * pz.v[e];
+                        }
+                }
+            }
+            const bool dup = st_reduce<RW * 4, G>(acc, lane);
+            const int base = st_base<RW * 4, G>(lane);
+            if (!dup && orow < rend) {
+                T *dst = reinterpret_cast<T *>(orow < d.n ? y + ocol : uvec + d.u_off + (orow - d.n));
+#pragma unroll
+                for (int j = 0; j < H; ++j) {
+                    const int comp = (base + j) & 3;
+                    if (comp < 3) dst[comp] = orow < d.n ? acc[j] : -acc[j];
+                }
+            }
+        }
+        __syncthreads();  // f is rewritten by the CTA's next tile
+    }
+    if (!waited) pdl_wait();
+}
+
+// Backward product of a stratum: x = M^T v for TC columns of a group, v = y on
+// its own rows and -x on the rows below it (solved by the launches before).
+// 16 bytes of a row per thread, TC / E threads per row, the rows dealt to the
+// thread groups in turn; their sums meet in shared memory in a fixed order.
+// Bound as the forward product; 64 columns per tile where that leaves two
+// CTAs per SM (bar 143 -> 139 us per iteration, 16 bars 318 -> 305, against
+// 32), fewer for small strata.
+// x goes to the solution and the positions (mode 0: pc64 = x, 1: pc64 += x).
+template <typename T, int TC>
+__global__ void __launch_bounds__(kStThreads)
+k_strata_bwd(int ntiles, int vmax, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
+             const int32_t *__restrict__ gcol, const int32_t *__restrict__ rows, const Vec4<T> *__restrict__ y,
+             Vec4<T> *sol, Vec4<double> *__restrict__ pc64, int mode) {
+    extern __shared__ __align__(128) unsigned char st_raw[];
+    constexpr int E = StPack<T>::E, QC = TC / E, NS = kStThreads / QC, U = 8;
+    Vec4<T> *v = reinterpret_cast<Vec4<T> *>(st_raw);
+    T *red = reinterpret_cast<T *>(v + vmax);  // NS x (TC columns x 4)
+    pdl_trigger();
+    const int tid = threadIdx.x, q = tid % QC, s = tid / QC;
+    bool waited = false;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const StTile d = st_tile(tiles + t);
+        const T *M = Mall + d.m_off + (int64_t)d.first * d.ld + d.first + q * E;
+        const int nrow = d.n + d.r - d.first;  // X is lower triangular: rows from the tile's first column on
+        const bool in = d.first + q * E < d.ld;
+        StPack<T> m[U];
+        auto load = [&](int r) {
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                if (in && r + i * NS < nrow) m[i].load(M + (int64_t)(r + i * NS) * d.ld);
+                else
+#pragma unroll
+                    for (int e = 0; e < E; ++e) m[i].v[e] = (T)0;
+            }
+        };
+        load(s);
+        // the vector's places before the wait, the vector after it
+        auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
+        constexpr int kPre = 4;
+        int at[kPre];
+#pragma unroll
+        for (int i = 0; i < kPre; ++i) {
+            const int r = tid + i * kStThreads, g = d.first + r;
+            at[i] = r < nrow ? (g < d.n ? column(g) : rows[d.row_off + g - d.n]) : 0;
+        }
+        if (!waited) {
+            pdl_wait();
+            waited = true;
+        }
+        // kSh threads per output value, each every kSh-th partial sum, kOut
+        // values per thread; the outputs' places and positions are loaded
+        // ahead of the product
+        constexpr int kSh = 4 * TC < kStThreads ? kStThreads / (4 * TC) : 1;
+        constexpr int kOut = 4 * TC > kStThreads ? 4 * TC / kStThreads : 1;
+        const int h = tid % kSh;
+        int ok[kOut];
+        double before[kOut];
+#pragma unroll
+        for (int j = 0; j < kOut; ++j) {
+            const int o = tid / kSh + j * kStThreads, oc = o >> 2, comp = o & 3;
+            ok[j] = h == 0 && comp < 3 && oc < d.count ? column(d.first + oc) : -1;
+            before[j] = ok[j] >= 0 && mode != 0 ? __ldcg(reinterpret_cast<const double *>(pc64 + ok[j]) + comp) : 0.0;
+        }
+        auto put = [&](int r, int k) {
+            const bool own = d.first + r < d.n;
+            Vec4<T> x = ldcg4((own ? y : (const Vec4<T> *)sol) + k);
+            if (!own) x = {-x.x, -x.y, -x.z, (T)0};
+            v[r] = x;
+        };
+#pragma unroll
+        for (int i = 0; i < kPre; ++i) {
+            const int r = tid + i * kStThreads;
+            if (r < nrow) put(r, at[i]);
+        }
+        for (int r = tid + kPre * kStThreads; r < nrow; r += kStThreads) {
+            const int g = d.first + r;
+            put(r, g < d.n ? column(g) : rows[d.row_off + g - d.n]);
+        }
+        __syncthreads();
+        T acc[E][3];
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e][0] = acc[e][1] = acc[e][2] = (T)0;
+        for (int r = s; r < nrow; r += U * NS) {
+            if (r != s) load(r);
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                if (r + i * NS >= nrow) break;
+                const Vec4<T> x = v[r + i * NS];
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    acc[e][0] += m[i].v[e] * x.x;
+                    acc[e][1] += m[i].v[e] * x.y;
+                    acc[e][2] += m[i].v[e] * x.z;
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) red[(s * TC + q * E + e) * 4 + c] = acc[e][c];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kOut; ++j) {
+            const int o = tid / kSh + j * kStThreads, comp = o & 3;
+            T sum = (T)0;
+#pragma unroll 8
+            for (int i = h; i < NS; i += kSh) sum += red[i * TC * 4 + o];
+#pragma unroll
+            for (int off = 1; off < kSh; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            if (ok[j] >= 0) {
+                reinterpret_cast<T *>(sol + ok[j])[comp] = sum;
+                reinterpret_cast<double *>(pc64 + ok[j])[comp] = mode == 0 ? (double)sum : before[j] + (double)sum;
+            }
+        }
+        __syncthreads();  // v and the sums are rewritten by the CTA's next tile
+    }
+    if (!waited) pdl_wait();
+}
+
+// RC columns [c0, c0 + RC) of supernode j's columns of its group's M: the
+// forward solve of L_gg Y = E (E the identity columns) along j's ancestors in
+// the group, supernode by supernode: Y_a = X_a F_a, U = F_b - L21_a Y_a with
+// F the update rows scattered into the parent's front. The Y are X's rows;
+// past the group's root, -U is W. Zeros of M (above the diagonal, and between
+// subtrees that do not meet) are never written: they are cleared once when
+// the matrices are laid out.
+template <typename T, int RC>
+__global__ void __launch_bounds__(kStThreads)
+k_strata_inverse(const int32_t *__restrict__ items, const SnInfo *__restrict__ sn, const StSn *__restrict__ ssn,
+                 const int32_t *__restrict__ relind, const T *__restrict__ Xall, const T *__restrict__ Lval,
+                 int ldx_max, int ld21_max, T *__restrict__ Mall) {
+    extern __shared__ __align__(128) unsigned char st_raw[];
+    T *Y = reinterpret_cast<T *>(st_raw);   // [row][RC], rows of the current supernode's columns
+    T *U = Y + (size_t)ldx_max * RC;        // [row][RC], its struct rows
+    T *F = U + (size_t)ld21_max * RC;       // the parent's front: columns
+    T *Fb = F + (size_t)ldx_max * RC;       // and struct rows
+    const int tid = threadIdx.x;
+    const int j = items[2 * blockIdx.x];
+    const SnInfo dj = sn[j];
+    const StSn gj = ssn[j];
+    for (int c0 = items[2 * blockIdx.x + 1], ce = min(c0 + kStInvCols, dj.ncol); c0 < ce; c0 += RC) {
+        const int w = min(RC, dj.ncol - c0);
+        T *M = Mall + gj.m_off + gj.pos + c0;  // the block's first column
+        {
+            const T *X = Xall + dj.x_off;
+            for (int q = tid; q < dj.ncol * RC; q += kStThreads) {
+                const int r = q / RC, c = q % RC;
+                const T x = (c < w && r >= c0 + c) ? X[(int64_t)(c0 + c) * dj.ldx + r] : (T)0;
+                Y[q] = x;
+                if (c < w && r >= c0 + c) M[(int64_t)(gj.pos + r) * gj.ld + c] = x;
+            }
+        }
+        __syncthreads();
+        int node = j, kfirst = c0;  // Y's rows before kfirst are zero
+        SnInfo dn = dj;
+        for (;;) {
+            const int nbn = dn.nrow - dn.ncol;
+            const T *L21 = Lval + dn.panel_off + dn.ncol;
+            const bool first = node == j, root = ssn[node].root != 0;
+            for (int r = tid; r < nbn; r += kStThreads) {
+                T acc[RC];
+#pragma unroll
+                for (int c = 0; c < RC; ++c) acc[c] = first ? (T)0 : Fb[r * RC + c];
+#pragma unroll 4
+                for (int k = kfirst; k < dn.ncol; ++k) {
+                    const T x = L21[(int64_t)k * dn.nrow + r];
+#pragma unroll
+                    for (int c = 0; c < RC; ++c) acc[c] -= x * Y[k * RC + c];
+                }
+                if (root) {
+                    T *row = M + (int64_t)(gj.n + r) * gj.ld;
+#pragma unroll
+                    for (int c = 0; c < RC; ++c)
+                        if (c < w) row[c] = -acc[c];
+                } else {
+#pragma unroll
+                    for (int c = 0; c < RC; ++c) U[r * RC + c] = acc[c];
+                }
+            }
+            if (root) break;
+            __syncthreads();
+            const int a = dn.parent;
+            const SnInfo da = sn[a];
+            const int nca = da.ncol, nba = da.nrow - da.ncol;
+            for (int q = tid; q < (nca + nba) * RC; q += kStThreads) (q < nca * RC ? F[q] : Fb[q - nca * RC]) = (T)0;
+            __syncthreads();
+            const int32_t *ri = relind + dn.relind_off;
+            for (int q = tid; q < nbn * RC; q += kStThreads) {
+                const int i = q / RC, c = q % RC, pos = ri[i];
+                (pos < nca ? F[pos * RC + c] : Fb[(pos - nca) * RC + c]) = U[q];
+            }
+            __syncthreads();
+            const T *X = Xall + da.x_off;
+            const int pa = ssn[a].pos;
+            for (int r = tid; r < nca; r += kStThreads) {
+                T acc[RC];
+#pragma unroll
+                for (int c = 0; c < RC; ++c) acc[c] = (T)0;
+#pragma unroll 4
+                for (int k = 0; k <= r; ++k) {  // X_a is lower triangular
+                    const T x = X[(int64_t)k * da.ldx + r];
+#pragma unroll
+                    for (int c = 0; c < RC; ++c) acc[c] += x * F[k * RC + c];
+                }
+                T *row = M + (int64_t)(pa + r) * gj.ld;
+#pragma unroll
+                for (int c = 0; c < RC; ++c) {
+                    Y[r * RC + c] = acc[c];
+                    if (c < w) row[c] = acc[c];
+                }
+            }
+            __syncthreads();
+            node = a;
+            dn = da;
+            kfirst = 0;
+        }
+        __syncthreads();  // the buffers are reused by the next pass
+    }
+}

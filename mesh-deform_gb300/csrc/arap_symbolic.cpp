@@ -821,7 +821,7 @@ bool build_symbolic(const Topology &topo, const std::vector<uint8_t> &constraine
                 add(kFdt, jb, dt);
                 add(kFrows, jb, rw);
             }
-            std::vector<FItem> sy, fx;
+            std::vector<FItem> sy;
             for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; ++q) {
                 const int sidx = sym.level_sn[q];
                 const SnInfo &d = sym.sn[sidx];
@@ -829,11 +829,17 @@ bool build_symbolic(const Topology &topo, const std::vector<uint8_t> &constraine
                 const int nt = (nb + kTileU - 1) / kTileU;
                 for (int rt = 0; rt < nt; ++rt)
                     for (int ct = 0; ct <= rt; ++ct) sy.push_back({sidx, rt, ct, 0});
-                for (int jb = 0; jb * kDiagBlock < d.ncol; ++jb) fx.push_back({sidx, jb, 0, 0});
             }
             add(kFsyrk, 0, sy);
-            add(kFx, 0, fx);
         }
+        // the inverses X need only the finished factor: one launch, the
+        // largest fronts (top levels) first
+        std::vector<FItem> fx;
+        for (int q = S - 1; q >= 0; --q) {
+            const int sidx = sym.level_sn[q];
+            for (int jb = 0; jb * kDiagBlock < sym.sn[sidx].ncol; ++jb) fx.push_back({sidx, jb, 0, 0});
+        }
+        add(kFx, 0, fx);
     }
     amap_th.t.join();
     if (!amap_ok) {

@@ -1,0 +1,95 @@
+"""The dense-phase solves (the default of a single request) against the
+supernodal sweeps and the oracle: sizes at the edges of the plan (one group,
+several phases, a last group large enough for the tiled top products), any CTA
+cap bit for bit, and both kinds of solve arrays used in turn on one context.
+
+Tolerances: both paths solve the same factored system; their sums differ in
+order, so FP64 positions agree to a few thousand roundings (1e-11 of the
+bounding box, as between the sweeps' own variants) and mixed ones to the mixed
+form's 1e-6."""
+import numpy as np
+import pytest
+
+import arap_workloads as W
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "sphere1": lambda: W.cfg_icosphere_l4(level=1, iterations=4),
+    "sphere3": lambda: W.cfg_icosphere_l4(level=3, iterations=5),
+    "sphere4": lambda: W.cfg_icosphere_l4(level=4, iterations=5),
+    "noisy5": lambda: W.cfg_noisy_sphere(level=5, iterations=4),
+    "bar.1": lambda: W.cfg_twisted_bar(h=0.1, iterations=4),
+    "bar.05": lambda: W.cfg_twisted_bar(h=0.05, iterations=4),
+}
+
+
+def make(gpu, w, precision):
+    ctx = gpu.ArapContext(w.V, w.faces)
+    ctx.set_precision(precision, 1)
+    ctx.set_rest_positions(w.positions)
+    ctx.set_constraints(w.cidx, w.ctargets)
+    return ctx
+
+
+@pytest.mark.parametrize("precision,tol,otol", [("fp64", 1e-11, 1e-10), ("mixed", 1e-6, 1e-6)])
+@pytest.mark.parametrize("name", CASES)
+def test_phases_match_sweeps_and_oracle(gpu, name, precision, tol, otol):
+    from oracle import oracle as O
+
+    w = CASES[name]()
+    ok, ref = O.run_deform(w.positions, w.faces, w.cidx, w.ctargets, w.iterations)
+    assert ok
+    with make(gpu, w, precision) as ctx:
+        ctx.set_dense_top(-1)  # asks for the sweeps
+        sweeps = ctx.deform(w.iterations)
+    outs = []
+    for cap in (0, 3, 64):
+        with make(gpu, w, precision) as ctx:
+            ctx.set_solve_ctas(cap)
+            a = ctx.deform(w.iterations)
+            ctx.invalidate()
+            np.testing.assert_array_equal(ctx.deform(w.iterations), a)
+            outs.append(a)
+    np.testing.assert_array_equal(outs[1], outs[0])
+    np.testing.assert_array_equal(outs[2], outs[0])
+    assert W.bbox_rel_error(outs[0], sweeps, w.positions) <= tol
+    assert W.bbox_rel_error(outs[0], ref, w.positions) <= otol
+
+
+def test_poses_and_deforms_in_turn(gpu):
+    """A pose batch needs the sweeps' arrays, a deform the phases': each is
+    formed from the resident factor when its call comes, and both give what a
+    context that ran nothing else gives."""
+    w = W.cfg_pose_batch(level=4, n_poses=5, iterations=4)
+    with make(gpu, w, "mixed") as ctx:
+        lone = ctx.deform(w.iterations)
+        ctx.set_targets(w.ctargets + 0.05)
+        lone2 = ctx.deform(w.iterations)
+    with make(gpu, w, "mixed") as ctx:
+        poses = ctx.deform_poses(w.poses, w.iterations)
+    with make(gpu, w, "mixed") as ctx:
+        ctx.set_targets(w.ctargets)
+        np.testing.assert_array_equal(ctx.deform(w.iterations), lone)
+        np.testing.assert_array_equal(ctx.deform_poses(w.poses, w.iterations), poses)
+        ctx.set_targets(w.ctargets + 0.05)
+        np.testing.assert_array_equal(ctx.deform(w.iterations), lone2)
+        ctx.invalidate()
+        np.testing.assert_array_equal(ctx.deform_poses(w.poses, w.iterations), poses)
+        ctx.set_targets(w.ctargets + 0.05)
+        np.testing.assert_array_equal(ctx.deform(w.iterations), lone2)
+
+
+def test_several_large_roots(gpu):
+    """Disjoint meshes: the last phase holds one group per mesh."""
+    from oracle import oracle as O
+
+    ws = [W.cfg_twisted_bar(h=0.1, iterations=3), W.cfg_noisy_sphere(level=4, iterations=3)]
+    with gpu.MeshBatch([(w.V, w.faces) for w in ws]) as mb:
+        mb.ctx.set_precision("fp64")
+        mb.set_rest_positions([w.positions for w in ws])
+        mb.set_constraints([w.cidx for w in ws], [w.ctargets for w in ws])
+        out = mb.deform(3)
+    for w, x in zip(ws, out):
+        ok, ref = O.run_deform(w.positions, w.faces, w.cidx, w.ctargets, 3)
+        assert ok and W.bbox_rel_error(x, ref, w.positions) <= 1e-10
