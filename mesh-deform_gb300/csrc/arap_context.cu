@@ -152,7 +152,7 @@ struct arap_ctx {
     DevBuf faces, ent_ptr, ent_fc, hc, w_orig;
     DevBuf rest, targets, out;
     DevBuf drow, dcol, dent, oldidx, amap, dmap, sn, rows, relind, child, level_sn, fitems;
-    DevBuf w64, w32, p64, pc64, p32, pc32, R, diag64, bfixed, b, sol, uvec, Lval, Dinv, Upd, Xinv, L21, L21T, redge;
+    DevBuf w64, w32, p64, pc64, p32, pc32, R, diag64, bfixed, b, sol, uvec, Lval, Dinv, Upd, Xinv, L21, L21T, redge, wsum;
     DevBuf Lval32, Dinv32;  // the mixed form's FP64 factor rounded to FP32 (the inverses for the solves are formed from it)
     DevBuf errw, ticket, flags, energy;
     DevBuf cidx_dev, handle_dev, tabs_dev;  // arap_pose_targets inputs
@@ -226,7 +226,7 @@ struct arap_ctx {
     std::vector<DevBuf *> buffers() {
         return {&faces, &ent_ptr, &ent_fc, &hc, &w_orig, &rest, &targets, &out, &drow, &dcol, &dent, &oldidx,
                 &amap, &dmap, &sn, &rows, &relind, &child, &level_sn, &fitems, &w64, &w32, &p64, &pc64, &p32,
-                &pc32, &R, &diag64, &bfixed, &b, &sol, &uvec, &Lval, &Dinv, &Upd, &Xinv, &L21, &L21T, &redge,
+                &pc32, &R, &diag64, &bfixed, &b, &sol, &uvec, &Lval, &Dinv, &Upd, &Xinv, &L21, &L21T, &redge, &wsum,
                 &errw, &ticket, &flags, &energy, &cidx_dev, &handle_dev, &tabs_dev, &vf_ptr, &vf_face, &fnorm,
                 &vnorm, &btargets, &bpc64, &bpc32, &bR, &bbfixed, &bb, &bsol, &buvec, &bout, &bftop, &bytop, &bws,
                 &batile,
@@ -429,7 +429,9 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
     add(ctx->R, V * 3 * sizeof(Vec4<T>));
     add(ctx->diag64, m1 * sizeof(double));
     add(ctx->bfixed, m1 * sizeof(Vec4<double>));
-    if (f32) add(ctx->redge, std::max<size_t>(nnz, 1) * sizeof(Vec4<float>));
+    // rest edges (mixed), weighted rest edges and their sums (FP64)
+    add(ctx->redge, std::max<size_t>(nnz, 1) * sizeof(Vec4<T>));
+    if (!f32) add(ctx->wsum, V * sizeof(Vec4<double>));
     add(ctx->b, m1 * sizeof(Vec4<T>));
     add(ctx->sol, m1 * sizeof(Vec4<T>));
     add(ctx->uvec, (size_t)std::max<int64_t>(s.uvec_size, 1) * sizeof(Vec4<T>));
@@ -870,7 +872,6 @@ int prepare_strata(arap_ctx *ctx) {
     StrataDev d{};
     d.nph = (int)p.ph.size();
     for (int k = 0; k < d.nph; ++k) d.ph[k] = p.ph[k];
-    d.grid_cap = ctx->solve_cap;
     d.overlap = ctx->solve_cap <= 0;
     d.big_n = p.big_n;
     d.big_off = p.big_off;
@@ -1037,8 +1038,11 @@ int setup_enqueue(arap_ctx *ctx, bool phases) {
         launch_setup_vertices<T>(d, ctx->rest.as<double>(), ctx->targets.as<double>(), ctx->p64.as<Vec4<double>>(),
                                  ctx->pc64.as<Vec4<double>>(), p_t, pc_t, ctx->R.as<Vec4<T>>(), st);
         if (sizeof(T) == 4) launch_rest_edges(d, ctx->p64.as<Vec4<double>>(), ctx->redge.as<Vec4<float>>(), st);
+        else
+            launch_weighted_edges(d, ctx->w64.as<double>(), ctx->p64.as<Vec4<double>>(),
+                                  ctx->redge.as<Vec4<double>>(), ctx->wsum.as<Vec4<double>>(), st);
     }
-    ctx->launches += sizeof(T) == 4 ? 3 : 2;
+    ctx->launches += 3;
     if (m > 0) {
         int rc;
         if (sizeof(T) == 4 && ctx->factor_bits == 64) {
@@ -1169,15 +1173,15 @@ int run_iterations<double>(arap_ctx *ctx, int iterations) {
     for (int it = 0; it < iterations; ++it) {
         {
             Prof pr(ctx, ARAP_K_LOCAL);
-            launch_local_step<double>(d, ctx->w64.as<double>(), ctx->p64.as<Vec4<double>>(),
-                                      ctx->pc64.as<Vec4<double>>(), ctx->R.as<Vec4<double>>(), st);
+            launch_local_step_fp64(d, ctx->redge.as<Vec4<double>>(), ctx->pc64.as<Vec4<double>>(),
+                                   ctx->R.as<Vec4<double>>(), st);
         }
         ctx->launches += 1;
         if (s.m == 0) continue;
         {
             Prof pr(ctx, ARAP_K_RHS);
-            launch_rhs<double>(d, ctx->w64.as<double>(), ctx->p64.as<Vec4<double>>(), ctx->R.as<Vec4<double>>(),
-                               ctx->bfixed.as<Vec4<double>>(), ctx->sol.as<Vec4<double>>(), st);
+            launch_rhs_fp64(d, ctx->redge.as<Vec4<double>>(), ctx->wsum.as<Vec4<double>>(),
+                            ctx->R.as<Vec4<double>>(), ctx->bfixed.as<Vec4<double>>(), ctx->sol.as<Vec4<double>>(), st);
         }
         if (phases) {
             {
@@ -2520,15 +2524,15 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         break;
     }
     case ARAP_K_LOCAL:
-        if (sz == 8.0)  // rest + current positions, rotations out, adjacency + weights
-            B = V * 3 * sz + P * V * (3 * sz + 9 * sz) + 4 * (V + 1) + nnz * (4 + sz);
+        if (sz == 8.0)  // current positions, rotations out, adjacency + weighted rest edges
+            B = P * V * (3 * sz + 9 * sz) + 4 * (V + 1) + nnz * (4 + 3 * sz);
         else  // FP32 rest edges + weights per entry; FP64 current positions, FP32 rotations per vertex and pose
             B = nnz * (4 + 4 + 12) + 4 * (V + 1) + P * V * (24 + 36);
         FL = P * (nnz * 24 + V * 600);
         break;
     case ARAP_K_RHS:
         if (sz == 8.0)
-            B = m * 3 * sz + P * m * (9 * sz + 3 * sz + 3 * sz) + 4 * (m + 1) + nnz * (4 + sz);
+            B = m * 3 * sz + P * m * (9 * sz + 3 * sz + 3 * sz) + 4 * (m + 1) + nnz * (4 + 3 * sz);
         else  // rest edges + weights per entry; rotations of every vertex, b of the free ones, per pose
             B = nnz * (4 + 4 + 12) + 4 * (m + 1) + P * (V * 36 + m * 12);
         FL = P * nnz * 24;

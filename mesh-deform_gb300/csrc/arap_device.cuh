@@ -274,33 +274,129 @@ __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32
         for (int b = 0; b < 3; ++b) Rm[a][b] = (float)R[a][b];
 }
 
-// FP64 rotation fit of the FP64 form: the FP32 fit of the covariance
-// (scaled to unit Frobenius norm before rounding), orthonormalised (one
-// Newton-Schulz step: 1e-7 -> 1e-14) and refined to FP64 accuracy by two
-// Newton steps on the rotation group (polar_newton); near rank-one
-// covariances, where the FP32 fit is a poor
-// seed, take the FP64 one-sided Jacobi fit. About a quarter of the FP64
-// instructions of the FP64 Jacobi fit, the same rotation to FP64 accuracy.
+// Conversions on the integer pipe: an FP64 conversion instruction takes an FP64
+// issue slot (about 64 clocks per warp and scheduler on this GPU).
+// x 2^(1023 - e) in FP32, truncated (e: a biased FP64 exponent; the result must
+// stay below 2^127; below 2^-126 it is 0)
+__device__ __forceinline__ float to_float_scaled(double x, int e) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int fe = (int)((hi >> 20) & 0x7ffu) - e + 127;
+    const unsigned bits = ((unsigned)fe << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    return __uint_as_float((hi & 0x80000000u) | (fe > 0 ? bits : 0u));
+}
+__device__ __forceinline__ double to_double(float x) {  // denormals as 0
+    const unsigned b = __float_as_uint(x), ex = (b >> 23) & 0xffu;
+    const unsigned hi = (b & 0x80000000u) | (ex ? ((ex + 896u) << 20) | ((b >> 3) & 0xfffffu) : 0u);
+    return __hiloint2double((int)hi, ex ? (int)(b << 29) : 0);
+}
+
+// Below this det(H) / tr(H)^3 the rotation is too poorly determined for FP32
+// Newton steps (0.037 at equal singular values, 0.010 at (sigma_2 + sigma_3) /
+// sigma_1 = 0.1 without a reflection).
+constexpr float kNewtonDet = 4e-3f;
+
+// FP64 rotation fit of the FP64 form, by iterative refinement of the FP32 fit:
+// FP64 only where the digits are made. With R = R0 exp([w]x) the objective's
+// gradient g (the axial vector of the skew part of (S R)^T) and R's deviation
+// from orthogonality E = R^T R - I are residuals, small numbers that FP64
+// products leave exact to FP64 rounding: 36 FP64 instructions a step. What is
+// made of them needs only a few digits, so the Hessian H = tr(Q) I - sym(Q),
+// w = H^-1 g, the Cayley map of w and the correction
+//     dR = R ((I - E/2 + 3 E^2/8) C(w) - I)
+// are formed in FP32, and R + dR costs 9 more. A step leaves the Newton and
+// FP32 remainders, about |dR| (1e-6 / conditioning): 1e-6 -> 1e-11 -> below
+// FP64 rounding in two steps. FP64 Newton steps (S R, adjugate, Cayley map and
+// products in FP64) took about 400 FP64 instructions for the same rotation.
+// Covariances close to rank one, or whose H is close to singular (a reflection
+// with close small singular values), take the FP64 one-sided Jacobi fit.
 __device__ __forceinline__ void rotation_fit_fp64(const double S[3][3], double R[3][3]) {
-    double f2 = 0.0;
+    int e = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b) f2 += S[a][b] * S[a][b];
-    if (f2 > 0.0 && f2 < 1e300) {
-        const double sc = 1.0 / sqrt(f2);
+        for (int b = 0; b < 3; ++b) e = max(e, (__double2hiint(S[a][b]) >> 20) & 0x7ff);
+    // normal numbers, and the gradient's FP32 exponents in range
+    if (e > 60 && e < 0x7f0) {
         float Sf[3][3], Rf[3][3], spread;
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) Sf[a][b] = (float)(S[a][b] * sc);
+            for (int b = 0; b < 3; ++b) Sf[a][b] = to_float_scaled(S[a][b], e);
         rotation_from_cov<float>(Sf, Rf, &spread);
-        if (spread >= kPolarFallback) {
+        float Q[3][3];  // (S R)^T
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) Q[a][b] = Sf[b][0] * Rf[0][a] + Sf[b][1] * Rf[1][a] + Sf[b][2] * Rf[2][a];
+        const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
+        const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
+                    h12 = -0.5f * (Q[1][2] + Q[2][1]);
+        const float c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
+        const float c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
+        const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
+        if (spread >= kPolarFallback && det > kNewtonDet * tr * tr * tr) {
+            const float id = 1.f / det;
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
-                for (int b = 0; b < 3; ++b) R[a][b] = (double)Rf[a][b];
-            polar_newton(S, R, 1, 2);
+                for (int b = 0; b < 3; ++b) R[a][b] = to_double(Rf[a][b]);
+#pragma unroll
+            for (int it = 0; it < 2; ++it) {
+                double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    g0 += S[1][k] * R[k][2];
+                    g1 += S[2][k] * R[k][0];
+                    g2 += S[0][k] * R[k][1];
+                    g0 -= S[2][k] * R[k][1];
+                    g1 -= S[0][k] * R[k][2];
+                    g2 -= S[1][k] * R[k][0];
+                }
+                float E[3][3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = a; b < 3; ++b) {
+                        double x = a == b ? -1.0 : 0.0;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
+                        E[a][b] = E[b][a] = to_float_scaled(x, 1023);
+                    }
+                // the gradient at the orthonormalised R (I - E/2): Q loses E Q / 2
+                float M[3][3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) M[a][b] = E[a][0] * Q[0][b] + E[a][1] * Q[1][b] + E[a][2] * Q[2][b];
+                const float f0 = (to_float_scaled(g0, e) - 0.5f * (M[2][1] - M[1][2])) * id,
+                            f1 = (to_float_scaled(g1, e) - 0.5f * (M[0][2] - M[2][0])) * id,
+                            f2 = (to_float_scaled(g2, e) - 0.5f * (M[1][0] - M[0][1])) * id;
+                // a = w / 2, w = H^-1 g; C(w) - I = f ([a]x + [a]x^2)
+                const float a0 = 0.5f * (c00 * f0 + c01 * f1 + c02 * f2), a1 = 0.5f * (c01 * f0 + c11 * f1 + c12 * f2),
+                            a2 = 0.5f * (c02 * f0 + c12 * f1 + c22 * f2);
+                const float f = 2.f / (1.f + a0 * a0 + a1 * a1 + a2 * a2);
+                const float K[3][3] = {{-f * (a1 * a1 + a2 * a2), f * (a0 * a1 - a2), f * (a0 * a2 + a1)},
+                                       {f * (a0 * a1 + a2), -f * (a0 * a0 + a2 * a2), f * (a1 * a2 - a0)},
+                                       {f * (a0 * a2 - a1), f * (a1 * a2 + a0), -f * (a0 * a0 + a1 * a1)}};
+                float D[3][3];  // -E/2 + 3 E^2/8, then the correction's factor
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+                        D[a][b] = -0.5f * E[a][b] +
+                                  0.375f * (E[a][0] * E[0][b] + E[a][1] * E[1][b] + E[a][2] * E[2][b]);
+                float N[3][3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+                        N[a][b] = K[a][b] + D[a][b] + (D[a][0] * K[0][b] + D[a][1] * K[1][b] + D[a][2] * K[2][b]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+                        R[a][b] += to_double(Rf[a][0] * N[0][b] + Rf[a][1] * N[1][b] + Rf[a][2] * N[2][b]);
+            }
             return;
         }
     }

@@ -70,6 +70,55 @@ template <> __device__ __forceinline__ Vec4<double> ldcg4(const Vec4<double> *p)
     return {a.x, a.y, b.x, b.y};
 }
 
+// Sums NV values over the G lanes of an aligned lane group by recursive
+// halving: while values are left to split, each exchange halves the values a
+// lane carries, so NV values cost about NV additions instead of NV log2 G
+// (FP64 additions are the scarce instructions here). Afterwards a lane holds
+// st_held values from st_base on; true: a copy of another lane's.
+template <int NV, int G, typename T>
+__device__ __forceinline__ bool st_reduce(T (&v)[NV], int lane) {
+    bool dup = false;
+    int h = NV;
+#pragma unroll
+    for (int off = G / 2; off >= 1; off >>= 1) {
+        if (h > 1) {
+            h >>= 1;
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < NV / 2; ++i)
+                if (i < h) {
+                    const T send = up ? v[i] : v[i + h];
+                    const T keep = up ? v[i + h] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+            dup = dup || (lane & off) != 0;
+        }
+    }
+    return dup;
+}
+// index of the first value a lane holds afterwards, and how many it holds
+template <int NV, int G>
+__device__ __forceinline__ int st_base(int lane) {
+    int base = 0, h = NV;
+#pragma unroll
+    for (int off = G / 2; off >= 1; off >>= 1)
+        if (h > 1) {
+            h >>= 1;
+            if (lane & off) base += h;
+        }
+    return base;
+}
+template <int NV, int G> constexpr int st_held() {
+    int h = NV, off = G;
+    while (h > 1 && off > 1) {
+        h /= 2;
+        off /= 2;
+    }
+    return h;
+}
+
 // ---------------------------------------------------------------------------
 // cotan weights
 
@@ -228,6 +277,27 @@ __global__ void k_rest_edges(int V, const int32_t *__restrict__ drow, const int3
         const Vec4<double> pl = p64[dcol[e]];
         redge[e] = {(float)(pk.x - pl.x), (float)(pk.y - pl.y), (float)(pk.z - pl.z), 0.f};
     }
+}
+
+// FP64 form: weighted rest edges w (p_k - p_l) per adjacency entry, and their
+// sum per vertex
+__global__ void k_weighted_edges(int V, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+                                 const double *__restrict__ w64, const Vec4<double> *__restrict__ p64,
+                                 Vec4<double> *__restrict__ wedge, Vec4<double> *__restrict__ wsum) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= V) return;
+    const Vec4<double> pk = p64[k];
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    for (int e = drow[k]; e < drow[k + 1]; ++e) {
+        const Vec4<double> pl = p64[dcol[e]];
+        const double w = w64[e];
+        const Vec4<double> we = {w * (pk.x - pl.x), w * (pk.y - pl.y), w * (pk.z - pl.z), 0.0};
+        wedge[e] = we;
+        sx += we.x;
+        sy += we.y;
+        sz += we.z;
+    }
+    wsum[k] = {sx, sy, sz, 0.0};
 }
 
 // ---------------------------------------------------------------------------
@@ -866,37 +936,34 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
 // ---------------------------------------------------------------------------
 // local step: estimateRotations, arap.h:354-384
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_local_step(int V, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const T *__restrict__ w,
-             const Vec4<T> *__restrict__ p, const Vec4<T> *__restrict__ pc, Vec4<T> *__restrict__ R) {
+// FP64 form: covariance from the weighted rest edges w (p_i - p_j), formed
+// once per set-up (they only change with the rest pose), and the rotation fit.
+// Bound by FP64 issue (about 64 clocks per warp instruction and scheduler):
+// 12 FP64 instructions per neighbour (18 with the edges formed here) and 90
+// for the fit. Small blocks spread the warps over every scheduler.
+__global__ void __launch_bounds__(128)
+k_local_step_fp64(int V, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+                  const Vec4<double> *__restrict__ wedge, const Vec4<double> *__restrict__ pc,
+                  Vec4<double> *__restrict__ R) {
     pdl_wait();  // the positions of the kernels before (an overlapped launch)
     pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= V) return;
-    const Vec4<T> pi = p[i], ci = pc[i];
-    T S[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) S[a][b] = (T)0;
+    const Vec4<double> ci = pc[i];
+    double S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     const int e1 = drow[i + 1];
     for (int e = drow[i]; e < e1; ++e) {
-        const int j = dcol[e];
-        const T wj = w[e];
-        const Vec4<T> pj = p[j], cj = pc[j];
-        const T ex = wj * (pi.x - pj.x), ey = wj * (pi.y - pj.y), ez = wj * (pi.z - pj.z);
-        const T fx = ci.x - cj.x, fy = ci.y - cj.y, fz = ci.z - cj.z;
-        S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
-        S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
-        S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
+        const Vec4<double> we = wedge[e], cj = pc[dcol[e]];
+        const double fx = ci.x - cj.x, fy = ci.y - cj.y, fz = ci.z - cj.z;
+        S[0][0] += we.x * fx; S[0][1] += we.x * fy; S[0][2] += we.x * fz;
+        S[1][0] += we.y * fx; S[1][1] += we.y * fy; S[1][2] += we.y * fz;
+        S[2][0] += we.z * fx; S[2][1] += we.z * fy; S[2][2] += we.z * fz;
     }
-    T Rm[3][3];
-    if constexpr (sizeof(T) == 8) dev::rotation_fit_fp64(S, Rm);
-    else rotation_from_cov(S, Rm);
-    R[3 * (int64_t)i + 0] = {Rm[0][0], Rm[0][1], Rm[0][2], (T)0};
-    R[3 * (int64_t)i + 1] = {Rm[1][0], Rm[1][1], Rm[1][2], (T)0};
-    R[3 * (int64_t)i + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], (T)0};
+    double Rm[3][3];
+    dev::rotation_fit_fp64(S, Rm);
+    R[3 * (int64_t)i + 0] = {Rm[0][0], Rm[0][1], Rm[0][2], 0.0};
+    R[3 * (int64_t)i + 1] = {Rm[1][0], Rm[1][1], Rm[1][2], 0.0};
+    R[3 * (int64_t)i + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], 0.0};
 }
 
 // Local step of the mixed form: the covariance in FP32 from the FP32 rest
@@ -996,32 +1063,46 @@ k_rhs_mixed(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__
     if (live && l == 0) b[i] = {ax, ay, az, 0.f};
 }
 
-// estimatePositions RHS, arap.h:395-414
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_rhs(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const T *__restrict__ w,
-      const Vec4<T> *__restrict__ p, const Vec4<T> *__restrict__ R, const Vec4<T> *__restrict__ bfixed,
-      Vec4<T> *__restrict__ b) {
+// estimatePositions RHS, arap.h:395-414, FP64 form: sum_j 1/2 w (R_i + R_j)
+// (p_i - p_j) = 1/2 (R_i sum_j w e_ij + sum_j R_j w e_ij) over the weighted
+// rest edges, whose sum per vertex is formed once per set-up: 9 FP64
+// instructions per neighbour and 12 per vertex (25 per neighbour with the
+// edges and rotation sums formed here). G lanes share a vertex (neighbours
+// l, l + G, ...) where there are too few vertices to fill every scheduler.
+template <int G>
+__global__ void __launch_bounds__(128)
+k_rhs_fp64(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+           const Vec4<double> *__restrict__ wedge, const Vec4<double> *__restrict__ wsum,
+           const Vec4<double> *__restrict__ R, const Vec4<double> *__restrict__ bfixed, Vec4<double> *__restrict__ b) {
     pdl_wait();     // the positions and rotations of the kernels before
     pdl_trigger();  // the forward sweep may take its first tasks meanwhile
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const Vec4<T> pi = p[i];
-    const Vec4<T> r0 = R[3 * (int64_t)i], r1 = R[3 * (int64_t)i + 1], r2 = R[3 * (int64_t)i + 2];
-    Vec4<T> acc = bfixed[i];
-    const int e1 = drow[i + 1];
-    for (int e = drow[i]; e < e1; ++e) {
-        const int j = dcol[e];
-        if (j == i) continue;
-        const T h = w[e] * (T)0.5;
-        const Vec4<T> pj = p[j];
-        const Vec4<T> q0 = R[3 * (int64_t)j], q1 = R[3 * (int64_t)j + 1], q2 = R[3 * (int64_t)j + 2];
-        const T dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        acc.x += ((r0.x + q0.x) * dx + (r0.y + q0.y) * dy + (r0.z + q0.z) * dz) * h;
-        acc.y += ((r1.x + q1.x) * dx + (r1.y + q1.y) * dy + (r1.z + q1.z) * dz) * h;
-        acc.z += ((r2.x + q2.x) * dx + (r2.y + q2.y) * dy + (r2.z + q2.z) * dz) * h;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int i = t / G, l = t % G;
+    const bool live = i < m;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (live) {
+        const int e1 = drow[i + 1];
+        for (int e = drow[i] + l; e < e1; e += G) {
+            const int j = dcol[e];
+            const Vec4<double> we = wedge[e];
+            const Vec4<double> q0 = R[3 * (int64_t)j], q1 = R[3 * (int64_t)j + 1], q2 = R[3 * (int64_t)j + 2];
+            acc[0] += q0.x * we.x; acc[0] += q0.y * we.y; acc[0] += q0.z * we.z;
+            acc[1] += q1.x * we.x; acc[1] += q1.y * we.y; acc[1] += q1.z * we.z;
+            acc[2] += q2.x * we.x; acc[2] += q2.y * we.y; acc[2] += q2.z * we.z;
+        }
     }
-    b[i] = acc;
+    const bool dup = st_reduce<4, G>(acc, lane);
+    const int base = st_base<4, G>(lane);
+    if (!live || dup) return;
+    const Vec4<double> ws = wsum[i];
+#pragma unroll
+    for (int j = 0; j < st_held<4, G>(); ++j) {
+        const int c = base + j;
+        if (c == 3) continue;
+        const Vec4<double> r = R[3 * (int64_t)i + c];
+        const double sum = r.x * ws.x + r.y * ws.y + r.z * ws.z + acc[j];
+        reinterpret_cast<double *>(b + i)[c] = reinterpret_cast<const double *>(bfixed + i)[c] + 0.5 * sum;
+    }
 }
 
 // r = b - A x in FP64 over the free vertices (A = constrained Laplacian)
@@ -2914,20 +2995,41 @@ template void launch_solve_blocks<float>(int, const int32_t *, const int32_t *, 
 template void launch_solve_blocks<double>(int, const int32_t *, const int32_t *, const SnInfo *, const SnInfo *,
                                           const int32_t *, const double *, double *, double *, double *, cudaStream_t);
 
-template <typename T>
-void launch_local_step(const DevSym &s, const T *w, const Vec4<T> *p, const Vec4<T> *pc, Vec4<T> *R,
-                       cudaStream_t st) {
+void launch_weighted_edges(const DevSym &s, const double *w64, const Vec4<double> *p64, Vec4<double> *wedge,
+                           Vec4<double> *wsum, cudaStream_t st) {
     if (s.V == 0) return;
-    launch_pdl(k_local_step<T>, s.overlap != 0, blocks_for(s.V, 256), 256, 0, st, s.V, (const int32_t *)s.drow,
-               (const int32_t *)s.dcol, w, p, pc, R);
+    k_weighted_edges<<<blocks_for(s.V, 64), 64, 0, st>>>(s.V, s.drow, s.dcol, w64, p64, wedge, wsum);
 }
 
-template <typename T>
-void launch_rhs(const DevSym &s, const T *w, const Vec4<T> *p, const Vec4<T> *R, const Vec4<T> *bfixed,
-                Vec4<T> *b, cudaStream_t st) {
+// threads per block of the FP64 per-vertex kernels: one warp where that still
+// leaves schedulers empty, else two
+static int fp64_block(int64_t threads) { return threads < 32 * 4 * 152 ? 32 : 64; }
+
+void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *pc, Vec4<double> *R,
+                            cudaStream_t st) {
+    if (s.V == 0) return;
+    const int block = fp64_block(s.V);
+    launch_pdl(k_local_step_fp64, s.overlap != 0, blocks_for(s.V, block), block, 0, st, s.V, (const int32_t *)s.drow,
+               (const int32_t *)s.dcol, wedge, pc, R);
+}
+
+void launch_rhs_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *wsum, const Vec4<double> *R,
+                     const Vec4<double> *bfixed, Vec4<double> *b, cudaStream_t st) {
     if (s.m == 0) return;
-    launch_pdl(k_rhs<T>, s.overlap != 0, blocks_for(s.m, 256), 256, 0, st, s.m, (const int32_t *)s.drow,
-               (const int32_t *)s.dcol, w, p, R, bfixed, b);
+    // lanes per vertex: the fewest that give every scheduler four warps
+    int g = 1;
+    while (g < 8 && (int64_t)s.m * g < (int64_t)32 * 4 * 152 * 4) g *= 2;
+    const int block = fp64_block((int64_t)s.m * g), grid = blocks_for((int64_t)s.m * g, block);
+#define ARAP_RHS64(G)                                                                                          \
+    launch_pdl(k_rhs_fp64<G>, s.overlap != 0, grid, block, 0, st, s.m, (const int32_t *)s.drow,                \
+               (const int32_t *)s.dcol, wedge, wsum, R, bfixed, b)
+    switch (g) {
+    case 1: ARAP_RHS64(1); break;
+    case 2: ARAP_RHS64(2); break;
+    case 4: ARAP_RHS64(4); break;
+    default: ARAP_RHS64(8); break;
+    }
+#undef ARAP_RHS64
 }
 
 void launch_residual(const DevSym &s, const double *w64, const double *diag64, const Vec4<double> *bfixed,
@@ -3290,11 +3392,10 @@ void launch_strata_fwd(const StrataDev &d, const T *M, Vec4<T> *sol, Vec4<T> *y,
         if (k > 0)  // no update lands on the first stratum
             launch_pdl(k_strata_gather<T>, d.overlap != 0, blocks_for(4 * (int64_t)p.cn, kStThreads), kStThreads, 0, st, p.c0, p.cn,
                        d.col, d.gptr, d.gidx, (const Vec4<T> *)uvec, sol);
-        const int grid = d.grid_cap > 0 ? std::min(d.grid_cap, (int)p.fn) : p.fn;
         const size_t smem = st_fwd_smem(p, sizeof(T));
 #define ARAP_STF(G, RW)                                                                                        \
-    launch_pdl(k_strata_fwd<T, G, RW>, d.overlap != 0, grid, kStThreads, smem, st, (int)p.fn, st_ldf(p),       \
-               d.tiles + p.f0, M, d.col, (const Vec4<T> *)sol, y, uvec)
+    launch_pdl(k_strata_fwd<T, G, RW>, d.overlap != 0, (int)p.fn, kStThreads, smem, st, st_ldf(p), d.tiles + p.f0, \
+               M, d.col, (const Vec4<T> *)sol, y, uvec)
         if constexpr (sizeof(T) == 8) {  // one row per lane group (build_strata)
             if (p.G == 1) ARAP_STF(1, 1);
             else if (p.G == 4) ARAP_STF(4, 1);
@@ -3331,11 +3432,10 @@ void launch_strata_bwd(const StrataDev &d, const DevSym &s, const T *M, Vec4<T> 
                            M + d.big_off, ytop, part, cnt, d.top_col, sol, pc64, pc32, mode);
             continue;
         }
-        const int grid = d.grid_cap > 0 ? std::min(d.grid_cap, (int)p.bn) : p.bn;
         const size_t smem = st_bwd_smem(p, sizeof(T));
 #define ARAP_STB(TC)                                                                                             \
-    launch_pdl(k_strata_bwd<T, TC>, d.overlap != 0, grid, kStThreads, smem, st, (int)p.bn, (int)p.vmax,          \
-               d.tiles + p.b0, M, d.col, s.rows, y, sol, pc64, mode)
+    launch_pdl(k_strata_bwd<T, TC>, d.overlap != 0, (int)p.bn, kStThreads, smem, st, (int)p.vmax, d.tiles + p.b0,  \
+               M, d.col, s.rows, y, sol, pc64, mode)
         if (p.TC == 64) ARAP_STB(64);
         else if (p.TC == 32) ARAP_STB(32);
         else if (p.TC == 16) ARAP_STB(16);
@@ -3471,14 +3571,6 @@ template void launch_factor_step<float>(const DevSym &, const FactorLaunch &, co
                                         float *, float *, float *, float *, int *, cudaStream_t);
 template void launch_factor_step<double>(const DevSym &, const FactorLaunch &, const FItem *, double *, double *,
                                          double *, double *, double *, double *, int *, cudaStream_t);
-template void launch_local_step<float>(const DevSym &, const float *, const Vec4<float> *, const Vec4<float> *,
-                                       Vec4<float> *, cudaStream_t);
-template void launch_local_step<double>(const DevSym &, const double *, const Vec4<double> *, const Vec4<double> *,
-                                        Vec4<double> *, cudaStream_t);
-template void launch_rhs<float>(const DevSym &, const float *, const Vec4<float> *, const Vec4<float> *,
-                                const Vec4<float> *, Vec4<float> *, cudaStream_t);
-template void launch_rhs<double>(const DevSym &, const double *, const Vec4<double> *, const Vec4<double> *,
-                                 const Vec4<double> *, Vec4<double> *, cudaStream_t);
 template void launch_solve_fwd<float>(const DevSym &, const float *, const float *, Vec4<float> *, Vec4<float> *,
                                       unsigned long long *, unsigned *, int *, cudaStream_t, const float *,
                                       Vec4<float> *);

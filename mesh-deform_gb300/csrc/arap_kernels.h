@@ -160,14 +160,15 @@ void launch_solve_blocks(int nblocks, const int32_t *items, const int32_t *membe
 // FP64 factor outputs (X, L21, L21^T, the dense top's T) rounded to the FP32
 // copies the mixed form's solves read: count <= 4 arrays of n[a] elements
 void launch_demote(int count, const double *const *src, float *const *dst, const int64_t *n, cudaStream_t st);
-// local step: covariance + rotation fit (estimateRotations arap.h:354-384)
-template <typename T>
-void launch_local_step(const DevSym &s, const T *w, const Vec4<T> *p, const Vec4<T> *pc, Vec4<T> *R,
-                       cudaStream_t st);
-// RHS (estimatePositions arap.h:395-414): b = bFixed + sum 1/2 w (Ri+Rj)(pi-pj)
-template <typename T>
-void launch_rhs(const DevSym &s, const T *w, const Vec4<T> *p, const Vec4<T> *R, const Vec4<T> *bfixed,
-                Vec4<T> *b, cudaStream_t st);
+// FP64 form: weighted rest edges per adjacency entry and their sums per vertex
+void launch_weighted_edges(const DevSym &s, const double *w64, const Vec4<double> *p64, Vec4<double> *wedge,
+                           Vec4<double> *wsum, cudaStream_t st);
+// FP64 local step: covariance + rotation fit (estimateRotations arap.h:354-384)
+void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *pc, Vec4<double> *R,
+                            cudaStream_t st);
+// FP64 RHS (estimatePositions arap.h:395-414): b = bFixed + sum 1/2 w (Ri+Rj)(pi-pj)
+void launch_rhs_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *wsum, const Vec4<double> *R,
+                     const Vec4<double> *bfixed, Vec4<double> *b, cudaStream_t st);
 // FP64 residual of the global system: r = (bFixed + b) - A x over the free vertices
 void launch_residual(const DevSym &s, const double *w64, const double *diag64, const Vec4<double> *bfixed,
                      const Vec4<float> *b, const Vec4<double> *x64, Vec4<float> *r, cudaStream_t st);
@@ -215,7 +216,6 @@ void launch_top_inverse(const DevSym &s, const T *X, const T *L21, T *Tt, cudaSt
 struct StrataDev {
     int nph;
     StPhase ph[kStMaxPhases];
-    int grid_cap;  // most CTAs per launch (0: a CTA per tile)
     int overlap;   // as DevSym::overlap
     int big_n, big_pair32, big_pair64;
     int64_t big_off;

@@ -43,55 +43,6 @@ __device__ __forceinline__ StTile st_tile(const StTile *p) {
     return t;
 }
 
-// Sums NV values over the G lanes of an aligned lane group by recursive
-// halving: while values are left to split, each exchange halves the values a
-// lane carries, so NV values cost about NV additions instead of NV log2 G
-// (FP64 additions are the scarce instructions here). Afterwards a lane holds
-// st_held values from st_base on; true: a copy of another lane's.
-template <int NV, int G, typename T>
-__device__ __forceinline__ bool st_reduce(T (&v)[NV], int lane) {
-    bool dup = false;
-    int h = NV;
-#pragma unroll
-    for (int off = G / 2; off >= 1; off >>= 1) {
-        if (h > 1) {
-            h >>= 1;
-            const bool up = (lane & off) != 0;
-#pragma unroll
-            for (int i = 0; i < NV / 2; ++i)
-                if (i < h) {
-                    const T send = up ? v[i] : v[i + h];
-                    const T keep = up ? v[i + h] : v[i];
-                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-                }
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
-            dup = dup || (lane & off) != 0;
-        }
-    }
-    return dup;
-}
-// index of the first value a lane holds afterwards, and how many it holds
-template <int NV, int G>
-__device__ __forceinline__ int st_base(int lane) {
-    int base = 0, h = NV;
-#pragma unroll
-    for (int off = G / 2; off >= 1; off >>= 1)
-        if (h > 1) {
-            h >>= 1;
-            if (lane & off) base += h;
-        }
-    return base;
-}
-template <int NV, int G> constexpr int st_held() {
-    int h = NV, off = G;
-    while (h > 1 && off > 1) {
-        h /= 2;
-        off /= 2;
-    }
-    return h;
-}
-
 // b[k] += the update entries of column k, for a stratum's columns, as a launch
 // of its own: four threads per column, each an index quad at a time (its
 // entries' loads in flight together), so that no thread runs a long chain of
@@ -149,7 +100,7 @@ k_strata_gather(int c0, int cn, const int32_t *__restrict__ gcol, const int32_t 
 // and scheduler), so lanes that share a row are as few as fill the device.
 template <typename T, int G, int RW>
 __global__ void __launch_bounds__(kStThreads, 8)
-k_strata_fwd(int ntiles, int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
+k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
              const int32_t *__restrict__ gcol, const Vec4<T> *__restrict__ b, Vec4<T> *__restrict__ y,
              Vec4<T> *__restrict__ uvec) {
     extern __shared__ __align__(128) unsigned char st_raw[];
@@ -159,99 +110,91 @@ k_strata_fwd(int ntiles, int ldf, const StTile *__restrict__ tiles, const T *__r
     T *fx = reinterpret_cast<T *>(st_raw), *fy = fx + ldf, *fz = fy + ldf;
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, l = tid % G, grp = tid / G;
-    bool waited = false;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const StTile d = st_tile(tiles + t);
-        const T *M = Mall + d.m_off;
-        const int rend = d.first + d.count;
-        // X is lower triangular: a warp's columns end at its last row's
-        auto cols_to = [&](int last) {
-            const int nc = last > d.n ? d.n : last;
-            return (nc + G * E - 1) / (G * E) * (G * E);
-        };
-        const int ncol = rend > d.n ? d.n : rend, fspan = cols_to(rend);
-        int span = cols_to(min(rend, d.first + (grp | (32 / G - 1)) * RW + RW));
-        // column c of the group: consecutive ones in the first phase (whole subtrees)
-        auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
-        StPack<T> m[NB][RW];
-        auto load = [&](int row, int c) {
+    const StTile d = st_tile(tiles + blockIdx.x);
+    const T *M = Mall + d.m_off;
+    const int rend = d.first + d.count;
+    // X is lower triangular: a warp's columns end at its last row's
+    auto cols_to = [&](int last) {
+        const int nc = last > d.n ? d.n : last;
+        return (nc + G * E - 1) / (G * E) * (G * E);
+    };
+    const int ncol = rend > d.n ? d.n : rend, fspan = cols_to(rend);
+    int span = cols_to(min(rend, d.first + (grp | (32 / G - 1)) * RW + RW));
+    // column c of the group: consecutive ones in the first phase (whole subtrees)
+    auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
+    StPack<T> m[NB][RW];
+    auto load = [&](int row, int c) {
 #pragma unroll
-            for (int k = 0; k < NB; ++k)
+        for (int k = 0; k < NB; ++k)
 #pragma unroll
-                for (int i = 0; i < RW; ++i) {
-                    const int cc = c + k * G * E;
-                    if (cc < d.ld && cc < span && row + i < rend) m[k][i].load(M + (int64_t)(row + i) * d.ld + cc);
-                    else
+            for (int i = 0; i < RW; ++i) {
+                const int cc = c + k * G * E;
+                if (cc < d.ld && cc < span && row + i < rend) m[k][i].load(M + (int64_t)(row + i) * d.ld + cc);
+                else
 #pragma unroll
-                        for (int e = 0; e < E; ++e) m[k][i].v[e] = (T)0;
-                }
-        };
-        int row = d.first + grp * RW;
-        load(row, l * E);
-        // the places of f before the wait, f after it
-        constexpr int kPre = 2;
-        int at[kPre];
-#pragma unroll
-        for (int i = 0; i < kPre; ++i) at[i] = tid + i * kStThreads < ncol ? column(tid + i * kStThreads) : -1;
-        if (!waited) {
-            pdl_wait();
-            waited = true;
-        }
-        auto put = [&](int c, int k) {
-            const Vec4<T> v = k >= 0 ? ldcg4(b + k) : Vec4<T>{(T)0, (T)0, (T)0, (T)0};
-            fx[c] = v.x;
-            fy[c] = v.y;
-            fz[c] = v.z;
-        };
-#pragma unroll
-        for (int i = 0; i < kPre; ++i)
-            if (tid + i * kStThreads < fspan) put(tid + i * kStThreads, at[i]);
-        for (int c = tid + kPre * kStThreads; c < fspan; c += kStThreads) put(c, c < ncol ? column(c) : -1);
-        __syncthreads();
-        for (int r0 = d.first; r0 < rend; r0 += kRows) {
-            row = r0 + grp * RW;
-            span = cols_to(min(rend, r0 + (grp | (32 / G - 1)) * RW + RW));
-            constexpr int H = st_held<RW * 4, G>();
-            // the value(s) this lane will hold after the reduction go to one row
-            const int orow = row + (st_base<RW * 4, G>(lane) >> 2);
-            const int ocol = orow < rend && orow < d.n ? column(orow) : 0;
-            T acc[RW * 4];
-#pragma unroll
-            for (int i = 0; i < RW * 4; ++i) acc[i] = (T)0;
-            for (int c = l * E; c < span; c += NB * G * E) {
-                if (r0 > d.first || c >= NB * G * E) load(row, c);
-#pragma unroll
-                for (int k = 0; k < NB; ++k) {
-                    const int cc = c + k * G * E;
-                    if (cc >= span) break;
-                    StPack<T> px, py, pz;
-                    px.lds(fx + cc);
-                    py.lds(fy + cc);
-                    pz.lds(fz + cc);
-#pragma unroll
-                    for (int i = 0; i < RW; ++i)
-#pragma unroll
-                        for (int e = 0; e < E; ++e) {
-                            acc[4 * i] += m[k][i].v[e] * px.v[e];
-                            acc[4 * i + 1] += m[k][i].v[e] * py.v[e];
-                            acc[4 * i + 2] += m[k][i].v[e] * pz.v[e];
-                        }
-                }
+                    for (int e = 0; e < E; ++e) m[k][i].v[e] = (T)0;
             }
-            const bool dup = st_reduce<RW * 4, G>(acc, lane);
-            const int base = st_base<RW * 4, G>(lane);
-            if (!dup && orow < rend) {
-                T *dst = reinterpret_cast<T *>(orow < d.n ? y + ocol : uvec + d.u_off + (orow - d.n));
+    };
+    int row = d.first + grp * RW;
+    load(row, l * E);
+    // the places of f before the wait, f after it
+    constexpr int kPre = 2;
+    int at[kPre];
 #pragma unroll
-                for (int j = 0; j < H; ++j) {
-                    const int comp = (base + j) & 3;
-                    if (comp < 3) dst[comp] = orow < d.n ? acc[j] : -acc[j];
-                }
+    for (int i = 0; i < kPre; ++i) at[i] = tid + i * kStThreads < ncol ? column(tid + i * kStThreads) : -1;
+    pdl_wait();
+    auto put = [&](int c, int k) {
+        const Vec4<T> v = k >= 0 ? ldcg4(b + k) : Vec4<T>{(T)0, (T)0, (T)0, (T)0};
+        fx[c] = v.x;
+        fy[c] = v.y;
+        fz[c] = v.z;
+    };
+#pragma unroll
+    for (int i = 0; i < kPre; ++i)
+        if (tid + i * kStThreads < fspan) put(tid + i * kStThreads, at[i]);
+    for (int c = tid + kPre * kStThreads; c < fspan; c += kStThreads) put(c, c < ncol ? column(c) : -1);
+    __syncthreads();
+    for (int r0 = d.first; r0 < rend; r0 += kRows) {
+        row = r0 + grp * RW;
+        span = cols_to(min(rend, r0 + (grp | (32 / G - 1)) * RW + RW));
+        constexpr int H = st_held<RW * 4, G>();
+        // the value(s) this lane will hold after the reduction go to one row
+        const int orow = row + (st_base<RW * 4, G>(lane) >> 2);
+        const int ocol = orow < rend && orow < d.n ? column(orow) : 0;
+        T acc[RW * 4];
+#pragma unroll
+        for (int i = 0; i < RW * 4; ++i) acc[i] = (T)0;
+        for (int c = l * E; c < span; c += NB * G * E) {
+            if (r0 > d.first || c >= NB * G * E) load(row, c);
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                const int cc = c + k * G * E;
+                if (cc >= span) break;
+                StPack<T> px, py, pz;
+                px.lds(fx + cc);
+                py.lds(fy + cc);
+                pz.lds(fz + cc);
+#pragma unroll
+                for (int i = 0; i < RW; ++i)
+#pragma unroll
+                    for (int e = 0; e < E; ++e) {
+                        acc[4 * i] += m[k][i].v[e] * px.v[e];
+                        acc[4 * i + 1] += m[k][i].v[e] * py.v[e];
+                        acc[4 * i + 2] += m[k][i].v[e] * pz.v[e];
+                    }
             }
         }
-        __syncthreads();  // f is rewritten by the CTA's next tile
+        const bool dup = st_reduce<RW * 4, G>(acc, lane);
+        const int base = st_base<RW * 4, G>(lane);
+        if (!dup && orow < rend) {
+            T *dst = reinterpret_cast<T *>(orow < d.n ? y + ocol : uvec + d.u_off + (orow - d.n));
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                const int comp = (base + j) & 3;
+                if (comp < 3) dst[comp] = orow < d.n ? acc[j] : -acc[j];
+            }
+        }
     }
-    if (!waited) pdl_wait();
 }
 
 // Backward product of a stratum: x = M^T v for TC columns of a group, v = y on
@@ -264,7 +207,7 @@ k_strata_fwd(int ntiles, int ldf, const StTile *__restrict__ tiles, const T *__r
 // x goes to the solution and the positions (mode 0: pc64 = x, 1: pc64 += x).
 template <typename T, int TC>
 __global__ void __launch_bounds__(kStThreads)
-k_strata_bwd(int ntiles, int vmax, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
+k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
              const int32_t *__restrict__ gcol, const int32_t *__restrict__ rows, const Vec4<T> *__restrict__ y,
              Vec4<T> *sol, Vec4<double> *__restrict__ pc64, int mode) {
     extern __shared__ __align__(128) unsigned char st_raw[];
@@ -273,104 +216,96 @@ k_strata_bwd(int ntiles, int vmax, const StTile *__restrict__ tiles, const T *__
     T *red = reinterpret_cast<T *>(v + vmax);  // NS x (TC columns x 4)
     pdl_trigger();
     const int tid = threadIdx.x, q = tid % QC, s = tid / QC;
-    bool waited = false;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const StTile d = st_tile(tiles + t);
-        const T *M = Mall + d.m_off + (int64_t)d.first * d.ld + d.first + q * E;
-        const int nrow = d.n + d.r - d.first;  // X is lower triangular: rows from the tile's first column on
-        const bool in = d.first + q * E < d.ld;
-        StPack<T> m[U];
-        auto load = [&](int r) {
+    const StTile d = st_tile(tiles + blockIdx.x);
+    const T *M = Mall + d.m_off + (int64_t)d.first * d.ld + d.first + q * E;
+    const int nrow = d.n + d.r - d.first;  // X is lower triangular: rows from the tile's first column on
+    const bool in = d.first + q * E < d.ld;
+    StPack<T> m[U];
+    auto load = [&](int r) {
 #pragma unroll
-            for (int i = 0; i < U; ++i) {
-                if (in && r + i * NS < nrow) m[i].load(M + (int64_t)(r + i * NS) * d.ld);
-                else
+        for (int i = 0; i < U; ++i) {
+            if (in && r + i * NS < nrow) m[i].load(M + (int64_t)(r + i * NS) * d.ld);
+            else
 #pragma unroll
-                    for (int e = 0; e < E; ++e) m[i].v[e] = (T)0;
-            }
-        };
-        load(s);
-        // the vector's places before the wait, the vector after it
-        auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
-        constexpr int kPre = 4;
-        int at[kPre];
-#pragma unroll
-        for (int i = 0; i < kPre; ++i) {
-            const int r = tid + i * kStThreads, g = d.first + r;
-            at[i] = r < nrow ? (g < d.n ? column(g) : rows[d.row_off + g - d.n]) : 0;
+                for (int e = 0; e < E; ++e) m[i].v[e] = (T)0;
         }
-        if (!waited) {
-            pdl_wait();
-            waited = true;
-        }
-        // kSh threads per output value, each every kSh-th partial sum, kOut
-        // values per thread; the outputs' places and positions are loaded
-        // ahead of the product
-        constexpr int kSh = 4 * TC < kStThreads ? kStThreads / (4 * TC) : 1;
-        constexpr int kOut = 4 * TC > kStThreads ? 4 * TC / kStThreads : 1;
-        const int h = tid % kSh;
-        int ok[kOut];
-        double before[kOut];
+    };
+    load(s);
+    // the vector's places before the wait, the vector after it
+    auto column = [&](int c) { return d.base >= 0 ? d.base + c : gcol[d.col_off + c]; };
+    constexpr int kPre = 4;
+    int at[kPre];
 #pragma unroll
-        for (int j = 0; j < kOut; ++j) {
-            const int o = tid / kSh + j * kStThreads, oc = o >> 2, comp = o & 3;
-            ok[j] = h == 0 && comp < 3 && oc < d.count ? column(d.first + oc) : -1;
-            before[j] = ok[j] >= 0 && mode != 0 ? __ldcg(reinterpret_cast<const double *>(pc64 + ok[j]) + comp) : 0.0;
-        }
-        auto put = [&](int r, int k) {
-            const bool own = d.first + r < d.n;
-            Vec4<T> x = ldcg4((own ? y : (const Vec4<T> *)sol) + k);
-            if (!own) x = {-x.x, -x.y, -x.z, (T)0};
-            v[r] = x;
-        };
-#pragma unroll
-        for (int i = 0; i < kPre; ++i) {
-            const int r = tid + i * kStThreads;
-            if (r < nrow) put(r, at[i]);
-        }
-        for (int r = tid + kPre * kStThreads; r < nrow; r += kStThreads) {
-            const int g = d.first + r;
-            put(r, g < d.n ? column(g) : rows[d.row_off + g - d.n]);
-        }
-        __syncthreads();
-        T acc[E][3];
-#pragma unroll
-        for (int e = 0; e < E; ++e) acc[e][0] = acc[e][1] = acc[e][2] = (T)0;
-        for (int r = s; r < nrow; r += U * NS) {
-            if (r != s) load(r);
-#pragma unroll
-            for (int i = 0; i < U; ++i) {
-                if (r + i * NS >= nrow) break;
-                const Vec4<T> x = v[r + i * NS];
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    acc[e][0] += m[i].v[e] * x.x;
-                    acc[e][1] += m[i].v[e] * x.y;
-                    acc[e][2] += m[i].v[e] * x.z;
-                }
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) red[(s * TC + q * E + e) * 4 + c] = acc[e][c];
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kOut; ++j) {
-            const int o = tid / kSh + j * kStThreads, comp = o & 3;
-            T sum = (T)0;
-#pragma unroll 8
-            for (int i = h; i < NS; i += kSh) sum += red[i * TC * 4 + o];
-#pragma unroll
-            for (int off = 1; off < kSh; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            if (ok[j] >= 0) {
-                reinterpret_cast<T *>(sol + ok[j])[comp] = sum;
-                reinterpret_cast<double *>(pc64 + ok[j])[comp] = mode == 0 ? (double)sum : before[j] + (double)sum;
-            }
-        }
-        __syncthreads();  // v and the sums are rewritten by the CTA's next tile
+    for (int i = 0; i < kPre; ++i) {
+        const int r = tid + i * kStThreads, g = d.first + r;
+        at[i] = r < nrow ? (g < d.n ? column(g) : rows[d.row_off + g - d.n]) : 0;
     }
-    if (!waited) pdl_wait();
+    pdl_wait();
+    // kSh threads per output value, each every kSh-th partial sum, kOut
+    // values per thread; the outputs' places and positions are loaded
+    // ahead of the product
+    constexpr int kSh = 4 * TC < kStThreads ? kStThreads / (4 * TC) : 1;
+    constexpr int kOut = 4 * TC > kStThreads ? 4 * TC / kStThreads : 1;
+    const int h = tid % kSh;
+    int ok[kOut];
+    double before[kOut];
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+        const int o = tid / kSh + j * kStThreads, oc = o >> 2, comp = o & 3;
+        ok[j] = h == 0 && comp < 3 && oc < d.count ? column(d.first + oc) : -1;
+        before[j] = ok[j] >= 0 && mode != 0 ? __ldcg(reinterpret_cast<const double *>(pc64 + ok[j]) + comp) : 0.0;
+    }
+    auto put = [&](int r, int k) {
+        const bool own = d.first + r < d.n;
+        Vec4<T> x = ldcg4((own ? y : (const Vec4<T> *)sol) + k);
+        if (!own) x = {-x.x, -x.y, -x.z, (T)0};
+        v[r] = x;
+    };
+#pragma unroll
+    for (int i = 0; i < kPre; ++i) {
+        const int r = tid + i * kStThreads;
+        if (r < nrow) put(r, at[i]);
+    }
+    for (int r = tid + kPre * kStThreads; r < nrow; r += kStThreads) {
+        const int g = d.first + r;
+        put(r, g < d.n ? column(g) : rows[d.row_off + g - d.n]);
+    }
+    __syncthreads();
+    T acc[E][3];
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e][0] = acc[e][1] = acc[e][2] = (T)0;
+    for (int r = s; r < nrow; r += U * NS) {
+        if (r != s) load(r);
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            if (r + i * NS >= nrow) break;
+            const Vec4<T> x = v[r + i * NS];
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                acc[e][0] += m[i].v[e] * x.x;
+                acc[e][1] += m[i].v[e] * x.y;
+                acc[e][2] += m[i].v[e] * x.z;
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) red[(s * TC + q * E + e) * 4 + c] = acc[e][c];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+        const int o = tid / kSh + j * kStThreads, comp = o & 3;
+        T sum = (T)0;
+#pragma unroll 8
+        for (int i = h; i < NS; i += kSh) sum += red[i * TC * 4 + o];
+#pragma unroll
+        for (int off = 1; off < kSh; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        if (ok[j] >= 0) {
+            reinterpret_cast<T *>(sol + ok[j])[comp] = sum;
+            reinterpret_cast<double *>(pc64 + ok[j])[comp] = mode == 0 ? (double)sum : before[j] + (double)sum;
+        }
+    }
 }
 
 // RC columns [c0, c0 + RC) of supernode j's columns of its group's M: the
