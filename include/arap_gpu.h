@@ -173,14 +173,24 @@ int arap_set_done_callback(arap_ctx *ctx, arap_done_fn fn, void *user);
    is what arap_wait returns. */
 int arap_query(arap_ctx *ctx, int32_t *done);
 
-/* Most CTAs one triangular-solve launch uses (0, the default: as many as fit
-   on the device). Each CTA works through the supernodes in schedule order, so
+/* The triangular solves of a single request (arap.h:417-429) run as dense
+   phases: the elimination tree is cut into a few strata of subtrees, each
+   subtree solved through its dense inverse, one launch per stratum and
+   direction. Setting any of the options of the supernodal sweeps below to
+   other than its default (arap_set_dense_top, arap_set_cluster_threshold,
+   arap_set_warp_rows, arap_set_solve_schedule, arap_set_solve_blocks) runs
+   the sweeps instead; arap_deform_poses always does. The results are equal up
+   to the order of sums.
+
+   Most CTAs one launch of the sweeps uses (0, the default: as many as fit on
+   the device). Each CTA works through the supernodes in schedule order, so
    any count gives the same result; a smaller count leaves room for the
-   launches of other contexts running at the same time. With 0 the context
-   assumes it owns the device: its sweeps and dense-top products start while
-   the kernel before them finishes (programmatic dependent launch); with a cap
-   every launch waits for the previous one as usual. Takes effect at the next
-   deform (which sets the problem up again). */
+   launches of other contexts running at the same time. The dense phases'
+   CTAs are short and never wait for one another: a cap leaves their grids as
+   they are. With 0 the context assumes it owns the device: its solves start
+   while the kernel before them finishes (programmatic dependent launch); with
+   a cap every launch waits for the previous one as usual. Takes effect at the
+   next deform (which sets the problem up again). */
 int arap_set_solve_ctas(arap_ctx *ctx, int32_t max_ctas);
 
 /* Poses per task of the batched triangular solves of arap_deform_poses: 1, 2,

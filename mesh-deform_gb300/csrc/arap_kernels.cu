@@ -3286,7 +3286,7 @@ cudaError_t configure_dense_smem(int inv32, int inv64) {
 static int st_ldf(const StPhase &p) { return (p.nmax + 127) & ~127; }
 static size_t st_fwd_smem(const StPhase &p, int sb) { return (size_t)3 * st_ldf(p) * sb; }
 static size_t st_bwd_smem(const StPhase &p, int sb) {
-    return (size_t)p.vmax * 4 * sb + (size_t)kStThreads * (16 / sb) * 4 * sb;
+    return (size_t)p.vmax * 4 * sb + (size_t)p.ntb * (16 / sb) * 4 * sb;
 }
 // columns per pass of the inversion whose buffers fit shared memory (0: none)
 static int st_inv_cols(const StPhase &p, int sb) {
@@ -3302,43 +3302,57 @@ bool strata_fits(const Strata &st, int sb) {
     return true;
 }
 
-template <typename T, int G, int RW> static cudaError_t raise_st_fwd(int bytes) {
-    return raise_smem_limit((const void *)k_strata_fwd<T, G, RW>, bytes);
-}
+// the phases' kernels by their launch shape
+template <typename T> struct StKernels {
+    using Fwd = void (*)(int, const StTile *, const T *, const int32_t *, const Vec4<T> *, Vec4<T> *, Vec4<T> *);
+    using Bwd = void (*)(int, const StTile *, const T *, const int32_t *, const int32_t *, const Vec4<T> *, Vec4<T> *,
+                         Vec4<double> *, int);
+    template <int NT> static Fwd fwd_nt(int G, int RW) {
+        if constexpr (sizeof(T) == 8) {  // one row per lane group (build_strata)
+            if (G == 1) return k_strata_fwd<T, NT, 1, 1>;
+            if (G == 4) return k_strata_fwd<T, NT, 4, 1>;
+            return G == 8 ? k_strata_fwd<T, NT, 8, 1> : k_strata_fwd<T, NT, 32, 1>;
+        } else {
+            if (G == 8)
+                return RW == 4 ? k_strata_fwd<T, NT, 8, 4> : RW == 2 ? k_strata_fwd<T, NT, 8, 2> : k_strata_fwd<T, NT, 8, 1>;
+            return RW == 4 ? k_strata_fwd<T, NT, 32, 4> : RW == 2 ? k_strata_fwd<T, NT, 32, 2> : k_strata_fwd<T, NT, 32, 1>;
+        }
+    }
+    template <int NT> static Bwd bwd_nt(int TC) {
+        switch (TC) {
+        case 64: return k_strata_bwd<T, NT, 64>;
+        case 32: return k_strata_bwd<T, NT, 32>;
+        case 16: return k_strata_bwd<T, NT, 16>;
+        case 8: return k_strata_bwd<T, NT, 8>;
+        default: return k_strata_bwd<T, NT, 4>;
+        }
+    }
+    static Fwd fwd(const StPhase &p) {
+        return p.ntf == kStThreads ? fwd_nt<kStThreads>(p.G, p.RW) : fwd_nt<kStThreadsLarge>(p.G, p.RW);
+    }
+    static Bwd bwd(const StPhase &p) {
+        return p.ntb == kStThreads ? bwd_nt<kStThreads>(p.TC) : bwd_nt<kStThreadsLarge>(p.TC);
+    }
+};
+
 template <typename T> static cudaError_t configure_strata_t(const Strata &st) {
-    size_t f = 0, b = 0, v = 0;
-    for (const StPhase &p : st.ph) {
-        v = std::max(v, dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), st_inv_cols(p, sizeof(T))));
-        if (p.big) continue;
-        f = std::max(f, st_fwd_smem(p, sizeof(T)));
-        b = std::max(b, st_bwd_smem(p, sizeof(T)));
-    }
     cudaError_t e = cudaSuccess;
-    auto up = [&](cudaError_t r) {
-        if (e == cudaSuccess) e = r;
+    auto up = [&](const void *f, size_t bytes) {
+        if (e == cudaSuccess) e = raise_smem_limit(f, (int)bytes);
     };
-    if constexpr (sizeof(T) == 8) {
-        up(raise_st_fwd<T, 1, 1>((int)f));
-        up(raise_st_fwd<T, 4, 1>((int)f));
-    } else {
-        up(raise_st_fwd<T, 8, 2>((int)f));
-        up(raise_st_fwd<T, 8, 4>((int)f));
-        up(raise_st_fwd<T, 32, 2>((int)f));
-        up(raise_st_fwd<T, 32, 4>((int)f));
-    }
-    up(raise_st_fwd<T, 8, 1>((int)f));
-    up(raise_st_fwd<T, 32, 1>((int)f));
-    up(raise_smem_limit((const void *)k_strata_bwd<T, 4>, (int)b));
-    up(raise_smem_limit((const void *)k_strata_bwd<T, 8>, (int)b));
-    up(raise_smem_limit((const void *)k_strata_bwd<T, 16>, (int)b));
-    up(raise_smem_limit((const void *)k_strata_bwd<T, 32>, (int)b));
-    up(raise_smem_limit((const void *)k_strata_bwd<T, 64>, (int)b));
-    up(raise_smem_limit((const void *)k_strata_inverse<T, 8>, (int)v));
-    up(raise_smem_limit((const void *)k_strata_inverse<T, 4>, (int)v));
-    up(raise_smem_limit((const void *)k_strata_inverse<T, 2>, (int)v));
-    if (st.big_n > 0) {
-        up(raise_smem_limit((const void *)k_top_pair_fwd<T>, (int)top_pair_smem(sizeof(T))));
-        up(raise_smem_limit((const void *)k_top_pair_bwd<T>, (int)top_pair_smem(sizeof(T))));
+    for (const StPhase &p : st.ph) {
+        const int rc = st_inv_cols(p, sizeof(T));
+        const void *inv = rc == 8   ? (const void *)k_strata_inverse<T, 8>
+                          : rc == 4 ? (const void *)k_strata_inverse<T, 4>
+                                    : (const void *)k_strata_inverse<T, 2>;
+        up(inv, dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), rc));
+        if (p.big) {
+            up((const void *)k_top_pair_fwd<T>, top_pair_smem(sizeof(T)));
+            up((const void *)k_top_pair_bwd<T>, top_pair_smem(sizeof(T)));
+            continue;
+        }
+        up((const void *)StKernels<T>::fwd(p), st_fwd_smem(p, sizeof(T)));
+        up((const void *)StKernels<T>::bwd(p), st_bwd_smem(p, sizeof(T)));
     }
     return e;
 }
@@ -3392,25 +3406,8 @@ void launch_strata_fwd(const StrataDev &d, const T *M, Vec4<T> *sol, Vec4<T> *y,
         if (k > 0)  // no update lands on the first stratum
             launch_pdl(k_strata_gather<T>, d.overlap != 0, blocks_for(4 * (int64_t)p.cn, kStThreads), kStThreads, 0, st, p.c0, p.cn,
                        d.col, d.gptr, d.gidx, (const Vec4<T> *)uvec, sol);
-        const size_t smem = st_fwd_smem(p, sizeof(T));
-#define ARAP_STF(G, RW)                                                                                        \
-    launch_pdl(k_strata_fwd<T, G, RW>, d.overlap != 0, (int)p.fn, kStThreads, smem, st, st_ldf(p), d.tiles + p.f0, \
-               M, d.col, (const Vec4<T> *)sol, y, uvec)
-        if constexpr (sizeof(T) == 8) {  // one row per lane group (build_strata)
-            if (p.G == 1) ARAP_STF(1, 1);
-            else if (p.G == 4) ARAP_STF(4, 1);
-            else if (p.G == 8) ARAP_STF(8, 1);
-            else ARAP_STF(32, 1);
-        } else if (p.G == 8) {
-            if (p.RW == 4) ARAP_STF(8, 4);
-            else if (p.RW == 2) ARAP_STF(8, 2);
-            else ARAP_STF(8, 1);
-        } else {
-            if (p.RW == 4) ARAP_STF(32, 4);
-            else if (p.RW == 2) ARAP_STF(32, 2);
-            else ARAP_STF(32, 1);
-        }
-#undef ARAP_STF
+        launch_pdl(StKernels<T>::fwd(p), d.overlap != 0, (int)p.fn, p.ntf, st_fwd_smem(p, sizeof(T)), st, st_ldf(p),
+                   d.tiles + p.f0, M, d.col, (const Vec4<T> *)sol, y, uvec);
     }
 }
 
@@ -3432,16 +3429,8 @@ void launch_strata_bwd(const StrataDev &d, const DevSym &s, const T *M, Vec4<T> 
                            M + d.big_off, ytop, part, cnt, d.top_col, sol, pc64, pc32, mode);
             continue;
         }
-        const size_t smem = st_bwd_smem(p, sizeof(T));
-#define ARAP_STB(TC)                                                                                             \
-    launch_pdl(k_strata_bwd<T, TC>, d.overlap != 0, (int)p.bn, kStThreads, smem, st, (int)p.vmax, d.tiles + p.b0,  \
-               M, d.col, s.rows, y, sol, pc64, mode)
-        if (p.TC == 64) ARAP_STB(64);
-        else if (p.TC == 32) ARAP_STB(32);
-        else if (p.TC == 16) ARAP_STB(16);
-        else if (p.TC == 8) ARAP_STB(8);
-        else ARAP_STB(4);
-#undef ARAP_STB
+        launch_pdl(StKernels<T>::bwd(p), d.overlap != 0, (int)p.bn, p.ntb, st_bwd_smem(p, sizeof(T)), st, (int)p.vmax,
+                   d.tiles + p.b0, M, d.col, s.rows, y, sol, pc64, mode);
     }
 }
 

@@ -12,14 +12,16 @@ namespace arapgpu {
 namespace {
 
 // Cost of a sweep's phase in us: a latency per launch (measured 4 to 6 us a
-// phase with overlapped launches), the matrix entries at the rate that bounds
-// them (FP32: bytes from L2; FP64: three FMAs per entry at about 0.55 T FMA/s),
-// and the entries' formation spread over the sweeps of a deform. The minimum
-// is flat: 2 us less or 3 more per phase moves the bar by +6% / +5% and the
-// level-7 sphere by +4% / -6%.
-constexpr double kPhaseUs = 5.0, kGatherUs = 2.5, kBigTopUs = 3.0;
-constexpr double kBytesPerUs = 5e6, kFma64PerUs = 0.55e6, kFma32PerUs = 8e6;
-constexpr double kSweepsPerFactor = 40.0;
+// phase with overlapped launches) and per gather, the matrix entries at the
+// rate that bounds them (FP32: bytes from L2; FP64: three FMAs per entry at
+// about 0.55 T FMA/s), and the entries' formation spread over the sweeps of a
+// deform. The minimum is flat in FP32: 3 us for 5, or 3 TB/s for 5, move the
+// bar and the level-7 sphere by 2%; 10 us for 5 takes one phase less of the
+// level-6 sphere, 113 -> 143 us per iteration. FP64: a tiled last phase with
+// the FP32 constants 290 against 271 us (bar).
+constexpr double kPhaseUs = 5.0, kBytesPerUs = 5e6, kFma64PerUs = 0.55e6, kFma32PerUs = 8e6;
+constexpr double kGatherUs[2] = {1.0, 2.5}, kBigTopUs[2] = {0.0, 3.0};  // FP32, FP64
+constexpr double kSweepsPerFactor[2] = {40.0, 20.0};
 
 int ld_of(int n) { return (n + 3) & ~3; }
 
@@ -90,9 +92,9 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
             }
             if (!fits) continue;
             double c = kPhaseUs + std::max(ent * (fp64 ? 8 : 4) / kBytesPerUs, fp64 ? ent * 3 / kFma64PerUs : 0.0) +
-                       form / (fp64 ? kFma64PerUs : kFma32PerUs) / kSweepsPerFactor;
-            if (j == K - 1 && cnt == 1 && nmax > kStBigTop) c += kBigTopUs;
-            else if (i > 0) c += 0.5 * kGatherUs;  // forward sweeps only
+                       form / (fp64 ? kFma64PerUs : kFma32PerUs) / kSweepsPerFactor[fp64];
+            if (j == K - 1 && cnt == 1 && nmax > kStBigTop) c += kBigTopUs[fp64];
+            else if (i > 0) c += 0.5 * kGatherUs[fp64];  // forward sweeps only
             if (best[i] + c < best[j]) {
                 best[j] = best[i] + c;
                 from[j] = i;
@@ -212,7 +214,12 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
         }
         int64_t rows = 0;
         for (const int32_t g : groups[k]) rows += gcols[g] + sn[g].nrow - sn[g].ncol;
-        auto step = [&](int rw) { return kStThreads / p.G * rw; };
+        // 512 threads where groups are large: the vectors' loads and the rows
+        // per thread, a CTA's serial part, are a quarter (level-7 sphere 277 ->
+        // 235 us per iteration, FP64 sphere level 3 46 -> 37)
+        p.ntf = p.nmax > kStLargeCols ? kStThreadsLarge : kStThreads;
+        p.ntb = p.vmax > kStLargeRows ? kStThreadsLarge : kStThreads;
+        auto step = [&](int rw) { return p.ntf / p.G * rw; };
         if (fp64) {
             // a lane group's sums cost FP64 additions, the scarce
             // instructions: as few lanes per row as give every scheduler a
@@ -222,15 +229,14 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
                 if (rows * p.G < (int64_t)32 * 4 * sms * 2) p.G = g;
         } else {
             // lane groups of 8 for groups of few columns; as many rows per
-            // lane group as leave four CTAs per SM (two: repose of the
-            // level-6 sphere 112 against 109 us per iteration; eight: 113)
+            // lane group as leave four warps per scheduler
             p.G = p.nmax <= 128 ? 8 : 32;
             p.RW = 4;
-            while (p.RW > 1 && rows / step(p.RW) < 4 * sms) p.RW /= 2;
+            while (p.RW > 1 && rows / (32 / p.G * p.RW) < 4 * 4 * sms) p.RW /= 2;
         }
         const int per = step(p.RW) * (int)std::min<int64_t>(8, std::max<int64_t>(1, rows / ((int64_t)step(p.RW) * 4 * sms)));
         p.TC = fp64 ? 32 : 64;
-        while (p.TC > (fp64 ? 4 : 8) && p.cn / p.TC < 2 * sms) p.TC /= 2;
+        while (p.TC > (fp64 ? 4 : 8) && (int64_t)p.cn / p.TC * p.ntb < (int64_t)(fp64 ? 4 : 2) * kStThreads * sms) p.TC /= 2;
         auto tile = [&](int32_t g, int first, int count) {
             StTile t{};
             t.m_off = gm_off[g];

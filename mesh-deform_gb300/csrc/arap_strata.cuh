@@ -94,19 +94,19 @@ k_strata_gather(int c0, int cn, const int32_t *__restrict__ gcol, const int32_t 
 // first loads of M (which only the factorisation writes) are issued before it
 // waits for the kernel before it.
 // FP32: bound by the launch's latency chain (tile, vector, product, store),
-// not by L2: the bar's first stratum, 12 MB in 7.7 us. Eight CTAs per SM with
-// four loads in flight per lane beat four with eight (bar 164 -> 145 us per
+// not by L2: the bar's first stratum, 12 MB in 6.7 us. Four loads in flight
+// per lane and 1,024 threads per SM beat eight and 512 (bar 164 -> 145 us per
 // iteration). FP64: bound by FP64 issue (about 64 clocks per warp instruction
 // and scheduler), so lanes that share a row are as few as fill the device.
-template <typename T, int G, int RW>
-__global__ void __launch_bounds__(kStThreads, 8)
+template <typename T, int NT, int G, int RW>
+__global__ void __launch_bounds__(NT, 1024 / NT)
 k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
              const int32_t *__restrict__ gcol, const Vec4<T> *__restrict__ b, Vec4<T> *__restrict__ y,
              Vec4<T> *__restrict__ uvec) {
     extern __shared__ __align__(128) unsigned char st_raw[];
     constexpr int E = StPack<T>::E;
     constexpr int NB = 4 / RW;  // steps of one batch of loads: four 16-byte loads in flight per lane
-    constexpr int kRows = kStThreads / G * RW;
+    constexpr int kRows = NT / G * RW;
     T *fx = reinterpret_cast<T *>(st_raw), *fy = fx + ldf, *fz = fy + ldf;
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, l = tid % G, grp = tid / G;
@@ -141,7 +141,7 @@ k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Ma
     constexpr int kPre = 2;
     int at[kPre];
 #pragma unroll
-    for (int i = 0; i < kPre; ++i) at[i] = tid + i * kStThreads < ncol ? column(tid + i * kStThreads) : -1;
+    for (int i = 0; i < kPre; ++i) at[i] = tid + i * NT < ncol ? column(tid + i * NT) : -1;
     pdl_wait();
     auto put = [&](int c, int k) {
         const Vec4<T> v = k >= 0 ? ldcg4(b + k) : Vec4<T>{(T)0, (T)0, (T)0, (T)0};
@@ -151,8 +151,8 @@ k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Ma
     };
 #pragma unroll
     for (int i = 0; i < kPre; ++i)
-        if (tid + i * kStThreads < fspan) put(tid + i * kStThreads, at[i]);
-    for (int c = tid + kPre * kStThreads; c < fspan; c += kStThreads) put(c, c < ncol ? column(c) : -1);
+        if (tid + i * NT < fspan) put(tid + i * NT, at[i]);
+    for (int c = tid + kPre * NT; c < fspan; c += NT) put(c, c < ncol ? column(c) : -1);
     __syncthreads();
     for (int r0 = d.first; r0 < rend; r0 += kRows) {
         row = r0 + grp * RW;
@@ -202,16 +202,16 @@ k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Ma
 // 16 bytes of a row per thread, TC / E threads per row, the rows dealt to the
 // thread groups in turn; their sums meet in shared memory in a fixed order.
 // Bound as the forward product; 64 columns per tile where that leaves two
-// CTAs per SM (bar 143 -> 139 us per iteration, 16 bars 318 -> 305, against
-// 32), fewer for small strata.
+// CTAs per SM (16 bars 318 -> 305 us per iteration against 32), fewer for
+// small strata.
 // x goes to the solution and the positions (mode 0: pc64 = x, 1: pc64 += x).
-template <typename T, int TC>
-__global__ void __launch_bounds__(kStThreads)
+template <typename T, int NT, int TC>
+__global__ void __launch_bounds__(NT, 1024 / NT)
 k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ Mall,
              const int32_t *__restrict__ gcol, const int32_t *__restrict__ rows, const Vec4<T> *__restrict__ y,
              Vec4<T> *sol, Vec4<double> *__restrict__ pc64, int mode) {
     extern __shared__ __align__(128) unsigned char st_raw[];
-    constexpr int E = StPack<T>::E, QC = TC / E, NS = kStThreads / QC, U = 8;
+    constexpr int E = StPack<T>::E, QC = TC / E, NS = NT / QC, U = 8;
     Vec4<T> *v = reinterpret_cast<Vec4<T> *>(st_raw);
     T *red = reinterpret_cast<T *>(v + vmax);  // NS x (TC columns x 4)
     pdl_trigger();
@@ -237,21 +237,21 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
     int at[kPre];
 #pragma unroll
     for (int i = 0; i < kPre; ++i) {
-        const int r = tid + i * kStThreads, g = d.first + r;
+        const int r = tid + i * NT, g = d.first + r;
         at[i] = r < nrow ? (g < d.n ? column(g) : rows[d.row_off + g - d.n]) : 0;
     }
     pdl_wait();
     // kSh threads per output value, each every kSh-th partial sum, kOut
     // values per thread; the outputs' places and positions are loaded
     // ahead of the product
-    constexpr int kSh = 4 * TC < kStThreads ? kStThreads / (4 * TC) : 1;
-    constexpr int kOut = 4 * TC > kStThreads ? 4 * TC / kStThreads : 1;
+    constexpr int kSh = 4 * TC < NT ? NT / (4 * TC) : 1;
+    constexpr int kOut = 4 * TC > NT ? 4 * TC / NT : 1;
     const int h = tid % kSh;
     int ok[kOut];
     double before[kOut];
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
-        const int o = tid / kSh + j * kStThreads, oc = o >> 2, comp = o & 3;
+        const int o = tid / kSh + j * NT, oc = o >> 2, comp = o & 3;
         ok[j] = h == 0 && comp < 3 && oc < d.count ? column(d.first + oc) : -1;
         before[j] = ok[j] >= 0 && mode != 0 ? __ldcg(reinterpret_cast<const double *>(pc64 + ok[j]) + comp) : 0.0;
     }
@@ -263,10 +263,10 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
     };
 #pragma unroll
     for (int i = 0; i < kPre; ++i) {
-        const int r = tid + i * kStThreads;
+        const int r = tid + i * NT;
         if (r < nrow) put(r, at[i]);
     }
-    for (int r = tid + kPre * kStThreads; r < nrow; r += kStThreads) {
+    for (int r = tid + kPre * NT; r < nrow; r += NT) {
         const int g = d.first + r;
         put(r, g < d.n ? column(g) : rows[d.row_off + g - d.n]);
     }
@@ -295,7 +295,7 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
-        const int o = tid / kSh + j * kStThreads, comp = o & 3;
+        const int o = tid / kSh + j * NT, comp = o & 3;
         T sum = (T)0;
 #pragma unroll 8
         for (int i = h; i < NS; i += kSh) sum += red[i * TC * 4 + o];

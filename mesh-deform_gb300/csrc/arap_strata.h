@@ -43,19 +43,21 @@ struct StSn {
 
 constexpr int kStMaxPhases = 16;
 constexpr int kStMaxCols = 4096;   // most columns of a group
-constexpr int kStThreads = 128;
+constexpr int kStThreads = 128;     // CTAs of the phases' kernels,
+constexpr int kStThreadsLarge = 512;  // and where groups are large
 constexpr int kStBigTop = 1024;    // a lone last group with more columns runs the tiled top products
+constexpr int kStLargeCols = 256, kStLargeRows = 400;  // columns / rows from which a group is large
 constexpr int kStInvCols = 8;      // columns of M one CTA of the inversion forms
 
 struct StPhase {
     int32_t f0, fn, b0, bn;   // tiles of the forward / backward product
     int32_t G, RW, TC;        // lanes per row group, rows per group; columns per backward tile
+    int32_t ntf, ntb;         // threads per CTA of the forward / backward product
     int32_t c0, cn;           // its columns in the column list
     int32_t nmax, vmax;       // largest n and n + r
     int32_t i0, in;           // its work items of the inversion
     int32_t ldx, ld21;        // largest supernode of the phase
     int32_t big;              // the tiled top products run this phase
-    int32_t pad;
 };
 
 struct Strata {
