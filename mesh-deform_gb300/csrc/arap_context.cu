@@ -448,7 +448,6 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
     }
     if (phases) {
         const Strata &p = ctx->strata;
-        add(ctx->Xinv, (size_t)std::max<int64_t>(s.x_size, 1) * sizeof(T));
         add(ctx->st_y, m1 * sizeof(Vec4<T>));
         add(ctx->st_m, (size_t)p.m_size * sizeof(T));
         add(ctx->st_ytop, std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16));
@@ -971,22 +970,12 @@ int factor_inverses(arap_ctx *ctx, const TI *Lval, const TI *Dinv, TI *X, TI *L2
 }
 
 // The dense phases' matrices (arap_strata.h) from a factor in the solves'
-// precision: X = inv(L11) per supernode, then M = [X; W] per group.
+// precision: M = [X; W] per group.
 template <typename TI>
 int form_strata(arap_ctx *ctx, const TI *Lval, const TI *Dinv) {
-    const DevSym &d = ctx->ds;
-    cudaStream_t st = ctx->stream;
-    TI *X = ctx->Xinv.as<TI>();
-    for (const FactorLaunch &fl : ctx->sym.fplan) {
-        if (fl.kind != kFx) continue;
-        Prof pr(ctx, ARAP_K_FACTOR);
-        launch_factor_step<TI>(d, fl, ctx->fitems.as<FItem>(), const_cast<TI *>(Lval), nullptr, const_cast<TI *>(Dinv),
-                               X, nullptr, nullptr, ctx->errw.as<int>(), st);
-        ctx->launches += 1;
-    }
     {
         Prof pr(ctx, ARAP_K_FACTOR);
-        launch_strata_inverse<TI>(ctx->std_, d, X, Lval, ctx->st_m.as<TI>(), st);
+        launch_strata_inverse<TI>(ctx->std_, ctx->ds, Lval, Dinv, ctx->st_m.as<TI>(), ctx->stream);
     }
     ctx->launches += ctx->std_.nph;
     CK(cudaGetLastError());

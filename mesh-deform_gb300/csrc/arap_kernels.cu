@@ -303,16 +303,10 @@ __global__ void k_weighted_edges(int V, const int32_t *__restrict__ drow, const 
 // ---------------------------------------------------------------------------
 // multifrontal Cholesky, level by level, many CTAs per front
 
+// Every kernel of the factorisation may start while the one before it
+// finishes (an overlapped launch): it loads its item and the supernode's
+// description, which only the analysis writes, and waits.
 constexpr int kFactorThreads = 256;
-// Tile shapes of the factorisation plan (arap_symbolic.cpp builds the items
-// with the same sizes): rows of a block-column update tile, rows of a tile of
-// the solve below a diagonal block, and the square tiles of the Schur
-// complement. Small tiles spread a front's work over many CTAs, which the
-// FP64 factor needs: a GB300 SM issues about two FP64 FMAs per clock.
-constexpr int kUpdRows = kFactorUpdRows;
-constexpr int kRowsTile = kFactorRowsTile;
-constexpr int kSyrkTile = kFactorSyrkTile;
-static_assert(kUpdRows == 32 && kRowsTile == 64 && kSyrkTile == 32, "thread mappings below assume these sizes");
 
 // Front of supernode d: the nrow x ncol panel P (column-major, ld nrow; rows are
 // the supernode's columns then its struct rows) and the nb x nb update matrix U.
@@ -332,6 +326,8 @@ k_fea(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const int3
     __shared__ int s_k0, s_k1;
     const FItem it = items[blockIdx.x];
     const SnInfo d = sn[it.sn];
+    pdl_wait();
+    pdl_trigger();
     const int n = d.nrow, nc = d.ncol, nb = n - nc;
     TF *P = Lval + d.panel_off;
     TF *U = Upd + d.upd_off;
@@ -446,258 +442,301 @@ __device__ __forceinline__ int tile_entries(int vr, int vc, bool tri, int er[4],
     return ne;
 }
 
-// Left-looking update of block column jb: rows [j0 + 32 rt, +32) of columns
-// [j0, j0+w) lose sum_{k < j0} P(r, k) P(j0+c, k).
-template <typename TF>
-__global__ void __launch_bounds__(kFactorThreads)
-k_fupd(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF *__restrict__ Lval) {
-    __shared__ TF As[NB][kUpdRows];
+// Right-looking update by block column jb: the R x 32 tile (row tile rt of
+// the rows from block column cb on) of block column cb loses
+// sum_{k in block jb} P(r, k) P(c, k). One 32-wide slice per launch, however
+// many block columns came before (left-looking updates summed them all in
+// front of the next diagonal block: 25 launches of 26 us on the bar).
+template <int R, typename TF>
+__global__ void __launch_bounds__(R == 32 ? 256 : 128)
+k_ftrail(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF *__restrict__ Lval) {
+    constexpr int NT = R == 32 ? 256 : 128;
+    __shared__ TF As[NB][R];
     __shared__ TF Bs[NB][NB + 1];
     const FItem it = items[blockIdx.x];
     const SnInfo d = sn[it.sn];
-    const int n = d.nrow, nc = d.ncol;
-    const int j0 = jb * NB, w = min(NB, nc - j0);
-    const int r0 = j0 + it.a * kUpdRows;
+    const int n = d.nrow, j0 = jb * NB, c0 = it.b * NB, w = min(NB, d.ncol - c0);
+    const int r0 = c0 + it.a * R;
     TF *P = Lval + d.panel_off;
     const int tid = threadIdx.x;
-    // the tile's entries: rows r0.. (at most kUpdRows, inside the front),
-    // columns of the block; the first row tile is the diagonal block, of
-    // which the lower triangle is needed
+    // the tile's entries inside the front and its lower triangle
     int er[4], ec[4];
-    const int ne = tile_entries(min(kUpdRows, n - r0), w, it.a == 0, er, ec);
-    TF acc[4] = {0, 0, 0, 0};
-    // the next k-slice is loaded into registers while the current one is
-    // multiplied, so its global round trip overlaps the products
-    constexpr int kPa = NB * kUpdRows / kFactorThreads, kPb = NB * NB / kFactorThreads;
-    TF pa[kPa], pb[kPb];
-    auto load_slice = [&](int k0) {
-#pragma unroll
-        for (int u = 0; u < kPa; ++u) {
-            const int q = tid + u * kFactorThreads, t = q / kUpdRows, r = q % kUpdRows;
-            pa[u] = (r0 + r < n) ? P[(int64_t)(k0 + t) * n + r0 + r] : (TF)0;
+    int ne = 0;
+    if (r0 >= c0 + w) {
+        ne = tile_entries(min(R, n - r0), w, false, er, ec);
+    } else {
+        // rows and columns of the diagonal block: entry (r, c) with r0 + r >= c0 + c
+        const int vr = min(R, n - r0);
+        int seen = 0;
+        for (int c = 0; c < w && ne < 4; ++c) {
+            const int lo = max(0, c0 + c - r0), cnt = vr - lo;
+            if (cnt <= 0) continue;
+            for (int e = (tid - seen % NT + NT) % NT; e < cnt && ne < 4; e += NT) {
+                er[ne] = lo + e;
+                ec[ne] = c;
+                ++ne;
+            }
+            seen += cnt;
         }
-#pragma unroll
-        for (int u = 0; u < kPb; ++u) {
-            const int q = tid + u * kFactorThreads, t = q / NB, c = q % NB;
-            pb[u] = (c < w) ? P[(int64_t)(k0 + t) * n + j0 + c] : (TF)0;
-        }
-    };
-    if (j0 > 0) load_slice(0);
-    for (int k0 = 0; k0 < j0; k0 += NB) {
-#pragma unroll
-        for (int u = 0; u < kPa; ++u) {
-            const int q = tid + u * kFactorThreads;
-            As[q / kUpdRows][q % kUpdRows] = pa[u];
-        }
-#pragma unroll
-        for (int u = 0; u < kPb; ++u) {
-            const int q = tid + u * kFactorThreads;
-            Bs[q / NB][q % NB] = pb[u];
-        }
-        __syncthreads();
-        if (k0 + NB < j0) load_slice(k0 + NB);
-        tile_fma(ne, NB, &As[0][0], kUpdRows, &Bs[0][0], NB + 1, er, ec, acc);
-        __syncthreads();
     }
+    pdl_wait();
+    pdl_trigger();
+    for (int q = tid; q < NB * R; q += NT) {
+        const int t = q / R, r = q % R;
+        As[t][r] = r0 + r < n ? P[(int64_t)(j0 + t) * n + r0 + r] : (TF)0;
+    }
+    for (int q = tid; q < NB * NB; q += NT) {
+        const int t = q / NB, c = q % NB;
+        Bs[t][c] = c < w ? P[(int64_t)(j0 + t) * n + c0 + c] : (TF)0;
+    }
+    TF old[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-        if (q < ne) P[(int64_t)(j0 + ec[q]) * n + r0 + er[q]] -= acc[q];
+        if (q < ne) old[q] = P[(int64_t)(c0 + ec[q]) * n + r0 + er[q]];
+    __syncthreads();
+    TF acc[4] = {0, 0, 0, 0};
+    tile_fma(ne, NB, &As[0][0], R, &Bs[0][0], NB + 1, er, ec, acc);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (q < ne) P[(int64_t)(c0 + ec[q]) * n + r0 + er[q]] = old[q] - acc[q];
 }
 
-// 1/sqrt(a) for the pivots: an FP32 seed refined by two Newton steps in the
-// working precision (a double's 53 bits from the seed's 22), which on GB300
-// costs far fewer FP64 instructions than a correctly rounded sqrt and a
-// division. Pivots outside the FP32 range take the plain route.
+// 1/sqrt(a) for the pivots: an FP32 seed r (relative error about 2^-21) and
+// one third-order step, r (1 + e/2 + 3 e^2/8) with e = 1 - a r^2, which leaves
+// about e^3: five dependent FP64 instructions where two Newton steps take
+// eight. The conversions run on the integer pipe. Pivots outside the FP32
+// range take the plain route.
 template <typename TF> __device__ __forceinline__ TF pivot_rsqrt(TF a);
 template <> __device__ __forceinline__ float pivot_rsqrt(float a) { return rsqrtf(a); }
 template <> __device__ __forceinline__ double pivot_rsqrt(double a) {
-    if (!(a > 1e-30 && a < 1e30)) return 1.0 / sqrt(a);
-    double r = (double)rsqrtf((float)a);
-    r = r * (1.5 - 0.5 * a * r * r);
-    r = r * (1.5 - 0.5 * a * r * r);
-    return r;
+    const int ex = __double2hiint(a) >> 20;  // biased exponent (the sign would make it negative or large)
+    if (!(ex > 924 && ex < 1122)) return 1.0 / sqrt(a);
+    const double r = dev::to_double(rsqrtf(dev::to_float_scaled(a, 1023)));
+    const double e = fma(-(a * r), r, 1.0);
+    return fma(r, e * fma(e, 0.375, 0.5), r);
+}
+__device__ __forceinline__ bool pivot_ok(float a) { return a > 0.f; }
+__device__ __forceinline__ bool pivot_ok(double a) {
+    const int hi = __double2hiint(a);
+    return hi > 0 && hi < 0x7ff00000 ? true : a > 0.0;
 }
 
 constexpr int kFdtThreads = 128;
-constexpr int kTri = NB * (NB + 1) / 2;  // entries of a block's lower triangle
 
 // Diagonal block jb of a front: its Cholesky factor and that factor's inverse
-// (written to Dinv for k_frows, which solves the rows below, and for k_fx).
-// Four warps share each step through shared memory, every lane with a useful
-// entry, so the FP64 form's arithmetic uses all four schedulers of the SM (a
-// GB300 SM issues about two FP64 FMAs per clock; a single warp's FP64 chain
-// runs at a quarter of that). Right-looking: step k takes the pivot, scales
-// column k and updates the trailing lower triangle, the operations of a
-// column-by-column Cholesky in the same order. The trailing entries of step k
-// are the first (31-k)(32-k)/2 of a table of the triangle ordered by column,
-// last column first. The inverse X = inv(L) is formed row by row: row i is
-// -rinv(i) times row i of L times the rows above, with the sum over k split
-// in four quarters (one per warp) added in a fixed order.
+// (written to Dinv for k_frows, which solves the rows below, and for the
+// groups' inverses). Bound by the chain of 32 pivots: an FP64 instruction
+// holds a scheduler's FP64 pipe for about 64 clocks, so a chain runs at that
+// pace and work on the same scheduler adds to it.
+// Lane i holds row i in registers, warp wp the columns c = wp mod 4. Step k:
+// the owner of column k + 1 first updates that column by column k, takes its
+// pivot and publishes it; then all warps update their other columns by column
+// k: one barrier per step, the updates of three warps beside the pivot chain
+// of the fourth (before: three barriers per step with the block in shared
+// memory, and two barriers per row of the inverse: 44 us per launch).
+// The inverse by halves: 8 x 8 blocks by substitution (a lane per column),
+// then X21 = -X22 (L21 X11) for blocks of 8 and of 16, products that use all
+// four schedulers.
 template <typename TF>
 __global__ void __launch_bounds__(kFdtThreads)
 k_fdt(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF *__restrict__ Lval,
       TF *__restrict__ Dinv, int *err) {
-    __shared__ TF A[NB][NB + 1];   // the block, A[r][c] = L(r, c) once factored
-    __shared__ TF X[NB][NB + 1];   // its inverse, X[r][c]
-    __shared__ TF part[4][NB];     // quarter sums of the inverse's current row
-    __shared__ TF rinv[NB];        // 1 / L(r, r)
-    __shared__ uint8_t tri_i[kTri], tri_j[kTri];
-    __shared__ int s_bad;
+    __shared__ TF col[2][NB];      // column k and k + 1 of L
+    __shared__ TF Ls[NB][NB + 1];  // the factored block, [r][c]
+    __shared__ TF X[NB][NB + 1];   // its inverse, [r][c]
+    __shared__ TF Ts[16][17];
+    __shared__ TF rinv[NB];        // 1 / L(r, r), 0 past the block
     const SnInfo d = sn[items[blockIdx.x].sn];
     const int n = d.nrow, nc = d.ncol;
     const int j0 = jb * NB, w = min(NB, nc - j0);
-    TF *P = Lval + d.panel_off;
-    const int tid = threadIdx.x;
-    if (tid == 0) s_bad = 0;
-    for (int q = tid; q < NB * NB; q += kFdtThreads) {
-        const int r = q % NB, c = q / NB;
-        A[r][c] = (r < w && c <= r) ? P[(int64_t)(j0 + c) * n + j0 + r] : (TF)0;
-        X[r][c] = (TF)0;
+    TF *P = Lval + d.panel_off + (int64_t)j0 * n + j0;
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    if (tid < NB) rinv[tid] = (TF)0;
+    pdl_wait();
+    pdl_trigger();
+    TF a[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int c = 4 * q + wp;
+        a[q] = (c < w && lane >= c && lane < w) ? P[(int64_t)c * n + lane] : (TF)0;
     }
-    // triangle table of the block's w columns: column jj from w-1 down to 0,
-    // rows jj..w-1 (a narrow block issues no FP64 work for absent rows)
-    for (int t = tid; t < w * (w + 1) / 2; t += kFdtThreads) {
-        int jj = w - 1, base = 0;
-        while (t >= base + (w - jj)) {
-            base += w - jj;
-            --jj;
+    for (int q = tid; q < NB * NB; q += kFdtThreads) X[q / NB][q % NB] = (TF)0;
+    bool bad = false;
+    auto pivot = [&](int k, TF &ak) {
+        TF p = __shfl_sync(0xffffffffu, ak, k);
+        if (!pivot_ok(p)) {
+            bad = true;
+            p = (TF)1;
         }
-        tri_j[t] = (uint8_t)jj;
-        tri_i[t] = (uint8_t)(jj + (t - base));
+        const TF r = pivot_rsqrt(p);
+        TF l = (lane == k ? p : ak) * r;
+        if (lane < k) l = (TF)0;
+        ak = l;
+        col[k & 1][lane] = l;
+        if (lane == k) rinv[k] = r;
+    };
+    __syncthreads();  // rinv is cleared
+    if (wp == 0) pivot(0, a[0]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NB - 1; ++k) {
+        if (k + 1 >= w) break;
+        const TF *ck = col[k & 1];
+        const TF li = ck[lane];
+        if (wp == ((k + 1) & 3)) {
+            TF &an = a[(k + 1) >> 2];
+            an -= li * ck[k + 1];
+            pivot(k + 1, an);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = 4 * q + wp;
+            if (4 * q + 3 > k + 1 && c > k + 1 && c < w) a[q] -= li * ck[c];
+        }
+        __syncthreads();
+    }
+    if (bad && lane == 0) atomicOr(err, kErrNotSpd);
+    // the factored block back into the panel and, for the inverse, into shared memory
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int c = 4 * q + wp;
+        const bool in = c < w && lane >= c && lane < w;
+        Ls[lane][c] = in ? a[q] : (TF)0;
+        if (in) P[(int64_t)c * n + lane] = a[q];
     }
     __syncthreads();
-    for (int k = 0; k < w; ++k) {
-        if (tid == 0) {
-            TF a = A[k][k];
-            if (!(a > (TF)0)) {
-                s_bad = 1;
-                a = (TF)1;
-            }
-            const TF r = pivot_rsqrt(a);
-            A[k][k] = a * r;
-            rinv[k] = r;
+    if (wp == 0) {
+        const int b = lane & ~7, o = lane & 7;
+        TF x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            TF s = i == o ? (TF)1 : (TF)0;
+#pragma unroll
+            for (int k = 0; k < i; ++k) s -= Ls[b + i][b + k] * x[k];
+            x[i] = s * rinv[b + i];
+            X[b + i][lane] = x[i];
         }
-        __syncthreads();
-        const TF r = rinv[k];
-        for (int i = k + 1 + tid; i < w; i += kFdtThreads) A[i][k] *= r;
-        __syncthreads();
-        const int T = (w - 1 - k) * (w - k) / 2;  // entries of columns k+1..w-1
-        for (int t = tid; t < T; t += kFdtThreads) {
-            const int i = tri_i[t], jj = tri_j[t];
-            A[i][jj] -= A[i][k] * A[jj][k];
-        }
-        __syncthreads();
     }
-    if (s_bad && tid == 0) atomicOr(err, kErrNotSpd);
-    // the factored block back into the panel
-    for (int q = tid; q < NB * NB; q += kFdtThreads) {
-        const int r = q % NB, c = q / NB;
-        if (r < w && c <= r) P[(int64_t)(j0 + c) * n + j0 + r] = A[r][c];
-    }
-    // X row by row: X(i, c) = -rinv(i) sum_{c <= k < i} L(i, k) X(k, c), X(i, i) = rinv(i)
-    const int c = tid & 31, qk = tid >> 5;  // column, quarter of the k range
-    for (int i = 0; i < w; ++i) {
-        TF acc = (TF)0;
-        for (int k = c + ((qk - c) & 3); k < i; k += 4) acc += A[i][k] * X[k][c];  // k >= c, k = qk mod 4
-        part[qk][c] = acc;
+    __syncthreads();
+    {  // blocks of 8: rows 8..15 and 24..31
+        const int B = (tid >> 6) * 16, i = (tid >> 3) & 7, c = tid & 7;
+        TF s = (TF)0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += Ls[B + 8 + i][B + k] * X[B + k][B + c];
+        Ts[(tid >> 6) * 8 + i][c] = s;
         __syncthreads();
-        if (tid < NB && c <= i) {
-            const TF sum = (part[0][c] + part[1][c]) + (part[2][c] + part[3][c]);
-            X[i][c] = (c == i) ? rinv[i] : -sum * rinv[i];
+        s = (TF)0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += X[B + 8 + i][B + 8 + k] * Ts[(tid >> 6) * 8 + k][c];
+        X[B + 8 + i][B + c] = -s;
+    }
+    __syncthreads();
+    if (w > 16) {  // blocks of 16: columns c and 15 - c of L21 X11, then rows i and 15 - i
+        {
+            const int i = tid >> 3, c = tid & 7;
+            TF s0 = (TF)0, s1 = (TF)0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s0 += Ls[16 + i][k] * X[k][c];
+#pragma unroll
+            for (int k = 8; k < 16; ++k) s1 += Ls[16 + i][k] * X[k][15 - c];
+            Ts[i][c] = s0;
+            Ts[i][15 - c] = s1;
         }
+        __syncthreads();
+        const int i = tid >> 4, c = tid & 15;
+        TF s0 = (TF)0, s1 = (TF)0;
+        for (int k = 0; k <= 2 * wp + 1; ++k) s0 += X[16 + i][16 + k] * Ts[k][c];
+        for (int k = 0; k <= 15 - 2 * wp; ++k) s1 += X[31 - i][16 + k] * Ts[k][c];
+        X[16 + i][c] = -s0;
+        X[31 - i][c] = -s1;
         __syncthreads();
     }
     TF *D = Dinv + d.dinv_off + (int64_t)jb * NB * NB;  // column-major: D[c * NB + r] = X(r, c)
     for (int q = tid; q < NB * NB; q += kFdtThreads) D[q] = X[q % NB][q / NB];
 }
 
-// The rows below diagonal block jb of a front, 64 rows per CTA, when the plan
-// takes them out of k_fdt (fronts with many rows): L(i, j0 + c) =
-// sum_k A(i, j0 + k) X(c, k) with X = inv(L_bb) from Dinv, written in place.
-// One matrix product per tile, so the rows spread over many CTAs instead of
-// one CTA's forward substitution.
-template <typename TF>
-__global__ void __launch_bounds__(kFactorThreads)
+// The rows below diagonal block jb of a front, R rows per CTA: L(i, j0 + c) =
+// sum_{k <= c} A(i, j0 + k) X(c, k) with X = inv(L_bb) from Dinv, in place.
+// Bound by FP64 issue: X is lower triangular, so warp wp takes the column
+// groups wp and 7 - wp (four columns each), whose sums are 36 terms together
+// whatever wp is; a half warp takes two columns of each group, a lane a row.
+template <int R, typename TF>
+__global__ void __launch_bounds__(128)
 k_frows(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF *__restrict__ Lval,
         const TF *__restrict__ Dinv) {
-    __shared__ TF As[NB][kRowsTile];
+    __shared__ TF As[NB][R];
     __shared__ TF Bs[NB][NB + 1];
     const FItem it = items[blockIdx.x];
     const SnInfo d = sn[it.sn];
     const int n = d.nrow, nc = d.ncol;
     const int j0 = jb * NB, w = min(NB, nc - j0);
-    const int r0 = j0 + w + it.a * kRowsTile;
+    const int r0 = j0 + w + it.a * R;
     TF *P = Lval + d.panel_off;
     const TF *D = Dinv + d.dinv_off + (int64_t)jb * NB * NB;  // column-major: D[k * NB + c] = X(c, k)
-    // warp wp: columns 4wp..4wp+3; lane: rows lane and lane + 32. X is lower
-    // triangular, so column c needs k <= c only: a warp's k range ends at its
-    // last column (the same bound for all its lanes), and warps past the
-    // block's columns or rows skip their work, which saves FP64 instructions,
-    // the scarce kind on this GPU
-    const int tid = threadIdx.x, wp = tid >> 5, lane = tid & 31;
-    for (int q = tid; q < NB * kRowsTile; q += kFactorThreads) {
-        const int t = q / kRowsTile, r = q % kRowsTile;
+    const int tid = threadIdx.x, wp = tid >> 5, lane = tid & 31, lr = lane & 15, h = lane >> 4;
+    pdl_wait();
+    pdl_trigger();
+    for (int q = tid; q < NB * R; q += 128) {
+        const int t = q / R, r = q % R;
         As[t][r] = (t < w && r0 + r < n) ? P[(int64_t)(j0 + t) * n + r0 + r] : (TF)0;
     }
-    for (int q = tid; q < NB * NB; q += kFactorThreads) Bs[q / NB][q % NB] = D[q];
+    for (int q = tid; q < NB * NB; q += 128) Bs[q / NB][q % NB] = D[q];
     __syncthreads();
-    const int c0 = 4 * wp;
-    if (c0 >= w) return;
-    const int kend = min(c0 + 4, w);
-    const bool two = r0 + 32 < n;  // rows lane + 32 hold entries for some lane
-    TF acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    for (int t = 0; t < kend; ++t) {
-        const TF a0 = As[t][lane];
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) acc[0][cc] += a0 * Bs[t][c0 + cc];
-        if (two) {
-            const TF a1 = As[t][lane + 32];
+    for (int rr = 0; rr < R; rr += 16) {
+        if (r0 + rr >= n) break;
+        const int r = r0 + rr + lr;
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) acc[1][cc] += a1 * Bs[t][c0 + cc];
-        }
-    }
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-        const int r = r0 + lane + 32 * rr;
-        if (r >= n) continue;
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const int c = c0 + cc;
-            if (c < w) P[(int64_t)(j0 + c) * n + r] = acc[rr][cc];
+        for (int half = 0; half < 2; ++half) {
+            const int g = half == 0 ? wp : 7 - wp, c = 4 * g + 2 * h, kend = min(4 * g + 4, w);
+            if (4 * g >= w) continue;
+            TF s0 = (TF)0, s1 = (TF)0;
+            for (int t = 0; t < kend; ++t) {
+                const TF x = As[t][rr + lr];
+                s0 += x * Bs[t][c];
+                s1 += x * Bs[t][c + 1];
+            }
+            if (r < n && c < w) P[(int64_t)(j0 + c) * n + r] = s0;
+            if (r < n && c + 1 < w) P[(int64_t)(j0 + c + 1) * n + r] = s1;
         }
     }
 }
 
-// Schur complement of a front: the 32x32 tile (rt, ct), rt >= ct, of U loses
-// sum_{k < nc} L21(r, k) L21(c, k); each entry is read and written once.
-template <typename TF>
-__global__ void __launch_bounds__(kFactorThreads)
+// Schur complement of a front: the S x S tile (rt, ct), rt >= ct, of U loses
+// sum_{k < nc} L21(r, k) L21(c, k); each entry is read and written once. Bound
+// by FP64 issue; S = 16 where 32 would leave SMs idle (a 32 x 32 tile of a
+// 200-column front holds its SM for 60 us).
+template <int S, typename TF>
+__global__ void __launch_bounds__(S * 8)
 k_fsyrk(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *__restrict__ Lval,
         TF *__restrict__ Upd) {
-    __shared__ TF As[NB][kSyrkTile];
-    __shared__ TF Bs[NB][kSyrkTile];
+    constexpr int NT = S * 8;
+    __shared__ TF As[NB][S];
+    __shared__ TF Bs[NB][S];
     const FItem it = items[blockIdx.x];
     const SnInfo d = sn[it.sn];
     const int n = d.nrow, nc = d.ncol, nb = n - nc;
     const TF *P = Lval + d.panel_off;
     TF *U = Upd + d.upd_off;
-    const int rb = it.a * kSyrkTile, cb = it.b * kSyrkTile;  // within U
-    const int vr = min(kSyrkTile, nb - rb), vc = min(kSyrkTile, nb - cb);
+    const int rb = it.a * S, cb = it.b * S;  // within U
+    const int vr = min(S, nb - rb), vc = min(S, nb - cb);
     const bool diag = rb == cb;
     const int tid = threadIdx.x;
     // only the tile's entries inside U and its lower triangle are computed
     int er[4], ec[4];
     const int ne = tile_entries(vr, vc, diag, er, ec);
     TF acc[4] = {(TF)0, (TF)0, (TF)0, (TF)0};
+    pdl_wait();
+    pdl_trigger();
     // the next k-slice is loaded into registers while the current one is
     // multiplied, so its global round trip overlaps the products
-    constexpr int kPer = NB * kSyrkTile / kFactorThreads;
+    constexpr int kPer = NB * S / NT;
     TF pa[kPer], pb[kPer];
     auto load_slice = [&](int k0) {
         const int kw = min(NB, nc - k0);
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
-            const int q = tid + u * kFactorThreads, t = q / kSyrkTile, r = q % kSyrkTile;
+            const int q = tid + u * NT, t = q / S, r = q % S;
             pa[u] = pb[u] = (TF)0;
             if (t < kw) {
                 const TF *col = P + (int64_t)(k0 + t) * n + nc;
@@ -711,13 +750,13 @@ k_fsyrk(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF
         const int kw = min(NB, nc - k0);
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
-            const int q = tid + u * kFactorThreads;
-            As[q / kSyrkTile][q % kSyrkTile] = pa[u];
-            Bs[q / kSyrkTile][q % kSyrkTile] = pb[u];
+            const int q = tid + u * NT;
+            As[q / S][q % S] = pa[u];
+            Bs[q / S][q % S] = pb[u];
         }
         __syncthreads();
         if (k0 + NB < nc) load_slice(k0 + NB);
-        tile_fma(ne, kw, &As[0][0], kSyrkTile, &Bs[0][0], kSyrkTile, er, ec, acc);
+        tile_fma(ne, kw, &As[0][0], S, &Bs[0][0], S, er, ec, acc);
         __syncthreads();
     }
 #pragma unroll
@@ -862,7 +901,7 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
             const int c = cg * 4 + cc, i = i0 + r;
             if (c >= wj) continue;
             X[(int64_t)(j0 + c) * ldx + i] = v[cc];
-            if (L21all && i >= j0 + c) XT[(int64_t)i * ldx + j0 + c] = v[cc];
+            if (i >= j0 + c) XT[(int64_t)i * ldx + j0 + c] = v[cc];
         }
     };
     {
@@ -922,7 +961,6 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
         __syncthreads();  // Ts and Ds are rewritten by the next block row
     }
     // rows of X above the block column stay as set up: zero (X is lower triangular)
-    if (!L21all) return;  // the dense phases read X alone
     TF *L21 = L21all + d.l21_off, *L21T = L21Tall + d.l21t_off;
     const int ld21 = d.ld21;
     for (int q = tid; q < wj * nb; q += kFactorThreads) {
@@ -2973,13 +3011,26 @@ void launch_factor_step(const DevSym &s, const FactorLaunch &fl, const FItem *it
                         TF *X, TF *L21, TF *L21T, int *err, cudaStream_t st) {
     if (fl.count == 0) return;
     const FItem *it = items + fl.item_off;
+    const bool ov = s.overlap != 0;
+    const SnInfo *sn = s.sn;
+    const int jb = fl.jb, n = fl.count;
     switch (fl.kind) {
-    case kFea: k_fea<TF><<<fl.count, kFactorThreads, 0, st>>>(it, s.sn, s.child, s.relind, Lval, Upd); break;
-    case kFupd: k_fupd<TF><<<fl.count, kFactorThreads, 0, st>>>(it, fl.jb, s.sn, Lval); break;
-    case kFdt: k_fdt<TF><<<fl.count, kFdtThreads, 0, st>>>(it, fl.jb, s.sn, Lval, Dinv, err); break;
-    case kFrows: k_frows<TF><<<fl.count, kFactorThreads, 0, st>>>(it, fl.jb, s.sn, Lval, Dinv); break;
-    case kFsyrk: k_fsyrk<TF><<<fl.count, kFactorThreads, 0, st>>>(it, s.sn, Lval, Upd); break;
-    case kFx: k_fx<TF><<<fl.count, kFactorThreads, 0, st>>>(it, s.sn, Lval, Dinv, X, L21, L21T); break;
+    case kFea: launch_pdl(k_fea<TF>, ov, n, kFactorThreads, 0, st, it, sn, s.child, s.relind, Lval, Upd); break;
+    case kFtrail:
+        if (fl.tile == 32) launch_pdl(k_ftrail<32, TF>, ov, n, 256, 0, st, it, jb, sn, Lval);
+        else if (fl.tile == 16) launch_pdl(k_ftrail<16, TF>, ov, n, 128, 0, st, it, jb, sn, Lval);
+        else launch_pdl(k_ftrail<8, TF>, ov, n, 128, 0, st, it, jb, sn, Lval);
+        break;
+    case kFdt: launch_pdl(k_fdt<TF>, ov, n, kFdtThreads, 0, st, it, jb, sn, Lval, Dinv, err); break;
+    case kFrows:
+        if (fl.tile == 32) launch_pdl(k_frows<32, TF>, ov, n, 128, 0, st, it, jb, sn, Lval, (const TF *)Dinv);
+        else launch_pdl(k_frows<16, TF>, ov, n, 128, 0, st, it, jb, sn, Lval, (const TF *)Dinv);
+        break;
+    case kFsyrk:
+        if (fl.tile == 32) launch_pdl(k_fsyrk<32, TF>, ov, n, 256, 0, st, it, sn, (const TF *)Lval, Upd);
+        else launch_pdl(k_fsyrk<16, TF>, ov, n, 128, 0, st, it, sn, (const TF *)Lval, Upd);
+        break;
+    case kFx: k_fx<TF><<<n, kFactorThreads, 0, st>>>(it, sn, Lval, Dinv, X, L21, L21T); break;
     }
 }
 
@@ -3288,16 +3339,11 @@ static size_t st_fwd_smem(const StPhase &p, int sb) { return (size_t)3 * st_ldf(
 static size_t st_bwd_smem(const StPhase &p, int sb) {
     return (size_t)p.vmax * 4 * sb + (size_t)p.ntb * (16 / sb) * 4 * sb;
 }
-// columns per pass of the inversion whose buffers fit shared memory (0: none)
-static int st_inv_cols(const StPhase &p, int sb) {
-    for (int rc = kStInvCols; rc >= 2; rc /= 2)
-        if (dense_inverse_smem_bytes(p.ldx, p.ld21, sb, rc) <= 200 * 1024) return rc;
-    return 0;
-}
+static size_t st_inv_smem(const StPhase &p, int sb) { return (size_t)(2 * p.front + NB) * p.rc * sb; }
 
 bool strata_fits(const Strata &st, int sb) {
     for (const StPhase &p : st.ph)
-        if (st_inv_cols(p, sb) == 0 || (!p.big && (st_fwd_smem(p, sb) > 200 * 1024 || st_bwd_smem(p, sb) > 200 * 1024)))
+        if (st_inv_smem(p, sb) > 200 * 1024 || (!p.big && (st_fwd_smem(p, sb) > 200 * 1024 || st_bwd_smem(p, sb) > 200 * 1024)))
             return false;
     return true;
 }
@@ -3327,6 +3373,11 @@ template <typename T> struct StKernels {
         default: return k_strata_bwd<T, NT, 4>;
         }
     }
+    using Inv = void (*)(const int32_t *, const SnInfo *, const StSn *, const int32_t *, const T *, const T *, int, int,
+                         T *);
+    static Inv inverse(const StPhase &p) {
+        return p.rc == 8 ? k_strata_inverse<T, 8> : p.rc == 4 ? k_strata_inverse<T, 4> : k_strata_inverse<T, 2>;
+    }
     static Fwd fwd(const StPhase &p) {
         return p.ntf == kStThreads ? fwd_nt<kStThreads>(p.G, p.RW) : fwd_nt<kStThreadsLarge>(p.G, p.RW);
     }
@@ -3341,11 +3392,7 @@ template <typename T> static cudaError_t configure_strata_t(const Strata &st) {
         if (e == cudaSuccess) e = raise_smem_limit(f, (int)bytes);
     };
     for (const StPhase &p : st.ph) {
-        const int rc = st_inv_cols(p, sizeof(T));
-        const void *inv = rc == 8   ? (const void *)k_strata_inverse<T, 8>
-                          : rc == 4 ? (const void *)k_strata_inverse<T, 4>
-                                    : (const void *)k_strata_inverse<T, 2>;
-        up(inv, dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), rc));
+        up((const void *)StKernels<T>::inverse(p), st_inv_smem(p, sizeof(T)));
         if (p.big) {
             up((const void *)k_top_pair_fwd<T>, top_pair_smem(sizeof(T)));
             up((const void *)k_top_pair_bwd<T>, top_pair_smem(sizeof(T)));
@@ -3367,20 +3414,12 @@ int strata_launches(const StrataDev &d, bool forward) {
 }
 
 template <typename T>
-void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *X, const T *Lval, T *M, cudaStream_t st) {
+void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *Lval, const T *Dinv, T *M, cudaStream_t st) {
+    // the last strata first: few CTAs with the longest chains
     for (int k = d.nph - 1; k >= 0; --k) {
         const StPhase &p = d.ph[k];
-        const int rc = st_inv_cols(p, sizeof(T));
-        const size_t smem = dense_inverse_smem_bytes(p.ldx, p.ld21, sizeof(T), rc);
-#define ARAP_STINV(R)                                                                                              \
-    k_strata_inverse<T, R><<<p.in, kStThreads, smem, st>>>(d.items + 2 * (size_t)p.i0, s.sn, d.sn, s.relind, X, Lval, \
-                                                           p.ldx, p.ld21, M)
-        switch (rc) {
-        case 8: ARAP_STINV(8); break;
-        case 4: ARAP_STINV(4); break;
-        default: ARAP_STINV(2); break;
-        }
-#undef ARAP_STINV
+        launch_pdl(StKernels<T>::inverse(p), d.overlap != 0, (int)p.in, kStThreads, st_inv_smem(p, sizeof(T)), st,
+                   d.items + 2 * (size_t)p.i0, s.sn, d.sn, s.relind, Lval, Dinv, (int)p.front, (int)(k == d.nph - 1), M);
     }
 }
 

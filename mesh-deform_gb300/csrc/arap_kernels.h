@@ -229,9 +229,9 @@ struct StrataDev {
 bool strata_fits(const Strata &p, int scalar_bytes);
 cudaError_t configure_strata(const Strata &p, int scalar_bytes);
 int strata_launches(const StrataDev &d, bool forward);
-// M of every group from the supernodes' X (k_fx) and panels; M's zeros stay as they are
+// M of every group from the panels and inverted diagonal blocks; M's zeros stay as they are
 template <typename T>
-void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *X, const T *Lval, T *M, cudaStream_t st);
+void launch_strata_inverse(const StrataDev &d, const DevSym &s, const T *Lval, const T *Dinv, T *M, cudaStream_t st);
 // sol: right-hand side in, solution out; y: the forward sweep's result
 template <typename T>
 void launch_strata_fwd(const StrataDev &d, const T *M, Vec4<T> *sol, Vec4<T> *y, Vec4<T> *uvec, Vec4<T> *ytop,

@@ -187,12 +187,17 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
     // tiles
     for (int k = 0; k < np; ++k) {
         StPhase &p = out.ph[k];
+        // columns of M per work item: as many as leave four CTAs per SM and
+        // fit shared memory (two fronts and a block of that many columns)
+        p.rc = kStInvCols;
+        for (int s = 0; s < S; ++s)
+            if (phase[s] == k) p.front = std::max(p.front, (int32_t)sn[s].nrow);
+        while (p.rc > 2 && (p.cn / p.rc < 4 * sms || (int64_t)(2 * p.front + kDiagBlock) * p.rc * (fp64 ? 8 : 4) > 200 * 1024))
+            p.rc /= 2;
         p.i0 = (int32_t)out.items.size() / 2;
         for (int s = 0; s < S; ++s) {
             if (phase[s] != k) continue;
-            p.ldx = std::max(p.ldx, (int32_t)sn[s].ldx);
-            p.ld21 = std::max(p.ld21, (int32_t)sn[s].ld21);
-            for (int c0 = 0; c0 < sn[s].ncol; c0 += kStInvCols) {
+            for (int c0 = 0; c0 < sn[s].ncol; c0 += p.rc) {
                 out.items.push_back(s);
                 out.items.push_back(c0);
             }

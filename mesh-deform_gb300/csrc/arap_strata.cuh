@@ -308,103 +308,90 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
     }
 }
 
-// RC columns [c0, c0 + RC) of supernode j's columns of its group's M: the
-// forward solve of L_gg Y = E (E the identity columns) along j's ancestors in
-// the group, supernode by supernode: Y_a = X_a F_a, U = F_b - L21_a Y_a with
-// F the update rows scattered into the parent's front. The Y are X's rows;
-// past the group's root, -U is W. Zeros of M (above the diagonal, and between
-// subtrees that do not meet) are never written: they are cleared once when
-// the matrices are laid out.
+// RC columns [c0, c0 + RC) of supernode j's columns of its group's M: forward
+// substitution L_gg Y = E (E the identity columns) along j's ancestors in the
+// group, block column by block column of 32: Y_b = inv(L_bb) F_b with the
+// factorisation's inverted diagonal blocks, then the rows below lose L Y_b;
+// a supernode's rows below its columns go into its parent's front. The Y are
+// X's rows; past the group's root, -F is W. Zeros of M (above the diagonal,
+// and between subtrees that do not meet) are never written: they are cleared
+// once when the matrices are laid out.
+// Bound by FP64 issue (FP64 form) or by the chain of blocks; a phase's columns
+// per CTA are cut until it has four CTAs per SM. The strata are independent:
+// their launches overlap (`first` waits for the factor, the others only
+// before they end).
 template <typename T, int RC>
 __global__ void __launch_bounds__(kStThreads)
 k_strata_inverse(const int32_t *__restrict__ items, const SnInfo *__restrict__ sn, const StSn *__restrict__ ssn,
-                 const int32_t *__restrict__ relind, const T *__restrict__ Xall, const T *__restrict__ Lval,
-                 int ldx_max, int ld21_max, T *__restrict__ Mall) {
+                 const int32_t *__restrict__ relind, const T *__restrict__ Lval, const T *__restrict__ Dinv,
+                 int front, int first, T *__restrict__ Mall) {
     extern __shared__ __align__(128) unsigned char st_raw[];
-    T *Y = reinterpret_cast<T *>(st_raw);   // [row][RC], rows of the current supernode's columns
-    T *U = Y + (size_t)ldx_max * RC;        // [row][RC], its struct rows
-    T *F = U + (size_t)ld21_max * RC;       // the parent's front: columns
-    T *Fb = F + (size_t)ldx_max * RC;       // and struct rows
+    T *F = reinterpret_cast<T *>(st_raw);  // [row][RC], the current supernode's front
+    T *G = F + (size_t)front * RC;         // its parent's
+    T *Y = G + (size_t)front * RC;         // [row][RC], the current block's solution
     const int tid = threadIdx.x;
-    const int j = items[2 * blockIdx.x];
-    const SnInfo dj = sn[j];
+    const int j = items[2 * blockIdx.x], c0 = items[2 * blockIdx.x + 1];
+    SnInfo dn = sn[j];
     const StSn gj = ssn[j];
-    for (int c0 = items[2 * blockIdx.x + 1], ce = min(c0 + kStInvCols, dj.ncol); c0 < ce; c0 += RC) {
-        const int w = min(RC, dj.ncol - c0);
-        T *M = Mall + gj.m_off + gj.pos + c0;  // the block's first column
-        {
-            const T *X = Xall + dj.x_off;
-            for (int q = tid; q < dj.ncol * RC; q += kStThreads) {
-                const int r = q / RC, c = q % RC;
-                const T x = (c < w && r >= c0 + c) ? X[(int64_t)(c0 + c) * dj.ldx + r] : (T)0;
-                Y[q] = x;
-                if (c < w && r >= c0 + c) M[(int64_t)(gj.pos + r) * gj.ld + c] = x;
+    const int w = min(RC, dn.ncol - c0);
+    T *M = Mall + gj.m_off + gj.pos + c0;  // the block's first column
+    for (int q = tid; q < dn.nrow * RC; q += kStThreads) F[q] = q / RC == c0 + q % RC ? (T)1 : (T)0;
+    if (first) pdl_wait();
+    pdl_trigger();
+    __syncthreads();
+    int node = j, jb = c0 / NB;
+    for (;;) {
+        const int n = dn.nrow, nc = dn.ncol, pos = ssn[node].pos;
+        const T *P = Lval + dn.panel_off;
+        for (; jb * NB < nc; ++jb) {
+            const int j0 = jb * NB, wb = min(NB, nc - j0);
+            const T *D = Dinv + dn.dinv_off + (int64_t)jb * NB * NB;  // D[k * NB + r] = inv(L_bb)(r, k)
+            for (int o = tid; o < NB * RC; o += kStThreads) {
+                const int r = o % NB, c = o / NB;
+                T dk[NB];
+#pragma unroll
+                for (int k = 0; k < NB; ++k) dk[k] = D[k * NB + r];
+                T s = (T)0;
+#pragma unroll
+                for (int k = 0; k < NB; ++k)
+                    if (k < wb) s += dk[k] * F[(j0 + k) * RC + c];
+                Y[r * RC + c] = s;
+                if (r < wb && c < w) M[(int64_t)(pos + j0 + r) * gj.ld + c] = s;
             }
+            __syncthreads();
+            for (int i = j0 + wb + tid; i < n; i += kStThreads) {
+                const T *Li = P + (int64_t)j0 * n + i;
+                T acc[RC];
+#pragma unroll
+                for (int c = 0; c < RC; ++c) acc[c] = F[i * RC + c];
+#pragma unroll 8
+                for (int k = 0; k < wb; ++k) {
+                    const T l = Li[(int64_t)k * n];
+#pragma unroll
+                    for (int c = 0; c < RC; ++c) acc[c] -= l * Y[k * RC + c];
+                }
+#pragma unroll
+                for (int c = 0; c < RC; ++c) F[i * RC + c] = acc[c];
+            }
+            __syncthreads();
         }
+        const int nb = n - nc;
+        if (ssn[node].root) {
+            for (int q = tid; q < nb * RC; q += kStThreads)
+                if (q % RC < w) M[(int64_t)(gj.n + q / RC) * gj.ld + q % RC] = -F[nc * RC + q];
+            break;
+        }
+        const int32_t *ri = relind + dn.relind_off;
+        node = dn.parent;
+        dn = sn[node];
+        for (int q = tid; q < dn.nrow * RC; q += kStThreads) G[q] = (T)0;
         __syncthreads();
-        int node = j, kfirst = c0;  // Y's rows before kfirst are zero
-        SnInfo dn = dj;
-        for (;;) {
-            const int nbn = dn.nrow - dn.ncol;
-            const T *L21 = Lval + dn.panel_off + dn.ncol;
-            const bool first = node == j, root = ssn[node].root != 0;
-            for (int r = tid; r < nbn; r += kStThreads) {
-                T acc[RC];
-#pragma unroll
-                for (int c = 0; c < RC; ++c) acc[c] = first ? (T)0 : Fb[r * RC + c];
-#pragma unroll 4
-                for (int k = kfirst; k < dn.ncol; ++k) {
-                    const T x = L21[(int64_t)k * dn.nrow + r];
-#pragma unroll
-                    for (int c = 0; c < RC; ++c) acc[c] -= x * Y[k * RC + c];
-                }
-                if (root) {
-                    T *row = M + (int64_t)(gj.n + r) * gj.ld;
-#pragma unroll
-                    for (int c = 0; c < RC; ++c)
-                        if (c < w) row[c] = -acc[c];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < RC; ++c) U[r * RC + c] = acc[c];
-                }
-            }
-            if (root) break;
-            __syncthreads();
-            const int a = dn.parent;
-            const SnInfo da = sn[a];
-            const int nca = da.ncol, nba = da.nrow - da.ncol;
-            for (int q = tid; q < (nca + nba) * RC; q += kStThreads) (q < nca * RC ? F[q] : Fb[q - nca * RC]) = (T)0;
-            __syncthreads();
-            const int32_t *ri = relind + dn.relind_off;
-            for (int q = tid; q < nbn * RC; q += kStThreads) {
-                const int i = q / RC, c = q % RC, pos = ri[i];
-                (pos < nca ? F[pos * RC + c] : Fb[(pos - nca) * RC + c]) = U[q];
-            }
-            __syncthreads();
-            const T *X = Xall + da.x_off;
-            const int pa = ssn[a].pos;
-            for (int r = tid; r < nca; r += kStThreads) {
-                T acc[RC];
-#pragma unroll
-                for (int c = 0; c < RC; ++c) acc[c] = (T)0;
-#pragma unroll 4
-                for (int k = 0; k <= r; ++k) {  // X_a is lower triangular
-                    const T x = X[(int64_t)k * da.ldx + r];
-#pragma unroll
-                    for (int c = 0; c < RC; ++c) acc[c] += x * F[k * RC + c];
-                }
-                T *row = M + (int64_t)(pa + r) * gj.ld;
-#pragma unroll
-                for (int c = 0; c < RC; ++c) {
-                    Y[r * RC + c] = acc[c];
-                    if (c < w) row[c] = acc[c];
-                }
-            }
-            __syncthreads();
-            node = a;
-            dn = da;
-            kfirst = 0;
-        }
-        __syncthreads();  // the buffers are reused by the next pass
+        for (int q = tid; q < nb * RC; q += kStThreads) G[ri[q / RC] * RC + q % RC] = F[nc * RC + q];
+        __syncthreads();
+        T *t = F;
+        F = G;
+        G = t;
+        jb = 0;
     }
+    if (!first) pdl_wait();
 }

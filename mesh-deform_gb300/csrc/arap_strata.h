@@ -47,7 +47,7 @@ constexpr int kStThreads = 128;     // CTAs of the phases' kernels,
 constexpr int kStThreadsLarge = 512;  // and where groups are large
 constexpr int kStBigTop = 1024;    // a lone last group with more columns runs the tiled top products
 constexpr int kStLargeCols = 256, kStLargeRows = 400;  // columns / rows from which a group is large
-constexpr int kStInvCols = 8;      // columns of M one CTA of the inversion forms
+constexpr int kStInvCols = 8;      // most columns of M one CTA of the inversion forms (8, 4 or 2)
 
 struct StPhase {
     int32_t f0, fn, b0, bn;   // tiles of the forward / backward product
@@ -56,7 +56,7 @@ struct StPhase {
     int32_t c0, cn;           // its columns in the column list
     int32_t nmax, vmax;       // largest n and n + r
     int32_t i0, in;           // its work items of the inversion
-    int32_t ldx, ld21;        // largest supernode of the phase
+    int32_t front, rc;        // its largest front, columns of M per item
     int32_t big;              // the tiled top products run this phase
 };
 

@@ -787,50 +787,68 @@ bool build_symbolic(const Topology &topo, const std::vector<uint8_t> &constraine
     // factorisation launch plan
     {
         const int nlev = (int)sym.level_ptr.size() - 1;
-        auto add = [&](int kind, int jb, const std::vector<FItem> &items) {
+        auto add = [&](int kind, int jb, const std::vector<FItem> &items, int tile) {
             if (items.empty()) return;
-            sym.fplan.push_back({kind, jb, (int32_t)sym.fitems.size(), (int32_t)items.size()});
+            sym.fplan.push_back({kind, jb, (int32_t)sym.fitems.size(), (int32_t)items.size(), tile});
             sym.fitems.insert(sym.fitems.end(), items.begin(), items.end());
         };
-        constexpr int kSlice = 32, kRowTile = kFactorUpdRows, kTileU = kFactorSyrkTile;
+        // items of one launch, its tiles halved from `most` down to `least`
+        // while they are too few (gen appends the items for a tile size)
+        std::vector<FItem> it;
+        auto launch = [&](int kind, int jb, int most, int least, auto &&gen) {
+            int tile = most;
+            for (;; tile /= 2) {
+                it.clear();
+                gen(tile);
+                if (tile <= least || (int)it.size() >= kFactorCtas) break;
+            }
+            add(kind, jb, it, tile);
+        };
         for (int l = 0; l < nlev; ++l) {
-            std::vector<FItem> it;
+            const int q0 = sym.level_ptr[l], q1 = sym.level_ptr[l + 1];
             int nblk_max = 0;
-            for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; ++q) {
-                const int sidx = sym.level_sn[q];
-                const SnInfo &d = sym.sn[sidx];
-                nblk_max = std::max(nblk_max, (d.ncol + kDiagBlock - 1) / kDiagBlock);
-                if (d.child_begin == d.child_end) continue;
-                for (int lo = 0; lo < d.nrow; lo += kSlice) it.push_back({sidx, lo, std::min(d.nrow, lo + kSlice), 0});
-            }
-            add(kFea, 0, it);
-            for (int jb = 0; jb < nblk_max; ++jb) {
-                std::vector<FItem> up, dt, rw;
-                for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; ++q) {
-                    const int sidx = sym.level_sn[q];
+            for (int q = q0; q < q1; ++q)
+                nblk_max = std::max(nblk_max, (sym.sn[sym.level_sn[q]].ncol + kDiagBlock - 1) / kDiagBlock);
+            launch(kFea, 0, 32, 4, [&](int t) {
+                for (int q = q0; q < q1; ++q) {
+                    const int32_t sidx = sym.level_sn[q];
                     const SnInfo &d = sym.sn[sidx];
-                    const int j0 = jb * kDiagBlock;
-                    if (j0 >= d.ncol) continue;
-                    const int below = d.nrow - std::min(d.ncol, j0 + kDiagBlock);
-                    dt.push_back({sidx, 0, 0, 0});
-                    for (int rt = 0; rt * kFactorRowsTile < below; ++rt) rw.push_back({sidx, rt, 0, 0});
-                    if (jb > 0)
-                        for (int rt = 0; j0 + rt * kRowTile < d.nrow; ++rt) up.push_back({sidx, rt, 0, 0});
+                    if (d.child_begin == d.child_end) continue;
+                    for (int lo = 0; lo < d.nrow; lo += t) it.push_back({sidx, lo, std::min(d.nrow, lo + t), 0});
                 }
-                add(kFupd, jb, up);
-                add(kFdt, jb, dt);
-                add(kFrows, jb, rw);
+            });
+            for (int jb = 0; jb < nblk_max; ++jb) {
+                const int j0 = jb * kDiagBlock;
+                it.clear();
+                for (int q = q0; q < q1; ++q)
+                    if (j0 < sym.sn[sym.level_sn[q]].ncol) it.push_back({sym.level_sn[q], 0, 0, 0});
+                add(kFdt, jb, it, kDiagBlock);
+                launch(kFrows, jb, 32, 16, [&](int t) {
+                    for (int q = q0; q < q1; ++q) {
+                        const int32_t sidx = sym.level_sn[q];
+                        const SnInfo &d = sym.sn[sidx];
+                        if (j0 >= d.ncol) continue;
+                        const int below = d.nrow - std::min(d.ncol, j0 + kDiagBlock);
+                        for (int rt = 0; rt * t < below; ++rt) it.push_back({sidx, rt, 0, 0});
+                    }
+                });
+                launch(kFtrail, jb, 32, 8, [&](int t) {
+                    for (int q = q0; q < q1; ++q) {
+                        const int32_t sidx = sym.level_sn[q];
+                        const SnInfo &d = sym.sn[sidx];
+                        for (int cb = jb + 1; cb * kDiagBlock < d.ncol; ++cb)
+                            for (int rt = 0; cb * kDiagBlock + rt * t < d.nrow; ++rt) it.push_back({sidx, rt, cb, 0});
+                    }
+                });
             }
-            std::vector<FItem> sy;
-            for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; ++q) {
-                const int sidx = sym.level_sn[q];
-                const SnInfo &d = sym.sn[sidx];
-                const int nb = d.nrow - d.ncol;
-                const int nt = (nb + kTileU - 1) / kTileU;
-                for (int rt = 0; rt < nt; ++rt)
-                    for (int ct = 0; ct <= rt; ++ct) sy.push_back({sidx, rt, ct, 0});
-            }
-            add(kFsyrk, 0, sy);
+            launch(kFsyrk, 0, 32, 16, [&](int t) {
+                for (int q = q0; q < q1; ++q) {
+                    const int32_t sidx = sym.level_sn[q];
+                    const int nt = (sym.sn[sidx].nrow - sym.sn[sidx].ncol + t - 1) / t;
+                    for (int rt = 0; rt < nt; ++rt)
+                        for (int ct = 0; ct <= rt; ++ct) it.push_back({sidx, rt, ct, 0});
+                }
+            });
         }
         // the inverses X need only the finished factor: one launch, the
         // largest fronts (top levels) first
@@ -839,7 +857,7 @@ bool build_symbolic(const Topology &topo, const std::vector<uint8_t> &constraine
             const int sidx = sym.level_sn[q];
             for (int jb = 0; jb * kDiagBlock < sym.sn[sidx].ncol; ++jb) fx.push_back({sidx, jb, 0, 0});
         }
-        add(kFx, 0, fx);
+        add(kFx, 0, fx, kDiagBlock);
     }
     amap_th.t.join();
     if (!amap_ok) {

@@ -84,20 +84,22 @@ struct FItem {
 };
 
 // Factorisation launch plan, level by level (leaves first):
-//   kFea   extend-add, item = (sn, first parent column, end parent column)
-//   kFupd  left-looking update of block column jb, item = (sn, row tile)
-//   kFdt   diagonal block jb: factor and invert, item = (sn)
-//   kFsyrk Schur complement U -= L21 L21^T, item = (sn, row tile, column tile)
-//   kFx    X = inv(L11) column block jb and the solve copies, item = (sn, jb)
-//   kFrows the rows below diagonal block jb, item = (sn, row tile)
-enum FactorKind { kFea = 0, kFupd = 1, kFdt = 2, kFsyrk = 3, kFx = 4, kFrows = 5 };
-// Tile sizes of the plan's items: rows of a kFupd tile, rows of a kFrows
-// tile, side of a kFsyrk tile
-constexpr int kFactorUpdRows = 32;
-constexpr int kFactorRowsTile = 64;
-constexpr int kFactorSyrkTile = 32;
+//   kFea    extend-add, item = (sn, first parent column, end parent column)
+//   kFdt    diagonal block jb: factor and invert, item = (sn)
+//   kFrows  the rows below diagonal block jb, item = (sn, row tile)
+//   kFtrail right-looking update by block column jb of a later block column,
+//           item = (sn, row tile, block column)
+//   kFsyrk  Schur complement U -= L21 L21^T, item = (sn, row tile, column tile)
+//   kFx     X = inv(L11) column block jb and the solve copies, item = (sn, jb)
+// `tile`: rows of a kFrows / kFtrail tile, side of a kFsyrk tile.
+enum FactorKind { kFea = 0, kFtrail = 1, kFdt = 2, kFsyrk = 3, kFx = 4, kFrows = 5 };
+// A launch's tiles are cut smaller (columns of a kFea slice, rows or sides of
+// the others) until it has this many CTAs, four per SM: FP64 instructions
+// issue at about one per 64 clocks and scheduler, so a tile's time is its
+// share of the work per scheduler.
+constexpr int kFactorCtas = 4 * 152;
 struct FactorLaunch {
-    int32_t kind, jb, item_off, count;
+    int32_t kind, jb, item_off, count, tile;
 };
 
 struct Symbolic {

@@ -85,8 +85,9 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
         for (int q = ph.i0; q < ph.i0 + ph.in; ++q) {
             const int j = p.items[2 * q], c0 = p.items[2 * q + 1];
             const SnInfo &d = s.sn[j];
-            REQUIRE(d.ldx <= ph.ldx && d.ld21 <= ph.ld21 && c0 % kStInvCols == 0 && c0 < d.ncol);
-            for (int c = c0; c < std::min(c0 + kStInvCols, (int)d.ncol); ++c) {
+            REQUIRE(d.nrow <= ph.front && c0 % ph.rc == 0 && c0 < d.ncol);
+            REQUIRE(ph.rc == 8 || ph.rc == 4 || ph.rc == 2);
+            for (int c = c0; c < std::min(c0 + ph.rc, (int)d.ncol); ++c) {
                 ++seen[d.first + c];
                 // column of M: forward substitution along j's ancestors in the group
                 const StSn &g = p.sn[j];
