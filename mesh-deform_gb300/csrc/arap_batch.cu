@@ -401,7 +401,7 @@ __global__ void k_bsetup(int V, int m, int P, const Vec4<double> *__restrict__ p
         v = {g[0], g[1], g[2], 0.0};
     }
     pc64[t] = v;
-    pc32[t] = {(float)v.x, (float)v.y, (float)v.z, 0.f};
+    if (pc32) pc32[t] = {(float)v.x, (float)v.y, (float)v.z, 0.f};
     R[3 * t + 0] = {1.f, 0.f, 0.f, 0.f};
     R[3 * t + 1] = {0.f, 1.f, 0.f, 0.f};
     R[3 * t + 2] = {0.f, 0.f, 1.f, 0.f};
@@ -427,23 +427,36 @@ __global__ void k_bbfixed(int m, int P, const int32_t *__restrict__ drow, const 
     bfixed[t] = {bx, by, bz, 0.0};
 }
 
+// The iteration's kernels take a block of kVb consecutive vertices (neighbours
+// in the elimination order, so their one-rings overlap in L1) for up to 32
+// poses: thread q of the block is (vertex q / pb, pose q % pb).
+constexpr int kVb = 8;
+__device__ __forceinline__ bool vertex_pose(int n, int P, int pb, int &i, int &p) {
+    const int q = threadIdx.x;
+    i = blockIdx.x * kVb + q / pb;
+    p = blockIdx.y * pb + q % pb;
+    return q < kVb * pb && i < n && p < P;
+}
+
 // estimateRotations per pose (arap.h:354-384): FP32 covariance from the FP32
-// rest edges and the pose's current edges differenced in FP64
+// rest edges and the pose's current edges, differences of the FP64 positions
+// rounded to FP32 (dev::Split: no FP64 instruction).
 __global__ void __launch_bounds__(256)
-k_blocal(int V, int P, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const float *__restrict__ w,
-         const Vec4<float> *__restrict__ redge, const Vec4<double> *__restrict__ pc64, Vec4<float> *__restrict__ R,
-         const double *__restrict__ w64, const Vec4<double> *__restrict__ p64) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)V * P) return;
-    const int i = (int)(t / P), p = (int)(t % P);
+k_blocal(int V, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+         const float *__restrict__ w, const Vec4<float> *__restrict__ redge, const Vec4<double> *__restrict__ pc64,
+         Vec4<float> *__restrict__ R, const double *__restrict__ w64, const Vec4<double> *__restrict__ p64) {
+    int i, p;
+    if (!vertex_pose(V, P, pb, i, p)) return;
+    const int64_t t = (int64_t)i * P + p;
     const Vec4<double> ci = pc64[t];
+    const dev::Split cx(ci.x), cy(ci.y), cz(ci.z);
     float S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     for (int e = drow[i]; e < drow[i + 1]; ++e) {
         const float wj = w[e];
         const Vec4<float> re = redge[e];
         const Vec4<double> cj = pc64[(int64_t)dcol[e] * P + p];
         const float ex = wj * re.x, ey = wj * re.y, ez = wj * re.z;
-        const float fx = (float)(ci.x - cj.x), fy = (float)(ci.y - cj.y), fz = (float)(ci.z - cj.z);
+        const float fx = cx - dev::Split(cj.x), fy = cy - dev::Split(cj.y), fz = cz - dev::Split(cj.z);
         S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
         S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
         S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
@@ -459,11 +472,12 @@ k_blocal(int V, int P, const int32_t *__restrict__ drow, const int32_t *__restri
 // estimatePositions RHS terms per pose (arap.h:395-414), bFixed added in FP64
 // by the residual
 __global__ void __launch_bounds__(256)
-k_brhs(int m, int P, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const float *__restrict__ w,
-       const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R, Vec4<float> *__restrict__ b) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)m * P) return;
-    const int i = (int)(t / P), p = (int)(t % P);
+k_brhs(int m, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+       const float *__restrict__ w, const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R,
+       Vec4<float> *__restrict__ b) {
+    int i, p;
+    if (!vertex_pose(m, P, pb, i, p)) return;
+    const int64_t t = (int64_t)i * P + p;
     const Vec4<float> r0 = R[3 * t], r1 = R[3 * t + 1], r2 = R[3 * t + 2];
     float ax = 0.f, ay = 0.f, az = 0.f;
     for (int e = drow[i]; e < drow[i + 1]; ++e) {
@@ -480,14 +494,15 @@ k_brhs(int m, int P, const int32_t *__restrict__ drow, const int32_t *__restrict
     b[t] = {ax, ay, az, 0.f};
 }
 
-// r = b - A x in FP64 per pose
+// r = b - A x in FP64 per pose; the conversions from and to FP32 on the
+// integer pipe (24 instead of 33 FP64 instructions per vertex and pose)
 __global__ void __launch_bounds__(256)
-k_bresidual(int m, int P, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+k_bresidual(int m, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
             const double *__restrict__ w64, const double *__restrict__ diag64, const Vec4<double> *__restrict__ bfixed,
             const Vec4<float> *__restrict__ b, const Vec4<double> *__restrict__ x, Vec4<float> *__restrict__ r) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)m * P) return;
-    const int i = (int)(t / P), p = (int)(t % P);
+    int i, p;
+    if (!vertex_pose(m, P, pb, i, p)) return;
+    const int64_t t = (int64_t)i * P + p;
     const Vec4<double> xi = x[t];
     const double dg = diag64[i];
     double ax = dg * xi.x, ay = dg * xi.y, az = dg * xi.z;
@@ -502,8 +517,8 @@ k_bresidual(int m, int P, const int32_t *__restrict__ drow, const int32_t *__res
     }
     const Vec4<float> bi = b[t];
     const Vec4<double> bf = bfixed[t];
-    r[t] = {(float)((bf.x + (double)bi.x) - ax), (float)((bf.y + (double)bi.y) - ay),
-            (float)((bf.z + (double)bi.z) - az), 0.f};
+    r[t] = {dev::to_float_rn((bf.x + dev::to_double(bi.x)) - ax), dev::to_float_rn((bf.y + dev::to_double(bi.y)) - ay),
+            dev::to_float_rn((bf.z + dev::to_double(bi.z)) - az), 0.f};
 }
 
 // positions of every pose back to vertex order: out[p][v][3]
@@ -519,11 +534,64 @@ __global__ void k_bgather(int V, int P, const int32_t *__restrict__ oldidx, cons
     o[2] = x.z;
 }
 
+#include "arap_bstrata.cuh"
+
+// poses, threads and grid of the (vertex block, pose) kernels: pose tiles of
+// equal size, at most 32
+inline int bv_poses(int P) {
+    const int t = (P + 31) / 32;
+    return (P + t - 1) / t;
+}
+inline int bv_threads(int P) { return (kVb * bv_poses(P) + 31) / 32 * 32; }
+inline dim3 bv_grid(int n, int P) { return dim3((n + kVb - 1) / kVb, (P + bv_poses(P) - 1) / bv_poses(P)); }
+
 inline int nblocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
+
+static size_t bs_smem(const StPhase &p) {
+    return (size_t)kBsRing * (kBsK * kBsPoses * sizeof(Vec4<float>) + bs_m_floats() * sizeof(float)) + (size_t)p.vmax * sizeof(int);
+}
+
+bool bstrata_fits(const Strata &st) {
+    for (const StPhase &p : st.ph)
+        if (bs_smem(p) > 200 * 1024) return false;
+    return true;
+}
+
+cudaError_t configure_bstrata(const Strata &st) {
+    cudaError_t e = cudaSuccess;
+    for (const StPhase &p : st.ph) {
+        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_bstrata<false>, (int)bs_smem(p));
+        if (e == cudaSuccess) e = raise_smem_limit((const void *)k_bstrata<true>, (int)bs_smem(p));
+    }
+    return e;
+}
+
+void launch_bstrata_fwd(const StrataDev &d, int P, const float *M, Vec4<float> *sol, Vec4<float> *y,
+                        Vec4<float> *uvec, cudaStream_t st) {
+    const unsigned np = (unsigned)((P + kBsPoses - 1) / kBsPoses);
+    for (int k = 0; k < d.nph; ++k) {
+        const StPhase &p = d.ph[k];
+        if (k > 0)
+            k_bstrata_gather<<<nblocks((int64_t)p.cn * P, 256), 256, 0, st>>>(p.c0, p.cn, P, d.col, d.gptr, d.gidx, uvec,
+                                                                             sol);
+        k_bstrata<false><<<dim3(p.fn, np), kBsThreads, bs_smem(p), st>>>(P, d.tiles + p.f0, M, d.col, nullptr, sol,
+                                                                        nullptr, y, uvec, nullptr);
+    }
+}
+
+void launch_bstrata_bwd(const StrataDev &d, const DevSym &s, int P, const float *M, Vec4<float> *sol,
+                        const Vec4<float> *y, Vec4<double> *pc64, cudaStream_t st) {
+    const unsigned np = (unsigned)((P + kBsPoses - 1) / kBsPoses);
+    for (int k = d.nph - 1; k >= 0; --k) {
+        const StPhase &p = d.ph[k];
+        k_bstrata<true><<<dim3(p.bn, np), kBsThreads, bs_smem(p), st>>>(P, d.tiles + p.b0, M, d.col, s.rows, y, sol, sol,
+                                                                       nullptr, pc64);
+    }
+}
 
 bool batch_pose_tile_fits(int max_ldx, int max_ld21, int pt) {
     if (pt != 1 && pt != 2 && pt != 4 && pt != 8 && pt != 16) return false;
@@ -617,19 +685,19 @@ void launch_bbfixed(const DevSym &s, int P, const double *w64, const Vec4<double
 void launch_blocal(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<double> *pc64,
                    Vec4<float> *R, const double *w64, const Vec4<double> *p64, cudaStream_t st) {
     const int64_t n = (int64_t)s.V * P;
-    if (n) k_blocal<<<nblocks(n, 256), 256, 0, st>>>(s.V, P, s.drow, s.dcol, w32, redge, pc64, R, w64, p64);
+    if (n) k_blocal<<<bv_grid(s.V, P), bv_threads(P), 0, st>>>(s.V, P, bv_poses(P), s.drow, s.dcol, w32, redge, pc64, R, w64, p64);
 }
 
 void launch_brhs(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
                  Vec4<float> *b, cudaStream_t st) {
     const int64_t n = (int64_t)s.m * P;
-    if (n) k_brhs<<<nblocks(n, 256), 256, 0, st>>>(s.m, P, s.drow, s.dcol, w32, redge, R, b);
+    if (n) k_brhs<<<bv_grid(s.m, P), bv_threads(P), 0, st>>>(s.m, P, bv_poses(P), s.drow, s.dcol, w32, redge, R, b);
 }
 
 void launch_bresidual(const DevSym &s, int P, const double *w64, const double *diag64, const Vec4<double> *bfixed,
                       const Vec4<float> *b, const Vec4<double> *x, Vec4<float> *r, cudaStream_t st) {
     const int64_t n = (int64_t)s.m * P;
-    if (n) k_bresidual<<<nblocks(n, 256), 256, 0, st>>>(s.m, P, s.drow, s.dcol, w64, diag64, bfixed, b, x, r);
+    if (n) k_bresidual<<<bv_grid(s.m, P), bv_threads(P), 0, st>>>(s.m, P, bv_poses(P), s.drow, s.dcol, w64, diag64, bfixed, b, x, r);
 }
 
 void launch_bgather(const DevSym &s, int P, const Vec4<double> *pc64, double *out, cudaStream_t st) {

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -197,7 +198,15 @@ struct arap_ctx {
     StrataDev std_{};
     bool strata_ready = false, sweeps_ready = false;
     bool strata_formed = false, sweeps_formed = false;
-    DevBuf st_tiles, st_sn, st_col, st_gptr, st_gidx, st_items, st_top_gptr, st_top_gidx, st_m, st_y, st_ytop;
+    // the same for pose batches, whose cuts differ
+    Strata bstrata;
+    bool bstrata_built = false, bstrata_ready = false, bstrata_formed = false;
+    StrataDev bstd{};
+    // the plans' device arrays: single requests, pose batches
+    struct StrataBufs {
+        DevBuf tiles, sn, col, gptr, gidx, items, top_gptr, top_gidx, m;
+    } stb, bstb;
+    DevBuf st_y, st_ytop, bst_y;
     int ordering = ARAP_ORDER_PER_CONSTRAINT_SET;
     arap_done_fn done_fn = nullptr;  // called from a CUDA thread when an async deform finished
     void *done_user = nullptr;
@@ -231,8 +240,9 @@ struct arap_ctx {
                 &vnorm, &btargets, &bpc64, &bpc32, &bR, &bbfixed, &bb, &bsol, &buvec, &bout, &bftop, &bytop, &bws,
                 &batile,
                 &bticket, &bflags, &top_col, &top_gptr, &top_gidx, &tdpos, &top_items, &Ttop, &ytop, &Lval32,
-                &Dinv32, &ssn, &slevel_sn, &sbitems, &sbmembers, &st_tiles, &st_sn, &st_col, &st_gptr, &st_gidx,
-                &st_items, &st_top_gptr, &st_top_gidx, &st_m, &st_y, &st_ytop};
+                &Dinv32, &ssn, &slevel_sn, &sbitems, &sbmembers, &stb.tiles, &stb.sn, &stb.col, &stb.gptr,
+                &stb.gidx, &stb.items, &stb.top_gptr, &stb.top_gidx, &stb.m, &bstb.tiles, &bstb.sn, &bstb.col,
+                &bstb.gptr, &bstb.gidx, &bstb.items, &bstb.top_gptr, &bstb.top_gidx, &bstb.m, &st_y, &st_ytop, &bst_y};
     }
 };
 
@@ -312,6 +322,7 @@ int analyze_symbolic(arap_ctx *ctx) {
         return fail(ctx, singular ? ARAP_ERR_NOT_SPD : ARAP_ERR_CUDA, err);
     ctx->use_sb = ctx->sb_built = false;
     ctx->strata_bits = 0;
+    ctx->bstrata_built = false;
     ctx->sym_host = true;
     return ARAP_OK;
 }
@@ -339,18 +350,33 @@ int device_sms() {
 // the supernodal sweeps at its default (an explicit dense-top cap, cluster
 // threshold, warp-row limit, solve-block size or level schedule asks for the
 // sweeps) and fronts that fit the phases' kernels. Builds the plan.
+bool sweep_options(const arap_ctx *ctx) {
+    return ctx->dense_cols != 0 || ctx->top_bytes != 0 || ctx->warp_rows != kWarpRowsDefault ||
+           ctx->solve_schedule != kSolveScheduleDefault || ctx->solve_blocks != kSolveBlocksDefault;
+}
 bool use_strata(arap_ctx *ctx, bool fp64) {
-    if (ctx->dense_cols != 0 || ctx->top_bytes != 0 || ctx->warp_rows != kWarpRowsDefault ||
-        ctx->solve_schedule != kSolveScheduleDefault || ctx->solve_blocks != kSolveBlocksDefault)
-        return false;
+    if (sweep_options(ctx)) return false;
     const int bits = fp64 ? 64 : 32;
     if (ctx->strata_bits != bits) {
         ctx->strata_ready = ctx->strata_formed = false;
-        if (build_strata(ctx->sym, fp64, device_sms(), ctx->strata) && !strata_fits(ctx->strata, bits / 8))
+        if (build_strata(ctx->sym, fp64 ? kStFp64 : kStFp32, device_sms(), ctx->strata) && !strata_fits(ctx->strata, bits / 8))
             ctx->strata.ok = false;
         ctx->strata_bits = bits;
     }
     return ctx->strata.ok;
+}
+
+// The same for pose batches, where a pose tile asks for the sweeps too.
+bool use_bstrata(arap_ctx *ctx) {
+    if (sweep_options(ctx) || ctx->pose_tile != 0) return false;
+    if (!ctx->bstrata_built) {
+        ctx->bstrata_ready = ctx->bstrata_formed = false;
+        if (build_strata(ctx->sym, kStPoses, device_sms(), ctx->bstrata) &&
+            !(strata_fits(ctx->bstrata, 4, true) && bstrata_fits(ctx->bstrata)))
+            ctx->bstrata.ok = false;
+        ctx->bstrata_built = true;
+    }
+    return ctx->bstrata.ok;
 }
 
 // The dense top of the tree: the most top levels whose supernodes hold at most
@@ -399,6 +425,17 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
     const size_t V = (size_t)s.V, m1 = (size_t)std::max(s.m, 1), nnz = s.dcol.size(), S1 = (size_t)std::max(s.S, 1);
     out.clear();
     auto add = [&](DevBuf &b, size_t bytes) { out.push_back({&b, bytes}); };
+    auto add_strata = [&](const Strata &p, arap_ctx::StrataBufs &b, size_t sz) {
+        add(b.m, (size_t)p.m_size * sz);
+        add(b.tiles, p.tiles.size() * sizeof(StTile));
+        add(b.sn, p.sn.size() * sizeof(StSn));
+        add(b.col, p.col.size() * 4);
+        add(b.gptr, p.gptr.size() * 4);
+        add(b.gidx, p.gidx.size() * 4);
+        add(b.items, p.items.size() * 4);
+        add(b.top_gptr, p.top_gptr.size() * 4);
+        add(b.top_gidx, p.top_gidx.size() * 8);
+    };
     // symbolic uploads and solve scheduling state
     add(ctx->drow, s.drow.size() * 4);
     add(ctx->dcol, s.dcol.size() * 4);
@@ -449,16 +486,23 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
     if (phases) {
         const Strata &p = ctx->strata;
         add(ctx->st_y, m1 * sizeof(Vec4<T>));
-        add(ctx->st_m, (size_t)p.m_size * sizeof(T));
         add(ctx->st_ytop, std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16));
-        add(ctx->st_tiles, p.tiles.size() * sizeof(StTile));
-        add(ctx->st_sn, p.sn.size() * sizeof(StSn));
-        add(ctx->st_col, p.col.size() * 4);
-        add(ctx->st_gptr, p.gptr.size() * 4);
-        add(ctx->st_gidx, p.gidx.size() * 4);
-        add(ctx->st_items, p.items.size() * 4);
-        add(ctx->st_top_gptr, p.top_gptr.size() * 4);
-        add(ctx->st_top_gidx, p.top_gidx.size() * 8);
+        add_strata(p, ctx->stb, sizeof(T));
+    }
+    if (n_poses > 0) {
+        const size_t P = (size_t)n_poses, VP = V * P, MP = m1 * P, nc = V - (size_t)s.m;
+        add(ctx->bpc64, VP * sizeof(Vec4<double>));
+        add(ctx->bR, VP * 3 * sizeof(Vec4<float>));
+        add(ctx->bbfixed, MP * sizeof(Vec4<double>));
+        add(ctx->bb, MP * sizeof(Vec4<float>));
+        add(ctx->bsol, MP * sizeof(Vec4<float>));
+        add(ctx->buvec, (size_t)std::max<int64_t>(s.uvec_size, 1) * P * sizeof(Vec4<float>));
+        add(ctx->bout, VP * 3 * sizeof(double));
+        add(ctx->btargets, P * nc * 3 * sizeof(double));
+        if (!sweeps) {
+            add(ctx->bst_y, MP * sizeof(Vec4<float>));
+            add_strata(ctx->bstrata, ctx->bstb, 4);
+        }
     }
     if (!sweeps) return;
     // the sweeps' solve arrays, with the solve blocks after the supernodes' own
@@ -471,19 +515,11 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
     add(ctx->Ttop, std::max<size_t>(nt > 0 ? dense_top_elems(nt) : 0, 1) * sizeof(T));
     add(ctx->ytop, std::max<size_t>(top_vec_bytes(nt, sizeof(T)), 16));  // y_top, the tiles' partials, counters
     if (n_poses > 0) {
-        const size_t P = (size_t)n_poses, VP = V * P, MP = m1 * P, nc = V - (size_t)s.m;
+        const size_t P = (size_t)n_poses, VP = V * P;
         const int pt = std::max(batch_pose_tile(ctx->use_sb ? std::max(s.max_ldx, ctx->sb.max_ldx) : s.max_ldx,
                                                 ctx->use_sb ? std::max(s.max_ld21, ctx->sb.max_ld21) : s.max_ld21), 1);
         const size_t T_ = (P + pt - 1) / pt;
-        add(ctx->bpc64, VP * sizeof(Vec4<double>));
         add(ctx->bpc32, VP * sizeof(Vec4<float>));
-        add(ctx->bR, VP * 3 * sizeof(Vec4<float>));
-        add(ctx->bbfixed, MP * sizeof(Vec4<double>));
-        add(ctx->bb, MP * sizeof(Vec4<float>));
-        add(ctx->bsol, MP * sizeof(Vec4<float>));
-        add(ctx->buvec, (size_t)std::max<int64_t>(s.uvec_size, 1) * P * sizeof(Vec4<float>));
-        add(ctx->bout, VP * 3 * sizeof(double));
-        add(ctx->btargets, P * nc * 3 * sizeof(double));
         add(ctx->bticket, 2 * sizeof(unsigned long long));
         add(ctx->bflags, 2 * S1 * T_ * sizeof(unsigned));
         add(ctx->bftop, std::max<size_t>(btop_matrix_floats(nt, (int)P), 1) * sizeof(float));
@@ -642,7 +678,7 @@ int prepare_symbolic(arap_ctx *ctx) {
     Symbolic &s = ctx->sym;
     cudaStream_t st = ctx->stream;
     ctx->gen++;
-    ctx->strata_formed = ctx->sweeps_formed = false;
+    ctx->strata_formed = ctx->sweeps_formed = ctx->bstrata_formed = false;
     CK(upload(ctx->drow, s.drow, st));
     CK(upload(ctx->dcol, s.dcol, st));
     CK(upload(ctx->dent, s.dent, st));
@@ -691,7 +727,7 @@ int prepare_symbolic(arap_ctx *ctx) {
     d.relind = ctx->relind.as<int32_t>();
     d.child = ctx->child.as<int32_t>();
     d.level_sn = ctx->level_sn.as<int32_t>();
-    ctx->strata_ready = ctx->sweeps_ready = false;
+    ctx->strata_ready = ctx->sweeps_ready = ctx->bstrata_ready = false;
     ctx->sym_valid = true;
     return ARAP_OK;
 }
@@ -845,30 +881,22 @@ int prepare_sweeps(arap_ctx *ctx) {
     return ARAP_OK;
 }
 
-// The dense phases' plan on the device, their matrices cleared (the inversion
-// never writes their zeros).
-template <typename T>
-int prepare_strata(arap_ctx *ctx) {
-    if (ctx->strata_ready) return ARAP_OK;
-    const Strata &p = ctx->strata;
+// A plan of the dense phases on the device, its matrices cleared (the
+// inversion never writes their zeros).
+int upload_strata(arap_ctx *ctx, const Strata &p, arap_ctx::StrataBufs &b, size_t scalar, StrataDev &d) {
     cudaStream_t st = ctx->stream;
     ctx->gen++;
-    ctx->strata_formed = false;
-    CK(configure_strata(p, sizeof(T)));
-    CK(upload(ctx->st_tiles, p.tiles, st));
-    CK(upload(ctx->st_sn, p.sn, st));
-    CK(upload(ctx->st_col, p.col, st));
-    CK(upload(ctx->st_gptr, p.gptr, st));
-    CK(upload(ctx->st_gidx, p.gidx, st));
-    CK(upload(ctx->st_items, p.items, st));
-    CK(upload(ctx->st_top_gptr, p.top_gptr, st));
-    CK(upload(ctx->st_top_gidx, p.top_gidx, st));
-    CK(ctx->st_m.ensure((size_t)p.m_size * sizeof(T)));
-    CK(cudaMemsetAsync(ctx->st_m.p, 0, (size_t)p.m_size * sizeof(T), st));
-    // the big top's arrival counters start at zero (each launch resets them)
-    CK(ctx->st_ytop.ensure(std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16)));
-    CK(cudaMemsetAsync(ctx->st_ytop.p, 0, ctx->st_ytop.cap, st));
-    StrataDev d{};
+    CK(upload(b.tiles, p.tiles, st));
+    CK(upload(b.sn, p.sn, st));
+    CK(upload(b.col, p.col, st));
+    CK(upload(b.gptr, p.gptr, st));
+    CK(upload(b.gidx, p.gidx, st));
+    CK(upload(b.items, p.items, st));
+    CK(upload(b.top_gptr, p.top_gptr, st));
+    CK(upload(b.top_gidx, p.top_gidx, st));
+    CK(b.m.ensure((size_t)p.m_size * scalar));
+    CK(cudaMemsetAsync(b.m.p, 0, (size_t)p.m_size * scalar, st));
+    d = StrataDev{};
     d.nph = (int)p.ph.size();
     for (int k = 0; k < d.nph; ++k) d.ph[k] = p.ph[k];
     d.overlap = ctx->solve_cap <= 0;
@@ -876,17 +904,41 @@ int prepare_strata(arap_ctx *ctx) {
     d.big_off = p.big_off;
     d.big_pair32 = p.big_n > 0 && (int64_t)top_tiles(p.big_n) > top_tile_resident_ctas(4);
     d.big_pair64 = p.big_n > 0 && (int64_t)top_tiles(p.big_n) > top_tile_resident_ctas(8);
-    d.tiles = ctx->st_tiles.as<StTile>();
-    d.sn = ctx->st_sn.as<StSn>();
-    d.col = ctx->st_col.as<int32_t>();
-    d.gptr = ctx->st_gptr.as<int32_t>();
-    d.gidx = ctx->st_gidx.as<int32_t>();
-    d.items = ctx->st_items.as<int32_t>();
+    d.tiles = b.tiles.as<StTile>();
+    d.sn = b.sn.as<StSn>();
+    d.col = b.col.as<int32_t>();
+    d.gptr = b.gptr.as<int32_t>();
+    d.gidx = b.gidx.as<int32_t>();
+    d.items = b.items.as<int32_t>();
     d.top_col = d.col + p.big_col;
-    d.top_gptr = ctx->st_top_gptr.as<int32_t>();
-    d.top_gidx = ctx->st_top_gidx.as<int64_t>();
-    ctx->std_ = d;
+    d.top_gptr = b.top_gptr.as<int32_t>();
+    d.top_gidx = b.top_gidx.as<int64_t>();
+    return ARAP_OK;
+}
+
+template <typename T>
+int prepare_strata(arap_ctx *ctx) {
+    if (ctx->strata_ready) return ARAP_OK;
+    ctx->strata_formed = false;
+    CK(configure_strata(ctx->strata, sizeof(T)));
+    const int rc = upload_strata(ctx, ctx->strata, ctx->stb, sizeof(T), ctx->std_);
+    if (rc != ARAP_OK) return rc;
+    // the big top's arrival counters start at zero (each launch resets them)
+    CK(ctx->st_ytop.ensure(std::max<size_t>(top_vec_bytes(ctx->strata.big_n, sizeof(T)), 16)));
+    CK(cudaMemsetAsync(ctx->st_ytop.p, 0, ctx->st_ytop.cap, ctx->stream));
     ctx->strata_ready = true;
+    return ARAP_OK;
+}
+
+// the pose batches' plan, and its matrices from the resident factor
+int prepare_bstrata(arap_ctx *ctx) {
+    if (ctx->bstrata_ready) return ARAP_OK;
+    ctx->bstrata_formed = false;
+    CK(configure_strata(ctx->bstrata, 4, true));
+    CK(configure_bstrata(ctx->bstrata));
+    const int rc = upload_strata(ctx, ctx->bstrata, ctx->bstb, 4, ctx->bstd);
+    if (rc != ARAP_OK) return rc;
+    ctx->bstrata_ready = true;
     return ARAP_OK;
 }
 
@@ -975,20 +1027,31 @@ template <typename TI>
 int form_strata(arap_ctx *ctx, const TI *Lval, const TI *Dinv) {
     {
         Prof pr(ctx, ARAP_K_FACTOR);
-        launch_strata_inverse<TI>(ctx->std_, ctx->ds, Lval, Dinv, ctx->st_m.as<TI>(), ctx->stream);
+        launch_strata_inverse<TI>(ctx->std_, ctx->ds, Lval, Dinv, ctx->stb.m.as<TI>(), ctx->stream);
     }
     ctx->launches += ctx->std_.nph;
     CK(cudaGetLastError());
     return ARAP_OK;
 }
 
-// The solve arrays of the current factorisation, for the dense phases or for
-// the sweeps.
+// The solve arrays of the current factorisation: for the dense phases, the
+// sweeps, or a pose batch's dense phases.
+enum SolveArrays { kSweepArrays = 0, kPhaseArrays = 1, kPoseArrays = 2 };
 template <typename T>
-int form_solves(arap_ctx *ctx, bool phases) {
+int form_solves(arap_ctx *ctx, int kind) {
     const bool demoted = sizeof(T) == 4 && ctx->factor_bits == 64;
     const T *L = (demoted ? ctx->Lval32 : ctx->Lval).as<T>(), *D = (demoted ? ctx->Dinv32 : ctx->Dinv).as<T>();
-    if (phases) return form_strata<T>(ctx, L, D);
+    if (kind == kPhaseArrays) return form_strata<T>(ctx, L, D);
+    if constexpr (sizeof(T) == 4)
+        if (kind == kPoseArrays) {
+            {
+                Prof pr(ctx, ARAP_K_FACTOR);
+                launch_strata_inverse<float>(ctx->bstd, ctx->ds, L, D, ctx->bstb.m.as<float>(), ctx->stream);
+            }
+            ctx->launches += ctx->bstd.nph;
+            CK(cudaGetLastError());
+            return ARAP_OK;
+        }
     return factor_inverses<T>(ctx, L, D, ctx->Xinv.as<T>(), ctx->L21.as<T>(), ctx->L21T.as<T>(), ctx->Ttop.as<T>());
 }
 
@@ -999,7 +1062,7 @@ int form_solves(arap_ctx *ctx, bool phases) {
 // bFixed assembly, the factorisation plan. No host synchronisation; a failed
 // pivot shows up in the device error word.
 template <typename T>
-int setup_enqueue(arap_ctx *ctx, bool phases) {
+int setup_enqueue(arap_ctx *ctx, int kind) {
     const Symbolic &s = ctx->sym;
     const DevSym &d = ctx->ds;
     cudaStream_t st = ctx->stream;
@@ -1007,7 +1070,7 @@ int setup_enqueue(arap_ctx *ctx, bool phases) {
     // the solves' scheduling counters and flags restart with every set-up: a
     // launch consumes tickets in proportion to its grid, which differs
     // between the precisions
-    if (!phases) {
+    if (kind == kSweepArrays) {
         CK(cudaMemsetAsync(ctx->ticket.p, 0, kTickets * sizeof(unsigned long long), st));
         CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(unsigned) * (size_t)std::max(s.S, 1), st));
         // and the dense top's arrival counters
@@ -1054,7 +1117,7 @@ int setup_enqueue(arap_ctx *ctx, bool phases) {
             rc = factor_numeric<T>(ctx, ctx->Lval.as<T>(), ctx->Upd.as<T>(), ctx->Dinv.as<T>());
             if (rc != ARAP_OK) return rc;
         }
-        rc = form_solves<T>(ctx, phases);
+        rc = form_solves<T>(ctx, kind);
         if (rc != ARAP_OK) return rc;
     }
     CK(cudaGetLastError());
@@ -1069,7 +1132,7 @@ int ensure_solves(arap_ctx *ctx, bool phases) {
     if (phases ? ctx->strata_ready && ctx->strata_formed : ctx->sweeps_ready && ctx->sweeps_formed) return ARAP_OK;
     int rc = phases ? prepare_strata<T>(ctx) : prepare_sweeps(ctx);
     if (rc == ARAP_OK) rc = setup_alloc<T>(ctx, !phases, phases);
-    if (rc == ARAP_OK && ctx->sym.m > 0) rc = form_solves<T>(ctx, phases);
+    if (rc == ARAP_OK && ctx->sym.m > 0) rc = form_solves<T>(ctx, phases ? kPhaseArrays : kSweepArrays);
     if (rc != ARAP_OK) return rc;
     if (!phases && ctx->ytop.p) CK(cudaMemsetAsync(ctx->ytop.p, 0, ctx->ytop.cap, ctx->stream));
     (phases ? ctx->strata_formed : ctx->sweeps_formed) = true;
@@ -1175,12 +1238,12 @@ int run_iterations<double>(arap_ctx *ctx, int iterations) {
         if (phases) {
             {
                 Prof pr(ctx, ARAP_K_SOLVE_FWD);
-                launch_strata_fwd<double>(ctx->std_, ctx->st_m.as<double>(), ctx->sol.as<Vec4<double>>(),
+                launch_strata_fwd<double>(ctx->std_, ctx->stb.m.as<double>(), ctx->sol.as<Vec4<double>>(),
                                           ctx->st_y.as<Vec4<double>>(), ctx->uvec.as<Vec4<double>>(),
                                           ctx->st_ytop.as<Vec4<double>>(), ctx->errw.as<int>(), st);
             }
             Prof pr(ctx, ARAP_K_SOLVE_BWD);
-            launch_strata_bwd<double>(ctx->std_, d, ctx->st_m.as<double>(), ctx->sol.as<Vec4<double>>(),
+            launch_strata_bwd<double>(ctx->std_, d, ctx->stb.m.as<double>(), ctx->sol.as<Vec4<double>>(),
                                       ctx->st_y.as<Vec4<double>>(), ctx->st_ytop.as<Vec4<double>>(),
                                       ctx->pc64.as<Vec4<double>>(), nullptr, 0, ctx->errw.as<int>(), st);
             ctx->launches += strata_launches(ctx->std_, true) + strata_launches(ctx->std_, false) + 1;
@@ -1238,12 +1301,12 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
             if (phases) {
                 {
                     Prof pr(ctx, ARAP_K_SOLVE_FWD);
-                    launch_strata_fwd<float>(ctx->std_, ctx->st_m.as<float>(), ctx->sol.as<Vec4<float>>(),
+                    launch_strata_fwd<float>(ctx->std_, ctx->stb.m.as<float>(), ctx->sol.as<Vec4<float>>(),
                                              ctx->st_y.as<Vec4<float>>(), ctx->uvec.as<Vec4<float>>(),
                                              ctx->st_ytop.as<Vec4<float>>(), ctx->errw.as<int>(), st);
                 }
                 Prof pr(ctx, ARAP_K_SOLVE_BWD);
-                launch_strata_bwd<float>(ctx->std_, d, ctx->st_m.as<float>(), ctx->sol.as<Vec4<float>>(),
+                launch_strata_bwd<float>(ctx->std_, d, ctx->stb.m.as<float>(), ctx->sol.as<Vec4<float>>(),
                                          ctx->st_y.as<Vec4<float>>(), ctx->st_ytop.as<Vec4<float>>(),
                                          ctx->pc64.as<Vec4<double>>(), ctx->pc32.as<Vec4<float>>(), 1,
                                          ctx->errw.as<int>(), st);
@@ -1273,16 +1336,16 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
 // `iterations` local/global iterations of P poses at once (the loop of
 // arap.h:122-129 per pose), the two triangular solves each one persistent
 // launch over all (supernode, pose tile) tasks.
-int run_batch_iterations(arap_ctx *ctx, int P, int iterations) {
+int run_batch_iterations(arap_ctx *ctx, int P, int iterations, bool phases) {
     const Symbolic &s = ctx->sym;
     const DevSym &d = ctx->ds;
-    const DevSym &dv = ctx->use_sb ? ctx->dss : d;  // the batched sweeps' layout (with the solve blocks)
+    const DevSym &dv = !phases && ctx->use_sb ? ctx->dss : d;  // the batched sweeps' layout (with the solve blocks)
     cudaStream_t st = ctx->stream;
     const int m = s.m;
     unsigned long long *tk = ctx->bticket.as<unsigned long long>();
     unsigned *fl = ctx->bflags.as<unsigned>();
     const size_t fhalf = (size_t)std::max(s.S, 1) * ctx->bT;
-    if (d.n_top > 0 && m > 0 && iterations > 0) {
+    if (!phases && d.n_top > 0 && m > 0 && iterations > 0) {
         // T of this factorisation as the tensor-core products' operand tiles
         launch_btop_pack(d, ctx->Ttop.as<float>(), ctx->batile.as<float>(), st);
         ctx->launches += 2;
@@ -1307,6 +1370,18 @@ int run_batch_iterations(arap_ctx *ctx, int P, int iterations) {
                 launch_bresidual(d, P, ctx->w64.as<double>(), ctx->diag64.as<double>(),
                                  ctx->bbfixed.as<Vec4<double>>(), ctx->bb.as<Vec4<float>>(),
                                  ctx->bpc64.as<Vec4<double>>(), ctx->bsol.as<Vec4<float>>(), st);
+            }
+            if (phases) {
+                {
+                    Prof pr(ctx, ARAP_K_SOLVE_FWD);
+                    launch_bstrata_fwd(ctx->bstd, P, ctx->bstb.m.as<float>(), ctx->bsol.as<Vec4<float>>(),
+                                       ctx->bst_y.as<Vec4<float>>(), ctx->buvec.as<Vec4<float>>(), st);
+                }
+                Prof pr(ctx, ARAP_K_SOLVE_BWD);
+                launch_bstrata_bwd(ctx->bstd, d, P, ctx->bstb.m.as<float>(), ctx->bsol.as<Vec4<float>>(),
+                                   ctx->bst_y.as<Vec4<float>>(), ctx->bpc64.as<Vec4<double>>(), st);
+                ctx->launches += 3 * ctx->bstd.nph;
+                continue;
             }
             {
                 Prof pr(ctx, ARAP_K_SOLVE_FWD);
@@ -1615,57 +1690,74 @@ int arap_deform_poses_async(arap_ctx *ctx, int32_t n_poses, const double *target
         if (!ctx->sym_cache) ctx->sym_host = ctx->sym_valid = false;  // analyse again, as SimplicialLDLT::compute
         int rc = prepare_symbolic(ctx);
         if (rc != ARAP_OK) return rc;
-        rc = prepare_sweeps(ctx);
+        const bool phases = use_bstrata(ctx);
+        rc = phases ? prepare_bstrata(ctx) : prepare_sweeps(ctx);
         if (rc != ARAP_OK) return rc;
-        rc = setup_alloc<float>(ctx, true, false);
+        rc = setup_alloc<float>(ctx, !phases, false);
         if (rc != ARAP_OK) return rc;
-        rc = setup_enqueue<float>(ctx, false);
+        rc = setup_enqueue<float>(ctx, phases ? kPoseArrays : kSweepArrays);
         if (rc != ARAP_OK) return rc;
-        ctx->sweeps_formed = true;
+        ctx->sweeps_formed = !phases;
+        ctx->bstrata_formed = phases;
         ctx->strata_formed = false;
         // a failed pivot is reported by arap_wait (the device error word)
         ctx->retarget = false;
         ctx->state_prec = ARAP_PRECISION_MIXED;
         ctx->have_rotations = true;
         ctx->dirty = false;
-    } else {
+    } else if (!use_bstrata(ctx)) {
         const int rc = ensure_solves<float>(ctx, false);
         if (rc != ARAP_OK) return rc;
+    } else if (!(ctx->bstrata_ready && ctx->bstrata_formed)) {
+        int rc = prepare_bstrata(ctx);
+        if (rc == ARAP_OK && ctx->sym.m > 0) rc = form_solves<float>(ctx, kPoseArrays);
+        if (rc != ARAP_OK) return rc;
+        ctx->bstrata_formed = true;
     }
+    const bool phases = use_bstrata(ctx);
+    build_blocks(ctx);  // the refusal below goes by the sweeps' fronts
     const Symbolic &s = ctx->sym;
-    const DevSym &d = ctx->use_sb ? ctx->dss : ctx->ds;  // the batched sweeps' layout (with the solve blocks)
+    // the batched sweeps' layout (with the solve blocks)
+    const DevSym &d = !phases && ctx->use_sb ? ctx->dss : ctx->ds;
     const int V = s.V, m = s.m, P = n_poses, nc = V - m;
     int pt = ctx->pose_tile;
-    if (pt == 0) pt = batch_pose_tile(d.max_ldx, d.max_ld21);
+    if (phases)
+        pt = batch_pose_tile(std::max(s.max_ldx, ctx->sb.max_ldx), std::max(s.max_ld21, ctx->sb.max_ld21));
+    else if (pt == 0) pt = batch_pose_tile(d.max_ldx, d.max_ld21);
     else if (!batch_pose_tile_fits(d.max_ldx, d.max_ld21, pt))
         return fail(ctx, ARAP_ERR_UNSUPPORTED,
                     "pose tile " + std::to_string(pt) + " does not fit this mesh's largest supernode");
     if (pt == 0) return fail(ctx, ARAP_ERR_UNSUPPORTED, "supernode fronts too large for the batched solves");
-    if (ctx->bgen != ctx->gen || ctx->bP != P || ctx->bpt != pt || ctx->bntop != d.n_top) {
-        const size_t smem = batch_solve_smem_bytes(d.max_ldx, d.max_ld21, pt);
-        if (pt != ctx->bpt || smem > ctx->bsmem) {
+    if (phases) pt = 0;  // no sweeps' tiles, counters or dense top
+    const int n_top = phases ? 0 : d.n_top;
+    if (ctx->bgen != ctx->gen || ctx->bP != P || ctx->bpt != pt || ctx->bntop != n_top) {
+        const size_t smem = phases ? 0 : batch_solve_smem_bytes(d.max_ldx, d.max_ld21, pt);
+        if (!phases && (pt != ctx->bpt || smem > ctx->bsmem)) {
             CK(configure_batch_smem(d.max_ldx, d.max_ld21, pt));
             ctx->bsmem = smem;
         }
-        const int T = (P + pt - 1) / pt;
+        const int T = phases ? 0 : (P + pt - 1) / pt;
         const size_t VP = (size_t)V * P, MP = (size_t)std::max(m, 1) * P;
         const size_t nflags = (size_t)2 * std::max(s.S, 1) * T;
-        const std::pair<DevBuf *, size_t> plan[] = {
+        std::vector<std::pair<DevBuf *, size_t>> plan = {
             {&ctx->bpc64, VP * sizeof(Vec4<double>)},
-            {&ctx->bpc32, VP * sizeof(Vec4<float>)},
             {&ctx->bR, VP * 3 * sizeof(Vec4<float>)},
             {&ctx->bbfixed, MP * sizeof(Vec4<double>)},
             {&ctx->bb, MP * sizeof(Vec4<float>)},
             {&ctx->bsol, MP * sizeof(Vec4<float>)},
             {&ctx->buvec, (size_t)std::max<int64_t>(s.uvec_size, 1) * P * sizeof(Vec4<float>)},
             {&ctx->bout, VP * 3 * sizeof(double)},
-            {&ctx->btargets, (size_t)P * nc * 3 * sizeof(double)},
-            {&ctx->bticket, 2 * sizeof(unsigned long long)},
-            {&ctx->bflags, nflags * sizeof(unsigned)},
-            {&ctx->bftop, std::max<size_t>(btop_matrix_floats(d.n_top, P), 1) * sizeof(float)},
-            {&ctx->bytop, std::max<size_t>(btop_matrix_floats(d.n_top, P), 1) * sizeof(float)},
-            {&ctx->bws, std::max<size_t>(btop_workspace_floats(d.n_top, P), 1) * sizeof(float)},
-            {&ctx->batile, std::max<size_t>(btop_atile_floats(d.n_top), 1) * sizeof(float)}};
+            {&ctx->btargets, (size_t)P * nc * 3 * sizeof(double)}};
+        if (phases)
+            plan.push_back({&ctx->bst_y, MP * sizeof(Vec4<float>)});
+        else
+            plan.insert(plan.end(), {{&ctx->bpc32, VP * sizeof(Vec4<float>)},
+                                     {&ctx->bticket, 2 * sizeof(unsigned long long)},
+                                     {&ctx->bflags, nflags * sizeof(unsigned)},
+                                     {&ctx->bftop, std::max<size_t>(btop_matrix_floats(n_top, P), 1) * sizeof(float)},
+                                     {&ctx->bytop, std::max<size_t>(btop_matrix_floats(n_top, P), 1) * sizeof(float)},
+                                     {&ctx->bws, std::max<size_t>(btop_workspace_floats(n_top, P), 1) * sizeof(float)},
+                                     {&ctx->batile, std::max<size_t>(btop_atile_floats(n_top), 1) * sizeof(float)}});
         bool moved = false;
         void *const old_targets = ctx->btargets.p;
         for (const auto &pb : plan) {
@@ -1675,21 +1767,24 @@ int arap_deform_poses_async(arap_ctx *ctx, int32_t n_poses, const double *target
         }
         if (moved) ctx->gen++;  // captured graphs hold the old addresses
         if (ctx->btargets.p != old_targets) ctx->tP = -1;
-        // scheduling counters restart: each launch then consumes a fixed
-        // number of tickets (tasks + CTAs), so the grid is fixed with them
-        CK(cudaMemsetAsync(ctx->bticket.p, 0, 2 * sizeof(unsigned long long), st));
-        CK(cudaMemsetAsync(ctx->bflags.p, 0, nflags * sizeof(unsigned), st));
-        // the products' B tiles: entries past the top's rows and the poses'
-        // columns are never written and must read as zero
-        CK(cudaMemsetAsync(ctx->bftop.p, 0, ctx->bftop.cap, st));
-        CK(cudaMemsetAsync(ctx->bytop.p, 0, ctx->bytop.cap, st));
-        int grid = batch_grid(d, P, pt);
-        if (ctx->solve_cap > 0) grid = std::min(grid, ctx->solve_cap);
+        int grid = 0;
+        if (!phases) {
+            // scheduling counters restart: each launch then consumes a fixed
+            // number of tickets (tasks + CTAs), so the grid is fixed with them
+            CK(cudaMemsetAsync(ctx->bticket.p, 0, 2 * sizeof(unsigned long long), st));
+            CK(cudaMemsetAsync(ctx->bflags.p, 0, nflags * sizeof(unsigned), st));
+            // the products' B tiles: entries past the top's rows and the poses'
+            // columns are never written and must read as zero
+            CK(cudaMemsetAsync(ctx->bftop.p, 0, ctx->bftop.cap, st));
+            CK(cudaMemsetAsync(ctx->bytop.p, 0, ctx->bytop.cap, st));
+            grid = batch_grid(d, P, pt);
+            if (ctx->solve_cap > 0) grid = std::min(grid, ctx->solve_cap);
+        }
         ctx->bpt = pt;
         ctx->bT = T;
         ctx->bgrid = grid;
         ctx->bP = P;
-        ctx->bntop = d.n_top;
+        ctx->bntop = n_top;
         ctx->bgen = ctx->gen;
     }
     if (!targets && ctx->tP < 0) return fail(ctx, ARAP_ERR_INVALID_ARGUMENT, "no targets on the device yet");
@@ -1703,7 +1798,7 @@ int arap_deform_poses_async(arap_ctx *ctx, int32_t n_poses, const double *target
     {
         Prof pr(ctx, ARAP_K_ASSEMBLE);
         launch_bsetup(d, P, ctx->p64.as<Vec4<double>>(), ctx->btargets.as<double>(), ctx->bpc64.as<Vec4<double>>(),
-                      ctx->bpc32.as<Vec4<float>>(), ctx->bR.as<Vec4<float>>(), st);
+                      phases ? nullptr : ctx->bpc32.as<Vec4<float>>(), ctx->bR.as<Vec4<float>>(), st);
         launch_bbfixed(d, P, ctx->w64.as<double>(), ctx->bpc64.as<Vec4<double>>(), ctx->bbfixed.as<Vec4<double>>(),
                        st);
     }
@@ -1719,7 +1814,7 @@ int arap_deform_poses_async(arap_ctx *ctx, int32_t n_poses, const double *target
         const int64_t key[4] = {ctx->gen, P, n + ((int64_t)ctx->refine << 32),
                                 ctx->bpt + ((int64_t)ctx->bgrid << 32)};
         const int rc = graph_or_direct(ctx, ctx->g_biter[k], ctx->g_biter_key[k], key, ctx->g_biter_launches[k],
-                                       [&] { return run_batch_iterations(ctx, P, n); });
+                                       [&] { return run_batch_iterations(ctx, P, n, phases); });
         if (rc != ARAP_OK) return rc;
         left -= n;
     }
@@ -1895,11 +1990,13 @@ int arap_deform_async(arap_ctx *ctx, int32_t iterations, double *out_xyz) {
         h2 = HClock::now();
         const int64_t key[4] = {ctx->gen, fp64 ? 1 : 2, fp64 ? 64 : ctx->factor_bits, phases ? 1 : 0};
         rc = graph_or_direct(ctx, ctx->g_setup, ctx->g_setup_key, key, ctx->g_setup_launches, [&] {
-            return fp64 ? setup_enqueue<double>(ctx, phases) : setup_enqueue<float>(ctx, phases);
+            return fp64 ? setup_enqueue<double>(ctx, phases ? kPhaseArrays : kSweepArrays)
+                        : setup_enqueue<float>(ctx, phases ? kPhaseArrays : kSweepArrays);
         });
         if (rc != ARAP_OK) return rc;
         ctx->strata_formed = phases;
         ctx->sweeps_formed = !phases;
+        ctx->bstrata_formed = false;
         ctx->state_prec = fp64 ? ARAP_PRECISION_FP64 : ARAP_PRECISION_MIXED;
         ctx->have_rotations = true;
         ctx->dirty = false;
@@ -2415,7 +2512,7 @@ int arap_plan_bytes(arap_ctx *ctx, int32_t n_poses, int64_t *bytes) {
         const bool fp64 = ctx->precision == ARAP_PRECISION_FP64 && n_poses == 0;
         const bool phases = use_strata(ctx, fp64);
         if (fp64) planned_sizes<double>(ctx, 0, !phases, phases, plan);
-        else planned_sizes<float>(ctx, n_poses, !phases || n_poses > 0, phases, plan);
+        else planned_sizes<float>(ctx, n_poses, !phases || (n_poses > 0 && !use_bstrata(ctx)), phases, plan);
     }
     for (DevBuf *b : ctx->buffers()) {
         size_t want = b->cap;
@@ -2535,6 +2632,9 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         if (!ctx->model_batched && use_strata(ctx, sz == 8.0)) {  // the groups' matrices once, vectors in and out
             B = ctx->strata.entries * sz + (m + ctx->strata.nb_sum) * 3 * sz * 2;
             FL = ctx->strata.entries * 6;
+        } else if (ctx->model_batched && use_bstrata(ctx)) {  // the groups' matrices once per 64 poses
+            B = ctx->bstrata.entries * sz * std::ceil(P / 64.0) + P * (m + ctx->bstrata.nb_sum) * 3 * sz * 2;
+            FL = P * ctx->bstrata.entries * 6;
         } else if (ctx->model_batched) {  // lower matrices once per pose tile, T once, vectors once per pose
             B = (T * (xlow_lo + l21_lo) + tri) * sz + P * vec;
             FL = P * (xlow_lo + l21_lo + tri) * 6;

@@ -18,6 +18,89 @@ template <typename T> struct Eps;
 template <> struct Eps<float> { static constexpr float v = 1.1920929e-07f; };
 template <> struct Eps<double> { static constexpr double v = 2.220446049250313e-16; };
 
+// Conversions on the integer pipe: an FP64 conversion instruction takes an FP64
+// issue slot (about 64 clocks per warp and scheduler on this GPU).
+// x 2^(1023 - e) in FP32, truncated (e: a biased FP64 exponent; the result must
+// stay below 2^127; below 2^-126 it is 0)
+__device__ __forceinline__ float to_float_scaled(double x, int e) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int fe = (int)((hi >> 20) & 0x7ffu) - e + 127;
+    const unsigned bits = ((unsigned)fe << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    return __uint_as_float((hi & 0x80000000u) | (fe > 0 ? bits : 0u));
+}
+__device__ __forceinline__ double to_double(float x) {  // denormals as 0
+    const unsigned b = __float_as_uint(x), ex = (b >> 23) & 0xffu;
+    const unsigned hi = (b & 0x80000000u) | (ex ? ((ex + 896u) << 20) | ((b >> 3) & 0xfffffu) : 0u);
+    return __hiloint2double((int)hi, ex ? (int)(b << 29) : 0);
+}
+
+// (float)x, rounded to nearest even; outside FP32's normal range the
+// conversion instruction
+__device__ __forceinline__ float to_float_rn(double x) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    b += 0x0fffffffull + ((b >> 29) & 1ull);
+    const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
+    const int fe = (int)((hi >> 20) & 0x7ffu) - 896;
+    if (fe <= 0 || fe >= 255) return (float)x;
+    return __uint_as_float((hi & 0x80000000u) | ((unsigned)fe << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+}
+
+// A double as hi + mid + low in FP32: its leading 24 bits, the next 23 and the
+// last 6. The difference of two is ((hi - hi') + (mid - mid')) + (low - low'):
+// neighbouring positions agree in their exponents, so the first differences
+// are exact and the sum carries the FP32 rounding that the rounded FP64
+// difference does, however short the edge, without an FP64 instruction.
+// Magnitudes below 2^-76 count as zero.
+struct Split {
+    float hi, mid, low;
+    __device__ __forceinline__ explicit Split(double x) {
+        const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+        const unsigned sign = h & 0x80000000u;
+        const int fe = (int)((h >> 20) & 0x7ffu) - 896;
+        const bool in = fe > 50;
+        const unsigned e0 = (unsigned)fe << 23, e1 = e0 - (23u << 23), e2 = e1 - (23u << 23);
+        hi = __uint_as_float(in ? sign | e0 | ((h & 0xfffffu) << 3) | (l >> 29) : 0u);
+        // bits as the fraction of a float of the right exponent, less its leading one
+        const float m = __uint_as_float(e1 | ((l >> 6) & 0x7fffffu)) - __uint_as_float(e1);
+        const float r = __uint_as_float(e2 | ((l << 17) & 0x7e0000u)) - __uint_as_float(e2);
+        mid = in ? __uint_as_float(__float_as_uint(m) | sign) : 0.f;
+        low = in ? __uint_as_float(__float_as_uint(r) | sign) : 0.f;
+    }
+    __device__ __forceinline__ float operator-(const Split &o) const {
+        return ((hi - o.hi) + (mid - o.mid)) + (low - o.low);
+    }
+};
+
+// Cosine and sine of the plane rotation that makes columns of squared norms a
+// and b and inner product g orthogonal; false where they are already, to
+// working precision. t = tan of the angle, the root of t^2 + 2 zeta t - 1 = 0
+// of smaller magnitude, zeta = (b - a) / 2g.
+__device__ __forceinline__ bool jacobi_angle(double a, double b, double g, double &c, double &sn) {
+    if (fabs(g) <= Eps<double>::v * sqrt(a * b)) return false;
+    const double zeta = (b - a) / (2.0 * g), az = fabs(zeta);
+    const double r = az > 1.0 ? az * sqrt(1.0 + 1.0 / (az * az)) : sqrt(1.0 + az * az);
+    const double t = (zeta < 0.0 ? -1.0 : 1.0) / (az + r);
+    c = 1.0 / sqrt(1.0 + t * t);
+    sn = c * t;
+    return true;
+}
+// FP32: t = 2g / (d + sign(d) sqrt(d^2 + 4 g^2)), d = b - a. Any t gives a
+// rotation; only c and sn = c t must be those of one angle to FP32 rounding,
+// so t takes the approximate reciprocal and root, and c a Newton step after
+// its approximate root. The columns are scaled to at most unit norm
+// (rotation_from_cov), so nothing overflows; where d^2 + 4 g^2 underflows the
+// columns are below FP32 resolution of the largest.
+__device__ __forceinline__ bool jacobi_angle(float a, float b, float g, float &c, float &sn) {
+    const float d = b - a, h = 2.f * g, q = fmaf(d, d, h * h);
+    if (g * g <= Eps<float>::v * Eps<float>::v * (a * b) || !(q > 1e-37f)) return false;
+    const float den = fabsf(d) + q * rsqrtf(q);
+    const float t = copysignf(__fdividef(fabsf(h), den), d < 0.f ? -g : g);
+    const float u = fmaf(t, t, 1.f), c0 = rsqrtf(u);
+    c = c0 * fmaf(-0.5f * u * c0, c0, 1.5f);
+    sn = c * t;
+    return true;
+}
+
 // One-sided (Hestenes) Jacobi on a 3x3 matrix (Golub & Van Loan, Sec. 8.6.3;
 // Demmel & Veselic 1992): plane rotations from the right orthogonalise the
 // columns of B = S J1 J2 ..., V accumulates the rotations. On exit the columns
@@ -41,16 +124,9 @@ __device__ __forceinline__ void hestenes3(T B[3][3], T V[3][3]) {
             const T a = B[0][p] * B[0][p] + B[1][p] * B[1][p] + B[2][p] * B[2][p];
             const T b = B[0][q] * B[0][q] + B[1][q] * B[1][q] + B[2][q] * B[2][q];
             const T g = B[0][p] * B[0][q] + B[1][p] * B[1][q] + B[2][p] * B[2][q];
-            if (fabs(g) <= Eps<T>::v * tsqrt(a * b)) continue;  // columns orthogonal to working precision
+            T c, sn;
+            if (!jacobi_angle(a, b, g, c, sn)) continue;  // columns orthogonal to working precision
             rotated = true;
-            // t = tan of the angle that makes the new columns orthogonal, the
-            // root of t^2 + 2 zeta t - 1 = 0 of smaller magnitude
-            const T zeta = (b - a) / ((T)2 * g);
-            const T az = fabs(zeta);
-            const T r = az > (T)1 ? az * tsqrt((T)1 + (T)1 / (az * az)) : tsqrt((T)1 + az * az);
-            const T t = (zeta < (T)0 ? (T)-1 : (T)1) / (az + r);
-            const T c = (T)1 / tsqrt((T)1 + t * t);
-            const T sn = c * t;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const T bp = B[i][p], bq = B[i][q];
@@ -272,22 +348,6 @@ __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int b = 0; b < 3; ++b) Rm[a][b] = (float)R[a][b];
-}
-
-// Conversions on the integer pipe: an FP64 conversion instruction takes an FP64
-// issue slot (about 64 clocks per warp and scheduler on this GPU).
-// x 2^(1023 - e) in FP32, truncated (e: a biased FP64 exponent; the result must
-// stay below 2^127; below 2^-126 it is 0)
-__device__ __forceinline__ float to_float_scaled(double x, int e) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int fe = (int)((hi >> 20) & 0x7ffu) - e + 127;
-    const unsigned bits = ((unsigned)fe << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-    return __uint_as_float((hi & 0x80000000u) | (fe > 0 ? bits : 0u));
-}
-__device__ __forceinline__ double to_double(float x) {  // denormals as 0
-    const unsigned b = __float_as_uint(x), ex = (b >> 23) & 0xffu;
-    const unsigned hi = (b & 0x80000000u) | (ex ? ((ex + 896u) << 20) | ((b >> 3) & 0xfffffu) : 0u);
-    return __hiloint2double((int)hi, ex ? (int)(b << 29) : 0);
 }
 
 // Below this det(H) / tr(H)^3 the rotation is too poorly determined for FP32

@@ -1005,8 +1005,8 @@ k_local_step_fp64(int V, const int32_t *__restrict__ drow, const int32_t *__rest
 }
 
 // Local step of the mixed form: the covariance in FP32 from the FP32 rest
-// edges and the current edges differenced in FP64 (the positions are kept in
-// FP64), then the FP32 rotation fit.
+// edges and the current edges, differences of the FP64 positions rounded to
+// FP32 (dev::Split: no FP64 instruction), then the FP32 rotation fit.
 template <int G>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -1038,13 +1038,14 @@ k_local_step_mixed(int V, const int32_t *__restrict__ drow, const int32_t *__res
     int e1 = 0;
     if (live) {
         const Vec4<double> ci = pc64[i];
+        const dev::Split cx(ci.x), cy(ci.y), cz(ci.z);
         e1 = drow[i + 1];
         for (int e = drow[i] + l; e < e1; e += G) {
             const float wj = w[e];
             const Vec4<float> re = redge[e];
             const Vec4<double> cj = pc64[dcol[e]];
             const float ex = wj * re.x, ey = wj * re.y, ez = wj * re.z;
-            const float fx = (float)(ci.x - cj.x), fy = (float)(ci.y - cj.y), fz = (float)(ci.z - cj.z);
+            const float fx = cx - dev::Split(cj.x), fy = cy - dev::Split(cj.y), fz = cz - dev::Split(cj.z);
             S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
             S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
             S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
@@ -1180,8 +1181,9 @@ k_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ 
     az += d * xi.z;
     const Vec4<float> bi = b[i];
     const Vec4<double> bf = bfixed[i];
-    r[i] = {(float)((bf.x + (double)bi.x) - ax), (float)((bf.y + (double)bi.y) - ay),
-            (float)((bf.z + (double)bi.z) - az), 0.f};
+    // (conversions on the integer pipe)
+    r[i] = {dev::to_float_rn((bf.x + dev::to_double(bi.x)) - ax), dev::to_float_rn((bf.y + dev::to_double(bi.y)) - ay),
+            dev::to_float_rn((bf.z + dev::to_double(bi.z)) - az), 0.f};
 }
 
 // ---------------------------------------------------------------------------
@@ -3341,9 +3343,9 @@ static size_t st_bwd_smem(const StPhase &p, int sb) {
 }
 static size_t st_inv_smem(const StPhase &p, int sb) { return (size_t)(2 * p.front + NB) * p.rc * sb; }
 
-bool strata_fits(const Strata &st, int sb) {
+bool strata_fits(const Strata &st, int sb, bool poses) {
     for (const StPhase &p : st.ph)
-        if (st_inv_smem(p, sb) > 200 * 1024 || (!p.big && (st_fwd_smem(p, sb) > 200 * 1024 || st_bwd_smem(p, sb) > 200 * 1024)))
+        if (st_inv_smem(p, sb) > 200 * 1024 || (!poses && !p.big && (st_fwd_smem(p, sb) > 200 * 1024 || st_bwd_smem(p, sb) > 200 * 1024)))
             return false;
     return true;
 }
@@ -3386,13 +3388,14 @@ template <typename T> struct StKernels {
     }
 };
 
-template <typename T> static cudaError_t configure_strata_t(const Strata &st) {
+template <typename T> static cudaError_t configure_strata_t(const Strata &st, bool poses) {
     cudaError_t e = cudaSuccess;
     auto up = [&](const void *f, size_t bytes) {
         if (e == cudaSuccess) e = raise_smem_limit(f, (int)bytes);
     };
     for (const StPhase &p : st.ph) {
         up((const void *)StKernels<T>::inverse(p), st_inv_smem(p, sizeof(T)));
+        if (poses) continue;  // only the inversion is shared
         if (p.big) {
             up((const void *)k_top_pair_fwd<T>, top_pair_smem(sizeof(T)));
             up((const void *)k_top_pair_bwd<T>, top_pair_smem(sizeof(T)));
@@ -3403,8 +3406,8 @@ template <typename T> static cudaError_t configure_strata_t(const Strata &st) {
     }
     return e;
 }
-cudaError_t configure_strata(const Strata &st, int sb) {
-    return sb == 4 ? configure_strata_t<float>(st) : configure_strata_t<double>(st);
+cudaError_t configure_strata(const Strata &st, int sb, bool poses) {
+    return sb == 4 ? configure_strata_t<float>(st, poses) : configure_strata_t<double>(st, poses);
 }
 
 int strata_launches(const StrataDev &d, bool forward) {

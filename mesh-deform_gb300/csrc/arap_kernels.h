@@ -226,8 +226,8 @@ struct StrataDev {
     const int64_t *top_gidx;
 };
 // whether the phases' kernels can hold their vectors, and their shared-memory limits
-bool strata_fits(const Strata &p, int scalar_bytes);
-cudaError_t configure_strata(const Strata &p, int scalar_bytes);
+bool strata_fits(const Strata &p, int scalar_bytes, bool poses = false);
+cudaError_t configure_strata(const Strata &p, int scalar_bytes, bool poses = false);
 int strata_launches(const StrataDev &d, bool forward);
 // M of every group from the panels and inverted diagonal blocks; M's zeros stay as they are
 template <typename T>
@@ -290,6 +290,14 @@ void launch_bsolve(const DevSym &s, int P, int pt, int grid, const float *X, con
                    Vec4<float> *sol, Vec4<float> *uvec, Vec4<double> *pc64, Vec4<float> *pc32,
                    unsigned long long *ticket, unsigned *flags, int *err, bool forward, cudaStream_t st,
                    const float *atiles, float *bftop, float *bytop, float *bws);
+// the dense phases for P poses (a plan of kStPoses): sol holds the right-hand
+// sides, then the solutions; x is added to pc64
+bool bstrata_fits(const Strata &p);
+cudaError_t configure_bstrata(const Strata &p);
+void launch_bstrata_fwd(const StrataDev &d, int P, const float *M, Vec4<float> *sol, Vec4<float> *y,
+                        Vec4<float> *uvec, cudaStream_t st);
+void launch_bstrata_bwd(const StrataDev &d, const DevSym &s, int P, const float *M, Vec4<float> *sol,
+                        const Vec4<float> *y, Vec4<double> *pc64, cudaStream_t st);
 // the dense top's T and T^T (row-major, FP32) split into TF32 head and rest
 // and laid out as the tensor-core products' A tiles (btop_atile_floats)
 void launch_btop_pack(const DevSym &s, const float *Ttop, float *atiles, cudaStream_t st);

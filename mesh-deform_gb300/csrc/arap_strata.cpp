@@ -22,13 +22,18 @@ namespace {
 constexpr double kPhaseUs = 5.0, kBytesPerUs = 5e6, kFma64PerUs = 0.55e6, kFma32PerUs = 8e6;
 constexpr double kGatherUs[2] = {1.0, 2.5}, kBigTopUs[2] = {0.0, 3.0};  // FP32, FP64
 constexpr double kSweepsPerFactor[2] = {40.0, 20.0};
+// many poses: FP32 FMAs at about half the peak, for 256 poses, and the chain of
+// a CTA's chunks by the largest group (without it 16 poses 300 instead of 276
+// us per iteration, 5 poses of 642 vertices 141 instead of 90)
+constexpr double kPosesUs = 8.0, kPosesGatherUs = 4.0, kPoses = 256.0, kPosesFmaPerUs = 18e6, kPosesColUs = 0.05;
 
 int ld_of(int n) { return (n + 3) & ~3; }
 
 }  // namespace
 
-bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
+bool build_strata(const Symbolic &sym, StrataKind kind, int sms, Strata &out) {
     out = Strata();
+    const bool fp64 = kind == kStFp64, poses = kind == kStPoses;
     const int S = sym.S, m = sym.m;
     if (S == 0 || sym.uvec_size >= std::numeric_limits<int32_t>::max()) return false;
     const std::vector<SnInfo> &sn = sym.sn;
@@ -91,10 +96,15 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
                 ++cnt;
             }
             if (!fits) continue;
-            double c = kPhaseUs + std::max(ent * (fp64 ? 8 : 4) / kBytesPerUs, fp64 ? ent * 3 / kFma64PerUs : 0.0) +
-                       form / (fp64 ? kFma64PerUs : kFma32PerUs) / kSweepsPerFactor[fp64];
-            if (j == K - 1 && cnt == 1 && nmax > kStBigTop) c += kBigTopUs[fp64];
-            else if (i > 0) c += 0.5 * kGatherUs[fp64];  // forward sweeps only
+            double c;
+            if (poses) {
+                c = kPosesUs + kPosesColUs * nmax + ent * 3 * kPoses / kPosesFmaPerUs + (i > 0 ? 0.5 * kPosesGatherUs : 0.0);
+            } else {
+                c = kPhaseUs + std::max(ent * (fp64 ? 8 : 4) / kBytesPerUs, fp64 ? ent * 3 / kFma64PerUs : 0.0) +
+                    form / (fp64 ? kFma64PerUs : kFma32PerUs) / kSweepsPerFactor[fp64];
+                if (j == K - 1 && cnt == 1 && nmax > kStBigTop) c += kBigTopUs[fp64];
+                else if (i > 0) c += 0.5 * kGatherUs[fp64];  // forward sweeps only
+            }
             if (best[i] + c < best[j]) {
                 best[j] = best[i] + c;
                 from[j] = i;
@@ -149,7 +159,7 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
             out.nb_sum += r;
         }
         p.cn = coff - p.c0;
-        p.big = k == np - 1 && groups[k].size() == 1 && p.nmax > kStBigTop;
+        p.big = !poses && k == np - 1 && groups[k].size() == 1 && p.nmax > kStBigTop;
         out.ph.push_back(p);
     }
     if (moff >= (int64_t)1 << 40) return false;
@@ -239,9 +249,10 @@ bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out) {
             p.RW = 4;
             while (p.RW > 1 && rows / (32 / p.G * p.RW) < 4 * 4 * sms) p.RW /= 2;
         }
-        const int per = step(p.RW) * (int)std::min<int64_t>(8, std::max<int64_t>(1, rows / ((int64_t)step(p.RW) * 4 * sms)));
+        int per = step(p.RW) * (int)std::min<int64_t>(8, std::max<int64_t>(1, rows / ((int64_t)step(p.RW) * 4 * sms)));
         p.TC = fp64 ? 32 : 64;
         while (p.TC > (fp64 ? 4 : 8) && (int64_t)p.cn / p.TC * p.ntb < (int64_t)(fp64 ? 4 : 2) * kStThreads * sms) p.TC /= 2;
+        if (poses) per = p.TC = 32;
         auto tile = [&](int32_t g, int first, int count) {
             StTile t{};
             t.m_off = gm_off[g];

@@ -86,8 +86,8 @@ k_strata_gather(int c0, int cn, const int32_t *__restrict__ gcol, const int32_t 
     if (j == 0 && c < cn) b[k] = v;
 }
 
-// Forward product of a stratum: out = M f for the rows of a tile, y = X f
-// into y and u = -W f into the update vectors. A group of G lanes takes RW
+// Forward product of a stratum: M f for the rows of a tile, X's rows into y
+// and -W's into the update vectors. A group of G lanes takes RW
 // rows at a time, each lane 16 bytes of every row per step (consecutive lanes
 // consecutive columns), with f as three arrays in shared memory so that a
 // lane's four (two) columns come with one 16-byte load per component. A CTA's
@@ -191,14 +191,14 @@ k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Ma
 #pragma unroll
             for (int j = 0; j < H; ++j) {
                 const int comp = (base + j) & 3;
-                if (comp < 3) dst[comp] = orow < d.n ? acc[j] : -acc[j];
+                if (comp < 3) dst[comp] = acc[j];
             }
         }
     }
 }
 
 // Backward product of a stratum: x = M^T v for TC columns of a group, v = y on
-// its own rows and -x on the rows below it (solved by the launches before).
+// its own rows and x on the rows below it (solved by the launches before).
 // 16 bytes of a row per thread, TC / E threads per row, the rows dealt to the
 // thread groups in turn; their sums meet in shared memory in a fixed order.
 // Bound as the forward product; 64 columns per tile where that leaves two
@@ -256,10 +256,7 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
         before[j] = ok[j] >= 0 && mode != 0 ? __ldcg(reinterpret_cast<const double *>(pc64 + ok[j]) + comp) : 0.0;
     }
     auto put = [&](int r, int k) {
-        const bool own = d.first + r < d.n;
-        Vec4<T> x = ldcg4((own ? y : (const Vec4<T> *)sol) + k);
-        if (!own) x = {-x.x, -x.y, -x.z, (T)0};
-        v[r] = x;
+        v[r] = ldcg4((d.first + r < d.n ? y : (const Vec4<T> *)sol) + k);
     };
 #pragma unroll
     for (int i = 0; i < kPre; ++i) {
@@ -313,7 +310,7 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
 // group, block column by block column of 32: Y_b = inv(L_bb) F_b with the
 // factorisation's inverted diagonal blocks, then the rows below lose L Y_b;
 // a supernode's rows below its columns go into its parent's front. The Y are
-// X's rows; past the group's root, -F is W. Zeros of M (above the diagonal,
+// X's rows; past the group's root, F is -W. Zeros of M (above the diagonal,
 // and between subtrees that do not meet) are never written: they are cleared
 // once when the matrices are laid out.
 // Bound by FP64 issue (FP64 form) or by the chain of blocks; a phase's columns
@@ -378,7 +375,7 @@ k_strata_inverse(const int32_t *__restrict__ items, const SnInfo *__restrict__ s
         const int nb = n - nc;
         if (ssn[node].root) {
             for (int q = tid; q < nb * RC; q += kStThreads)
-                if (q % RC < w) M[(int64_t)(gj.n + q / RC) * gj.ld + q % RC] = -F[nc * RC + q];
+                if (q % RC < w) M[(int64_t)(gj.n + q / RC) * gj.ld + q % RC] = F[nc * RC + q];
             break;
         }
         const int32_t *ri = relind + dn.relind_off;

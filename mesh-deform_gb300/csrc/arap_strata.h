@@ -4,12 +4,12 @@
 // group's columns holding at most a few hundred to a few thousand columns.
 // Per group the factorisation leaves one dense row-major matrix
 //
-//     M = [ X ]   X = inv(L_gg), n x n lower triangular
-//         [ W ]   W = L(rows below the group, group) X, r x n
+//     M = [  X ]   X = inv(L_gg), n x n lower triangular
+//         [ -W ]   W = L(rows below the group, group) X, r x n
 //
-// so a forward sweep is one product per stratum, y = X f and u = -W f (u goes
-// to the columns above), and a backward sweep one transposed product,
-// x = X^T y - W^T x_below. No task waits for another inside a stratum; strata
+// so a forward sweep is one product per stratum, [y; u] = M f (u goes to the
+// columns above), and a backward sweep one transposed product,
+// x = M^T [y; x_below]. No task waits for another inside a stratum; strata
 // follow each other as launches. A sweep over a tree of 13 levels takes 2 to 5
 // such phases instead of a chain of 13 dependent tasks.
 #pragma once
@@ -76,8 +76,13 @@ struct Strata {
     double entries = 0.0, nb_sum = 0.0;  // matrix entries of one sweep, update rows
 };
 
-// Cuts the tree for solves in FP64 or FP32 on a device with `sms` SMs; false
-// (and out.ok false) when some front does not fit the phases' kernels.
-bool build_strata(const Symbolic &sym, bool fp64, int sms, Strata &out);
+// What the phases solve: one request in FP32 or FP64, or many poses in FP32
+// (a plan that does not depend on how many: a pose's result is the same in
+// any batch).
+enum StrataKind { kStFp32 = 0, kStFp64 = 1, kStPoses = 2 };
+
+// Cuts the tree for a device with `sms` SMs; false (and out.ok false) when
+// some front does not fit the phases' kernels.
+bool build_strata(const Symbolic &sym, StrataKind kind, int sms, Strata &out);
 
 }  // namespace arapgpu

@@ -29,7 +29,8 @@ static void grid(int nx, int ny, int off, std::vector<int32_t> &f) {
         }
 }
 
-static int check(int nx, int ny, int copies, bool fp64, int sms) {
+static int check(int nx, int ny, int copies, StrataKind kind, int sms) {
+    const bool fp64 = kind == kStFp64, poses = kind == kStPoses;
     std::vector<int32_t> faces;
     for (int c = 0; c < copies; ++c) grid(nx, ny, c * nx * ny, faces);
     const int V = copies * nx * ny;
@@ -42,7 +43,7 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
     bool singular;
     REQUIRE(build_symbolic(topo, fixed, s, err, singular));
     Strata p;
-    REQUIRE(build_strata(s, fp64, sms, p));
+    REQUIRE(build_strata(s, kind, sms, p));
     const int m = s.m;
     // the matrix in elimination order, its dense Cholesky factor
     std::mt19937 rng(7);
@@ -107,7 +108,7 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
                     }
                     if (p.sn[node].root) {
                         for (int i = 0; i < x.nrow - x.ncol; ++i)
-                            M[g.m_off + (int64_t)(g.n + i) * g.ld + g.pos + c] = -e[s.rows[x.rows_off + i]];
+                            M[g.m_off + (int64_t)(g.n + i) * g.ld + g.pos + c] = e[s.rows[x.rows_off + i]];
                         break;
                     }
                     node = x.parent;
@@ -149,12 +150,14 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
             }
             continue;
         }
-        REQUIRE(ph.G == 8 || ph.G == 32 || (fp64 && (ph.G == 1 || ph.G == 4)));
+        if (poses) REQUIRE(!ph.big && ph.TC == 32);
+        if (!poses) REQUIRE(ph.G == 8 || ph.G == 32 || (fp64 && (ph.G == 1 || ph.G == 4)));
         if (fp64) REQUIRE(ph.RW == 1);
-        REQUIRE(ph.RW == 1 || ph.RW == 2 || ph.RW == 4);
+        if (!poses) REQUIRE(ph.RW == 1 || ph.RW == 2 || ph.RW == 4);
         for (int t = ph.f0; t < ph.f0 + ph.fn; ++t) {
             const StTile &d = p.tiles[t];
             REQUIRE(d.count > 0 && d.first >= 0 && d.first + d.count <= d.n + d.r && d.ld == ((d.n + 3) & ~3));
+            if (poses) REQUIRE(d.count <= 32);
             REQUIRE(d.n <= ph.nmax && d.n + d.r <= ph.vmax && d.m_off % 4 == 0);
             REQUIRE(d.m_off + (int64_t)(d.n + d.r) * d.ld <= p.m_size);
             for (int c = 0; c < d.n; ++c) REQUIRE(d.base < 0 || p.col[d.col_off + c] == d.base + c);
@@ -167,7 +170,7 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
                     ++wrote[p.col[d.col_off + r]];
                 } else {
                     REQUIRE(d.u_off + r - d.n < s.uvec_size);
-                    uv[d.u_off + r - d.n] = -v;
+                    uv[d.u_off + r - d.n] = v;
                     ++uwrote[d.u_off + r - d.n];
                 }
             }
@@ -202,7 +205,7 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
                 double v = 0;
                 for (int r = d.first; r < d.n + d.r; ++r) {
                     if (r >= d.n) REQUIRE(solved[s.rows[d.row_off + r - d.n]] == 1);
-                    const double w = r < d.n ? y[p.col[d.col_off + r]] : -x[s.rows[d.row_off + r - d.n]];
+                    const double w = r < d.n ? y[p.col[d.col_off + r]] : x[s.rows[d.row_off + r - d.n]];
                     v += M[d.m_off + (int64_t)r * d.ld + c] * w;
                 }
                 x[p.col[d.col_off + c]] = v;
@@ -218,19 +221,19 @@ static int check(int nx, int ny, int copies, bool fp64, int sms) {
         for (int l = 0; l < m; ++l) r -= (l <= k ? A[(size_t)k * m + l] : A[(size_t)l * m + k]) * x[l];
         worst = std::max(worst, std::fabs(r));
     }
-    std::printf("%dx%d x%d fp%d sms %d: m %d, %d phases, residual %.1e\n", nx, ny, copies, fp64 ? 64 : 32, sms, m, np, worst);
+    std::printf("%dx%d x%d kind %d sms %d: m %d, %d phases, residual %.1e\n", nx, ny, copies, (int)kind, sms, m, np, worst);
     // x is O(m) at most here; 1e-16 x condition (about m) x sqrt(m) of rounding
     REQUIRE(worst < 1e-16 * (double)m * 64.0);
     return 0;
 }
 
 int main() {
-    for (int fp64 = 0; fp64 < 2; ++fp64) {
-        if (check(3, 2, 1, fp64, 152)) return 1;     // four unknowns
-        if (check(9, 8, 1, fp64, 152)) return 1;     // one leaf
-        if (check(23, 17, 2, fp64, 152)) return 1;   // two components
-        if (check(60, 33, 1, fp64, 152)) return 1;
-        if (check(47, 41, 1, fp64, 4)) return 1;     // tiles of several row steps
+    for (const StrataKind kind : {kStFp32, kStFp64, kStPoses}) {
+        if (check(3, 2, 1, kind, 152)) return 1;     // four unknowns
+        if (check(9, 8, 1, kind, 152)) return 1;     // one leaf
+        if (check(23, 17, 2, kind, 152)) return 1;   // two components
+        if (check(60, 33, 1, kind, 152)) return 1;
+        if (check(47, 41, 1, kind, 4)) return 1;     // tiles of several row steps
     }
     std::printf("ok\n");
     return 0;
