@@ -588,8 +588,8 @@ void launch_bstrata_bwd(const StrataDev &d, const DevSym &s, int P, const float 
     const unsigned np = (unsigned)((P + kBsPoses - 1) / kBsPoses);
     for (int k = d.nph - 1; k >= 0; --k) {
         const StPhase &p = d.ph[k];
-        k_bstrata<true><<<dim3(p.bn, np), kBsThreads, bs_smem(p), st>>>(P, d.tiles + p.b0, M, d.col, s.rows, y, sol, sol,
-                                                                       nullptr, pc64);
+        k_bstrata<true><<<dim3(p.bn, np), kBsThreads, bs_smem(p), st>>>(P, d.tiles + p.b0, M, d.col, s.rows, y, sol,
+                                                                       k > 0 ? sol : nullptr, nullptr, pc64);
     }
 }
 

@@ -43,7 +43,8 @@ k_bstrata_gather(int c0, int cn, int P, const int32_t *__restrict__ gcol, const 
 // One 32 x 32 tile of a group's product: BWD false, rows [first, first +
 // count) of M f, X's rows into `out` (y) and -W's into uvec; BWD true, columns
 // of M^T v, v = y on the group's rows and x (`below`) on the rows below, into
-// `out` (the solution) and added to the positions. 128 threads as 8 row groups
+// `out` (the solution; null where no stratum below reads it) and added to the
+// positions. 128 threads as 8 row groups
 // x 16 pose groups, each 4 rows x 2 poses (x, y, z of every pose in one
 // 16-byte load); K in chunks of 16 through a ring of four shared-memory
 // buffers filled by cp.async (two left a chunk waiting for its loads: 0.95 us
@@ -159,24 +160,40 @@ k_bstrata(int P, const StTile *__restrict__ tiles, const float *__restrict__ Mal
                 }
         }
     }
+    // two rows at a time: backward, their positions' loads ahead of the stores
 #pragma unroll
-    for (int i = 0; i < RT; ++i) {
-        const int o = row_of(i), r = d.first + o;
-        if (o >= d.count) continue;
-        const bool own_row = BWD || r < d.n;
-        const int k = own_row ? column(r) : d.u_off + (r - d.n);
-        Vec4<float> *dst = (own_row ? out : uvec) + (int64_t)k * P;
+    for (int i0 = 0; i0 < RT; i0 += 2) {
+        int at[2];  // row of `out` (or of uvec, < 0: ~row)
+        Vec4<double> v[2][PT];
 #pragma unroll
-        for (int j = 0; j < PT; ++j) {
-            const int p = p0 + pg + 16 * j;
-            if (p >= P) continue;
-            dst[p] = {acc[i][j][0], acc[i][j][1], acc[i][j][2], 0.f};
-            if (BWD) {
-                Vec4<double> v = pc64[(int64_t)k * P + p];
-                v.x += dev::to_double(acc[i][j][0]);
-                v.y += dev::to_double(acc[i][j][1]);
-                v.z += dev::to_double(acc[i][j][2]);
-                pc64[(int64_t)k * P + p] = v;
+        for (int i = 0; i < 2; ++i) {
+            const int o = row_of(i0 + i), r = d.first + o;
+            const bool in = o < d.count;
+            at[i] = !in ? 0 : BWD || r < d.n ? column(r) : ~(d.u_off + (r - d.n));
+            if (BWD)
+#pragma unroll
+                for (int j = 0; j < PT; ++j) {
+                    const int p = p0 + pg + 16 * j;
+                    if (in && p < P) v[i][j] = pc64[(int64_t)at[i] * P + p];
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (row_of(i0 + i) >= d.count) continue;
+            Vec4<float> *dst = at[i] >= 0 ? out + (int64_t)at[i] * P : uvec + (int64_t)~at[i] * P;
+#pragma unroll
+            for (int j = 0; j < PT; ++j) {
+                const int p = p0 + pg + 16 * j;
+                if (p >= P) continue;
+                const float *x = acc[i0 + i][j];
+                if (!BWD || out) dst[p] = {x[0], x[1], x[2], 0.f};
+                if (BWD) {
+                    Vec4<double> q = v[i][j];
+                    q.x += dev::to_double(x[0]);
+                    q.y += dev::to_double(x[1]);
+                    q.z += dev::to_double(x[2]);
+                    pc64[(int64_t)at[i] * P + p] = q;
+                }
             }
         }
     }
