@@ -235,7 +235,8 @@ int arap_set_warp_rows(arap_ctx *ctx, int32_t rows);
    threads_per_vertex = 1, 2, 4, 8 or 32 lanes of one warp per vertex, which
    split the vertex's adjacency entries and sum by shuffles (32: a warp per
    vertex); block_threads a multiple of 32, at most 256 for ARAP_K_LOCAL and
-   1024 for the others. Default 1 and 256 for all three. Any shape gives the
+   1024 for the others. Default: 1, with blocks of 32 to 256 by the mesh's
+   size, for all three. Any shape gives the
    same result up to the order of sums. The batched kernels of
    arap_deform_poses take one thread per (vertex, pose) and keep their shape.
    mesh-deform_gb300/arap_tune.py measures the best shape per kernel. */

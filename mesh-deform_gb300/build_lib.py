@@ -44,7 +44,7 @@ SOURCES = [
     ("g++", CSRC / "arap_strata.cpp"),
     ("g++", CSRC / "arap_server.cpp"),
 ]
-HEADERS = [CSRC / "arap_kernels.h", CSRC / "arap_strata.h", CSRC / "arap_strata.cuh", CSRC / "arap_bstrata.cuh", CSRC / "arap_btop.cuh",
+HEADERS = [CSRC / "arap_kernels.h", CSRC / "arap_strata.h", CSRC / "arap_strata.cuh", CSRC / "arap_bstrata.cuh", CSRC / "arap_launch.cuh", CSRC / "arap_btop.cuh",
            CSRC / "arap_wsolve.cuh", CSRC / "arap_btop_plan.h", CSRC / "arap_symbolic.h", CSRC / "arap_device.cuh", CSRC / "arap_server.h",
            ROOT / "include" / "arap_gpu.h"]
 

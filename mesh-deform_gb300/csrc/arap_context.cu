@@ -187,7 +187,7 @@ struct arap_ctx {
     DevSym dss;                                  // the single-request sweeps' layout with the blocks
     DevBuf ssn, slevel_sn, sbitems, sbmembers;
     // launch shape of the local step, RHS and residual (arap_set_vertex_launch)
-    VertexLaunch vlaunch[kVertexKernels] = {{1, 256}, {1, 256}, {1, 256}};
+    VertexLaunch vlaunch[kVertexKernels] = {{1, 0}, {1, 0}, {1, 0}};
     size_t dense_inv_smem[2] = {0, 0};  // configured limits (FP32, FP64)
     DevBuf top_col, top_gptr, top_gidx, tdpos, top_items, Ttop, ytop;
     // dense-phase solves (arap_strata.h): the plan of the current analysis and

@@ -4,6 +4,7 @@
 // it replaces. Layouts are described in arap_kernels.h.
 #include "arap_kernels.h"
 #include "arap_device.cuh"
+#include "arap_launch.cuh"
 
 #include <cooperative_groups.h>
 
@@ -50,14 +51,6 @@ __device__ __forceinline__ void wait_flag(const unsigned *p, unsigned target, in
     }
     atomicOr(err, kErrTimeout);
 }
-
-// Programmatic dependent launch: a kernel launched with programmatic stream
-// serialization may start once every CTA of the kernel before it has called
-// pdl_trigger (or exited); pdl_wait then blocks until that kernel has
-// finished and its memory is visible. Without the launch attribute pdl_wait
-// returns at once.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename T> __device__ __forceinline__ Vec4<T> ldcg4(const Vec4<T> *p);
 template <> __device__ __forceinline__ Vec4<float> ldcg4(const Vec4<float> *p) {
@@ -974,6 +967,23 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
 // ---------------------------------------------------------------------------
 // local step: estimateRotations, arap.h:354-384
 
+// One-ring entries e, e + G, ... (N of them, below e1) gathered together:
+// their neighbours' indices first, then everything load(k, entry, neighbour)
+// reads, so that a vertex waits for two round trips per N neighbours instead
+// of two per neighbour. Bound by that latency: an iteration of the 30,000
+// vertex bar, mixed form, 131.6 us one neighbour at a time, 123.6 by twos,
+// 122.1 by fours; of the level-7 sphere (163,842 vertices) 215.4, 204.2, 201.4.
+constexpr int kRing = 4;
+template <int G, int N = kRing, typename F>
+__device__ __forceinline__ void ring_gather(int e, int e1, const int32_t *__restrict__ dcol, F &&load) {
+    int j[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) j[k] = e + k * G < e1 ? dcol[e + k * G] : 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        if (e + k * G < e1) load(k, e + k * G, j[k]);
+}
+
 // FP64 form: covariance from the weighted rest edges w (p_i - p_j), formed
 // once per set-up (they only change with the rest pose), and the rotation fit.
 // Bound by FP64 issue (about 64 clocks per warp instruction and scheduler):
@@ -990,12 +1000,20 @@ k_local_step_fp64(int V, const int32_t *__restrict__ drow, const int32_t *__rest
     const Vec4<double> ci = pc[i];
     double S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     const int e1 = drow[i + 1];
-    for (int e = drow[i]; e < e1; ++e) {
-        const Vec4<double> we = wedge[e], cj = pc[dcol[e]];
-        const double fx = ci.x - cj.x, fy = ci.y - cj.y, fz = ci.z - cj.z;
-        S[0][0] += we.x * fx; S[0][1] += we.x * fy; S[0][2] += we.x * fz;
-        S[1][0] += we.y * fx; S[1][1] += we.y * fy; S[1][2] += we.y * fz;
-        S[2][0] += we.z * fx; S[2][1] += we.z * fy; S[2][2] += we.z * fz;
+    for (int e = drow[i]; e < e1; e += kRing) {
+        Vec4<double> we[kRing], cj[kRing];
+        ring_gather<1>(e, e1, dcol, [&](int k, int ek, int j) {
+            we[k] = wedge[ek];
+            cj[k] = pc[j];
+        });
+#pragma unroll
+        for (int k = 0; k < kRing; ++k) {
+            if (e + k >= e1) break;
+            const double fx = ci.x - cj[k].x, fy = ci.y - cj[k].y, fz = ci.z - cj[k].z;
+            S[0][0] += we[k].x * fx; S[0][1] += we[k].x * fy; S[0][2] += we[k].x * fz;
+            S[1][0] += we[k].y * fx; S[1][1] += we[k].y * fy; S[1][2] += we[k].y * fz;
+            S[2][0] += we[k].z * fx; S[2][1] += we[k].z * fy; S[2][2] += we[k].z * fz;
+        }
     }
     double Rm[3][3];
     dev::rotation_fit_fp64(S, Rm);
@@ -1040,15 +1058,24 @@ k_local_step_mixed(int V, const int32_t *__restrict__ drow, const int32_t *__res
         const Vec4<double> ci = pc64[i];
         const dev::Split cx(ci.x), cy(ci.y), cz(ci.z);
         e1 = drow[i + 1];
-        for (int e = drow[i] + l; e < e1; e += G) {
-            const float wj = w[e];
-            const Vec4<float> re = redge[e];
-            const Vec4<double> cj = pc64[dcol[e]];
-            const float ex = wj * re.x, ey = wj * re.y, ez = wj * re.z;
-            const float fx = cx - dev::Split(cj.x), fy = cy - dev::Split(cj.y), fz = cz - dev::Split(cj.z);
-            S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
-            S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
-            S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
+        for (int e = drow[i] + l; e < e1; e += G * kRing) {
+            float wj[kRing];
+            Vec4<float> re[kRing];
+            Vec4<double> cj[kRing];
+            ring_gather<G>(e, e1, dcol, [&](int k, int ek, int j) {
+                wj[k] = w[ek];
+                re[k] = redge[ek];
+                cj[k] = pc64[j];
+            });
+#pragma unroll
+            for (int k = 0; k < kRing; ++k) {
+                if (e + k * G >= e1) break;
+                const float ex = wj[k] * re[k].x, ey = wj[k] * re[k].y, ez = wj[k] * re[k].z;
+                const float fx = cx - dev::Split(cj[k].x), fy = cy - dev::Split(cj[k].y), fz = cz - dev::Split(cj[k].z);
+                S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
+                S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
+                S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
+            }
         }
     }
     if (G > 1) {
@@ -1083,15 +1110,24 @@ k_rhs_mixed(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__
     if (live) {
         const Vec4<float> r0 = R[3 * (int64_t)i], r1 = R[3 * (int64_t)i + 1], r2 = R[3 * (int64_t)i + 2];
         const int e1 = drow[i + 1];
-        for (int e = drow[i] + l; e < e1; e += G) {
-            const int j = dcol[e];
-            if (j == i) continue;
-            const float h = w[e] * 0.5f;
-            const Vec4<float> d = redge[e];
-            const Vec4<float> q0 = R[3 * (int64_t)j], q1 = R[3 * (int64_t)j + 1], q2 = R[3 * (int64_t)j + 2];
-            ax += ((r0.x + q0.x) * d.x + (r0.y + q0.y) * d.y + (r0.z + q0.z) * d.z) * h;
-            ay += ((r1.x + q1.x) * d.x + (r1.y + q1.y) * d.y + (r1.z + q1.z) * d.z) * h;
-            az += ((r2.x + q2.x) * d.x + (r2.y + q2.y) * d.y + (r2.z + q2.z) * d.z) * h;
+        constexpr int kR = 2;  // 48 bytes of rotation each: two neighbours in flight
+        for (int e = drow[i] + l; e < e1; e += G * kR) {
+            float h[kR];
+            Vec4<float> d[kR], q[kR][3];
+            ring_gather<G, kR>(e, e1, dcol, [&](int k, int ek, int j) {
+                h[k] = j == i ? 0.f : w[ek] * 0.5f;
+                d[k] = redge[ek];
+                q[k][0] = R[3 * (int64_t)j];
+                q[k][1] = R[3 * (int64_t)j + 1];
+                q[k][2] = R[3 * (int64_t)j + 2];
+            });
+#pragma unroll
+            for (int k = 0; k < kR; ++k) {
+                if (e + k * G >= e1) break;
+                ax += ((r0.x + q[k][0].x) * d[k].x + (r0.y + q[k][0].y) * d[k].y + (r0.z + q[k][0].z) * d[k].z) * h[k];
+                ay += ((r1.x + q[k][1].x) * d[k].x + (r1.y + q[k][1].y) * d[k].y + (r1.z + q[k][1].z) * d[k].z) * h[k];
+                az += ((r2.x + q[k][2].x) * d[k].x + (r2.y + q[k][2].y) * d[k].y + (r2.z + q[k][2].z) * d[k].z) * h[k];
+            }
         }
     }
     if (G > 1) {
@@ -1121,13 +1157,25 @@ k_rhs_fp64(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ 
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     if (live) {
         const int e1 = drow[i + 1];
-        for (int e = drow[i] + l; e < e1; e += G) {
-            const int j = dcol[e];
-            const Vec4<double> we = wedge[e];
-            const Vec4<double> q0 = R[3 * (int64_t)j], q1 = R[3 * (int64_t)j + 1], q2 = R[3 * (int64_t)j + 2];
-            acc[0] += q0.x * we.x; acc[0] += q0.y * we.y; acc[0] += q0.z * we.z;
-            acc[1] += q1.x * we.x; acc[1] += q1.y * we.y; acc[1] += q1.z * we.z;
-            acc[2] += q2.x * we.x; acc[2] += q2.y * we.y; acc[2] += q2.z * we.z;
+        constexpr int kR = 2;  // 96 bytes of rotation each: two neighbours in flight
+        for (int e = drow[i] + l; e < e1; e += G * kR) {
+            Vec4<double> we[kR], q[kR][3];
+            ring_gather<G, kR>(e, e1, dcol, [&](int k, int ek, int j) {
+                we[k] = wedge[ek];
+                q[k][0] = R[3 * (int64_t)j];
+                q[k][1] = R[3 * (int64_t)j + 1];
+                q[k][2] = R[3 * (int64_t)j + 2];
+            });
+#pragma unroll
+            for (int k = 0; k < kR; ++k) {
+                if (e + k * G >= e1) break;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    acc[c] += q[k][c].x * we[k].x;
+                    acc[c] += q[k][c].y * we[k].y;
+                    acc[c] += q[k][c].z * we[k].z;
+                }
+            }
         }
     }
     const bool dup = st_reduce<4, G>(acc, lane);
@@ -1158,14 +1206,23 @@ k_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ 
     double ax = 0.0, ay = 0.0, az = 0.0;
     if (live) {
         const int e1 = drow[i + 1];
-        for (int e = drow[i] + l; e < e1; e += G) {
-            const int j = dcol[e];
-            if (j == i || j >= m) continue;
-            const double wj = w64[e];
-            const Vec4<double> xj = x[j];
-            ax -= wj * xj.x;
-            ay -= wj * xj.y;
-            az -= wj * xj.z;
+        for (int e = drow[i] + l; e < e1; e += G * kRing) {
+            double wj[kRing];
+            Vec4<double> xj[kRing];
+            bool in[kRing];
+            ring_gather<G>(e, e1, dcol, [&](int k, int ek, int j) {
+                in[k] = j != i && j < m;
+                wj[k] = w64[ek];
+                xj[k] = x[j];  // x holds every vertex
+            });
+#pragma unroll
+            for (int k = 0; k < kRing; ++k) {
+                if (e + k * G >= e1) break;
+                if (!in[k]) continue;
+                ax -= wj[k] * xj[k].x;
+                ay -= wj[k] * xj[k].y;
+                az -= wj[k] * xj[k].z;
+            }
         }
     }
     if (G > 1) {
@@ -2953,32 +3010,30 @@ void launch_rest_edges(const DevSym &s, const Vec4<double> *p64, Vec4<float> *re
     k_rest_edges<<<blocks_for(s.V, 256), 256, 0, st>>>(s.V, s.drow, s.dcol, p64, redge);
 }
 
-// A launch with programmatic stream serialization when `overlap` is set: the
-// kernel may then start while the kernel before it in the stream still runs
-// (see pdl_wait); otherwise an ordinary launch.
-template <typename... KArgs, typename... Args>
-static void launch_pdl(void (*kern)(KArgs...), bool overlap, int grid, int block, size_t smem, cudaStream_t st,
-                       Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = overlap ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kern, args...);
+// threads per block of the FP64 per-vertex kernels: one warp where that still
+// leaves schedulers empty, else two
+static int fp64_block(int64_t threads) { return threads < 32 * 4 * 152 ? 32 : 64; }
+
+// Threads per block of the mixed per-vertex kernels where the caller chose
+// none: 256, halved down to one warp while the blocks are fewer than the
+// device's schedulers, so that a small mesh's warps do not share one. The
+// 8,000-vertex sheet's iteration takes 57.5 us with blocks of 256 and 52.6 so;
+// a 900-vertex sheet's 38.6 and 31.1. From 155,648 vertices on it is 256.
+static int vertex_block(const VertexLaunch &vl, int64_t vertices) {
+    if (vl.block > 0) return vl.block;
+    const int64_t n = vertices * vl.tpv;
+    int block = 256;
+    while (block > 32 && n < (int64_t)block * 4 * 152) block /= 2;
+    return block;
 }
 
 void launch_local_step_mixed(const DevSym &s, const float *w32, const Vec4<float> *redge, const Vec4<double> *pc64,
                              Vec4<float> *R, const double *w64, const Vec4<double> *p64, cudaStream_t st) {
     if (s.V == 0) return;
     const VertexLaunch vl = s.vlaunch[kVertexLocal];
-    const int grid = (int)(((int64_t)s.V * vl.tpv + vl.block - 1) / vl.block);
+    const int block = vertex_block(vl, s.V), grid = blocks_for((int64_t)s.V * vl.tpv, block);
 #define ARAP_LOCAL(G)                                                                                  \
-    launch_pdl(k_local_step_mixed<G>, s.overlap != 0, grid, vl.block, 0, st, s.V, (const int32_t *)s.drow,  \
+    launch_pdl(k_local_step_mixed<G>, s.overlap != 0, grid, block, 0, st, s.V, (const int32_t *)s.drow,  \
                (const int32_t *)s.dcol, w32, redge, pc64, R, w64, p64)
     switch (vl.tpv) {
     case 2: ARAP_LOCAL(2); break;
@@ -2994,9 +3049,9 @@ void launch_rhs_mixed(const DevSym &s, const float *w32, const Vec4<float> *redg
                       Vec4<float> *b, cudaStream_t st) {
     if (s.m == 0) return;
     const VertexLaunch vl = s.vlaunch[kVertexRhs];
-    const int grid = (int)(((int64_t)s.m * vl.tpv + vl.block - 1) / vl.block);
+    const int block = vertex_block(vl, s.m), grid = blocks_for((int64_t)s.m * vl.tpv, block);
 #define ARAP_RHS(G)                                                                                    \
-    launch_pdl(k_rhs_mixed<G>, s.overlap != 0, grid, vl.block, 0, st, s.m, (const int32_t *)s.drow,         \
+    launch_pdl(k_rhs_mixed<G>, s.overlap != 0, grid, block, 0, st, s.m, (const int32_t *)s.drow,         \
                (const int32_t *)s.dcol, w32, redge, (const Vec4<float> *)R, b)
     switch (vl.tpv) {
     case 2: ARAP_RHS(2); break;
@@ -3054,10 +3109,6 @@ void launch_weighted_edges(const DevSym &s, const double *w64, const Vec4<double
     k_weighted_edges<<<blocks_for(s.V, 64), 64, 0, st>>>(s.V, s.drow, s.dcol, w64, p64, wedge, wsum);
 }
 
-// threads per block of the FP64 per-vertex kernels: one warp where that still
-// leaves schedulers empty, else two
-static int fp64_block(int64_t threads) { return threads < 32 * 4 * 152 ? 32 : 64; }
-
 void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *pc, Vec4<double> *R,
                             cudaStream_t st) {
     if (s.V == 0) return;
@@ -3089,9 +3140,9 @@ void launch_residual(const DevSym &s, const double *w64, const double *diag64, c
                      const Vec4<float> *b, const Vec4<double> *x64, Vec4<float> *r, cudaStream_t st) {
     if (s.m == 0) return;
     const VertexLaunch vl = s.vlaunch[kVertexResidual];
-    const int grid = (int)(((int64_t)s.m * vl.tpv + vl.block - 1) / vl.block);
+    const int block = vertex_block(vl, s.m), grid = blocks_for((int64_t)s.m * vl.tpv, block);
 #define ARAP_RES(G)                                                                                    \
-    launch_pdl(k_residual<G>, s.overlap != 0, grid, vl.block, 0, st, s.m, (const int32_t *)s.drow,          \
+    launch_pdl(k_residual<G>, s.overlap != 0, grid, block, 0, st, s.m, (const int32_t *)s.drow,          \
                (const int32_t *)s.dcol, w64, diag64, bfixed, b, x64, r)
     switch (vl.tpv) {
     case 2: ARAP_RES(2); break;

@@ -49,7 +49,7 @@ constexpr int kLevelTicket0 = 8;
 
 // launch shape of a per-vertex kernel of the single-request iterations
 // (arap_set_vertex_launch): tpv lanes of one warp per vertex (1, 2, 4, 8 or
-// 32), block threads a multiple of 32 (and of tpv) up to 1024
+// 32), block threads a multiple of 32 (and of tpv) up to 1024; 0: by the size
 struct VertexLaunch {
     int tpv, block;
 };

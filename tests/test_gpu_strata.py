@@ -58,8 +58,8 @@ def test_phases_match_sweeps_and_oracle(gpu, name, precision, tol, otol):
 
 
 def test_poses_and_deforms_in_turn(gpu):
-    """A pose batch needs the sweeps' arrays, a deform the phases': each is
-    formed from the resident factor when its call comes, and both give what a
+    """A pose batch and a deform have plans of their own, whose arrays are each
+    formed from the resident factor when its call comes; both give what a
     context that ran nothing else gives."""
     w = W.cfg_pose_batch(level=4, n_poses=5, iterations=4)
     with make(gpu, w, "mixed") as ctx:
@@ -93,3 +93,16 @@ def test_several_large_roots(gpu):
     for w, x in zip(ws, out):
         ok, ref = O.run_deform(w.positions, w.faces, w.cidx, w.ctargets, 3)
         assert ok and W.bbox_rel_error(x, ref, w.positions) <= 1e-10
+
+
+@pytest.mark.parametrize("level", [0, 3, 5, 6])
+def test_vertex_blocks_by_size(gpu, level):
+    """Per-vertex kernels' blocks chosen by the mesh's size (12, 642, 10,242 and
+    40,962 vertices: blocks of 32 and 128) give the bits of blocks of 256."""
+    w = W.cfg_noisy_sphere(level=level, iterations=3) if level else W.cfg_icosphere_l4(level=0, iterations=3)
+    with make(gpu, w, "mixed") as ctx:
+        a = ctx.deform(w.iterations)
+    with make(gpu, w, "mixed") as ctx:
+        for k in ("local", "rhs", "residual"):
+            ctx.set_vertex_launch(k, 1, 256)
+        np.testing.assert_array_equal(ctx.deform(w.iterations), a)
