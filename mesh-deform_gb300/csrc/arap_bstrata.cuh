@@ -18,14 +18,16 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
 // the poses.
 __global__ void __launch_bounds__(256)
 k_bstrata_gather(int c0, int cn, int P, const int32_t *__restrict__ gcol, const int32_t *__restrict__ gptr,
-                 const int32_t *__restrict__ gidx, const Vec4<float> *__restrict__ uvec, Vec4<float> *__restrict__ b) {
+                 const int32_t *__restrict__ gidx, const Vec4<float> *uvec, Vec4<float> *b) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (t >= (int64_t)cn * P) return;
     const int c = (int)(t / P), p = (int)(t % P);
     const int q0 = gptr[c0 + c], q1 = gptr[c0 + c + 1];
     if (q0 == q1) return;
     Vec4<float> *dst = b + (int64_t)gcol[c0 + c] * P + p;
-    Vec4<float> v = *dst;
+    Vec4<float> v = ldcg4(dst);
     const Vec4<float> zero{0.f, 0.f, 0.f, 0.f};
     for (int q = q0; q < q1; ++q) {
         const int4 id = __ldg(reinterpret_cast<const int4 *>(gidx) + q);
@@ -80,6 +82,8 @@ k_bstrata(int P, const StTile *__restrict__ tiles, const float *__restrict__ Mal
         const int r = BWD ? d.first + k : k;
         idx[k] = r < d.n ? column(r) : ~rows[d.row_off + r - d.n];
     }
+    pdl_wait();  // the vectors of the kernels before (an overlapped launch)
+    pdl_trigger();
     __syncthreads();
     const int nk = (K + KC - 1) / KC;
     auto issue = [&](int c) {

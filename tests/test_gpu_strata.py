@@ -80,6 +80,19 @@ def test_poses_and_deforms_in_turn(gpu):
         np.testing.assert_array_equal(ctx.deform(w.iterations), lone2)
 
 
+@pytest.mark.parametrize("n_poses", [1, 7, 33])
+def test_pose_phases_overlap(gpu, n_poses):
+    """Phases whose launches overlap give the bits of launches that do not (a
+    CTA cap turns the overlap off)."""
+    w = W.cfg_pose_batch(level=4, n_poses=n_poses, iterations=4)
+    outs = []
+    for cap in (0, 64):
+        with make(gpu, w, "mixed") as ctx:
+            ctx.set_solve_ctas(cap)
+            outs.append(ctx.deform_poses(w.poses, w.iterations))
+    np.testing.assert_array_equal(outs[1], outs[0])
+
+
 def test_several_large_roots(gpu):
     """Disjoint meshes: the last phase holds one group per mesh."""
     from oracle import oracle as O
