@@ -514,6 +514,27 @@ __device__ __forceinline__ bool pivot_ok(double a) {
     return hi > 0 && hi < 0x7ff00000 ? true : a > 0.0;
 }
 
+// 1/a for the pivot chain: an FP32 seed r and one third-order step,
+// r (1 + e + e^2) with e = 1 - a r: three dependent FP64 instructions.
+template <typename TF> __device__ __forceinline__ TF pivot_rcp(TF a);
+template <> __device__ __forceinline__ float pivot_rcp(float a) { return 1.f / a; }
+template <> __device__ __forceinline__ double pivot_rcp(double a) {
+    const int ex = __double2hiint(a) >> 20;
+    if (!(ex > 924 && ex < 1122)) return 1.0 / a;
+    const double r = dev::to_double(__frcp_rn(dev::to_float_scaled(a, 1023)));
+    const double e = fma(-a, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// named barriers (1..15) of one CTA: `threads` arrivals complete a turn, and
+// only bar_sync waits for it
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 constexpr int kFdtThreads = 128;
 
 // Diagonal block jb of a front: its Cholesky factor and that factor's inverse
@@ -521,12 +542,22 @@ constexpr int kFdtThreads = 128;
 // groups' inverses). Bound by the chain of 32 pivots: an FP64 instruction
 // holds a scheduler's FP64 pipe for about 64 clocks, so a chain runs at that
 // pace and work on the same scheduler adds to it.
-// Lane i holds row i in registers, warp wp the columns c = wp mod 4. Step k:
-// the owner of column k + 1 first updates that column by column k, takes its
-// pivot and publishes it; then all warps update their other columns by column
-// k: one barrier per step, the updates of three warps beside the pivot chain
-// of the fourth (before: three barriers per step with the block in shared
-// memory, and two barriers per row of the inverse: 44 us per launch).
+// The block is eliminated without square roots (L = U sqrt(D)^-1 in the end):
+// column k of U is u, and column j loses u u_j / d_k. Warp 0 does nothing but
+// the chain: with lane i at row i, it takes column k + 1 from smem, subtracts
+// (u u_{k+1}) r, r = 1/d_k, and has the next pivot: four dependent FP64
+// instructions per pivot, u u_{k+1} beside the reciprocal's seed. Warps 1 to 3
+// hold columns 2.. in registers (column 1 + wp + 3 q), subtract column k from
+// them and hand column k + 2 over before the others. 32.1 -> 21.3 us a launch
+// on the bar (before: the chain went through a square root and the owner's
+// other columns, seven instructions and up to seven more per pivot).
+// Barriers: P(k), column k and its r are there (warp 0 arrives, warps 1..3
+// wait), k = 0..w-2; N(c), column c has lost columns 0..c-2 (its owner
+// arrives, warp 0 waits), c = 2..w-1. Each has two numbers, taken in turn:
+// warp 0 arrives at P(k + 1) before P(k) need be complete, but after N(k + 1),
+// whose owner has passed P(k - 1); the owner of c + 1 arrives at N(c + 1)
+// before warp 0 need have taken N(c), but that of c + 2 only after P(c), at
+// which warp 0 arrives after N(c).
 // The inverse by halves: 8 x 8 blocks by substitution (a lane per column),
 // then X21 = -X22 (L21 X11) for blocks of 8 and of 16, products that use all
 // four schedulers.
@@ -534,80 +565,103 @@ template <typename TF>
 __global__ void __launch_bounds__(kFdtThreads)
 k_fdt(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF *__restrict__ Lval,
       TF *__restrict__ Dinv, int *err) {
-    __shared__ TF col[2][NB];      // column k and k + 1 of L
+    __shared__ TF U[NB][NB + 1];   // column k of U in row k
     __shared__ TF Ls[NB][NB + 1];  // the factored block, [r][c]
     __shared__ TF X[NB][NB + 1];   // its inverse, [r][c]
     __shared__ TF Ts[16][17];
-    __shared__ TF rinv[NB];        // 1 / L(r, r), 0 past the block
+    __shared__ TF piv[NB], rcp[NB];  // d_k, 1 / d_k
+    __shared__ TF rinv[NB];          // 1 / L(r, r), 0 past the block
     const SnInfo d = sn[items[blockIdx.x].sn];
     const int n = d.nrow, nc = d.ncol;
     const int j0 = jb * NB, w = min(NB, nc - j0);
     TF *P = Lval + d.panel_off + (int64_t)j0 * n + j0;
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    if (tid < NB) rinv[tid] = (TF)0;
     pdl_wait();
     pdl_trigger();
-    TF a[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int c = 4 * q + wp;
-        a[q] = (c < w && lane >= c && lane < w) ? P[(int64_t)c * n + lane] : (TF)0;
-    }
-    for (int q = tid; q < NB * NB; q += kFdtThreads) X[q / NB][q % NB] = (TF)0;
-    bool bad = false;
-    auto pivot = [&](int k, TF &ak) {
-        TF p = __shfl_sync(0xffffffffu, ak, k);
-        if (!pivot_ok(p)) {
-            bad = true;
-            p = (TF)1;
+    if (wp == 0) {
+        TF u = lane < w ? P[lane] : (TF)0;
+        const TF first = (lane >= 1 && lane < w) ? P[n + lane] : (TF)0;
+        bool bad = false;
+        for (int k = 0; k < w; ++k) {
+            TF p = __shfl_sync(0xffffffffu, u, k);
+            const TF un = __shfl_sync(0xffffffffu, u, (k + 1) & 31);
+            if (!pivot_ok(p)) {
+                bad = true;
+                p = (TF)1;
+                if (lane == k) u = (TF)1;
+            }
+            U[k][lane] = u;
+            const TF q = u * un;
+            const TF r = pivot_rcp(p);
+            if (lane == 0) {
+                piv[k] = p;
+                rcp[k] = r;
+            }
+            if (k + 1 == w) break;
+            __syncwarp();
+            bar_arrive(1 + (k & 1), 128);  // P(k)
+            TF a = first;
+            if (k > 0) {
+                bar_sync(3 + ((k + 1) & 1), 64);  // N(k + 1)
+                a = U[k + 1][lane];
+            }
+            a -= q * r;
+            u = lane > k ? a : (TF)0;
         }
-        const TF r = pivot_rsqrt(p);
-        TF l = (lane == k ? p : ak) * r;
-        if (lane < k) l = (TF)0;
-        ak = l;
-        col[k & 1][lane] = l;
-        if (lane == k) rinv[k] = r;
-    };
-    __syncthreads();  // rinv is cleared
-    if (wp == 0) pivot(0, a[0]);
+        if (bad && lane == 0) atomicOr(err, kErrNotSpd);
+    } else {
+        TF a[10];
+#pragma unroll
+        for (int q = 0; q < 10; ++q) {
+            const int c = 1 + wp + 3 * q;
+            a[q] = (c < w && lane >= c && lane < w) ? P[(int64_t)c * n + lane] : (TF)0;
+        }
+        for (int q = tid - 32; q < NB * NB; q += kFdtThreads - 32) X[q / NB][q % NB] = (TF)0;
+#pragma unroll
+        for (int k = 0; k < NB - 1; ++k) {
+            if (k + 1 >= w) break;
+            bar_sync(1 + (k & 1), 128);  // P(k)
+            if (k + 2 >= w) break;
+            const TF u = U[k][lane], v = u * rcp[k];
+            if (wp - 1 == k % 3) {
+                a[k / 3] -= u * __shfl_sync(0xffffffffu, v, k + 2);
+                U[k + 2][lane] = a[k / 3];
+                __syncwarp();
+                bar_arrive(3 + (k & 1), 64);  // N(k + 2)
+            }
+#pragma unroll
+            for (int q = 0; q < 10; ++q) {
+                const int c = 1 + wp + 3 * q;
+                if (4 + 3 * q > k + 2 && c > k + 2 && c < w) a[q] -= u * __shfl_sync(0xffffffffu, v, c);
+            }
+        }
+    }
     __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NB - 1; ++k) {
-        if (k + 1 >= w) break;
-        const TF *ck = col[k & 1];
-        const TF li = ck[lane];
-        if (wp == ((k + 1) & 3)) {
-            TF &an = a[(k + 1) >> 2];
-            an -= li * ck[k + 1];
-            pivot(k + 1, an);
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int c = 4 * q + wp;
-            if (4 * q + 3 > k + 1 && c > k + 1 && c < w) a[q] -= li * ck[c];
-        }
-        __syncthreads();
-    }
-    if (bad && lane == 0) atomicOr(err, kErrNotSpd);
+    if (tid < NB) rinv[tid] = tid < w ? pivot_rsqrt(piv[tid]) : (TF)0;
+    __syncthreads();
     // the factored block back into the panel and, for the inverse, into shared memory
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int c = 4 * q + wp;
-        const bool in = c < w && lane >= c && lane < w;
-        Ls[lane][c] = in ? a[q] : (TF)0;
-        if (in) P[(int64_t)c * n + lane] = a[q];
+        TF l = (TF)0;
+        if (c < w && lane >= c && lane < w) {
+            l = U[c][lane] * rinv[c];
+            P[(int64_t)c * n + lane] = l;
+        }
+        Ls[lane][c] = l;
     }
     __syncthreads();
     if (wp == 0) {
         const int b = lane & ~7, o = lane & 7;
         TF x[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            TF s = i == o ? (TF)1 : (TF)0;
+        for (int i = 0; i < 8; ++i) x[i] = i == o ? (TF)1 : (TF)0;
 #pragma unroll
-            for (int k = 0; k < i; ++k) s -= Ls[b + i][b + k] * x[k];
-            x[i] = s * rinv[b + i];
+        for (int i = 0; i < 8; ++i) {
+            x[i] *= rinv[b + i];
             X[b + i][lane] = x[i];
+#pragma unroll
+            for (int k = i + 1; k < 8; ++k) x[k] -= Ls[b + k][b + i] * x[i];
         }
     }
     __syncthreads();
