@@ -442,7 +442,7 @@ __device__ __forceinline__ bool vertex_pose(int n, int P, int pb, int &i, int &p
 // estimateRotations per pose (arap.h:354-384): FP32 covariance from the FP32
 // rest edges and the pose's current edges, differences of the FP64 positions
 // rounded to FP32 (dev::Split: no FP64 instruction).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 k_blocal(int V, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
          const float *__restrict__ w, const Vec4<float> *__restrict__ redge, const Vec4<double> *__restrict__ pc64,
          Vec4<float> *__restrict__ R, const double *__restrict__ w64, const Vec4<double> *__restrict__ p64) {
@@ -452,19 +452,39 @@ k_blocal(int V, int P, int pb, const int32_t *__restrict__ drow, const int32_t *
     const Vec4<double> ci = pc64[t];
     const dev::Split cx(ci.x), cy(ci.y), cz(ci.z);
     float S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int e = drow[i]; e < drow[i + 1]; ++e) {
-        const float wj = w[e];
-        const Vec4<float> re = redge[e];
-        const Vec4<double> cj = pc64[(int64_t)dcol[e] * P + p];
-        const float ex = wj * re.x, ey = wj * re.y, ez = wj * re.z;
-        const float fx = cx - dev::Split(cj.x), fy = cy - dev::Split(cj.y), fz = cz - dev::Split(cj.z);
-        S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
-        S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
-        S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
+    const int e1 = drow[i + 1];
+    constexpr int kR = 2;  // neighbours in flight
+    for (int e = drow[i]; e < e1; e += kR) {
+        Vec4<double> cj[kR];
+#pragma unroll
+        for (int k = 0; k < kR; ++k)
+            if (e + k < e1) cj[k] = pc64[(int64_t)dcol[e + k] * P + p];
+#pragma unroll
+        for (int k = 0; k < kR; ++k) {
+            if (e + k >= e1) break;
+            const float wj = w[e + k];
+            const Vec4<float> re = redge[e + k];
+            const float ex = wj * re.x, ey = wj * re.y, ez = wj * re.z;
+            const float fx = cx - dev::Split(cj[k].x), fy = cy - dev::Split(cj[k].y), fz = cz - dev::Split(cj[k].z);
+            S[0][0] += ex * fx; S[0][1] += ex * fy; S[0][2] += ex * fz;
+            S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
+            S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
+        }
     }
-    float Rm[3][3], spread;
-    dev::rotation_from_cov<float>(S, Rm, &spread);
-    if (!(spread >= dev::kPolarFallback)) dev::rotation_fp64<false>(i, drow[i], drow[i + 1], dcol, w64, p64, pc64, P, p, Rm);
+    float Rm[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const Vec4<float> r = R[3 * t + a];
+        Rm[a][0] = r.x;
+        Rm[a][1] = r.y;
+        Rm[a][2] = r.z;
+    }
+    if (!dev::rotation_warm(S, Rm)) {
+        float spread;
+        dev::rotation_from_cov<float>(S, Rm, &spread);
+        if (!(spread >= dev::kPolarFallback))
+            dev::rotation_fp64(i, drow[i], e1, dcol, w64, p64, pc64, P, p, Rm);
+    }
     R[3 * t + 0] = {Rm[0][0], Rm[0][1], Rm[0][2], 0.f};
     R[3 * t + 1] = {Rm[1][0], Rm[1][1], Rm[1][2], 0.f};
     R[3 * t + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], 0.f};

@@ -306,14 +306,206 @@ __device__ __forceinline__ void polar_newton(const T S[3][3], T R[3][3], int ns_
     }
 }
 
+// The rotation of rotation_from_cov by Newton's method in FP32 from a nearby
+// one, the vertex's rotation of the iteration before (the identity at first),
+// in place. The steps are polar_newton's; about 130 FP32 instructions each,
+// one to three in most iterations, against some 1,500 of the Jacobi fit
+// (256 poses of 10,242 vertices: local step 185 -> 154 us). The
+// step after which the last one's remainder is below FP32 resolution
+// orthonormalises R to first order and ends. A point with g = 0 and a positive
+// definite H is the maximum (tr(R S) has no other local maximum on the proper
+// rotations). False, and R undefined, where five steps do not end, or H is not
+// safely positive definite: det(H) / tr(H)^3 above kWarmDet bounds
+// (sigma_2 + sigma_3) / sigma_1 from below by kPolarFallback (with
+// x = (sigma_2 +- sigma_3) / sigma_1 it is at most x (1 + x/2)^2 / (2 + 2x)^3,
+// 0.01035 at x = 0.1), so that what needs the FP64 fallback goes to the Jacobi
+// fit, which tells.
+constexpr float kWarmDet = 0.0104f;
+__device__ __forceinline__ bool rotation_warm(const float S_in[3][3], float R[3][3]) {
+    float f2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) f2 += S_in[i][j] * S_in[i][j];
+    if (!(f2 > 1e-30f && f2 < 1e30f)) return false;
+    const float sc = rsqrtf(f2);
+    float S[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) S[i][j] = S_in[i][j] * sc;
+#pragma unroll 1
+    for (int it = 0; it < 5; ++it) {
+        float Q[3][3];  // (S R)^T
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) Q[a][b] = S[b][0] * R[0][a] + S[b][1] * R[1][a] + S[b][2] * R[2][a];
+        const float g0 = Q[2][1] - Q[1][2], g1 = Q[0][2] - Q[2][0], g2 = Q[1][0] - Q[0][1];
+        const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
+        const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
+                    h12 = -0.5f * (Q[1][2] + Q[2][1]);
+        const float c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
+        const float c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
+        const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = h00 + h11 + h22;
+        if (!(h00 > 0.f && c22 > 0.f && det > kWarmDet * tr * tr * tr)) return false;
+        // a = w / 2, w = H^-1 g; C(w) - I = f ([a]x + [a]x^2)
+        const float id = __fdividef(0.5f, det);
+        const float a0 = id * (c00 * g0 + c01 * g1 + c02 * g2), a1 = id * (c01 * g0 + c11 * g1 + c12 * g2),
+                    a2 = id * (c02 * g0 + c12 * g1 + c22 * g2);
+        const float n2 = a0 * a0 + a1 * a1 + a2 * a2, f = __fdividef(2.f, 1.f + n2);
+        float K[3][3] = {{-f * (a1 * a1 + a2 * a2), f * (a0 * a1 - a2), f * (a0 * a2 + a1)},
+                         {f * (a0 * a1 + a2), -f * (a0 * a0 + a2 * a2), f * (a1 * a2 - a0)},
+                         {f * (a0 * a2 - a1), f * (a1 * a2 + a0), -f * (a0 * a0 + a1 * a1)}};
+        const bool last = n2 < 4e-9f;
+        if (last) {  // less half of R^T R - I
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = a; b < 3; ++b) {
+                    float x = a == b ? -1.f : 0.f;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) x = fmaf(R[k][a], R[k][b], x);
+                    K[a][b] -= 0.5f * x;
+                    if (a != b) K[b][a] -= 0.5f * x;
+                }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float r0 = R[a][0], r1 = R[a][1], r2 = R[a][2];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) R[a][b] += r0 * K[0][b] + r1 * K[1][b] + r2 * K[2][b];
+        }
+        if (last) return true;
+    }
+    return false;
+}
+
+// FP64 rotation from an FP32 fit Rf by iterative refinement: FP64 only where
+// the digits are made. With R = R0 exp([w]x) the objective's gradient g (the
+// axial vector of the skew part of (S R)^T) and R's deviation from
+// orthogonality E = R^T R - I are residuals, small numbers that FP64 products
+// leave exact to FP64 rounding: 36 FP64 instructions a step. What is made of
+// them needs only a few digits, so the Hessian H = tr(Q) I - sym(Q),
+// w = H^-1 g, the Cayley map of w and the correction
+//     dR = R ((I - E/2 + 3 E^2/8) C(w) - I)
+// are formed in FP32 (H and R at Rf), and R + dR costs 9 more. A step leaves
+// about |dR| (1e-6 / conditioning): with det(H) / tr(H)^3 above kNewtonDet
+// (0.037 at equal singular values, 0.010 at (sigma_2 + sigma_3) / sigma_1 = 0.1
+// without a reflection) 1e-6 -> 1e-11 -> below FP64 rounding in two steps, the
+// first of which is all a result of FP32 needs. Down to kRefineDet, a tenth of
+// the conditioning, steps go on until they are that small. FP64 Newton steps
+// (S R, adjugate, Cayley map and products in FP64) take about 400 FP64
+// instructions for the same rotation, the FP64 Jacobi fit some thousands: the
+// one-rings stretched by a handle's move made the first iterations' local step
+// 62 to 67 us on the 61,600-vertex bar against 25 later, FP64 form.
+// S's largest entry has the biased exponent e, Sf is S at that scale. False,
+// and R undefined, below kRefineDet or where eight steps do not end.
+constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f;
+template <bool FULL>
+__device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, const float Sf[3][3],
+                                                const float Rf[3][3], double R[3][3]) {
+    float Q[3][3];  // (S R)^T
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) Q[a][b] = Sf[b][0] * Rf[0][a] + Sf[b][1] * Rf[1][a] + Sf[b][2] * Rf[2][a];
+    const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
+    const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
+                h12 = -0.5f * (Q[1][2] + Q[2][1]);
+    const float c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
+    const float c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
+    const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
+    if (!(h00 > 0.f && c22 > 0.f && det > kRefineDet * tr * tr * tr)) return false;
+    const bool plain = det > kNewtonDet * tr * tr * tr;
+    const float id = 1.f / det;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) R[a][b] = to_double(Rf[a][b]);
+#pragma unroll 1
+    for (int it = 0; it < 8; ++it) {
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            g0 += S[1][k] * R[k][2];
+            g1 += S[2][k] * R[k][0];
+            g2 += S[0][k] * R[k][1];
+            g0 -= S[2][k] * R[k][1];
+            g1 -= S[0][k] * R[k][2];
+            g2 -= S[1][k] * R[k][0];
+        }
+        float E[3][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = a; b < 3; ++b) {
+                double x = a == b ? -1.0 : 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
+                E[a][b] = E[b][a] = to_float_scaled(x, 1023);
+            }
+        // the gradient at the orthonormalised R (I - E/2): Q loses E Q / 2
+        float M[3][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) M[a][b] = E[a][0] * Q[0][b] + E[a][1] * Q[1][b] + E[a][2] * Q[2][b];
+        const float f0 = (to_float_scaled(g0, e) - 0.5f * (M[2][1] - M[1][2])) * id,
+                    f1 = (to_float_scaled(g1, e) - 0.5f * (M[0][2] - M[2][0])) * id,
+                    f2 = (to_float_scaled(g2, e) - 0.5f * (M[1][0] - M[0][1])) * id;
+        // a = w / 2, w = H^-1 g; C(w) - I = f ([a]x + [a]x^2)
+        const float a0 = 0.5f * (c00 * f0 + c01 * f1 + c02 * f2), a1 = 0.5f * (c01 * f0 + c11 * f1 + c12 * f2),
+                    a2 = 0.5f * (c02 * f0 + c12 * f1 + c22 * f2);
+        const float n2 = a0 * a0 + a1 * a1 + a2 * a2, f = 2.f / (1.f + n2);
+        const float K[3][3] = {{-f * (a1 * a1 + a2 * a2), f * (a0 * a1 - a2), f * (a0 * a2 + a1)},
+                               {f * (a0 * a1 + a2), -f * (a0 * a0 + a2 * a2), f * (a1 * a2 - a0)},
+                               {f * (a0 * a2 - a1), f * (a1 * a2 + a0), -f * (a0 * a0 + a1 * a1)}};
+        float D[3][3];  // -E/2 + 3 E^2/8, then the correction's factor
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                D[a][b] = -0.5f * E[a][b] + 0.375f * (E[a][0] * E[0][b] + E[a][1] * E[1][b] + E[a][2] * E[2][b]);
+        float N[3][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                N[a][b] = K[a][b] + D[a][b] + (D[a][0] * K[0][b] + D[a][1] * K[1][b] + D[a][2] * K[2][b]);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                R[a][b] += to_double(Rf[a][0] * N[0][b] + Rf[a][1] * N[1][b] + Rf[a][2] * N[2][b]);
+        if (plain ? it == (FULL ? 1 : 0) : n2 < (FULL ? 2.5e-27f : 1e-16f)) return true;
+    }
+    return false;
+}
+
+// Exponent and FP32 form of S for rotation_refine; false where the gradient's
+// FP32 exponents would leave their range
+__device__ __forceinline__ bool refine_scale(const double S[3][3], int &e, float Sf[3][3]) {
+    e = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) e = max(e, (__double2hiint(S[a][b]) >> 20) & 0x7ff);
+    if (!(e > 60 && e < 0x7f0)) return false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) Sf[a][b] = to_float_scaled(S[a][b], e);
+    return true;
+}
+
 // FP64 covariance of vertex i's one-ring (estimateRotations, arap.h:358-374)
 // and its rotation refined from the FP32 fit Rm (in place), from the rest
 // positions p, current positions pc (element k of vertex k's pose at
-// k * stride + off) and the FP64 weights.
-// NEWTON: the refinement below; else the FP64 one-sided Jacobi fit of the
-// FP64 covariance (measured faster in the batched local step, where the 32
-// lanes of a warp are 32 poses of one vertex, slower for one request).
-template <bool NEWTON>
+// k * stride + off) and the FP64 weights: by rotation_refine, below its range
+// by an orthonormalisation and a Newton step in FP64, which leave an error of
+// about 1e-12 of the fit's few 1e-6 (the FP64 Jacobi fit instead made a local
+// step of 256 poses of 10,242 vertices 154 us on average against 137).
 __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32_t *__restrict__ dcol,
                                               const double *__restrict__ w64, const Vec4<double> *__restrict__ p,
                                               const Vec4<double> *__restrict__ pc, int64_t stride, int64_t off,
@@ -330,135 +522,37 @@ __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32
         S[1][0] += ey * fx; S[1][1] += ey * fy; S[1][2] += ey * fz;
         S[2][0] += ez * fx; S[2][1] += ez * fy; S[2][2] += ez * fz;
     }
-    // Newton's method on the rotation group from the FP32 fit, which is close
-    // (a few 1e-6 at worst): one orthonormalisation and one Newton step leave
-    // an error of about 1e-12, far below what the mixed form's FP32 rotations
-    // carry anyway, for ~300 FP64 instructions (the scarce kind on this GPU).
     double R[3][3];
-    if constexpr (NEWTON) {
+    int ex;
+    float Sf[3][3];
+    if (!(refine_scale(S, ex, Sf) && rotation_refine<false>(S, ex, Sf, Rm, R))) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) R[a][b] = (double)Rm[a][b];
         polar_newton(S, R, 1, 1);
-    } else {
-        rotation_from_cov<double>(S, R);
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 3; ++b) Rm[a][b] = (float)R[a][b];
+        for (int b = 0; b < 3; ++b) Rm[a][b] = to_float_rn(R[a][b]);
 }
 
-// Below this det(H) / tr(H)^3 the rotation is too poorly determined for FP32
-// Newton steps (0.037 at equal singular values, 0.010 at (sigma_2 + sigma_3) /
-// sigma_1 = 0.1 without a reflection).
-constexpr float kNewtonDet = 4e-3f;
-
-// FP64 rotation fit of the FP64 form, by iterative refinement of the FP32 fit:
-// FP64 only where the digits are made. With R = R0 exp([w]x) the objective's
-// gradient g (the axial vector of the skew part of (S R)^T) and R's deviation
-// from orthogonality E = R^T R - I are residuals, small numbers that FP64
-// products leave exact to FP64 rounding: 36 FP64 instructions a step. What is
-// made of them needs only a few digits, so the Hessian H = tr(Q) I - sym(Q),
-// w = H^-1 g, the Cayley map of w and the correction
-//     dR = R ((I - E/2 + 3 E^2/8) C(w) - I)
-// are formed in FP32, and R + dR costs 9 more. A step leaves the Newton and
-// FP32 remainders, about |dR| (1e-6 / conditioning): 1e-6 -> 1e-11 -> below
-// FP64 rounding in two steps. FP64 Newton steps (S R, adjugate, Cayley map and
-// products in FP64) took about 400 FP64 instructions for the same rotation.
-// Covariances close to rank one, or whose H is close to singular (a reflection
-// with close small singular values), take the FP64 one-sided Jacobi fit.
+// Rotation fit of the FP64 form, from the FP32 fit (R: the rotation of the
+// iteration before). Covariances closer to rank one than the refinement takes,
+// or whose H is close to singular (a reflection with close small singular
+// values), take the FP64 one-sided Jacobi fit.
 __device__ __forceinline__ void rotation_fit_fp64(const double S[3][3], double R[3][3]) {
-    int e = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) e = max(e, (__double2hiint(S[a][b]) >> 20) & 0x7ff);
-    // normal numbers, and the gradient's FP32 exponents in range
-    if (e > 60 && e < 0x7f0) {
-        float Sf[3][3], Rf[3][3], spread;
+    int e;
+    float Sf[3][3];
+    if (refine_scale(S, e, Sf)) {
+        float Rf[3][3];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) Sf[a][b] = to_float_scaled(S[a][b], e);
-        rotation_from_cov<float>(Sf, Rf, &spread);
-        float Q[3][3];  // (S R)^T
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) Q[a][b] = Sf[b][0] * Rf[0][a] + Sf[b][1] * Rf[1][a] + Sf[b][2] * Rf[2][a];
-        const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
-        const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
-                    h12 = -0.5f * (Q[1][2] + Q[2][1]);
-        const float c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
-        const float c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
-        const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
-        if (spread >= kPolarFallback && det > kNewtonDet * tr * tr * tr) {
-            const float id = 1.f / det;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) R[a][b] = to_double(Rf[a][b]);
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-                double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    g0 += S[1][k] * R[k][2];
-                    g1 += S[2][k] * R[k][0];
-                    g2 += S[0][k] * R[k][1];
-                    g0 -= S[2][k] * R[k][1];
-                    g1 -= S[0][k] * R[k][2];
-                    g2 -= S[1][k] * R[k][0];
-                }
-                float E[3][3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = a; b < 3; ++b) {
-                        double x = a == b ? -1.0 : 0.0;
-#pragma unroll
-                        for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
-                        E[a][b] = E[b][a] = to_float_scaled(x, 1023);
-                    }
-                // the gradient at the orthonormalised R (I - E/2): Q loses E Q / 2
-                float M[3][3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b) M[a][b] = E[a][0] * Q[0][b] + E[a][1] * Q[1][b] + E[a][2] * Q[2][b];
-                const float f0 = (to_float_scaled(g0, e) - 0.5f * (M[2][1] - M[1][2])) * id,
-                            f1 = (to_float_scaled(g1, e) - 0.5f * (M[0][2] - M[2][0])) * id,
-                            f2 = (to_float_scaled(g2, e) - 0.5f * (M[1][0] - M[0][1])) * id;
-                // a = w / 2, w = H^-1 g; C(w) - I = f ([a]x + [a]x^2)
-                const float a0 = 0.5f * (c00 * f0 + c01 * f1 + c02 * f2), a1 = 0.5f * (c01 * f0 + c11 * f1 + c12 * f2),
-                            a2 = 0.5f * (c02 * f0 + c12 * f1 + c22 * f2);
-                const float f = 2.f / (1.f + a0 * a0 + a1 * a1 + a2 * a2);
-                const float K[3][3] = {{-f * (a1 * a1 + a2 * a2), f * (a0 * a1 - a2), f * (a0 * a2 + a1)},
-                                       {f * (a0 * a1 + a2), -f * (a0 * a0 + a2 * a2), f * (a1 * a2 - a0)},
-                                       {f * (a0 * a2 - a1), f * (a1 * a2 + a0), -f * (a0 * a0 + a1 * a1)}};
-                float D[3][3];  // -E/2 + 3 E^2/8, then the correction's factor
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-                        D[a][b] = -0.5f * E[a][b] +
-                                  0.375f * (E[a][0] * E[0][b] + E[a][1] * E[1][b] + E[a][2] * E[2][b]);
-                float N[3][3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-                        N[a][b] = K[a][b] + D[a][b] + (D[a][0] * K[0][b] + D[a][1] * K[1][b] + D[a][2] * K[2][b]);
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-                        R[a][b] += to_double(Rf[a][0] * N[0][b] + Rf[a][1] * N[1][b] + Rf[a][2] * N[2][b]);
-            }
-            return;
-        }
+            for (int b = 0; b < 3; ++b) Rf[a][b] = to_float_scaled(R[a][b], 1023);
+        if (!rotation_warm(Sf, Rf)) rotation_from_cov<float>(Sf, Rf);
+        if (rotation_refine<true>(S, e, Sf, Rf, R)) return;
     }
     rotation_from_cov<double>(S, R);
 }

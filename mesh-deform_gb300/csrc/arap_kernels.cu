@@ -1070,6 +1070,13 @@ k_local_step_fp64(int V, const int32_t *__restrict__ drow, const int32_t *__rest
         }
     }
     double Rm[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const Vec4<double> r = R[3 * (int64_t)i + a];
+        Rm[a][0] = r.x;
+        Rm[a][1] = r.y;
+        Rm[a][2] = r.z;
+    }
     dev::rotation_fit_fp64(S, Rm);
     R[3 * (int64_t)i + 0] = {Rm[0][0], Rm[0][1], Rm[0][2], 0.0};
     R[3 * (int64_t)i + 1] = {Rm[1][0], Rm[1][1], Rm[1][2], 0.0};
@@ -1139,9 +1146,19 @@ k_local_step_mixed(int V, const int32_t *__restrict__ drow, const int32_t *__res
             for (int b = 0; b < 3; ++b) S[a][b] = group_sum<G>(S[a][b]);
     }
     if (!live || l != 0) return;
-    float Rm[3][3], spread;
-    rotation_from_cov(S, Rm, &spread);
-    if (!(spread >= dev::kPolarFallback)) dev::rotation_fp64<true>(i, drow[i], e1, dcol, w64, p64, pc64, 1, 0, Rm);
+    float Rm[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const Vec4<float> r = R[3 * (int64_t)i + a];
+        Rm[a][0] = r.x;
+        Rm[a][1] = r.y;
+        Rm[a][2] = r.z;
+    }
+    if (!dev::rotation_warm(S, Rm)) {
+        float spread;
+        rotation_from_cov(S, Rm, &spread);
+        if (!(spread >= dev::kPolarFallback)) dev::rotation_fp64(i, drow[i], e1, dcol, w64, p64, pc64, 1, 0, Rm);
+    }
     R[3 * (int64_t)i + 0] = {Rm[0][0], Rm[0][1], Rm[0][2], 0.f};
     R[3 * (int64_t)i + 1] = {Rm[1][0], Rm[1][1], Rm[1][2], 0.f};
     R[3 * (int64_t)i + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], 0.f};

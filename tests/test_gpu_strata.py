@@ -119,3 +119,30 @@ def test_vertex_blocks_by_size(gpu, level):
         for k in ("local", "rhs", "residual"):
             ctx.set_vertex_launch(k, 1, 256)
         np.testing.assert_array_equal(ctx.deform(w.iterations), a)
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-6)])
+@pytest.mark.parametrize("pull", [0.02, 0.3, 1.0])
+def test_rotation_seeds(gpu, precision, tol, pull):
+    """Local steps from the rotations before: a small move (every fit ends in
+    the Newton steps), a large one and one that stretches the one-rings at the
+    handles to near rank one (refinement, Jacobi fits), against the oracle's
+    SVD; one deform of n iterations gives the bits of n deforms of one."""
+    from oracle import oracle as O
+
+    w = W.cfg_icosphere_l4(level=3, iterations=6)
+    targets = w.ctargets + pull * np.array([0.3, 1.0, -0.2]) * (np.arange(len(w.cidx)) % 2)[:, None]
+    ok, ref = O.run_deform(w.positions, w.faces, w.cidx, targets, w.iterations)
+    assert ok
+    outs = []
+    for parts in ([6], [1, 1, 1, 3]):
+        with make(gpu, w, precision) as ctx:
+            ctx.set_constraints(w.cidx, targets)
+            for n in parts:
+                out = ctx.deform(n)
+            outs.append(out)
+    np.testing.assert_array_equal(outs[1], outs[0])
+    assert W.bbox_rel_error(outs[0], ref, w.positions) <= tol
+    with make(gpu, w, "mixed") as ctx:
+        poses = np.stack([targets, w.ctargets])
+        got = ctx.deform_poses(poses, w.iterations)
+    assert W.bbox_rel_error(got[0], ref, w.positions) <= 1e-6
