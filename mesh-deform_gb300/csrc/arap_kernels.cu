@@ -3478,15 +3478,9 @@ template <typename T> struct StKernels {
     using Bwd = void (*)(int, const StTile *, const T *, const int32_t *, const int32_t *, const Vec4<T> *, Vec4<T> *,
                          Vec4<double> *, int);
     template <int NT> static Fwd fwd_nt(int G, int RW) {
-        if constexpr (sizeof(T) == 8) {  // one row per lane group (build_strata)
-            if (G == 1) return k_strata_fwd<T, NT, 1, 1>;
-            if (G == 4) return k_strata_fwd<T, NT, 4, 1>;
-            return G == 8 ? k_strata_fwd<T, NT, 8, 1> : k_strata_fwd<T, NT, 32, 1>;
-        } else {
-            if (G == 8)
-                return RW == 4 ? k_strata_fwd<T, NT, 8, 4> : RW == 2 ? k_strata_fwd<T, NT, 8, 2> : k_strata_fwd<T, NT, 8, 1>;
-            return RW == 4 ? k_strata_fwd<T, NT, 32, 4> : RW == 2 ? k_strata_fwd<T, NT, 32, 2> : k_strata_fwd<T, NT, 32, 1>;
-        }
+        if (G == 8)
+            return RW == 4 ? k_strata_fwd<T, NT, 8, 4> : RW == 2 ? k_strata_fwd<T, NT, 8, 2> : k_strata_fwd<T, NT, 8, 1>;
+        return RW == 4 ? k_strata_fwd<T, NT, 32, 4> : RW == 2 ? k_strata_fwd<T, NT, 32, 2> : k_strata_fwd<T, NT, 32, 1>;
     }
     template <int NT> static Bwd bwd_nt(int TC) {
         switch (TC) {
@@ -3503,7 +3497,10 @@ template <typename T> struct StKernels {
         return p.rc == 8 ? k_strata_inverse<T, 8> : p.rc == 4 ? k_strata_inverse<T, 4> : k_strata_inverse<T, 2>;
     }
     static Fwd fwd(const StPhase &p) {
-        return p.ntf == kStThreads ? fwd_nt<kStThreads>(p.G, p.RW) : fwd_nt<kStThreadsLarge>(p.G, p.RW);
+        if constexpr (sizeof(T) == 8)  // one row per lane group (build_strata)
+            return p.ntf == kStThreadsSmall ? k_strata_fwd<T, kStThreadsSmall, 8, 1> : k_strata_fwd<T, kStThreadsLarge, 32, 1>;
+        else
+            return p.ntf == kStThreads ? fwd_nt<kStThreads>(p.G, p.RW) : fwd_nt<kStThreadsLarge>(p.G, p.RW);
     }
     static Bwd bwd(const StPhase &p) {
         return p.ntb == kStThreads ? bwd_nt<kStThreads>(p.TC) : bwd_nt<kStThreadsLarge>(p.TC);

@@ -235,21 +235,29 @@ bool build_strata(const Symbolic &sym, StrataKind kind, int sms, Strata &out) {
         p.ntf = p.nmax > kStLargeCols ? kStThreadsLarge : kStThreads;
         p.ntb = p.vmax > kStLargeRows ? kStThreadsLarge : kStThreads;
         auto step = [&](int rw) { return p.ntf / p.G * rw; };
+        int per;
         if (fp64) {
-            // a lane group's sums cost FP64 additions, the scarce
-            // instructions: as few lanes per row as give every scheduler a
-            // warp or two
-            p.RW = p.G = 1;
-            for (const int g : {4, 8, 32})
-                if (rows * p.G < (int64_t)32 * 4 * sms * 2) p.G = g;
+            // Bound by FP64 issue, so the work has to come in shares small
+            // enough to even out over the schedulers: 8 lanes per row and 8
+            // rows per CTA of 64 threads (one row per lane of 128-thread CTAs
+            // left one scheduler in four without rows: bar 259 -> 224 us per
+            // iteration, level-6 sphere 200 -> 167, 2,562 vertices 41 -> 40;
+            // with 4 or 2 lanes per row 229 and 232).
+            p.RW = 1;
+            p.G = 32;
+            if (p.nmax <= kStLargeCols) {
+                p.ntf = kStThreadsSmall;
+                p.G = 8;
+            }
+            per = step(1);
         } else {
             // lane groups of 8 for groups of few columns; as many rows per
             // lane group as leave four warps per scheduler
             p.G = p.nmax <= 128 ? 8 : 32;
             p.RW = 4;
             while (p.RW > 1 && rows / (32 / p.G * p.RW) < 4 * 4 * sms) p.RW /= 2;
+            per = step(p.RW) * (int)std::min<int64_t>(8, std::max<int64_t>(1, rows / ((int64_t)step(p.RW) * 4 * sms)));
         }
-        int per = step(p.RW) * (int)std::min<int64_t>(8, std::max<int64_t>(1, rows / ((int64_t)step(p.RW) * 4 * sms)));
         p.TC = fp64 ? 32 : 64;
         while (p.TC > (fp64 ? 4 : 8) && (int64_t)p.cn / p.TC * p.ntb < (int64_t)(fp64 ? 4 : 2) * kStThreads * sms) p.TC /= 2;
         if (poses) per = p.TC = 32;

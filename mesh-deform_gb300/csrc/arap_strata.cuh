@@ -97,7 +97,7 @@ k_strata_gather(int c0, int cn, const int32_t *__restrict__ gcol, const int32_t 
 // not by L2: the bar's first stratum, 12 MB in 6.7 us. Four loads in flight
 // per lane and 1,024 threads per SM beat eight and 512 (bar 164 -> 145 us per
 // iteration). FP64: bound by FP64 issue (about 64 clocks per warp instruction
-// and scheduler), so lanes that share a row are as few as fill the device.
+// and scheduler): tiles of 8 rows, so that the schedulers' shares even out.
 template <typename T, int NT, int G, int RW>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 k_strata_fwd(int ldf, const StTile *__restrict__ tiles, const T *__restrict__ Mall,

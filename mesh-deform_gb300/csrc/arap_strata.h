@@ -44,7 +44,8 @@ struct StSn {
 constexpr int kStMaxPhases = 16;
 constexpr int kStMaxCols = 4096;   // most columns of a group
 constexpr int kStThreads = 128;     // CTAs of the phases' kernels,
-constexpr int kStThreadsLarge = 512;  // and where groups are large
+constexpr int kStThreadsLarge = 512;  // where groups are large,
+constexpr int kStThreadsSmall = 64;   // and of the FP64 forward product where they are not
 constexpr int kStBigTop = 1024;    // a lone last group with more columns runs the tiled top products
 constexpr int kStLargeCols = 256, kStLargeRows = 400;  // columns / rows from which a group is large
 constexpr int kStInvCols = 8;      // most columns of M one CTA of the inversion forms (8, 4 or 2)
