@@ -313,16 +313,21 @@ k_strata_bwd(int vmax, const StTile *__restrict__ tiles, const T *__restrict__ M
 // X's rows; past the group's root, F is -W. Zeros of M (above the diagonal,
 // and between subtrees that do not meet) are never written: they are cleared
 // once when the matrices are laid out.
+// The block that holds the columns starts from the identity: its Y are columns
+// of inv(L_bb), and their rows above c0 are zero (half the FP64 work of groups
+// with few columns: set-up of the bar in FP64 3.41 -> 2.83 ms).
 // Bound by FP64 issue (FP64 form) or by the chain of blocks; a phase's columns
-// per CTA are cut until it has four CTAs per SM. The strata are independent:
+// per CTA are cut until it has four CTAs per SM. In FP32 more CTAs on an SM
+// are worth more than loads ahead (bar's set-up 2.42 against 2.48 ms). The strata are independent:
 // their launches overlap (`first` waits for the factor, the others only
 // before they end).
 template <typename T, int RC>
-__global__ void __launch_bounds__(kStThreads)
+__global__ void __launch_bounds__(kStThreads, sizeof(T) == 8 ? 6 : 8)
 k_strata_inverse(const int32_t *__restrict__ items, const SnInfo *__restrict__ sn, const StSn *__restrict__ ssn,
                  const int32_t *__restrict__ relind, const T *__restrict__ Lval, const T *__restrict__ Dinv,
                  int front, int first, T *__restrict__ Mall) {
     extern __shared__ __align__(128) unsigned char st_raw[];
+    constexpr bool kAhead = sizeof(T) == 8;
     T *F = reinterpret_cast<T *>(st_raw);  // [row][RC], the current supernode's front
     T *G = F + (size_t)front * RC;         // its parent's
     T *Y = G + (size_t)front * RC;         // [row][RC], the current block's solution
@@ -337,35 +342,64 @@ k_strata_inverse(const int32_t *__restrict__ items, const SnInfo *__restrict__ s
     pdl_trigger();
     __syncthreads();
     int node = j, jb = c0 / NB;
+    bool start = true;
     for (;;) {
         const int n = dn.nrow, nc = dn.ncol, pos = ssn[node].pos;
         const T *P = Lval + dn.panel_off;
         for (; jb * NB < nc; ++jb) {
             const int j0 = jb * NB, wb = min(NB, nc - j0);
+            const int kb = start ? c0 - j0 : 0;  // the solution's rows above are zero
             const T *D = Dinv + dn.dinv_off + (int64_t)jb * NB * NB;  // D[k * NB + r] = inv(L_bb)(r, k)
+            // FP64: the row of L below the block that this thread takes first is
+            // loaded ahead of the block's solution
+            T l[NB];
+            auto load = [&](int i) {
+                const T *Li = P + (int64_t)j0 * n + i;
+#pragma unroll
+                for (int k = 0; k < NB; ++k) l[k] = k >= kb && k < wb ? Li[(int64_t)k * n] : (T)0;
+            };
+            const int i0 = j0 + wb + tid;
+            if (kAhead && i0 < n) load(i0);
             for (int o = tid; o < NB * RC; o += kStThreads) {
                 const int r = o % NB, c = o / NB;
-                T dk[NB];
-#pragma unroll
-                for (int k = 0; k < NB; ++k) dk[k] = D[k * NB + r];
                 T s = (T)0;
+                if (start) {  // F is the identity's columns
+                    if (c < w) s = D[(kb + c) * NB + r];
+                } else {
+                    T dk[NB];
 #pragma unroll
-                for (int k = 0; k < NB; ++k)
-                    if (k < wb) s += dk[k] * F[(j0 + k) * RC + c];
+                    for (int k = 0; k < NB; ++k) dk[k] = D[k * NB + r];
+#pragma unroll
+                    for (int k = 0; k < NB; ++k)
+                        if (k < wb) s += dk[k] * F[(j0 + k) * RC + c];
+                }
                 Y[r * RC + c] = s;
                 if (r < wb && c < w) M[(int64_t)(pos + j0 + r) * gj.ld + c] = s;
             }
+            start = false;
             __syncthreads();
-            for (int i = j0 + wb + tid; i < n; i += kStThreads) {
-                const T *Li = P + (int64_t)j0 * n + i;
+            for (int i = i0; i < n; i += kStThreads) {
                 T acc[RC];
 #pragma unroll
                 for (int c = 0; c < RC; ++c) acc[c] = F[i * RC + c];
-#pragma unroll 8
-                for (int k = 0; k < wb; ++k) {
-                    const T l = Li[(int64_t)k * n];
+                if constexpr (kAhead) {
+                    if (i != i0) load(i);
 #pragma unroll
-                    for (int c = 0; c < RC; ++c) acc[c] -= l * Y[k * RC + c];
+                    for (int k0 = 0; k0 < NB; k0 += 4) {
+                        if (k0 + 4 <= kb || k0 >= wb) continue;
+#pragma unroll
+                        for (int k = k0; k < k0 + 4; ++k)
+#pragma unroll
+                            for (int c = 0; c < RC; ++c) acc[c] -= l[k] * Y[k * RC + c];
+                    }
+                } else {
+                    const T *Li = P + (int64_t)j0 * n + i;
+#pragma unroll 8
+                    for (int k = kb; k < wb; ++k) {
+                        const T lk = Li[(int64_t)k * n];
+#pragma unroll
+                        for (int c = 0; c < RC; ++c) acc[c] -= lk * Y[k * RC + c];
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < RC; ++c) F[i * RC + c] = acc[c];
