@@ -402,58 +402,39 @@ __device__ __forceinline__ bool rotation_warm(const float S_in[3][3], float R[3]
 // S's largest entry has the biased exponent e, Sf is S at that scale. False,
 // and R undefined, below kRefineDet or where eight steps do not end.
 constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f;
-template <bool FULL>
-__device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, const float Sf[3][3],
-                                                const float Rf[3][3], double R[3][3]) {
-    float Q[3][3];  // (S R)^T
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) Q[a][b] = Sf[b][0] * Rf[0][a] + Sf[b][1] * Rf[1][a] + Sf[b][2] * Rf[2][a];
-    const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
-    const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
-                h12 = -0.5f * (Q[1][2] + Q[2][1]);
-    const float c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
-    const float c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
-    const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
-    if (!(h00 > 0.f && c22 > 0.f && det > kRefineDet * tr * tr * tr)) return false;
-    const bool plain = det > kNewtonDet * tr * tr * tr;
-    const float id = 1.f / det;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) R[a][b] = to_double(Rf[a][b]);
-#pragma unroll 1
-    for (int it = 0; it < 8; ++it) {
-        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            g0 += S[1][k] * R[k][2];
-            g1 += S[2][k] * R[k][0];
-            g2 += S[0][k] * R[k][1];
-            g0 -= S[2][k] * R[k][1];
-            g1 -= S[0][k] * R[k][2];
-            g2 -= S[1][k] * R[k][0];
-        }
-        float E[3][3];
+constexpr int kRefineSteps = 8;
+
+// What the steps share: Q = (S R)^T at Rf, adj(H), 1 / det(H)
+struct RefineFrame {
+    float Q[3][3], c00, c01, c02, c11, c12, c22, id;
+    bool plain;  // a fixed number of steps suffices
+    __device__ __forceinline__ bool init(const float Sf[3][3], const float Rf[3][3]) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = a; b < 3; ++b) {
-                double x = a == b ? -1.0 : 0.0;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
-                E[a][b] = E[b][a] = to_float_scaled(x, 1023);
-            }
+            for (int b = 0; b < 3; ++b) Q[a][b] = Sf[b][0] * Rf[0][a] + Sf[b][1] * Rf[1][a] + Sf[b][2] * Rf[2][a];
+        const float h00 = Q[1][1] + Q[2][2], h11 = Q[0][0] + Q[2][2], h22 = Q[0][0] + Q[1][1];
+        const float h01 = -0.5f * (Q[0][1] + Q[1][0]), h02 = -0.5f * (Q[0][2] + Q[2][0]),
+                    h12 = -0.5f * (Q[1][2] + Q[2][1]);
+        c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
+        c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
+        const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
+        if (!(h00 > 0.f && c22 > 0.f && det > kRefineDet * tr * tr * tr)) return false;
+        plain = det > kNewtonDet * tr * tr * tr;
+        id = 1.f / det;
+        return true;
+    }
+    // the correction to R from g and E; returns |w / 2|^2
+    __device__ __forceinline__ float correction(const float Rf[3][3], const float E[3][3], float g0, float g1, float g2,
+                                                float dR[3][3]) const {
         // the gradient at the orthonormalised R (I - E/2): Q loses E Q / 2
         float M[3][3];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) M[a][b] = E[a][0] * Q[0][b] + E[a][1] * Q[1][b] + E[a][2] * Q[2][b];
-        const float f0 = (to_float_scaled(g0, e) - 0.5f * (M[2][1] - M[1][2])) * id,
-                    f1 = (to_float_scaled(g1, e) - 0.5f * (M[0][2] - M[2][0])) * id,
-                    f2 = (to_float_scaled(g2, e) - 0.5f * (M[1][0] - M[0][1])) * id;
+        const float f0 = (g0 - 0.5f * (M[2][1] - M[1][2])) * id, f1 = (g1 - 0.5f * (M[0][2] - M[2][0])) * id,
+                    f2 = (g2 - 0.5f * (M[1][0] - M[0][1])) * id;
         // a = w / 2, w = H^-1 g; C(w) - I = f ([a]x + [a]x^2)
         const float a0 = 0.5f * (c00 * f0 + c01 * f1 + c02 * f2), a1 = 0.5f * (c01 * f0 + c11 * f1 + c12 * f2),
                     a2 = 0.5f * (c02 * f0 + c12 * f1 + c22 * f2);
@@ -476,9 +457,52 @@ __device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, con
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b)
-                R[a][b] += to_double(Rf[a][0] * N[0][b] + Rf[a][1] * N[1][b] + Rf[a][2] * N[2][b]);
-        if (plain ? it == (FULL ? 1 : 0) : n2 < (FULL ? 2.5e-27f : 1e-16f)) return true;
+            for (int b = 0; b < 3; ++b) dR[a][b] = Rf[a][0] * N[0][b] + Rf[a][1] * N[1][b] + Rf[a][2] * N[2][b];
+        return n2;
+    }
+    template <bool FULL> __device__ __forceinline__ bool done(int it, float n2) const {
+        return plain ? it == (FULL ? 1 : 0) : n2 < (FULL ? 2.5e-27f : 1e-16f);
+    }
+};
+
+template <bool FULL>
+__device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, const float Sf[3][3],
+                                                const float Rf[3][3], double R[3][3]) {
+    RefineFrame fr;
+    if (!fr.init(Sf, Rf)) return false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) R[a][b] = to_double(Rf[a][b]);
+#pragma unroll 1
+    for (int it = 0; it < kRefineSteps; ++it) {
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            g0 += S[1][k] * R[k][2];
+            g1 += S[2][k] * R[k][0];
+            g2 += S[0][k] * R[k][1];
+            g0 -= S[2][k] * R[k][1];
+            g1 -= S[0][k] * R[k][2];
+            g2 -= S[1][k] * R[k][0];
+        }
+        float E[3][3], dR[3][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = a; b < 3; ++b) {
+                double x = a == b ? -1.0 : 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
+                E[a][b] = E[b][a] = to_float_scaled(x, 1023);
+            }
+        const float n2 =
+            fr.correction(Rf, E, to_float_scaled(g0, e), to_float_scaled(g1, e), to_float_scaled(g2, e), dR);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) R[a][b] += to_double(dR[a][b]);
+        if (fr.done<FULL>(it, n2)) return true;
     }
     return false;
 }
@@ -555,6 +579,88 @@ __device__ __forceinline__ void rotation_fit_fp64(const double S[3][3], double R
         if (rotation_refine<true>(S, e, Sf, Rf, R)) return;
     }
     rotation_from_cov<double>(S, R);
+}
+
+// The same by four lanes of a warp: lane l < 3 has row l of S and gets column l
+// of R (lane 3 goes along with lane 0); R holds the rotation before on every
+// lane. Column l's lane makes component l of g, E(l, l), E(l, l + 1) and its
+// column's corrections: 15 FP64 instructions a step instead of 45, for small
+// meshes, whose warps leave the FP64 pipes idle while each waits for its own
+// chain.
+__device__ __forceinline__ void rotation_fit_fp64_quad(const double row[3], int lane, const float Rb[3][3],
+                                                       double col[3]) {
+    const int q0 = lane & ~3, l = lane & 3, c = l == 3 ? 0 : l, c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+    const unsigned mask = 0xfu << q0;
+    int e = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) e = max(e, (__double2hiint(row[k]) >> 20) & 0x7ff);
+    e = max(e, __shfl_xor_sync(mask, e, 1));
+    e = max(e, __shfl_xor_sync(mask, e, 2));
+    if (e > 60 && e < 0x7f0) {  // as refine_scale
+        float Sf[3][3], Rf[3][3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float x = to_float_scaled(row[k], e);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                Sf[a][k] = __shfl_sync(mask, x, q0 + a);
+                Rf[a][k] = Rb[a][k];
+            }
+        }
+        if (!rotation_warm(Sf, Rf)) rotation_from_cov<float>(Sf, Rf);
+        RefineFrame fr;
+        if (fr.init(Sf, Rf)) {
+            double Sa[3], Sb[3], C0[3], C1[3], C2[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                Sa[k] = __shfl_sync(mask, row[k], q0 + c1);
+                Sb[k] = __shfl_sync(mask, row[k], q0 + c2);
+                C0[k] = to_double(c == 0 ? Rf[k][0] : c == 1 ? Rf[k][1] : Rf[k][2]);
+                C1[k] = to_double(c == 0 ? Rf[k][1] : c == 1 ? Rf[k][2] : Rf[k][0]);
+                C2[k] = to_double(c == 0 ? Rf[k][2] : c == 1 ? Rf[k][0] : Rf[k][1]);
+            }
+#pragma unroll 1
+            for (int it = 0; it < kRefineSteps; ++it) {
+                double g = 0.0, x0 = -1.0, x1 = 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    g += Sa[k] * C2[k];
+                    x0 += C0[k] * C0[k];
+                    g -= Sb[k] * C1[k];
+                    x1 += C0[k] * C1[k];
+                }
+                const float gf = to_float_scaled(g, e), f0 = to_float_scaled(x0, 1023), f1 = to_float_scaled(x1, 1023);
+                float E[3][3], dR[3][3], gs[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    gs[a] = __shfl_sync(mask, gf, q0 + a);
+                    E[a][a] = __shfl_sync(mask, f0, q0 + a);
+                    const int b = a == 2 ? 0 : a + 1;
+                    E[a][b] = E[b][a] = __shfl_sync(mask, f1, q0 + a);
+                }
+                const float n2 = fr.correction(Rf, E, gs[0], gs[1], gs[2], dR);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    C0[k] += to_double(c == 0 ? dR[k][0] : c == 1 ? dR[k][1] : dR[k][2]);
+                    C1[k] = __shfl_sync(mask, C0[k], q0 + c1);
+                    C2[k] = __shfl_sync(mask, C0[k], q0 + c2);
+                }
+                if (fr.done<true>(it, n2)) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) col[k] = C0[k];
+                    return;
+                }
+            }
+        }
+    }
+    double S[3][3], R[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) S[a][k] = __shfl_sync(mask, row[k], q0 + a);
+    rotation_from_cov<double>(S, R);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) col[k] = c == 0 ? R[k][0] : c == 1 ? R[k][1] : R[k][2];
 }
 
 }  // namespace dev

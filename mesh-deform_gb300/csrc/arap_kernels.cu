@@ -1083,6 +1083,54 @@ k_local_step_fp64(int V, const int32_t *__restrict__ drow, const int32_t *__rest
     R[3 * (int64_t)i + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], 0.0};
 }
 
+// the same with four lanes per vertex, for small meshes (launch_local_step_fp64)
+__global__ void __launch_bounds__(64)
+k_local_step_fp64_quad(int V, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+                       const Vec4<double> *__restrict__ wedge, const Vec4<double> *__restrict__ pc,
+                       Vec4<double> *__restrict__ R) {
+    pdl_wait();  // the positions of the kernels before (an overlapped launch)
+    pdl_trigger();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, l = lane & 3, i = t >> 2;
+    double S[12];  // row by row, and three zeros
+#pragma unroll
+    for (int k = 0; k < 12; ++k) S[k] = 0.0;
+    float Rb[3][3];
+    if (i < V) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const Vec4<double> r = R[3 * (int64_t)i + a];
+            Rb[a][0] = dev::to_float_scaled(r.x, 1023);
+            Rb[a][1] = dev::to_float_scaled(r.y, 1023);
+            Rb[a][2] = dev::to_float_scaled(r.z, 1023);
+        }
+        const Vec4<double> ci = pc[i];
+        constexpr int kR = 2;
+        const int e1 = drow[i + 1];
+        for (int e = drow[i] + l; e < e1; e += 4 * kR) {
+            Vec4<double> we[kR], cj[kR];
+            ring_gather<4, kR>(e, e1, dcol, [&](int k, int ek, int j) {
+                we[k] = wedge[ek];
+                cj[k] = pc[j];
+            });
+#pragma unroll
+            for (int k = 0; k < kR; ++k) {
+                if (e + 4 * k >= e1) break;
+                const double fx = ci.x - cj[k].x, fy = ci.y - cj[k].y, fz = ci.z - cj[k].z;
+                S[0] += we[k].x * fx; S[1] += we[k].x * fy; S[2] += we[k].x * fz;
+                S[3] += we[k].y * fx; S[4] += we[k].y * fy; S[5] += we[k].y * fz;
+                S[6] += we[k].z * fx; S[7] += we[k].z * fy; S[8] += we[k].z * fz;
+            }
+        }
+    }
+    st_reduce<12, 4>(S, lane);  // lane l has entries 3 l .. 3 l + 2
+    if (i >= V) return;
+    double col[3];
+    dev::rotation_fit_fp64_quad(S, lane, Rb, col);
+    if (l < 3)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) reinterpret_cast<double *>(R + 3 * (int64_t)i + k)[l] = col[k];
+}
+
 // Local step of the mixed form: the covariance in FP32 from the FP32 rest
 // edges and the current edges, differences of the FP64 positions rounded to
 // FP32 (dev::Split: no FP64 instruction), then the FP32 rotation fit.
@@ -3183,7 +3231,18 @@ void launch_weighted_edges(const DevSym &s, const double *w64, const Vec4<double
 void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *pc, Vec4<double> *R,
                             cudaStream_t st) {
     if (s.V == 0) return;
-    const int block = fp64_block(s.V);
+    // Four lanes per vertex (62 FP64 instructions a warp instead of 174) while
+    // one lane each would not give every scheduler a warp. FP64 iterations with
+    // one and with four: 380 vertices 22.3 and 19.7 us, 1,600 31.8 and 29.3,
+    // 8,280 90.9 and 74.0, 18,200 107.5 and 94.9; slower at some sizes (9,500
+    // vertices 77.5 and 82.6).
+    if (s.V <= 32 * 4 * 152) {
+        const int block = fp64_block(4 * (int64_t)s.V);
+        launch_pdl(k_local_step_fp64_quad, s.overlap != 0, blocks_for(4 * (int64_t)s.V, block), block, 0, st, s.V,
+                   (const int32_t *)s.drow, (const int32_t *)s.dcol, wedge, pc, R);
+        return;
+    }
+    const int block = 64;
     launch_pdl(k_local_step_fp64, s.overlap != 0, blocks_for(s.V, block), block, 0, st, s.V, (const int32_t *)s.drow,
                (const int32_t *)s.dcol, wedge, pc, R);
 }

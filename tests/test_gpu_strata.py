@@ -146,3 +146,16 @@ def test_rotation_seeds(gpu, precision, tol, pull):
         poses = np.stack([targets, w.ctargets])
         got = ctx.deform_poses(poses, w.iterations)
     assert W.bbox_rel_error(got[0], ref, w.positions) <= 1e-6
+
+
+@pytest.mark.parametrize("level", [0, 5, 6])
+def test_fp64_lanes_by_size(gpu, level):
+    """FP64 local steps with four lanes per vertex (12 and 10,242 vertices) and
+    with one (40,962), against the oracle."""
+    from oracle import oracle as O
+
+    w = W.cfg_noisy_sphere(level=level, iterations=3) if level else W.cfg_icosphere_l4(level=0, iterations=3)
+    ok, ref = O.run_deform(w.positions, w.faces, w.cidx, w.ctargets, w.iterations)
+    assert ok
+    with make(gpu, w, "fp64") as ctx:
+        assert W.bbox_rel_error(ctx.deform(w.iterations), ref, w.positions) <= 1e-10
