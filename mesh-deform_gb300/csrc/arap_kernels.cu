@@ -1362,6 +1362,51 @@ k_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ 
             dev::to_float_rn((bf.z + dev::to_double(bi.z)) - az), 0.f};
 }
 
+// RHS and the first residual of an iteration in one pass over the one-rings
+// (both read the same entries, and a launch's latency is most of either); the
+// sums are k_rhs_mixed's and k_residual's, in their order. Iterations with two
+// launches and with one: 380 vertices 19.7 and 18.0 us, 2,562 43.5 and 41.0,
+// 8,000 52.0 and 49.1, 18,200 67.9 and 64.3, the 67,202-vertex bar 118.8 and
+// 113.9 (but a 900-vertex sheet 28.8 and 31.6). Neighbours by twos gather no
+// faster here (113.0; 16 bars 215.7 and 218.5).
+__global__ void __launch_bounds__(256)
+k_rhs_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const float *__restrict__ w,
+               const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R,
+               const double *__restrict__ w64, const double *__restrict__ diag64, const Vec4<double> *__restrict__ bfixed,
+               const Vec4<double> *__restrict__ x, Vec4<float> *__restrict__ b, Vec4<float> *__restrict__ r) {
+    pdl_wait();  // the rotations of the local step (an overlapped launch)
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const Vec4<float> r0 = R[3 * (int64_t)i], r1 = R[3 * (int64_t)i + 1], r2 = R[3 * (int64_t)i + 2];
+    const Vec4<double> xi = x[i], bf = bfixed[i];
+    const double dg = diag64[i];
+    float bx = 0.f, by = 0.f, bz = 0.f;
+    double ax = 0.0, ay = 0.0, az = 0.0;
+    const int e1 = drow[i + 1];
+    for (int e = drow[i]; e < e1; ++e) {
+        const int j = dcol[e];
+        const float h = j == i ? 0.f : w[e] * 0.5f;
+        const double wj = w64[e];
+        const Vec4<float> d = redge[e];
+        const Vec4<float> q0 = R[3 * (int64_t)j], q1 = R[3 * (int64_t)j + 1], q2 = R[3 * (int64_t)j + 2];
+        const Vec4<double> xj = x[j];  // x holds every vertex
+        bx += ((r0.x + q0.x) * d.x + (r0.y + q0.y) * d.y + (r0.z + q0.z) * d.z) * h;
+        by += ((r1.x + q1.x) * d.x + (r1.y + q1.y) * d.y + (r1.z + q1.z) * d.z) * h;
+        bz += ((r2.x + q2.x) * d.x + (r2.y + q2.y) * d.y + (r2.z + q2.z) * d.z) * h;
+        if (j == i || j >= m) continue;
+        ax -= wj * xj.x;
+        ay -= wj * xj.y;
+        az -= wj * xj.z;
+    }
+    ax += dg * xi.x;
+    ay += dg * xi.y;
+    az += dg * xi.z;
+    b[i] = {bx, by, bz, 0.f};
+    r[i] = {dev::to_float_rn((bf.x + dev::to_double(bx)) - ax), dev::to_float_rn((bf.y + dev::to_double(by)) - ay),
+            dev::to_float_rn((bf.z + dev::to_double(bz)) - az), 0.f};
+}
+
 // ---------------------------------------------------------------------------
 // supernodal triangular solves
 //
@@ -3264,6 +3309,17 @@ void launch_rhs_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<doub
     default: ARAP_RHS64(8); break;
     }
 #undef ARAP_RHS64
+}
+
+bool rhs_with_residual(const VertexLaunch *vl) { return vl[kVertexRhs].block == 0 && vl[kVertexResidual].block == 0; }
+
+void launch_rhs_residual(const DevSym &s, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
+                         const double *w64, const double *diag64, const Vec4<double> *bfixed, const Vec4<double> *x64,
+                         Vec4<float> *b, Vec4<float> *r, cudaStream_t st) {
+    if (s.m == 0) return;
+    const int block = vertex_block(s.vlaunch[kVertexRhs], s.m);
+    launch_pdl(k_rhs_residual, s.overlap != 0, blocks_for(s.m, block), block, 0, st, s.m, (const int32_t *)s.drow,
+               (const int32_t *)s.dcol, w32, redge, R, w64, diag64, bfixed, x64, b, r);
 }
 
 void launch_residual(const DevSym &s, const double *w64, const double *diag64, const Vec4<double> *bfixed,

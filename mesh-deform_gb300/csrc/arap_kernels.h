@@ -169,6 +169,12 @@ void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Ve
 // FP64 RHS (estimatePositions arap.h:395-414): b = bFixed + sum 1/2 w (Ri+Rj)(pi-pj)
 void launch_rhs_fp64(const DevSym &s, const Vec4<double> *wedge, const Vec4<double> *wsum, const Vec4<double> *R,
                      const Vec4<double> *bfixed, Vec4<double> *b, cudaStream_t st);
+// The RHS and an iteration's first residual in one launch, where the caller
+// chose no shape for either
+bool rhs_with_residual(const VertexLaunch *vl);
+void launch_rhs_residual(const DevSym &s, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
+                         const double *w64, const double *diag64, const Vec4<double> *bfixed, const Vec4<double> *x64,
+                         Vec4<float> *b, Vec4<float> *r, cudaStream_t st);
 // FP64 residual of the global system: r = (bFixed + b) - A x over the free vertices
 void launch_residual(const DevSym &s, const double *w64, const double *diag64, const Vec4<double> *bfixed,
                      const Vec4<float> *b, const Vec4<double> *x64, Vec4<float> *r, cudaStream_t st);
@@ -280,8 +286,10 @@ void launch_bbfixed(const DevSym &s, int P, const double *w64, const Vec4<double
                     cudaStream_t st);
 void launch_blocal(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<double> *pc64,
                    Vec4<float> *R, const double *w64, const Vec4<double> *p64, cudaStream_t st);
-void launch_brhs(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
-                 Vec4<float> *b, cudaStream_t st);
+// the RHS and an iteration's first residual in one launch
+void launch_brhs_residual(const DevSym &s, int P, const float *w32, const Vec4<float> *redge, const Vec4<float> *R,
+                          const double *w64, const double *diag64, const Vec4<double> *bfixed, const Vec4<double> *x,
+                          Vec4<float> *b, Vec4<float> *r, cudaStream_t st);
 void launch_bresidual(const DevSym &s, int P, const double *w64, const double *diag64, const Vec4<double> *bfixed,
                       const Vec4<float> *b, const Vec4<double> *x, Vec4<float> *r, cudaStream_t st);
 // one persistent launch of `grid` CTAs (batch_grid) over all (supernode, pose

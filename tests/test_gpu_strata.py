@@ -111,7 +111,8 @@ def test_several_large_roots(gpu):
 @pytest.mark.parametrize("level", [0, 3, 5, 6])
 def test_vertex_blocks_by_size(gpu, level):
     """Per-vertex kernels' blocks chosen by the mesh's size (12, 642, 10,242 and
-    40,962 vertices: blocks of 32 and 128) give the bits of blocks of 256."""
+    40,962 vertices: blocks of 32 and 128), with the RHS and the first residual
+    in one launch, give the bits of blocks of 256 and of two launches."""
     w = W.cfg_noisy_sphere(level=level, iterations=3) if level else W.cfg_icosphere_l4(level=0, iterations=3)
     with make(gpu, w, "mixed") as ctx:
         a = ctx.deform(w.iterations)
