@@ -812,7 +812,7 @@ def main():
     ap.add_argument("--solve-schedule", default="auto", choices=["auto", "persistent", "levels"],
                     help="single-request solves: persistent CTAs per sweep or one launch per tree level "
                          "(auto: autotuned with the CTA count when requests run concurrently)")
-    ap.add_argument("--vertex-launch", default="auto", choices=["auto", "default"],
+    ap.add_argument("--vertex-launch", default="default", choices=["auto", "default"],
                     help="threads per vertex and block size of the local step, RHS and residual "
                          "(auto: autotuned per kernel before the timed region)")
     ap.add_argument("--solve-blocks", type=int, default=512,
@@ -1117,7 +1117,7 @@ def run_requests(args):
     analysis = "kept for the unchanged constraint set" if args.cached_analysis else \
         "redone on every request (ordering, elimination tree, supernodes, plan), as SimplicialLDLT::compute"
     extra = {"requests_per_step": N, "solve_blocks": args.solve_blocks,
-             "vertex_launch": vtuned or "1 thread per vertex, 256-thread blocks",
+             "vertex_launch": vtuned or "1 thread per vertex, blocks of 32 to 256 by mesh size",
              "solve_schedule": args.solve_schedule, "warp_rows": args.warp_rows,
              "solve_ctas": args.solve_ctas,
              "cuda_device_max_connections": os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS"),

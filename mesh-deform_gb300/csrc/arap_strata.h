@@ -10,7 +10,7 @@
 // so a forward sweep is one product per stratum, [y; u] = M f (u goes to the
 // columns above), and a backward sweep one transposed product,
 // x = M^T [y; x_below]. No task waits for another inside a stratum; strata
-// follow each other as launches. A sweep over a tree of 13 levels takes 2 to 5
+// follow each other as launches. A sweep over a tree of 13 levels takes 3 to 7
 // such phases instead of a chain of 13 dependent tasks.
 #pragma once
 
