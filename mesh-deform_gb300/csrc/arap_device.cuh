@@ -237,89 +237,23 @@ __device__ __forceinline__ void rotation_from_cov(const T S_in[3][3], T R[3][3],
 // it (a fraction of a percent of the vertices).
 constexpr float kPolarFallback = 0.1f;
 
-// Newton steps towards the rotation R of rotation_from_cov (the maximiser of
-// tr(R S) over proper rotations, so V diag(1,1,det) U^T for S = U Sigma V^T)
-// from a nearby R. With R = R0 exp([w]x) the objective's gradient at w = 0
-// is g, the axial vector of the skew part of Q = (S R0)^T, and its Hessian
-// -(tr(Q) I - sym(Q)); the step w = (tr(Q) I - sym(Q))^-1 g is applied
-// through the Cayley map, which keeps R orthogonal. Quadratic convergence:
-// from an FP32 fit (error e), one step leaves about e^2, two reach FP64
-// accuracy.
-template <typename T>
-__device__ __forceinline__ void polar_newton(const T S[3][3], T R[3][3], int ns_iters, int iters) {
-    // R orthogonal to working precision first (the Cayley steps keep R's
-    // deviation from orthogonality): Newton-Schulz, R <- R (3 I - R^T R) / 2,
-    // which squares the deviation (1e-7 of an FP32 fit -> 1e-14 -> 1e-28)
-    for (int it = 0; it < ns_iters; ++it) {
-        T G[3][3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-                G[a][b] = (a == b ? (T)1.5 : (T)0) - (T)0.5 * (R[0][a] * R[0][b] + R[1][a] * R[1][b] + R[2][a] * R[2][b]);
-        T Rn[3][3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) Rn[a][b] = R[a][0] * G[0][b] + R[a][1] * G[1][b] + R[a][2] * G[2][b];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) R[a][b] = Rn[a][b];
-    }
-    for (int it = 0; it < iters; ++it) {
-        T Q[3][3];  // Q = (S R)^T: Q[a][b] = sum_k S[b][k] R[k][a]
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) Q[a][b] = S[b][0] * R[0][a] + S[b][1] * R[1][a] + S[b][2] * R[2][a];
-        const T g0 = Q[2][1] - Q[1][2], g1 = Q[0][2] - Q[2][0], g2 = Q[1][0] - Q[0][1];
-        const T tr = Q[0][0] + Q[1][1] + Q[2][2];
-        // H = tr I - sym(Q), symmetric
-        const T h00 = tr - Q[0][0], h11 = tr - Q[1][1], h22 = tr - Q[2][2];
-        const T h01 = -(T)0.5 * (Q[0][1] + Q[1][0]), h02 = -(T)0.5 * (Q[0][2] + Q[2][0]),
-                h12 = -(T)0.5 * (Q[1][2] + Q[2][1]);
-        // w = adj(H) g / det(H)
-        const T c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
-        const T c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
-        const T det = h00 * c00 + h01 * c01 + h02 * c02;
-        const T scale = fabs(h00) + fabs(h11) + fabs(h22);
-        if (!(det > Eps<T>::v * scale * scale * scale)) break;  // not a maximum's neighbourhood: keep R
-        const T id = (T)1 / det;
-        const T w0 = (c00 * g0 + c01 * g1 + c02 * g2) * id, w1 = (c01 * g0 + c11 * g1 + c12 * g2) * id,
-                w2 = (c02 * g0 + c12 * g1 + c22 * g2) * id;
-        // Cayley: C = I + 2/(1+|a|^2) ([a]x + [a]x^2), a = w/2
-        const T a0 = (T)0.5 * w0, a1 = (T)0.5 * w1, a2 = (T)0.5 * w2;
-        const T f = (T)2 / ((T)1 + a0 * a0 + a1 * a1 + a2 * a2);
-        const T C[3][3] = {{(T)1 - f * (a1 * a1 + a2 * a2), f * (a0 * a1 - a2), f * (a0 * a2 + a1)},
-                           {f * (a0 * a1 + a2), (T)1 - f * (a0 * a0 + a2 * a2), f * (a1 * a2 - a0)},
-                           {f * (a0 * a2 - a1), f * (a1 * a2 + a0), (T)1 - f * (a0 * a0 + a1 * a1)}};
-        T Rn[3][3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) Rn[a][b] = R[a][0] * C[0][b] + R[a][1] * C[1][b] + R[a][2] * C[2][b];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) R[a][b] = Rn[a][b];
-    }
-}
-
 // The rotation of rotation_from_cov by Newton's method in FP32 from a nearby
 // one, the vertex's rotation of the iteration before (the identity at first),
-// in place. The steps are polar_newton's; about 130 FP32 instructions each,
-// one to three in most iterations, against some 1,500 of the Jacobi fit
-// (256 poses of 10,242 vertices: local step 185 -> 154 us). The
-// step after which the last one's remainder is below FP32 resolution
-// orthonormalises R to first order and ends. A point with g = 0 and a positive
-// definite H is the maximum (tr(R S) has no other local maximum on the proper
-// rotations). False, and R undefined, where five steps do not end, or H is not
-// safely positive definite: det(H) / tr(H)^3 above kWarmDet bounds
-// (sigma_2 + sigma_3) / sigma_1 from below by kPolarFallback (with
-// x = (sigma_2 +- sigma_3) / sigma_1 it is at most x (1 + x/2)^2 / (2 + 2x)^3,
-// 0.01035 at x = 0.1), so that what needs the FP64 fallback goes to the Jacobi
-// fit, which tells.
+// in place. R of rotation_from_cov maximises tr(R S) over proper rotations.
+// With R = R0 exp([w]x) the gradient at w = 0 is g, the axial vector of the
+// skew part of Q = (S R0)^T, and the Hessian -H, H = tr(Q) I - sym(Q); the step
+// w = H^-1 g is applied through the Cayley map, which keeps R orthogonal, and
+// an error e becomes about e^2. About 130 FP32 instructions a step, one to
+// three steps in most iterations, against some 1,500 of the Jacobi fit
+// (256 poses of 10,242 vertices: local step 185 -> 154 us). The step after
+// which the last one's remainder is below FP32 resolution orthonormalises R to
+// first order and ends. A point with g = 0 and a positive definite H is the
+// maximum (tr(R S) has no other local maximum on the proper rotations). False,
+// and R undefined, where five steps do not end, or H is not safely positive
+// definite: det(H) / tr(H)^3 above kWarmDet bounds (sigma_2 + sigma_3) / sigma_1
+// from below by kPolarFallback (with x = (sigma_2 +- sigma_3) / sigma_1 it is at
+// most x (1 + x/2)^2 / (2 + 2x)^3, 0.01035 at x = 0.1), so that what needs the
+// FP64 fallback goes to the Jacobi fit, which tells.
 constexpr float kWarmDet = 0.0104f;
 __device__ __forceinline__ bool rotation_warm(const float S_in[3][3], float R[3][3]) {
     float f2 = 0.f;
@@ -527,9 +461,9 @@ __device__ __forceinline__ bool refine_scale(const double S[3][3], int &e, float
 // and its rotation refined from the FP32 fit Rm (in place), from the rest
 // positions p, current positions pc (element k of vertex k's pose at
 // k * stride + off) and the FP64 weights: by rotation_refine, below its range
-// by an orthonormalisation and a Newton step in FP64, which leave an error of
-// about 1e-12 of the fit's few 1e-6 (the FP64 Jacobi fit instead made a local
-// step of 256 poses of 10,242 vertices 154 us on average against 137).
+// by the FP64 Jacobi fit. There the FP32 fit is no seed for Newton's method:
+// its error is FP32 rounding over (sigma_2 +- sigma_3) / sigma_1, and one step
+// from it was off by half a turn below 1e-5 (one-rings with cap triangles).
 __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32_t *__restrict__ dcol,
                                               const double *__restrict__ w64, const Vec4<double> *__restrict__ p,
                                               const Vec4<double> *__restrict__ pc, int64_t stride, int64_t off,
@@ -549,13 +483,7 @@ __device__ __forceinline__ void rotation_fp64(int i, int e0, int e1, const int32
     double R[3][3];
     int ex;
     float Sf[3][3];
-    if (!(refine_scale(S, ex, Sf) && rotation_refine<false>(S, ex, Sf, Rm, R))) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) R[a][b] = (double)Rm[a][b];
-        polar_newton(S, R, 1, 1);
-    }
+    if (!(refine_scale(S, ex, Sf) && rotation_refine<false>(S, ex, Sf, Rm, R))) rotation_from_cov<double>(S, R);
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
