@@ -334,8 +334,11 @@ __device__ __forceinline__ bool rotation_warm(const float S_in[3][3], float R[3]
 // one-rings stretched by a handle's move made the first iterations' local step
 // 62 to 67 us on the 61,600-vertex bar against 25 later, FP64 form.
 // S's largest entry has the biased exponent e, Sf is S at that scale. False,
-// and R undefined, below kRefineDet or where eight steps do not end.
-constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f;
+// and R undefined, below kRefineDet or where eight steps do not end, and
+// (FULL false) where Rf is no fit of Sf: one made from S in FP32 is within
+// 2e-5 of R above kRefineDet, |w / 2|^2 = 1e-10; the identity that stands for
+// the rotation of an FP32 covariance whose squares underflow is anywhere.
+constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f, kRefineSeed = 1e-8f;
 constexpr int kRefineSteps = 8;
 
 // What the steps share: Q = (S R)^T at Rf, adj(H), 1 / det(H)
@@ -432,6 +435,7 @@ __device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, con
             }
         const float n2 =
             fr.correction(Rf, E, to_float_scaled(g0, e), to_float_scaled(g1, e), to_float_scaled(g2, e), dR);
+        if (!FULL && it == 0 && !(n2 < kRefineSeed)) return false;
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll

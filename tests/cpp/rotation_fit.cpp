@@ -1,7 +1,8 @@
 // The local step's 3x3 rotation fits (csrc/arap_device.cuh) on the host, against
 // the rotation a covariance was built from: S = U diag(1, s2, s3) V^T has the
 // best rotation V diag(1, 1, det(U V^T)) U^T, for s2 from order one down to
-// 1e-7, s3 half of it or close to it, and both signs of the determinant.
+// 1e-7, s3 half of it or close to it, both signs of the determinant, and S of
+// order one or so small that its squares are zero in FP32.
 //
 // Tolerance: S's rounding and the fit's own turn R by some multiple of the
 // precision over the smallest eigenvalue of the objective's Hessian,
@@ -96,33 +97,35 @@ int main() {
     bool ok = true;
     for (int k = 0; k <= 7; ++k)
         for (const long double near : {0.5L, 0.999L})
-            for (const bool reflect : {false, true}) {
-                const long double s2 = k ? std::pow(10.0L, -k) / 2 : 0.5L, s3 = s2 * near,
-                                  gap = reflect ? s2 - s3 : s2 + s3;
-                const double tol64 = 64 * 0x1p-52 / (double)gap + 8 * 0x1p-52;
-                // below kPolarFallback the mixed form's fit is redone in FP64, above it
-                // the FP32 covariance's rounding stands
-                const double tol32 = s2 + s3 < 0.1L ? tol64 + 0x1p-24 : 64 * 0x1p-23 / (double)gap;
-                double worst64 = 0.0, worst32 = 0.0;
-                for (int t = 0; t < 2000; ++t) {
-                    const long double sig[3] = {1, s2, s3};
-                    double S[3][3], D[3][3];
-                    long double ref[3][3];
-                    covariance(sig, reflect, S, ref);
-                    for (int a = 0; a < 3; ++a)
-                        for (int b = 0; b < 3; ++b) D[a][b] = a == b;
-                    dev::rotation_fit_fp64(S, D);
-                    worst64 = std::max(worst64, distance(D, ref));
-                    float F[3][3];
-                    mixed_fit(S, F);
-                    worst32 = std::max(worst32, distance(F, ref));
+            for (const bool reflect : {false, true})
+                for (const double scale : {1.0, 1e-24}) {
+                    const long double s2 = k ? std::pow(10.0L, -k) / 2 : 0.5L, s3 = s2 * near,
+                                      gap = reflect ? s2 - s3 : s2 + s3;
+                    const double tol64 = 64 * 0x1p-52 / (double)gap + 8 * 0x1p-52;
+                    // the mixed form's fit is redone in FP64 below kPolarFallback and
+                    // where FP32 shows no covariance, else the FP32 covariance's rounding stands
+                    const bool redone = s2 + s3 < 0.1L || scale < 1.0;
+                    const double tol32 = redone ? tol64 + 0x1p-24 : 64 * 0x1p-23 / (double)gap;
+                    double worst64 = 0.0, worst32 = 0.0;
+                    for (int t = 0; t < 2000; ++t) {
+                        const long double sig[3] = {scale, scale * s2, scale * s3};
+                        double S[3][3], D[3][3];
+                        long double ref[3][3];
+                        covariance(sig, reflect, S, ref);
+                        for (int a = 0; a < 3; ++a)
+                            for (int b = 0; b < 3; ++b) D[a][b] = a == b;
+                        dev::rotation_fit_fp64(S, D);
+                        worst64 = std::max(worst64, distance(D, ref));
+                        float F[3][3];
+                        mixed_fit(S, F);
+                        worst32 = std::max(worst32, distance(F, ref));
+                    }
+                    const bool good = worst64 <= tol64 && worst32 <= tol32;
+                    ok = ok && good;
+                    std::printf("s2 %.0e s3 %.3f s2 %s scale %.0e: fp64 %.1e (%.1e), mixed %.1e (%.1e)%s\n", (double)s2,
+                                (double)near, reflect ? "-" : "+", scale, worst64, tol64, worst32, tol32,
+                                good ? "" : "  FAILED");
                 }
-                const bool good = worst64 <= tol64 && worst32 <= tol32;
-                ok = ok && good;
-                std::printf("s2 %.0e s3 %.3f s2 %s: fp64 %.1e (%.1e), mixed %.1e (%.1e)%s\n", (double)s2,
-                            (double)near, reflect ? "-" : "+", worst64, tol64, worst32, tol32,
-                            good ? "" : "  FAILED");
-            }
     std::printf(ok ? "ok\n" : "failed\n");
     return ok ? 0 : 1;
 }
