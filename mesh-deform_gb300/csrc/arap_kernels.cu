@@ -504,7 +504,7 @@ template <> __device__ __forceinline__ float pivot_rsqrt(float a) { return rsqrt
 template <> __device__ __forceinline__ double pivot_rsqrt(double a) {
     const int ex = __double2hiint(a) >> 20;  // biased exponent (the sign would make it negative or large)
     if (!(ex > 924 && ex < 1122)) return 1.0 / sqrt(a);
-    const double r = dev::to_double(rsqrtf(dev::to_float_scaled(a, 1023)));
+    const double r = dev::to_double_finite(rsqrtf(dev::to_float_scaled(a, 1023)));
     const double e = fma(-(a * r), r, 1.0);
     return fma(r, e * fma(e, 0.375, 0.5), r);
 }
@@ -521,7 +521,7 @@ template <> __device__ __forceinline__ float pivot_rcp(float a) { return 1.f / a
 template <> __device__ __forceinline__ double pivot_rcp(double a) {
     const int ex = __double2hiint(a) >> 20;
     if (!(ex > 924 && ex < 1122)) return 1.0 / a;
-    const double r = dev::to_double(__frcp_rn(dev::to_float_scaled(a, 1023)));
+    const double r = dev::to_double_finite(__frcp_rn(dev::to_float_scaled(a, 1023)));
     const double e = fma(-a, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
