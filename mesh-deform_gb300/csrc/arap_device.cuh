@@ -62,21 +62,21 @@ __device__ __forceinline__ float to_float_rn(double x) {
 // neighbouring positions agree in their exponents, so the first differences
 // are exact and the sum carries the FP32 rounding that the rounded FP64
 // difference does, however short the edge, without an FP64 instruction.
-// Magnitudes below 2^-76 count as zero.
+// A magnitude below 2^-76 other than zero or from 2^128 on, and what is not
+// finite, is NaN, and so is a covariance with it, which rotation_fp64 then
+// forms in FP64.
 struct Split {
     float hi, mid, low;
     __device__ __forceinline__ explicit Split(double x) {
-        const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
-        const unsigned sign = h & 0x80000000u;
-        const int fe = (int)((h >> 20) & 0x7ffu) - 896;
-        const bool in = fe > 50;
-        const unsigned e0 = (unsigned)fe << 23, e1 = e0 - (23u << 23), e2 = e1 - (23u << 23);
-        hi = __uint_as_float(in ? sign | e0 | ((h & 0xfffffu) << 3) | (l >> 29) : 0u);
-        // bits as the fraction of a float of the right exponent, less its leading one
-        const float m = __uint_as_float(e1 | ((l >> 6) & 0x7fffffu)) - __uint_as_float(e1);
-        const float r = __uint_as_float(e2 | ((l << 17) & 0x7e0000u)) - __uint_as_float(e2);
-        mid = in ? __uint_as_float(__float_as_uint(m) | sign) : 0.f;
-        low = in ? __uint_as_float(__float_as_uint(r) | sign) : 0.f;
+        const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), a = h & 0x7fffffffu;
+        const unsigned q = a - (896u << 20);  // FP32's exponent and the fraction's upper 20 bits
+        const unsigned f = (h & 0x80000000u) | (q << 3) | (l >> 29);
+        const bool in = q - (51u << 20) < 204u << 20;
+        hi = __uint_as_float(in ? f : (a | l) ? 0x7fffffffu : 0u);
+        // bits as the fraction of a float of the right exponent, less its leading one (of zero: none)
+        const unsigned e1 = (f & 0xff800000u) - (23u << 23), e2 = e1 - (23u << 23);
+        mid = __uint_as_float(e1 | ((l >> 6) & 0x7fffffu)) - __uint_as_float(e1);
+        low = __uint_as_float(e2 | ((l << 17) & 0x7e0000u)) - __uint_as_float(e2);
     }
     __device__ __forceinline__ float operator-(const Split &o) const {
         return ((hi - o.hi) + (mid - o.mid)) + (low - o.low);

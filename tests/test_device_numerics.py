@@ -9,7 +9,7 @@ ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "mesh-deform_gb300" / "csrc"
 
 
-@pytest.mark.parametrize("name", ["conversions"])
+@pytest.mark.parametrize("name", ["conversions", "split_difference"])
 def test_on_the_host(tmp_path, name):
     import build_lib
 

@@ -54,3 +54,19 @@ def test_tiny_meshes(gpu, exponent):
         poses = ctx.deform_poses(np.stack([t, p[w.cidx]]), w.iterations)
     assert W.bbox_rel_error(poses[0], ref, p) <= 1e-6
     assert W.bbox_rel_error(single, ref, p) <= 1e-6
+
+
+def test_huge_coordinates(gpu):
+    """Coordinates beyond FP32's range, whose differences are inside it."""
+    from oracle import oracle as O
+
+    w = W.cfg_icosphere_l4(level=3, iterations=4)
+    p, t = w.positions * 2.0 ** 120 + 2.0 ** 130, w.ctargets * 2.0 ** 120 + 2.0 ** 130
+    ok, ref = O.run_deform(p, w.faces, w.cidx, t, w.iterations)
+    assert ok
+    with gpu.ArapContext(w.V, w.faces) as ctx:
+        ctx.set_precision("mixed", 1)
+        ctx.set_rest_positions(p)
+        ctx.set_constraints(w.cidx, t)
+        got = ctx.deform_poses(t[None], w.iterations)[0]
+    assert W.bbox_rel_error(got, ref, p) <= 1e-6
