@@ -58,10 +58,12 @@ __device__ __forceinline__ float to_float_rn(double x) {
 }
 
 // A double as hi + mid + low in FP32: its leading 24 bits, the next 23 and the
-// last 6. The difference of two is ((hi - hi') + (mid - mid')) + (low - low'):
-// neighbouring positions agree in their exponents, so the first differences
-// are exact and the sum carries the FP32 rounding that the rounded FP64
-// difference does, however short the edge, without an FP64 instruction.
+// last 6. The difference of two is (hi - hi') + (mid - mid') + (low - low')
+// with the rounding of the first difference (two-sum; none where the exponents
+// agree) and of the first sum carried along, so that only the last addition
+// rounds: the rounded FP64 difference, however short the edge, without an FP64
+// instruction. 14 additions a component; the 5 of the plain sums rounded twice
+// where exponents differ, 1.2e-7 instead of 6e-8.
 // A magnitude below 2^-76 other than zero or from 2^128 on, and what is not
 // finite, is NaN, and so is a covariance with it, which rotation_fp64 then
 // forms in FP64.
@@ -79,7 +81,10 @@ struct Split {
         low = __uint_as_float(e2 | ((l << 17) & 0x7e0000u)) - __uint_as_float(e2);
     }
     __device__ __forceinline__ float operator-(const Split &o) const {
-        return ((hi - o.hi) + (mid - o.mid)) + (low - o.low);
+        const float d = hi - o.hi, r = d - hi;
+        const float s = (mid - o.mid) + ((hi - (d - r)) - (o.hi + r));
+        const float t = d + s;
+        return t + ((s - (t - d)) + (low - o.low));
     }
 };
 

@@ -28,7 +28,8 @@ void check(double a, double b, double ulps) {
 }  // namespace
 
 int main() {
-    constexpr double ulps = 2.0;
+    // half a unit of the result, and what the roundings of the lower parts leave
+    constexpr double ulps = 1.001;
     const double inf = std::numeric_limits<double>::infinity();
     const std::vector<double> special = {0.0, 1.0, 0x1.fffffffffffffp0, 0x1p-76, 0x1.fffffffffffffp-77, 0x1p-1022, 0x1p127,
                                          0x1.fffffffffffffp126, 0x1p128, 1e40, 1e300, inf,
@@ -44,6 +45,11 @@ int main() {
         const double b = i % 2 ? (unit() - 0.5) * std::pow(2.0, (int)(rng() % 40) - 20)
                                : a + (unit() - 0.5) * std::pow(10.0, -(double)(rng() % 9));
         check(a, b, ulps);
+    }
+    for (int i = 0; i < 2000000; ++i) {  // on both sides of a power of two, and of zero
+        const double c = std::pow(2.0, (int)(rng() % 9) - 4), s = std::pow(2.0, -(double)(rng() % 50));
+        check(c * (1.0 + s * unit()), c * (1.0 - s * unit()), ulps);
+        check(c * s * unit(), -c * s * unit(), ulps);
     }
     std::printf(failures ? "failed\n" : "ok\n");
     return failures ? 1 : 0;
