@@ -591,7 +591,7 @@ k_fdt(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF
                 if (lane == k) u = (TF)1;
             }
             U[k][lane] = u;
-            const TF q = u * un;
+            const TF q = sizeof(TF) == 8 ? u * un : un;
             const TF r = pivot_rcp(p);
             if (lane == 0) {
                 piv[k] = p;
@@ -605,7 +605,9 @@ k_fdt(const FItem *__restrict__ items, int jb, const SnInfo *__restrict__ sn, TF
                 bar_sync(3 + ((k + 1) & 1), 64);  // N(k + 1)
                 a = U[k + 1][lane];
             }
-            a -= q * r;
+            // FP32: the product of two entries may leave the range (weights above 1.8e19)
+            if constexpr (sizeof(TF) == 8) a -= q * r;
+            else a -= u * (q * r);
             u = lane > k ? a : (TF)0;
         }
         if (bad && lane == 0) atomicOr(err, kErrNotSpd);
