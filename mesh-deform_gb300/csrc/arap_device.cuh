@@ -344,25 +344,32 @@ __device__ __forceinline__ bool rotation_warm(const float S_in[3][3], float R[3]
 // about |dR| (1e-6 / conditioning): with det(H) / tr(H)^3 above kNewtonDet
 // (0.037 at equal singular values, 0.010 at (sigma_2 + sigma_3) / sigma_1 = 0.1
 // without a reflection) 1e-6 -> 1e-11 -> below FP64 rounding in two steps, the
-// first of which is all a result of FP32 needs. Down to kRefineDet, a tenth of
-// the conditioning, steps go on until they are that small. FP64 Newton steps
-// (S R, adjugate, Cayley map and products in FP64) take about 400 FP64
-// instructions for the same rotation, the FP64 Jacobi fit some thousands: the
-// one-rings stretched by a handle's move made the first iterations' local step
-// 62 to 67 us on the 61,600-vertex bar against 25 later, FP64 form.
+// first of which is all a result of FP32 needs. Below, steps go on until they
+// are that small. FP64 Newton steps (S R, adjugate, Cayley map and products in
+// FP64) take about 400 FP64 instructions for the same rotation, the FP64 Jacobi
+// fit some thousands: the one-rings stretched by a handle's move made the first
+// iterations' local step 62 to 67 us on the 61,600-vertex bar against 25 later,
+// FP64 form.
 // S's largest entry has the biased exponent e, Sf is S at that scale. False,
-// and R undefined, below kRefineDet or where eight steps do not end, and
-// (FULL false) where Rf is no fit of Sf: one made from S in FP32 is within
-// 2e-5 of R above kRefineDet, |w / 2|^2 = 1e-10; the identity that stands for
-// the rotation of an FP32 covariance whose squares underflow is anywhere.
-constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f, kRefineSeed = 1e-8f;
+// and R undefined, below kRefineDet or where eight steps do not end.
+// FULL false (the mixed form's refit, whose result is rounded to FP32) ends at
+// |w / 2| of 1e-8, or after a first step within 1e-5, and goes down to
+// kRefineDetFit, (sigma_2 +- sigma_3) / sigma_1 of about 8e-5: there H's FP32
+// rounding is a hundredth of its small eigenvalue, so a step still leaves a
+// hundredth, and errors stay below 3e-11 (random covariances of any smaller
+// singular values). With the Jacobi fit from kRefineDet down the first local
+// step of the twisted bar took 130 us more (set-up and one iteration 2,755 us,
+// 2,603 so). An Rf that is no fit of Sf is refused by its gradient, 1e-6 of |S|
+// for one made in FP32: the identity that stands for the rotation of an FP32
+// covariance whose squares underflow can be anywhere.
+constexpr float kNewtonDet = 4e-3f, kRefineDet = 6e-4f, kRefineDetFit = 1e-5f, kRefineSeed = 1e-10f;
 constexpr int kRefineSteps = 8;
 
 // What the steps share: Q = (S R)^T at Rf, adj(H), 1 / det(H)
 struct RefineFrame {
     float Q[3][3], c00, c01, c02, c11, c12, c22, id;
     bool plain;  // a fixed number of steps suffices
-    __device__ __forceinline__ bool init(const float Sf[3][3], const float Rf[3][3]) {
+    __device__ __forceinline__ bool init(const float Sf[3][3], const float Rf[3][3], float least) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -373,7 +380,7 @@ struct RefineFrame {
         c00 = h11 * h22 - h12 * h12, c01 = h02 * h12 - h01 * h22, c02 = h01 * h12 - h02 * h11;
         c11 = h00 * h22 - h02 * h02, c12 = h01 * h02 - h00 * h12, c22 = h00 * h11 - h01 * h01;
         const float det = h00 * c00 + h01 * c01 + h02 * c02, tr = fabsf(h00) + fabsf(h11) + fabsf(h22);
-        if (!(h00 > 0.f && c22 > 0.f && det > kRefineDet * tr * tr * tr)) return false;
+        if (!(h00 > 0.f && c22 > 0.f && det > least * tr * tr * tr)) return false;
         plain = det > kNewtonDet * tr * tr * tr;
         id = 1.f / det;
         return true;
@@ -415,7 +422,8 @@ struct RefineFrame {
         return n2;
     }
     template <bool FULL> __device__ __forceinline__ bool done(int it, float n2) const {
-        return plain ? it == (FULL ? 1 : 0) : n2 < (FULL ? 2.5e-27f : 1e-16f);
+        if (FULL) return plain ? it == 1 : n2 < 2.5e-27f;
+        return n2 < (plain && it == 0 ? 1e-10f : 1e-16f);
     }
 };
 
@@ -423,7 +431,7 @@ template <bool FULL>
 __device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, const float Sf[3][3],
                                                 const float Rf[3][3], double R[3][3]) {
     RefineFrame fr;
-    if (!fr.init(Sf, Rf)) return false;
+    if (!fr.init(Sf, Rf, FULL ? kRefineDet : kRefineDetFit)) return false;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -450,9 +458,9 @@ __device__ __forceinline__ bool rotation_refine(const double S[3][3], int e, con
                 for (int k = 0; k < 3; ++k) x += R[k][a] * R[k][b];
                 E[a][b] = E[b][a] = to_float_scaled(x, 1023);
             }
-        const float n2 =
-            fr.correction(Rf, E, to_float_scaled(g0, e), to_float_scaled(g1, e), to_float_scaled(g2, e), dR);
-        if (!FULL && it == 0 && !(n2 < kRefineSeed)) return false;
+        const float f0 = to_float_scaled(g0, e), f1 = to_float_scaled(g1, e), f2 = to_float_scaled(g2, e);
+        if (!FULL && it == 0 && !(f0 * f0 + f1 * f1 + f2 * f2 < kRefineSeed)) return false;
+        const float n2 = fr.correction(Rf, E, f0, f1, f2, dR);
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -558,7 +566,7 @@ __device__ __forceinline__ void rotation_fit_fp64_quad(const double row[3], int 
         }
         if (!rotation_warm(Sf, Rf)) rotation_from_cov<float>(Sf, Rf);
         RefineFrame fr;
-        if (fr.init(Sf, Rf)) {
+        if (fr.init(Sf, Rf, kRefineDet)) {
             double Sa[3], Sb[3], C0[3], C1[3], C2[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
