@@ -416,9 +416,10 @@ int dense_cap(const arap_ctx *ctx) {
 
 // Bytes of every device buffer the setup of precision T (and, for n_poses > 0,
 // arap_deform_poses with that many poses) holds, buffer by buffer.
-// sweeps / phases: the solve arrays of the supernodal sweeps / dense phases.
+// sweeps: with the solve arrays of the supernodal sweeps; single, poses: with
+// those of a plan of dense phases for a single request / a pose batch.
 template <typename T>
-void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
+void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, const Strata *single, const Strata *poses,
                    std::vector<std::pair<DevBuf *, size_t>> &out) {
     const Symbolic &s = ctx->sym;
     if (sweeps) build_blocks(ctx);
@@ -483,11 +484,10 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
         add(ctx->Lval32, (size_t)std::max<int64_t>(s.panel_size, 1) * sizeof(float));
         add(ctx->Dinv32, (size_t)std::max<int64_t>(s.dinv_size, 1) * sizeof(float));
     }
-    if (phases) {
-        const Strata &p = ctx->strata;
+    if (single) {
         add(ctx->st_y, m1 * sizeof(Vec4<T>));
-        add(ctx->st_ytop, std::max<size_t>(top_vec_bytes(p.big_n, sizeof(T)), 16));
-        add_strata(p, ctx->stb, sizeof(T));
+        add(ctx->st_ytop, std::max<size_t>(top_vec_bytes(single->big_n, sizeof(T)), 16));
+        add_strata(*single, ctx->stb, sizeof(T));
     }
     if (n_poses > 0) {
         const size_t P = (size_t)n_poses, VP = V * P, MP = m1 * P, nc = V - (size_t)s.m;
@@ -499,9 +499,9 @@ void planned_sizes(arap_ctx *ctx, int n_poses, bool sweeps, bool phases,
         add(ctx->buvec, (size_t)std::max<int64_t>(s.uvec_size, 1) * P * sizeof(Vec4<float>));
         add(ctx->bout, VP * 3 * sizeof(double));
         add(ctx->btargets, P * nc * 3 * sizeof(double));
-        if (!sweeps) {
+        if (poses) {
             add(ctx->bst_y, MP * sizeof(Vec4<float>));
-            add_strata(ctx->bstrata, ctx->bstb, 4);
+            add_strata(*poses, ctx->bstb, 4);
         }
     }
     if (!sweeps) return;
@@ -948,7 +948,7 @@ int prepare_bstrata(arap_ctx *ctx) {
 template <typename T>
 int setup_alloc(arap_ctx *ctx, bool sweeps, bool phases) {
     std::vector<std::pair<DevBuf *, size_t>> plan;
-    planned_sizes<T>(ctx, 0, sweeps, phases, plan);
+    planned_sizes<T>(ctx, 0, sweeps, phases ? &ctx->strata : nullptr, nullptr, plan);
     bool moved = false;
     for (auto &pb : plan) {
         void *before = pb.first->p;
@@ -2519,10 +2519,15 @@ int arap_plan_bytes(arap_ctx *ctx, int32_t n_poses, int64_t *bytes) {
     if (!ctx->cidx.empty()) {
         const int rc = analyze_symbolic(ctx);
         if (rc != ARAP_OK) return rc;
-        const bool fp64 = ctx->precision == ARAP_PRECISION_FP64 && n_poses == 0;
-        const bool phases = use_strata(ctx, fp64);
-        if (fp64) planned_sizes<double>(ctx, 0, !phases, phases, plan);
-        else planned_sizes<float>(ctx, n_poses, !phases || (n_poses > 0 && !use_bstrata(ctx)), phases, plan);
+        if (n_poses > 0) {  // a pose call forms its own solve arrays only; a single request's resident plan stays
+            const bool phases = use_bstrata(ctx);
+            planned_sizes<float>(ctx, n_poses, !phases, nullptr, phases ? &ctx->bstrata : nullptr, plan);
+        } else {
+            const bool fp64 = ctx->precision == ARAP_PRECISION_FP64;
+            const Strata *single = use_strata(ctx, fp64) ? &ctx->strata : nullptr;
+            if (fp64) planned_sizes<double>(ctx, 0, !single, single, nullptr, plan);
+            else planned_sizes<float>(ctx, 0, !single, single, nullptr, plan);
+        }
     }
     for (DevBuf *b : ctx->buffers()) {
         size_t want = b->cap;
