@@ -4,7 +4,7 @@
 // arap_batch.cu.
 
 constexpr int kBsThreads = 128, kBsK = 16;
-constexpr int kBsRows = 32, kBsPoses = 32, kBsRing = 4;  // tile, shared-memory buffers
+constexpr int kBsRows = 32, kBsPoses = kStPoseTile, kBsRing = 4;  // tile, shared-memory buffers
 // floats of a chunk of M in shared memory (forward rows padded to 20)
 constexpr int bs_m_floats() { return kBsRows * (kBsK + 4); }
 

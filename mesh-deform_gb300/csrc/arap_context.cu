@@ -2618,8 +2618,10 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         // writes the FP32 solve copies (and reads the FP64 ones back once)
         const bool f64f = ctx->state_prec == ARAP_PRECISION_MIXED && ctx->factor_bits == 64;
         const double fz = f64f ? 8.0 : sz;
-        B = (double)s.panel_size * fz * 2 + (double)s.upd_size * fz * 2 + (double)s.dinv_size * fz +
-            (xlow + l21) * sz;
+        // the solve arrays it ends with: the groups' matrices, or the sweeps' X and L21
+        const double solve = ctx->model_batched ? (use_bstrata(ctx) ? ctx->bstrata.entries : xlow + l21)
+                                                : (use_strata(ctx, sz == 8.0) ? ctx->strata.entries : xlow + l21);
+        B = (double)s.panel_size * fz * 2 + (double)s.upd_size * fz * 2 + (double)s.dinv_size * fz + solve * sz;
         if (f64f) B += (double)(s.panel_size + s.dinv_size) * (8 + 4);  // rounded to FP32 for the inverses
         FL = s.factor_flops;
         break;
@@ -2651,8 +2653,8 @@ int arap_get_kernel_model(arap_ctx *ctx, int32_t kernel_class, double *bytes, do
         if (!ctx->model_batched && use_strata(ctx, sz == 8.0)) {  // the groups' matrices once, vectors in and out
             B = ctx->strata.entries * sz + (m + ctx->strata.nb_sum) * 3 * sz * 2;
             FL = ctx->strata.entries * 6;
-        } else if (ctx->model_batched && use_bstrata(ctx)) {  // the groups' matrices once per 64 poses
-            B = ctx->bstrata.entries * sz * std::ceil(P / 64.0) + P * (m + ctx->bstrata.nb_sum) * 3 * sz * 2;
+        } else if (ctx->model_batched && use_bstrata(ctx)) {  // the groups' matrices once per pose tile
+            B = ctx->bstrata.entries * sz * std::ceil(P / kStPoseTile) + P * (m + ctx->bstrata.nb_sum) * 3 * sz * 2;
             FL = P * ctx->bstrata.entries * 6;
         } else if (ctx->model_batched) {  // lower matrices once per pose tile, T once, vectors once per pose
             B = (T * (xlow_lo + l21_lo) + tri) * sz + P * vec;

@@ -298,6 +298,7 @@ void launch_bsolve(const DevSym &s, int P, int pt, int grid, const float *X, con
                    Vec4<float> *sol, Vec4<float> *uvec, Vec4<double> *pc64, Vec4<float> *pc32,
                    unsigned long long *ticket, unsigned *flags, int *err, bool forward, cudaStream_t st,
                    const float *atiles, float *bftop, float *bytop, float *bws);
+constexpr int kStPoseTile = 32;  // poses one CTA of the phases' products takes
 // the dense phases for P poses (a plan of kStPoses): sol holds the right-hand
 // sides, then the solutions; x is added to pc64
 bool bstrata_fits(const Strata &p);
