@@ -173,14 +173,16 @@ int arap_set_done_callback(arap_ctx *ctx, arap_done_fn fn, void *user);
    is what arap_wait returns. */
 int arap_query(arap_ctx *ctx, int32_t *done);
 
-/* The triangular solves of a single request (arap.h:417-429) run as dense
-   phases: the elimination tree is cut into a few strata of subtrees, each
-   subtree solved through its dense inverse, one launch per stratum and
-   direction. Setting any of the options of the supernodal sweeps below to
-   other than its default (arap_set_dense_top, arap_set_cluster_threshold,
-   arap_set_warp_rows, arap_set_solve_schedule, arap_set_solve_blocks) runs
-   the sweeps instead; arap_deform_poses always does. The results are equal up
-   to the order of sums.
+/* The triangular solves (arap.h:417-429) of a single request and of a pose
+   batch run as dense phases: the elimination tree is cut into a few strata of
+   subtrees, each subtree solved through its dense inverse, one launch per
+   stratum and direction, and forward one more per stratum but the first that
+   gathers its updates. Setting any of the options of the supernodal sweeps
+   below to other than its default (arap_set_dense_top,
+   arap_set_cluster_threshold, arap_set_warp_rows, arap_set_solve_schedule,
+   arap_set_solve_blocks) runs the sweeps instead, for both;
+   arap_set_pose_tile does for pose batches alone. The results are equal up to
+   the order of sums.
 
    Most CTAs one launch of the sweeps uses (0, the default: as many as fit on
    the device). Each CTA works through the supernodes in schedule order, so
@@ -193,12 +195,15 @@ int arap_query(arap_ctx *ctx, int32_t *done);
    next deform (which sets the problem up again). */
 int arap_set_solve_ctas(arap_ctx *ctx, int32_t max_ctas);
 
-/* Poses per task of the batched triangular solves of arap_deform_poses: 1, 2,
-   4, 8 or 16 (0, the default: the largest the mesh's biggest supernode
-   allows). A larger tile streams each factor block once for more poses; a
-   smaller one gives more tasks to run at once. Any value gives the same
-   result. ARAP_ERR_UNSUPPORTED at the next arap_deform_poses when the tile
-   does not fit; ARAP_ERR_INVALID_ARGUMENT for other values. */
+/* Poses per task of the supernodal sweeps of arap_deform_poses: 1, 2, 4, 8 or
+   16 asks for the sweeps with that tile (their arrays are then formed from the
+   resident factor); 0, the default, leaves pose batches to the dense phases,
+   and where a sweep option asks for the sweeps takes the largest tile the
+   mesh's biggest supernode allows. A larger tile streams each factor block
+   once for more poses; a smaller one gives more tasks to run at once. Every
+   tile gives the same result, and the phases' up to the order of sums.
+   ARAP_ERR_UNSUPPORTED at the next arap_deform_poses when the tile does not
+   fit; ARAP_ERR_INVALID_ARGUMENT for other values. */
 int arap_set_pose_tile(arap_ctx *ctx, int32_t poses);
 
 /* The triangular solves take the top levels of the elimination tree (large

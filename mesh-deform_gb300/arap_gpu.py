@@ -363,7 +363,7 @@ class ArapContext:
         self._check(self.lib.arap_set_solve_ctas(self.h, int(n)))
 
     def set_pose_tile(self, poses: int):
-        """Poses per batched-solve task of deform_poses (0: automatic)."""
+        """Poses per task of deform_poses' supernodal sweeps (0: the dense phases)."""
         self._check(self.lib.arap_set_pose_tile(self.h, int(poses)))
 
     def set_targets(self, xyz):

@@ -733,7 +733,8 @@ int prepare_symbolic(arap_ctx *ctx) {
 }
 
 // The supernodal sweeps' layout and scheduling state for the current analysis
-// (pose batches, and single requests that ask for the sweeps).
+// (requests and pose batches that ask for the sweeps, or whose plan of dense
+// phases does not fit).
 int prepare_sweeps(arap_ctx *ctx) {
     if (ctx->sweeps_ready) return ARAP_OK;
     build_blocks(ctx);
@@ -1341,8 +1342,8 @@ int run_iterations<float>(arap_ctx *ctx, int iterations) {
 }
 
 // `iterations` local/global iterations of P poses at once (the loop of
-// arap.h:122-129 per pose), the two triangular solves each one persistent
-// launch over all (supernode, pose tile) tasks.
+// arap.h:122-129 per pose), the two triangular solves as dense phases or, each,
+// as one persistent launch over all (supernode, pose tile) tasks.
 int run_batch_iterations(arap_ctx *ctx, int P, int iterations, bool phases) {
     const Symbolic &s = ctx->sym;
     const DevSym &d = ctx->ds;

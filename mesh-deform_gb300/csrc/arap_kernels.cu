@@ -1026,7 +1026,7 @@ k_fx(const FItem *__restrict__ items, const SnInfo *__restrict__ sn, const TF *_
 // One-ring entries e, e + G, ... (N of them, below e1) gathered together:
 // their neighbours' indices first, then everything load(k, entry, neighbour)
 // reads, so that a vertex waits for two round trips per N neighbours instead
-// of two per neighbour. Bound by that latency: an iteration of the 30,000
+// of two per neighbour. Bound by that latency: an iteration of the 67,202
 // vertex bar, mixed form, 131.6 us one neighbour at a time, 123.6 by twos,
 // 122.1 by fours; of the level-7 sphere (163,842 vertices) 215.4, 204.2, 201.4.
 constexpr int kRing = 4;
@@ -1367,10 +1367,11 @@ k_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ 
 // RHS and the first residual of an iteration in one pass over the one-rings
 // (both read the same entries, and a launch's latency is most of either); the
 // sums are k_rhs_mixed's and k_residual's, in their order. Iterations with two
-// launches and with one: 380 vertices 19.7 and 18.0 us, 2,562 43.5 and 41.0,
-// 8,000 52.0 and 49.1, 18,200 67.9 and 64.3, the 67,202-vertex bar 118.8 and
-// 113.9 (but a 900-vertex sheet 28.8 and 31.6). Neighbours by twos gather no
-// faster here (113.0; 16 bars 215.7 and 218.5).
+// launches and with one, of sheets: 288 vertices 19.1 and 17.6 us, 957 33.7 and
+// 32.2, 2,500 44.9 and 43.0, 9,504 48.6 and 46.4, 18,900 71.6 and 68.9; the
+// 67,202-vertex bar 118.8 and 113.9. Of 18 sheets one was slower (840 vertices,
+// 27.5 and 29.0). Neighbours by twos gather no faster here (113.0; 16 bars 215.7
+// and 218.5).
 __global__ void __launch_bounds__(256)
 k_rhs_residual(int m, const int32_t *__restrict__ drow, const int32_t *__restrict__ dcol, const float *__restrict__ w,
                const Vec4<float> *__restrict__ redge, const Vec4<float> *__restrict__ R,
@@ -3280,9 +3281,10 @@ void launch_local_step_fp64(const DevSym &s, const Vec4<double> *wedge, const Ve
     if (s.V == 0) return;
     // Four lanes per vertex (62 FP64 instructions a warp instead of 174) while
     // one lane each would not give every scheduler a warp. FP64 iterations with
-    // one and with four: 380 vertices 22.3 and 19.7 us, 1,600 31.8 and 29.3,
-    // 8,280 90.9 and 74.0, 18,200 107.5 and 94.9; slower at some sizes (9,500
-    // vertices 77.5 and 82.6).
+    // one and with four, of sheets: 400 vertices 22.1 and 19.7 us, 1,600 31.8 and
+    // 29.2, 4,096 67.0 and 58.1, 9,504 91.2 and 81.7, 18,900 122.4 and 103.4. Of
+    // 18 sheets two were slower, by 1% (6,400 vertices 84.8 and 85.6, 12,100 85.9
+    // and 86.3).
     if (s.V <= 32 * 4 * 152) {
         const int block = fp64_block(4 * (int64_t)s.V);
         launch_pdl(k_local_step_fp64_quad, s.overlap != 0, blocks_for(4 * (int64_t)s.V, block), block, 0, st, s.V,

@@ -1,5 +1,5 @@
 // arap_strata.cpp -- cuts the elimination tree into the dense phases of the
-// single-request solves (arap_strata.h). Integer work on the host, O(S log m).
+// solves (arap_strata.h). Integer work on the host, O(S log m).
 #include "arap_strata.h"
 
 #include <algorithm>

@@ -1,4 +1,5 @@
-// arap_strata.h -- the single-request triangular solves in a few dense phases.
+// arap_strata.h -- the triangular solves of a request or of a pose batch in a few
+// dense phases.
 //
 // The elimination tree is cut into strata of rooted subtrees ("groups"), each
 // group's columns holding at most a few hundred to a few thousand columns.
